@@ -64,6 +64,7 @@ SYMBOLS = {
     "hipattn_select_stage": (i32, [vp, vp, i64, i32, i32, i32, i32, i32, vp, vp, vp, vp]),
     "hipattn_finalize_indices": (i32, [vp, vp, i64, i64, vp, i64, i64, i32, i32, i32, i32, i32, i32, i32, vp, vp, vp, vp]),
     "hipattn_bsa_attention": (i32, [C.POINTER(BsaParams), vp]),
+    "hipattn_attention_splits": (i32, [C.POINTER(BsaParams)]),
     "hipattn_merge_partials": (i32, [vp, vp, i64, i32, i32, i32, vp, i64, vp, vp]),
     "hipattn_mark_attention_access": (i32, [C.POINTER(BsaParams), vp, i64, i64, i32, i32, vp]),
     "hipattn_bsa_decode_noalloc": (i32, [C.POINTER(BsaParams), vp]),

@@ -559,7 +559,7 @@ int dispatch_row(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handl
 // Decode shapes: one query row, 1 / 2 / 4 / 8 query heads per KV head, K / V rows of 128, 256 or 512 bytes.
 int bsa_decode(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled) {
   *handled = false;
-  if (p.TQ != 1) return HIPATTN_OK;
+  if (p.TQ != 1 || p.k.fp8_e5m2 || p.v.fp8_e5m2) return HIPATTN_OK;
   const int G = p.H / p.HKV;
   if (p.dtype != HIPATTN_F32 && G <= 8 && (p.D == 64 || p.D == 128)) {
     *handled = true;

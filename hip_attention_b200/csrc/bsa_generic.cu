@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(kThreads) bsa_generic_kernel(const hipattn_bsa
     const float inv = l_run[r] > 0.f ? 1.f / l_run[r] : 0.f;
     const float lse = l_run[r] > 0.f ? m_run[r] + log2f(l_run[r]) : -INFINITY;
     if (p.n_splits > 1) {
-      const int64_t o = ((int64_t)b * p.H + hh) * p.n_splits + split;
+      const int64_t o = (((int64_t)b * p.TQ + ti) * p.H + hh) * p.n_splits + split;
       if (tx == 0) p.part_lse[o] = lse;
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
@@ -335,7 +335,6 @@ int dispatch_tile(const hipattn_bsa_params_t& p, cudaStream_t stream) {
     return launch<DT, D, 16>(p, 1, rows_in_block, 1, stream);
   if (p.heads_share_mask && p.TQ <= p.block_size_q && Gq * rows_in_block <= 64)
     return launch<DT, D, 64>(p, 1, rows_in_block, 1, stream);
-  HIPATTN_REQUIRE(p.n_splits == 1, HIPATTN_ERR_INVALID, "attention: key splits need one query row per head");
   if (rows_in_block <= 16) return launch<DT, D, 16>(p, 0, 0, 1, stream);
   return launch<DT, D, 64>(p, 0, 0, cdiv(p.block_size_q, 64), stream);
 }

@@ -51,6 +51,7 @@ __global__ void __launch_bounds__(M * 2) bsa_mma_kernel(const hipattn_bsa_params
   const int NBLK = cdiv(p.TQ, p.block_size_q);
   const int hslots = p.H / NH;
   int64_t bid = blockIdx.x;
+  const int split = (int)(bid % p.n_splits); bid /= p.n_splits;
   const int sub = (int)(bid % n_sub); bid /= n_sub;     // n_sub > 1 never happens with NH > 1
   const int d = (int)(bid % NBLK); bid /= NBLK;
   const int hs = (int)(bid % hslots); bid /= hslots;
@@ -103,7 +104,11 @@ __global__ void __launch_bounds__(M * 2) bsa_mma_kernel(const hipattn_bsa_params
   const int pmin = s_mm[0], pmax = s_mm[1];
   const int rmin = s_mm[2], rmax = s_mm[3];
   const KeyList kl = make_key_list(p, b, h0, d, pmin, pmax);
-  const int n_tiles = cdiv(kl.total, TKM);
+  // the tiles of this CTA's key range (all of them unless the caller asked for key splits)
+  const int all_tiles = cdiv(kl.total, TKM);
+  const int per_split = cdiv(all_tiles, p.n_splits);
+  const int tile0 = split * per_split;
+  const int n_tiles = max(0, min(per_split, all_tiles - tile0));
 
   // Q fragments
   uint32_t qf[KSTEPS][4];
@@ -117,7 +122,7 @@ __global__ void __launch_bounds__(M * 2) bsa_mma_kernel(const hipattn_bsa_params
     if (tid < TKM) {
       TileMeta& m = meta[tile % 3];
       bool w;
-      const int j = tile * TKM + tid;
+      const int j = (tile0 + tile) * TKM + tid;
       const int t = key_position(kl, j, &w);
       m.tpos[tid] = t;
       m.twin[tid] = (t >= 0 && w) ? 1 : 0;
@@ -269,6 +274,21 @@ __global__ void __launch_bounds__(M * 2) bsa_mma_kernel(const hipattn_bsa_params
   }
   cp_async_wait<0>();
 
+  if (p.n_splits > 1) {   // a normalised fp32 partial row per key range, merged by merge_kernel
+    const int r0 = warp * 16 + (lane >> 2);
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int r = r0 + half * 8, i = r % BQ;
+      if (i >= rows_here) continue;
+      const float inv = l_run[half] > 0.f ? 1.f / l_run[half] : 0.f;
+      const int64_t o_row = (((int64_t)b * p.TQ + row_t0 + i) * p.H + h0 + r / BQ) * p.n_splits + split;
+#pragma unroll
+      for (int nt = 0; nt < NO; ++nt)
+        *reinterpret_cast<float2*>(p.part_o + o_row * D + nt * 8 + (lane & 3) * 2) = make_float2(o[nt][half * 2] * inv, o[nt][half * 2 + 1] * inv);
+      if ((lane & 3) == 0) p.part_lse[o_row] = l_run[half] > 0.f ? m_run[half] + log2f(l_run[half]) : -INFINITY;
+    }
+    return;
+  }
   // ---- epilogue: normalise, stage through shared memory, 16-byte stores ----
   const float inv0 = l_run[0] > 0.f ? 1.f / l_run[0] : 0.f, inv1 = l_run[1] > 0.f ? 1.f / l_run[1] : 0.f;
   {
@@ -303,7 +323,7 @@ int launch(const hipattn_bsa_params_t& p, int BQ, int n_sub, cudaStream_t stream
   const size_t smem = (size_t)M * D * 2 + 4 * (size_t)TKM * D * 2 + 3 * sizeof(TileMeta);
   const int NH = M / BQ;
   const int NBLK = cdiv(p.TQ, p.block_size_q);
-  const int64_t grid = (int64_t)p.B * (p.H / NH) * NBLK * n_sub;
+  const int64_t grid = (int64_t)p.B * (p.H / NH) * NBLK * n_sub * p.n_splits;
   HIPATTN_REQUIRE(grid > 0 && grid < 0x7fffffffLL, HIPATTN_ERR_INVALID, "attention grid of %lld blocks", (long long)grid);
   auto kern = bsa_mma_kernel<DT, D, M>;
   HIPATTN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -311,30 +331,48 @@ int launch(const hipattn_bsa_params_t& p, int BQ, int n_sub, cudaStream_t stream
   return check_launch("bsa_mma_kernel");
 }
 
+// rows and heads of a CTA's tile (M rows, BQ per head) and tiles per attention block; false: another kernel's shape
+bool mma_shape(const hipattn_bsa_params_t& p, int* M, int* BQ, int* n_sub) {
+  if (p.dtype == HIPATTN_F32 || p.TQ < 16 || p.k.fp8_e5m2 || p.v.fp8_e5m2) return false;
+  if (p.D != 64 && p.D != 128) return false;
+  if (p.out && (((uintptr_t)p.out % 16) || (p.o_stride_b % 8) || (p.o_stride_t % 8) || (p.o_stride_h % 8))) return false;
+  const int Gq = p.H / p.HKV, bq = p.block_size_q;
+  *n_sub = 1;
+  if (bq == 64) {
+    *BQ = 64;
+    *M = p.heads_share_mask && (Gq % 2) == 0 ? 128 : 64;   // two heads per CTA where they share the key list
+    return true;
+  }
+  if (bq % 128 == 0) { *M = *BQ = 128; *n_sub = bq / 128; return true; }
+  return false;
+}
+
 template <int DT, int D>
-int dispatch(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled) {
-  const int Gq = p.H / p.HKV;
-  const int bq = p.block_size_q;
-  *handled = true;
-  if (bq == 64 && p.heads_share_mask && (Gq % 2) == 0) return launch<DT, D, 128>(p, 64, 1, stream);  // two heads per CTA
-  if (bq == 64) return launch<DT, D, 64>(p, 64, 1, stream);
-  if (bq % 128 == 0) return launch<DT, D, 128>(p, 128, bq / 128, stream);
-  *handled = false;
-  return HIPATTN_OK;
+int dispatch(const hipattn_bsa_params_t& p, int M, int BQ, int n_sub, cudaStream_t stream) {
+  return M == 128 ? launch<DT, D, 128>(p, BQ, n_sub, stream) : launch<DT, D, 64>(p, BQ, n_sub, stream);
 }
 
 }  // namespace
+
+// CTAs of the kernel without key splits, and how many the GPU holds at once (0: another kernel takes the call)
+int64_t bsa_mma_ctas(const hipattn_bsa_params_t& p, int* resident, int* tile_keys) {
+  int M, BQ, n_sub;
+  if (!mma_shape(p, &M, &BQ, &n_sub)) return 0;
+  *resident = 148 * (M == 128 ? 1 : 2) * (p.D == 64 ? 2 : 1);
+  *tile_keys = TKM;
+  return (int64_t)p.B * (p.H / (M / BQ)) * cdiv(p.TQ, p.block_size_q) * n_sub;
+}
 
 // Handles 16-bit prefill shapes (attention blocks of 64 or a multiple of 128 rows, head dim 64 or 128,
 // out rows 16-byte aligned); everything else is left to the general kernel.
 int bsa_mma(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled) {
   *handled = false;
-  if (p.n_splits != 1 || p.dtype == HIPATTN_F32 || p.TQ < 16) return HIPATTN_OK;
-  if (p.D != 64 && p.D != 128) return HIPATTN_OK;
-  if (((uintptr_t)p.out % 16) || (p.o_stride_b % 8) || (p.o_stride_t % 8) || (p.o_stride_h % 8)) return HIPATTN_OK;
-  if (p.dtype == HIPATTN_BF16) return p.D == 128 ? dispatch<HIPATTN_BF16, 128>(p, stream, handled) : dispatch<HIPATTN_BF16, 64>(p, stream, handled);
-  if (p.dtype == HIPATTN_F16) return p.D == 128 ? dispatch<HIPATTN_F16, 128>(p, stream, handled) : dispatch<HIPATTN_F16, 64>(p, stream, handled);
-  return HIPATTN_OK;
+  int M, BQ, n_sub;
+  if (!mma_shape(p, &M, &BQ, &n_sub)) return HIPATTN_OK;
+  *handled = true;
+  if (p.dtype == HIPATTN_BF16)
+    return p.D == 128 ? dispatch<HIPATTN_BF16, 128>(p, M, BQ, n_sub, stream) : dispatch<HIPATTN_BF16, 64>(p, M, BQ, n_sub, stream);
+  return p.D == 128 ? dispatch<HIPATTN_F16, 128>(p, M, BQ, n_sub, stream) : dispatch<HIPATTN_F16, 64>(p, M, BQ, n_sub, stream);
 }
 
 }  // namespace hipattn

@@ -1,4 +1,4 @@
-// Block-sparse attention, prefill, 16-bit types, head dim 128: warp-specialised tcgen05 / TMEM kernel.
+// Block-sparse attention, prefill, 16-bit types, head dim 64 or 128: warp-specialised tcgen05 / TMEM kernel.
 //
 // One CTA (8 warps: four softmax, one MMA issuer, three copy warps) owns 128 query rows -- two heads
 // of a KV group x 64 rows, or one head x 128 rows -- and walks the key list [sink | selected blocks | window] in tiles of 64 keys.  Two CTAs
@@ -8,7 +8,7 @@
 //               canonical layouts, K-major), accumulator double buffered in TMEM
 //   softmax     thread t owns row t = TMEM lane t: tcgen05.ld of its 64 logits, admission rule,
 //               base-2 online softmax with a lazily updated maximum, P written back to TMEM
-//   O += P V    tcgen05.mma (M 128, N 128, K 16) x 4, A operand = P in TMEM, V staged row-major
+//   O += P V    tcgen05.mma (M 128, N head dim, K 16) x 4, A operand = P in TMEM, V staged row-major
 //               (MN-major operand)
 //
 // K / V rows are gathered with 16-byte cp.async through the page table directly into the swizzled
@@ -20,6 +20,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "bsa_common.cuh"
 #include "tcgen05_common.cuh"
@@ -29,7 +30,6 @@ namespace hipattn {
 namespace {
 
 constexpr int TK5 = 64;            // keys per tile
-constexpr int D5 = 128;            // head dimension
 constexpr float kLog2e = 1.4426950408889634f;
 // log2 of the growth of a row's maximum that triggers a rescale of O: P = 2^(s - m) stays below 2^13 in fp16 (largest
 // finite value 2^16) and 2^24 in bf16; O and the row sums are fp32.  A reference maximum that lags the true one costs no
@@ -165,12 +165,22 @@ __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64
       ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u));
 }
 
-template <int DT, bool ROPE>
+// KV8 = K and V rows are e5m2 bytes: the copy warps load them into registers, widen them (exactly) and store the 16-bit
+// operand tiles themselves.  P then goes to TMEM as two 16-bit terms (value rounded, and what the rounding left), each
+// multiplied with V, so that an fp8 cache keeps softmax weights of at least 16 significant bits: the general kernel, which
+// served it before, multiplies fp32 weights.  (2 x 3001 queries, RoPE: 12.2 ms there, 1.43 ms here; output 5e-5 apart.)
+// Head dim 64: the same roles with half the MMAs and copies per tile; 2 x 2999 queries of 16 heads 0.44 ms with mma.sync,
+// 0.24 ms here.
+// SPLIT = the grid may cut key lists into ranges (p.n_splits); the variant without is 2 % faster on grids that need none.
+template <int DT, int D, bool ROPE, bool KV8, bool SPLIT>
 __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bsa_params_t p, int BQ, int n_sub) {
   using T = typename Elem<DT>::type;
   constexpr int NT = 256;
-  constexpr int Q_BYTES = 2 * 128 * 128;
-  constexpr int KT_BYTES = 2 * TK5 * 128;
+  static_assert(D == 128 || (D == 64 && !ROPE), "in-kernel RoPE pairs the two 128-byte halves of a 256-byte row");
+  constexpr int KB = D / 64;                  // 128-byte blocks per row
+  constexpr int PIECES = D / 8;               // 16-byte pieces per row
+  constexpr int Q_BYTES = KB * 128 * 128;
+  constexpr int KT_BYTES = KB * TK5 * 128;
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   unsigned char* smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
@@ -196,6 +206,8 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
   const int NBLK = cdiv(p.TQ, p.block_size_q);
   const int hslots = p.H / NH;
   int64_t bid = blockIdx.x;
+  int split = 0;
+  if constexpr (SPLIT) { split = (int)(bid % p.n_splits); bid /= p.n_splits; }
   const int sub = (int)(bid % n_sub); bid /= n_sub;
   const int d = (int)(bid % NBLK); bid /= NBLK;
   const int hs = (int)(bid % hslots); bid /= hslots;
@@ -266,8 +278,8 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
   }
   // the query tile: one batch of asynchronous 16-byte copies per thread (rows beyond the block are zero-filled), so that
   // the tile costs one trip to memory instead of one per loop iteration
-  for (int i = tid; i < 128 * 16; i += NT) {
-    const int r = i >> 4, pc = i & 15;
+  for (int i = tid; i < 128 * PIECES; i += NT) {
+    const int r = i >> (D == 128 ? 4 : 3), pc = i & (PIECES - 1);
     const bool live = (r % BQ) < rows_here;
     const T* qp = reinterpret_cast<const T*>(p.q) + (int64_t)b * p.q_stride_b + (int64_t)(row_t0 + (live ? r % BQ : 0)) * p.q_stride_t +
                   (int64_t)(h0 + r / BQ) * p.q_stride_h + pc * 8;
@@ -275,7 +287,7 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
   }
   cp_async_commit();
   cp_async_wait<0>();
-  if (ROPE) {   // in-kernel RoPE: every query row at its own position (attention_extend_bsa.py:797-856)
+  if constexpr (ROPE) {   // in-kernel RoPE: every query row at its own position (attention_extend_bsa.py:797-856)
     __syncthreads();
     RopeTile<DT, 4> rq;   // 128 rows x 8 pieces over 256 threads: 32 rows per pass
     rq.fetch(p, 0, 128, tid, NT, [&](int r) { return s_rowpos[r]; });
@@ -286,10 +298,15 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
   const int pmin = s_mm[0], pmax = s_mm[1];
   const int rmin = s_mm[2], rmax = s_mm[3];
   const KeyList kl = make_key_list(p, b, h0, d, pmin, pmax);
-  const int n_tiles = cdiv(kl.total, TK5);
+  // the tiles of this CTA's key range (all of them unless the caller asked for key splits)
+  const int all_tiles = cdiv(kl.total, TK5);
+  const int per_split = SPLIT ? cdiv(all_tiles, p.n_splits) : all_tiles;
+  const int tile0 = SPLIT ? split * per_split : 0;
+  const int n_tiles = SPLIT ? max(0, min(per_split, all_tiles - tile0)) : all_tiles;
+  constexpr int EB = KV8 ? 1 : 2;   // bytes of a K / V element
   constexpr int FMT = DT == HIPATTN_BF16 ? 1 : 0;
   const uint32_t idesc_s = make_idesc(FMT, 128, TK5, 0);
-  const uint32_t idesc_o = make_idesc(FMT, 128, D5, 1);
+  const uint32_t idesc_o = make_idesc(FMT, 128, D, 1);
   const uint32_t tmem_o = tmem + 128;
 
   const char* kbase = (const char*)(p.k.cache ? p.k.cache : p.k.dense);
@@ -304,13 +321,13 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
   long long seq_len = 0;
   if (paged_fast)
     seq_len = p.k.seq_lens_is_i64 ? ((const int64_t*)p.k.cache_seq_lens)[b] : (long long)((const int32_t*)p.k.cache_seq_lens)[b];
-  const long long k_base_off = ((long long)b * p.k.stride_b + (long long)hkv * p.k.stride_h) * 2, k_step = p.k.stride_t * 2;
-  const long long v_base_off = ((long long)b * p.v.stride_b + (long long)hkv * p.v.stride_h) * 2, v_step = p.v.stride_t * 2;
+  const long long k_base_off = ((long long)b * p.k.stride_b + (long long)hkv * p.k.stride_h) * EB, k_step = p.k.stride_t * EB;
+  const long long v_base_off = ((long long)b * p.v.stride_b + (long long)hkv * p.v.stride_h) * EB, v_step = p.v.stride_t * EB;
   // requests the block start of entry e of `tile` (if it is a selected entry) into the tile's record; the copy joins
   // the calling thread's next commit group and must be consumed by the same thread
   auto prefetch_start = [&](int tile, int e) {
     if (tile >= n_tiles) return;
-    const int blk = selected_block_of(kl, tile * TK5 + e);
+    const int blk = selected_block_of(kl, (tile0 + tile) * TK5 + e);
     if (blk >= 0)
       asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(smem_u32(&meta[tile & 3].start[e])), "l"(kl.idx + blk));
   };
@@ -319,7 +336,7 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
     Meta5& m = meta[tile & 3];
     MetaS& ms = metas[tile & 7];
     bool w;
-    const int j = tile * TK5 + e;
+    const int j = (tile0 + tile) * TK5 + e;
     const int t = prefetched ? key_position_at(kl, j, m.start[e], &w) : key_position(kl, j, &w);
     ms.tpos[e] = t;
     ms.twin[e] = (t >= 0 && w) ? 1 : 0;
@@ -342,8 +359,8 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
             page = 0;
           }
         }
-        ko = (page * p.k.stride_page + (long long)off * p.k.stride_off + (long long)hkv * p.k.stride_ch) * 2;
-        vo = (page * p.v.stride_page + (long long)off * p.v.stride_off + (long long)hkv * p.v.stride_ch) * 2;
+        ko = (page * p.k.stride_page + (long long)off * p.k.stride_off + (long long)hkv * p.k.stride_ch) * EB;
+        vo = (page * p.v.stride_page + (long long)off * p.v.stride_off + (long long)hkv * p.v.stride_ch) * EB;
       } else {
         ko = token_row(p.k, b, t, hkv, 2, p.status) - kbase;
         vo = token_row(p.v, b, t, hkv, 2, p.status) - vbase;
@@ -368,24 +385,70 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
     // multiprocessor carries one of each per CTA.
     const bool k_role = warp != 6;
     const int ptid = warp == 5 ? lane : (warp == 7 ? 32 + lane : lane);   // 0..63 in the K group, 0..31 in the V warp
-    // K group: thread ptid copies piece ptid & 15 of rows (ptid >> 4) + 4 i, i < 16;
-    // V warp:  thread ptid copies piece ptid & 15 of rows (ptid >> 4) + 2 i, i < 32 (two batches of sixteen)
-    const int g_pc = ptid & 15, g_r0 = ptid >> 4;
-    // All sixteen row addresses of a batch are read first and the copies follow without a branch between them.
-    auto gather_rows = [&](const char* const* rowp, unsigned char* dst, int row0, int rstep) {
+    // K group: thread ptid copies piece ptid % PIECES of rows ptid / PIECES + i * 64 / PIECES;
+    // V warp:  the same with 32 threads, in batches of at most sixteen rows
+    constexpr int KSTEP = 64 / PIECES, KN = TK5 / KSTEP;        // rows apart, rows per thread (K group)
+    constexpr int VN = TK5 * PIECES / 32, VB = VN > 16 ? 2 : 1; // rows per thread and batches (V warp)
+    constexpr int VSTEP = VB * 32 / PIECES, NB = VN / VB;       // rows apart within a batch, rows per batch
+    static_assert(KN <= 16 && NB <= 16, "a batch of copies is at most sixteen rows");
+    const int g_pc = ptid & (PIECES - 1), g_r0 = ptid >> (D == 128 ? 4 : 3);
+    // All row addresses of a batch are read first and the copies follow without a branch between them.
+    auto gather_rows = [&](const char* const* rowp, unsigned char* dst, int row0, auto step, auto count) {
+      constexpr int S = decltype(step)::value, N = decltype(count)::value;
       const uint32_t d0 = smem_u32(dst) + (g_pc >> 3) * (TK5 * 128);
-      const char* o[16];
+      const char* o[N];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) o[i] = rowp[row0 + rstep * i];
+      for (int i = 0; i < N; ++i) o[i] = rowp[row0 + S * i];
 #pragma unroll
-      for (int i = 0; i < 16; ++i)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d0 + sw128(row0 + rstep * i, g_pc & 7)), "l"(o[i] + g_pc * 16));
+      for (int i = 0; i < N; ++i)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d0 + sw128(row0 + S * i, g_pc & 7)), "l"(o[i] + g_pc * 16));
     };
-    auto gather_k = [&](int tile) { gather_rows(meta[tile & 3].kptr, sK + (tile & 1) * KT_BYTES, g_r0, 4); };
-    auto gather_v = [&](int tile) {
-      gather_rows(meta[tile & 3].vptr, sV + (tile & 1) * KT_BYTES, g_r0, 4);
-      gather_rows(meta[tile & 3].vptr, sV + (tile & 1) * KT_BYTES, g_r0 + 2, 4);
+    using KStep = std::integral_constant<int, KSTEP>;
+    using KCount = std::integral_constant<int, KN>;
+    using VStep = std::integral_constant<int, VSTEP>;
+    using VCount = std::integral_constant<int, NB>;
+    // fp8 rows: eight bytes become one 16-byte piece.  The loads of a batch are all in flight before the first is used,
+    // and they are issued before the wait for the tile's buffer (load_rows8 / store_rows8).
+    auto load_rows8 = [&](const char* const* rowp, int row0, auto step, auto count, uint2* w) {
+      constexpr int S = decltype(step)::value, N = decltype(count)::value;
+#pragma unroll
+      for (int i = 0; i < N; ++i) w[i] = __ldg(reinterpret_cast<const uint2*>(rowp[row0 + S * i] + g_pc * 8));
     };
+    auto store_rows8 = [&](const uint2* w, unsigned char* dst, int row0, auto step, auto count) {
+      constexpr int S = decltype(step)::value, N = decltype(count)::value;
+      const uint32_t d0 = smem_u32(dst) + (g_pc >> 3) * (TK5 * 128);
+#pragma unroll
+      for (int i = 0; i < N; ++i) sts128(d0 + sw128(row0 + S * i, g_pc & 7), widen_fp8_e5m2<DT>(w[i]));
+    };
+    // K(tile) / V(tile) into its buffer once wait() says the buffer is free
+    auto gather_k = [&](int tile, auto wait) {
+      unsigned char* dst = sK + (tile & 1) * KT_BYTES;
+      if constexpr (KV8) {
+        uint2 w[KN];
+        load_rows8(meta[tile & 3].kptr, g_r0, KStep{}, KCount{}, w);
+        wait();
+        store_rows8(w, dst, g_r0, KStep{}, KCount{});
+      } else {
+        wait();
+        gather_rows(meta[tile & 3].kptr, dst, g_r0, KStep{}, KCount{});
+      }
+    };
+    auto gather_v = [&](int tile, auto wait) {
+      unsigned char* dst = sV + (tile & 1) * KT_BYTES;
+      if constexpr (KV8) {
+        uint2 w[VB][NB];
+#pragma unroll
+        for (int i = 0; i < VB; ++i) load_rows8(meta[tile & 3].vptr, g_r0 + i * (32 / PIECES), VStep{}, VCount{}, w[i]);
+        wait();
+#pragma unroll
+        for (int i = 0; i < VB; ++i) store_rows8(w[i], dst, g_r0 + i * (32 / PIECES), VStep{}, VCount{});
+      } else {
+        wait();
+#pragma unroll
+        for (int i = 0; i < VB; ++i) gather_rows(meta[tile & 3].vptr, dst, g_r0 + i * (32 / PIECES), VStep{}, VCount{});
+      }
+    };
+    auto no_wait = [] {};
     // all 96 producer threads; returns the OR of the arguments
     auto producer_sync_or = [&](bool v) -> bool {
       uint32_t r;
@@ -406,17 +469,17 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
     }
     producer_sync_or(false);
     if (k_role) {
-      for (int t = 0; t < 2 && t < n_tiles; ++t) gather_k(t);
+      for (int t = 0; t < 2 && t < n_tiles; ++t) gather_k(t, no_wait);
       prefetch_start(3, ptid);
       cp_async_commit();
       cp_async_wait<0>();
-      if (ROPE) {
+      if constexpr (ROPE) {
         for (int t = 0; t < 2 && t < n_tiles; ++t) rotate_k_front(t);
       }
       fence_async_smem();
       for (int t = 0; t < 2 && t < n_tiles; ++t) mbar_arrive((ROPE ? mbar_kraw0 : mbar_k0) + 8 * t);
     } else {
-      if (n_tiles > 0) gather_v(0);
+      if (n_tiles > 0) gather_v(0, no_wait);
       cp_async_commit();
     }
     __syncthreads();  // B0: Q is in place
@@ -424,8 +487,11 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
       if (k_role) {
         // K(it + 2) goes where K(it) was: wait until S(it) has been computed
         if (it + 2 < n_tiles) {
-          mbar_wait(mbar_s0 + 8 * (it & 1), (it >> 1) & 1, &s_abort, p.status);
-          gather_k(it + 2);
+          if constexpr (KV8) gather_k(it + 2, [&] { mbar_wait(mbar_s0 + 8 * (it & 1), (it >> 1) & 1, &s_abort, p.status); });
+          else {
+            mbar_wait(mbar_s0 + 8 * (it & 1), (it >> 1) & 1, &s_abort, p.status);
+            gather_rows(meta[(it + 2) & 3].kptr, sK + ((it + 2) & 1) * KT_BYTES, g_r0, KStep{}, KCount{});
+          }
         }
         prefetch_start(it + 4, ptid);   // block start of this thread's entry of tile it + 4, used one tile from now
         cp_async_commit();
@@ -444,8 +510,11 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
         mbar_arrive(mbar_v0 + 8 * (it & 1));   // V(it) is in place
         // V(it + 1) goes where V(it - 1) was: wait until PV(it - 1) has completed
         if (it + 1 < n_tiles) {
-          if (it >= 1) mbar_wait(mbar_o(it - 1), phase_o(it - 1), &s_abort, p.status);
-          gather_v(it + 1);
+          if constexpr (KV8) gather_v(it + 1, [&] { if (it >= 1) mbar_wait(mbar_o(it - 1), phase_o(it - 1), &s_abort, p.status); });
+          else {
+            if (it >= 1) mbar_wait(mbar_o(it - 1), phase_o(it - 1), &s_abort, p.status);
+            gather_v(it + 1, no_wait);
+          }
         }
         cp_async_commit();
       }
@@ -462,7 +531,7 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
       const uint32_t kb = k_lo + (tile & 1) * (KT_BYTES >> 4);
       const uint32_t ts = tmem + (tile & 1) * 64;
 #pragma unroll
-      for (int kk = 0; kk < 8; ++kk) {
+      for (int kk = 0; kk < D / 16; ++kk) {
         const uint32_t off = (kk >> 2) * ((128 * 128) >> 4) + (kk & 3) * 2;
         const uint32_t offk = (kk >> 2) * ((TK5 * 128) >> 4) + (kk & 3) * 2;
         umma(ts, dk | (uint64_t)((q_lo + off) & 0x3fffu), dk | (uint64_t)((kb + offk) & 0x3fffu), idesc_s, kk > 0);
@@ -490,6 +559,10 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
           umma_ts(tmem_o, tp + kk * 8, dv | (uint64_t)((vb + kk * 128) & 0x3fffu), idesc_o, (it > 0 || kk > 0) ? 1u : 0u);
+        if (KV8) {   // the weights' second terms
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk) umma_ts(tmem_o, tp + 32 + kk * 8, dv | (uint64_t)((vb + kk * 128) & 0x3fffu), idesc_o, 1u);
+        }
         umma_commit(mbar_o(it));
         if (it + 2 < n_tiles) {
           if (!mbar_wait(mbar_k0 + 8 * (it & 1), ((it + 2) >> 1) & 1, &s_abort, p.status)) break;   // K(it + 2) is in place
@@ -549,7 +622,7 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
           __syncwarp();
           tc_fence_after();
 #pragma unroll 1
-          for (int c = 0; c < D5; c += 32) {
+          for (int c = 0; c < D; c += 32) {
             float o[32];
             tmem_ld32(tmem_o + lane_base + c, o);
 #pragma unroll
@@ -567,7 +640,7 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
       // the scaling and the row sum run two values per instruction
       const unsigned long long scale2 = f32x2(kLog2e, kLog2e), nbase2 = f32x2(-base, -base);
       unsigned long long sum2[4] = {0ull, 0ull, 0ull, 0ull};
-      float pk[32];
+      float pk[32], pk2[KV8 ? 32 : 1];
 #pragma unroll
       for (int j = 0; j < TK5; j += 2) {
         float x0, x1;
@@ -575,6 +648,11 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
         const float e0 = exp2_approx(x0), e1 = exp2_approx(x1);
         const uint32_t w = pack2<DT>(e0, e1);
         pk[j >> 1] = __uint_as_float(w);
+        if constexpr (KV8) {
+          pk2[j >> 1] = __uint_as_float(pack2<DT>(e0 - pair_lo<DT>(w), e1 - pair_hi<DT>(w)));
+          sum2[(j >> 1) & 3] = add_f32x2(sum2[(j >> 1) & 3], f32x2(e0, e1));
+          continue;
+        }
         // the row sum takes the ROUNDED weights, the ones P V is computed with: numerator and denominator then carry the
         // same rounding of a row's largest terms and it cancels in O / l
         sum2[(j >> 1) & 3] = add_f32x2(sum2[(j >> 1) & 3], f32x2(pair_lo<DT>(w), pair_hi<DT>(w)));
@@ -585,6 +663,7 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
         (void)b0; (void)b1;
         l_run += a0 + a1;
       }
+      if constexpr (KV8) tmem_st32<false>(ts + 32, pk2);   // ... and the second terms over the other half
       tmem_st32(ts, pk);        // P(it) over the first half of S(it)
       tc_fence_before();
       if (__any_sync(0xffffffffu, s_abort != 0)) break;   // warp-uniform: the TMEM accesses are warp-collective
@@ -601,13 +680,22 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
     const bool warp_ok = __all_sync(0xffffffffu, ok);
     const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
 #pragma unroll 1
-    for (int c = 0; c < D5; c += 32) {
+    for (int c = 0; c < D; c += 32) {
       float o[32];
       if (warp_ok) {
         tmem_ld32(tmem_o + lane_base + c, o);
       } else {
 #pragma unroll
         for (int j = 0; j < 32; ++j) o[j] = 0.f;
+      }
+      if (SPLIT && p.n_splits > 1) {   // a normalised fp32 partial row per key range, merged by merge_kernel
+        if ((tid % BQ) < rows_here) {
+          float* po = p.part_o + ((((int64_t)b * p.TQ + row_t0 + tid % BQ) * p.H + h0 + tid / BQ) * p.n_splits + split) * D + c;
+#pragma unroll
+          for (int j = 0; j < 32; j += 4)
+            *reinterpret_cast<float4*>(po + j) = make_float4(o[j] * inv, o[j + 1] * inv, o[j + 2] * inv, o[j + 3] * inv);
+        }
+        continue;
       }
 #pragma unroll
       for (int j = 0; j < 32; j += 8) {
@@ -618,13 +706,16 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
         *reinterpret_cast<uint4*>(sQ + (pc >> 3) * (128 * 128) + sw128(tid, pc & 7)) = w;
       }
     }
-    if (p.lse_out && (tid % BQ) < rows_here)
+    if (SPLIT && p.n_splits > 1 && (tid % BQ) < rows_here)
+      p.part_lse[(((int64_t)b * p.TQ + row_t0 + tid % BQ) * p.H + h0 + tid / BQ) * p.n_splits + split] =
+          l_run > 0.f ? m_ref + log2f(l_run) : -INFINITY;
+    if ((!SPLIT || p.n_splits == 1) && p.lse_out && (tid % BQ) < rows_here)
       p.lse_out[((int64_t)b * p.TQ + row_t0 + tid % BQ) * p.H + h0 + tid / BQ] = l_run > 0.f ? m_ref + log2f(l_run) : -INFINITY;
     tc_fence_before();
   }
   __syncthreads();  // all roles: output rows staged, every TMEM access finished
-  for (int i = tid; i < 128 * 16; i += NT) {
-    const int r = i >> 4, pc = i & 15;
+  for (int i = tid; i < 128 * PIECES && (!SPLIT || p.n_splits == 1); i += NT) {
+    const int r = i >> (D == 128 ? 4 : 3), pc = i & (PIECES - 1);
     if ((r % BQ) < rows_here) {
       T* op = reinterpret_cast<T*>(p.out) + (int64_t)b * p.o_stride_b + (int64_t)(row_t0 + r % BQ) * p.o_stride_t +
               (int64_t)(h0 + r / BQ) * p.o_stride_h + pc * 8;
@@ -637,14 +728,14 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
   }
 }
 
-template <int DT, bool ROPE>
+template <int DT, int D, bool ROPE, bool KV8, bool SPLIT>
 int launch5_ws(const hipattn_bsa_params_t& p, int BQ, int n_sub, cudaStream_t stream) {
-  const size_t smem = 1024 + 2 * 128 * 128 + 4 * (2 * TK5 * 128) + 4 * sizeof(Meta5) + 8 * sizeof(MetaS);
+  const size_t smem = 1024 + (D / 64) * (128 * 128 + 4 * TK5 * 128) + 4 * sizeof(Meta5) + 8 * sizeof(MetaS);
   const int NH = 128 / BQ;
   const int NBLK = cdiv(p.TQ, p.block_size_q);
-  const int64_t grid = (int64_t)p.B * (p.H / NH) * NBLK * n_sub;
+  const int64_t grid = (int64_t)p.B * (p.H / NH) * NBLK * n_sub * p.n_splits;
   HIPATTN_REQUIRE(grid > 0 && grid < 0x7fffffffLL, HIPATTN_ERR_INVALID, "attention grid of %lld blocks", (long long)grid);
-  auto kern = bsa_tcgen05_ws_kernel<DT, ROPE>;
+  auto kern = bsa_tcgen05_ws_kernel<DT, D, ROPE, KV8, SPLIT>;
   HIPATTN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kern<<<(unsigned)grid, 256, smem, stream>>>(p, BQ, n_sub);
   return check_launch("bsa_tcgen05_ws_kernel");
@@ -672,21 +763,46 @@ int bounded_wait_probe(uint32_t* status, cudaStream_t stream) {
   return check_launch("bounded_wait_probe_kernel");
 }
 
-// Takes 16-bit prefill with head dim 128 and attention blocks of 64 rows (two heads of a KV group that
-// share their key list per CTA) or a multiple of 128 rows.
+// Rows per CTA and CTAs per attention block, or false: 16-bit prefill with head dim 64 or 128 and attention blocks of 64 rows
+// (two heads of a KV group that share their key list per CTA) or a multiple of 128 rows.
+static bool tcgen05_shape(const hipattn_bsa_params_t& p, int* BQ, int* n_sub) {
+  if (p.dtype == HIPATTN_F32 || (p.D != 128 && (p.D != 64 || p.rope_cos)) || p.TQ < 64) return false;
+  if (p.k.fp8_e5m2 != p.v.fp8_e5m2) return false;
+  if (p.out && (((uintptr_t)p.out % 16) || (p.o_stride_b % 8) || (p.o_stride_t % 8) || (p.o_stride_h % 8))) return false;
+  const int Gq = p.H / p.HKV;
+  if (p.block_size_q == 64 && p.heads_share_mask && (Gq % 2) == 0) { *BQ = 64; *n_sub = 1; return true; }
+  if (p.block_size_q % 128 == 0) { *BQ = 128; *n_sub = p.block_size_q / 128; return true; }
+  return false;
+}
+
+// CTAs of the kernel without key splits, and how many the GPU holds at once (0: another kernel takes the call)
+int64_t bsa_tcgen05_ctas(const hipattn_bsa_params_t& p, int* resident, int* tile_keys) {
+  int BQ, n_sub;
+  if (!tcgen05_shape(p, &BQ, &n_sub)) return 0;
+  *resident = 148 * 2;
+  *tile_keys = TK5;
+  return (int64_t)p.B * (p.H / (128 / BQ)) * cdiv(p.TQ, p.block_size_q) * n_sub;
+}
+
+template <int DT>
+static int launch5(const hipattn_bsa_params_t& p, int BQ, int n_sub, cudaStream_t stream) {
+  const bool split = p.n_splits > 1;
+  if (p.D == 64) {
+    if (p.k.fp8_e5m2) return launch5_ws<DT, 64, false, true, true>(p, BQ, n_sub, stream);
+    return split ? launch5_ws<DT, 64, false, false, true>(p, BQ, n_sub, stream) : launch5_ws<DT, 64, false, false, false>(p, BQ, n_sub, stream);
+  }
+  if (p.k.fp8_e5m2)
+    return p.rope_cos ? launch5_ws<DT, 128, true, true, true>(p, BQ, n_sub, stream) : launch5_ws<DT, 128, false, true, true>(p, BQ, n_sub, stream);
+  if (p.rope_cos) return launch5_ws<DT, 128, true, false, true>(p, BQ, n_sub, stream);
+  return split ? launch5_ws<DT, 128, false, false, true>(p, BQ, n_sub, stream) : launch5_ws<DT, 128, false, false, false>(p, BQ, n_sub, stream);
+}
+
 int bsa_tcgen05(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled) {
   *handled = false;
-  if (p.n_splits != 1 || p.dtype == HIPATTN_F32 || p.D != 128 || p.TQ < 64) return HIPATTN_OK;
-  if (((uintptr_t)p.out % 16) || (p.o_stride_b % 8) || (p.o_stride_t % 8) || (p.o_stride_h % 8)) return HIPATTN_OK;
-  const int Gq = p.H / p.HKV;
   int BQ, n_sub;
-  if (p.block_size_q == 64 && p.heads_share_mask && (Gq % 2) == 0) { BQ = 64; n_sub = 1; }
-  else if (p.block_size_q % 128 == 0) { BQ = 128; n_sub = p.block_size_q / 128; }
-  else return HIPATTN_OK;
+  if (!tcgen05_shape(p, &BQ, &n_sub)) return HIPATTN_OK;
   *handled = true;
-  if (p.rope_cos)
-    return p.dtype == HIPATTN_BF16 ? launch5_ws<HIPATTN_BF16, true>(p, BQ, n_sub, stream) : launch5_ws<HIPATTN_F16, true>(p, BQ, n_sub, stream);
-  return p.dtype == HIPATTN_BF16 ? launch5_ws<HIPATTN_BF16, false>(p, BQ, n_sub, stream) : launch5_ws<HIPATTN_F16, false>(p, BQ, n_sub, stream);
+  return p.dtype == HIPATTN_BF16 ? launch5<HIPATTN_BF16>(p, BQ, n_sub, stream) : launch5<HIPATTN_F16>(p, BQ, n_sub, stream);
 }
 
 }  // namespace hipattn

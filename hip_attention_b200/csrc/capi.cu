@@ -50,9 +50,17 @@ int bsa_generic(const hipattn_bsa_params_t& p, cudaStream_t stream);
 int bsa_mma(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled);
 int bsa_decode(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled);
 int bsa_tcgen05(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled);
+int64_t bsa_tcgen05_ctas(const hipattn_bsa_params_t& p, int* resident, int* tile_keys);
+int64_t bsa_mma_ctas(const hipattn_bsa_params_t& p, int* resident, int* tile_keys);
 int bounded_wait_probe(uint32_t* status, cudaStream_t stream);
 
 namespace {
+
+// HIPATTN_PREFILL_KERNEL = tcgen05 (default: warp-specialised tcgen05 kernel) | mma (mma.sync kernel, for comparisons)
+bool tcgen05_prefill() {
+  const char* pk = getenv("HIPATTN_PREFILL_KERNEL");
+  return !(pk && strcmp(pk, "mma") == 0);
+}
 
 template <int DT>
 __global__ void merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse, int n_parts, int D,
@@ -147,8 +155,7 @@ extern "C" int hipattn_bsa_attention(const hipattn_bsa_params_t* p, void* stream
                   "attention: bad mask geometry");
   HIPATTN_REQUIRE(p->n_splits >= 1 && p->n_splits <= 64, HIPATTN_ERR_INVALID, "attention: n_splits %d outside [1, 64]", p->n_splits);
   if (p->n_splits > 1) {
-    HIPATTN_REQUIRE(p->TQ == 1 && p->part_o && p->part_lse, HIPATTN_ERR_INVALID,
-                    "attention: key splits need TQ == 1 and the part_o / part_lse buffers");
+    HIPATTN_REQUIRE(p->part_o && p->part_lse, HIPATTN_ERR_INVALID, "attention: key splits need the part_o / part_lse buffers");
   } else {
     HIPATTN_REQUIRE(p->out != nullptr, HIPATTN_ERR_INVALID, "attention: out is null");
   }
@@ -160,43 +167,74 @@ extern "C" int hipattn_bsa_attention(const hipattn_bsa_params_t* p, void* stream
   if (rc) return rc;
   rc = validate_tokens(p->v, eb, p->D, "v");
   if (rc) return rc;
-  if (p->k.fp8_e5m2 || p->v.fp8_e5m2) {
-    // an fp8 KV cache is read by the general kernel (prefill and decode, key splits included), RoPE or not
-    if (p->rope_cos || p->rope_sin)
-      HIPATTN_REQUIRE(p->rope_cos && p->rope_sin && p->rope_rows > 0, HIPATTN_ERR_INVALID, "attention: cos and sin tables go together");
-    return bsa_generic(*p, (cudaStream_t)stream);
-  }
   if (p->rope_cos || p->rope_sin) {
-    // in-kernel RoPE is built into the tcgen05 prefill kernel (head dim 128), the mma.sync decode and prefill kernels
-    // (16-bit, head dim 64 / 128) and the general kernel (everything else)
     HIPATTN_REQUIRE(p->rope_cos && p->rope_sin && p->rope_rows > 0, HIPATTN_ERR_INVALID, "attention: cos and sin tables go together");
     HIPATTN_REQUIRE(((uintptr_t)p->rope_cos % 16) == 0 && ((uintptr_t)p->rope_sin % 16) == 0 && p->rope_stride % ra == 0 &&
                         p->rope_stride >= p->D / 2,
                     HIPATTN_ERR_INVALID, "attention: cos / sin rows must start on 16-byte boundaries and hold D / 2 columns");
-    bool done = false;
-    rc = bsa_decode(*p, (cudaStream_t)stream, &done);
-    if (done) return rc;
-    const char* pk_ = getenv("HIPATTN_PREFILL_KERNEL");
-    if (!(pk_ && strcmp(pk_, "mma") == 0)) {
-      rc = bsa_tcgen05(*p, (cudaStream_t)stream, &done);
-      if (done) return rc;
-    }
-    rc = bsa_mma(*p, (cudaStream_t)stream, &done);
-    if (done) return rc;
-    return bsa_generic(*p, (cudaStream_t)stream);
   }
+  // In-kernel RoPE: the mma.sync decode and prefill kernels and (head dim 128) the tcgen05 prefill kernel.  An fp8 KV
+  // cache: the tcgen05 prefill kernel.  What none of them takes is the general kernel's.
   bool handled = false;
   rc = bsa_decode(*p, (cudaStream_t)stream, &handled);
   if (handled) return rc;
-  // HIPATTN_PREFILL_KERNEL = tcgen05 (default: warp-specialised tcgen05 kernel) | mma (mma.sync kernel, for comparisons)
-  const char* pk = getenv("HIPATTN_PREFILL_KERNEL");
-  if (!(pk && strcmp(pk, "mma") == 0)) {
+  if (tcgen05_prefill()) {
     rc = bsa_tcgen05(*p, (cudaStream_t)stream, &handled);
     if (handled) return rc;
   }
   rc = bsa_mma(*p, (cudaStream_t)stream, &handled);
   if (handled) return rc;
   return bsa_generic(*p, (cudaStream_t)stream);
+}
+
+// Key ranges for hipattn_bsa_attention.
+extern "C" int32_t hipattn_attention_splits(const hipattn_bsa_params_t* p) {
+  if (p == nullptr || p->B <= 0 || p->TQ <= 0 || p->H <= 0 || p->HKV <= 0 || p->H % p->HKV || p->block_size_q <= 0) return 1;
+  if (const char* forced = getenv(p->TQ == 1 ? "HIPATTN_DECODE_SPLITS" : "HIPATTN_PREFILL_SPLITS"); forced && *forced) {
+    const int n = atoi(forced);
+    return n < 1 ? 1 : (n > 64 ? 64 : n);
+  }
+  // most keys a block can attend: sink, selected blocks, the window of its first to its last row
+  const int64_t keys = (int64_t)(p->sink < p->T ? p->sink : p->T) + (int64_t)p->K * p->block_size_k +
+                       ((int64_t)p->window + p->block_size_q - 1 < p->T ? (int64_t)p->window + p->block_size_q - 1 : p->T);
+  if (p->TQ == 1) {
+    // Decode: one range when the batch alone fills the GPU; otherwise enough ranges for two CTAs per multiprocessor,
+    // each at least four tiles (256 keys) long.
+    const int64_t units = (int64_t)p->B * p->HKV;
+    if (units >= 148) return 1;
+    int64_t n = (148 * 2 + units - 1) / units;
+    if (n > keys / 256) n = keys / 256;
+    if (n > 32) n = 32;
+    return n < 1 ? 1 : (int32_t)n;
+  }
+  int resident = 0, tile_keys = 64;
+  int64_t ctas = tcgen05_prefill() ? bsa_tcgen05_ctas(*p, &resident, &tile_keys) : 0;
+  if (ctas == 0) ctas = bsa_mma_ctas(*p, &resident, &tile_keys);
+  if (ctas == 0) {   // the general kernel: 64-row tiles, one or two CTAs per multiprocessor
+    const int64_t blocks = (p->TQ + p->block_size_q - 1) / p->block_size_q;
+    ctas = (int64_t)p->B * p->H * blocks * ((p->block_size_q + 63) / 64);
+    resident = 148 * 2;
+    tile_keys = 32;
+  }
+  if (ctas == 0 || ctas >= 4 * (int64_t)resident) return 1;
+  // Prefill: the schedule's length in tiles = waves of CTAs x (tiles of a range + what a CTA costs before and after its
+  // tiles), the merge of the partial rows included.  A grid that fills the GPU keeps one range; the last queries of a
+  // prompt, which attend the whole context (16 CTAs of 1400 tiles: 3.5 ms), are cut into as many ranges as the GPU
+  // has room for (0.3 ms).
+  const int64_t tiles = (keys + tile_keys - 1) / tile_keys;
+  auto cost = [&](int64_t n) {
+    return (double)((ctas * n + resident - 1) / resident) * (double)((tiles + n - 1) / n + 6) + (n > 1 ? 6.0 : 0.0);
+  };
+  const double whole = cost(1);
+  double best = whole * 0.9;
+  int pick = 1;
+  for (int n = 2; n <= 64 && n * 4 <= tiles; ++n) {
+    if (cost(n) < best) {
+      best = cost(n);
+      pick = n;
+    }
+  }
+  return pick;
 }
 
 extern "C" int hipattn_merge_partials(const float* part_o, const float* part_lse, int64_t rows, int32_t n_parts, int32_t D,

@@ -434,18 +434,6 @@ def _restart_inputs(entry: HiPAttentionStageInputCache, rows: int) -> Tuple[Tens
     return l, r
 
 
-def _decode_splits(B: int, HKV: int, total_tokens: int) -> int:
-    """Key ranges per (sequence, KV head).  One range when the batch alone fills the GPU (two CTAs per
-    SM); otherwise enough ranges to do so, each at least four tiles (256 keys) long."""
-    forced = os.environ.get("HIPATTN_DECODE_SPLITS")
-    if forced:
-        return max(1, min(64, int(forced)))
-    units = max(1, B * HKV)
-    if units >= 148:
-        return 1
-    return int(max(1, min(32, _cdiv(148 * 2, units), total_tokens // 256)))
-
-
 def _attention(q: Tensor, ktok: L.Tokens, vtok: L.Tokens, T: int, HKV: int, pos: Tensor, indices: Tensor, ks: Tensor,
                *, sink: int, window: int, block_size_k: int, bsa_block_q: int, index_block_q: int, heads_share: bool,
                decode: bool, softcap: Optional[float], want_lse: bool,
@@ -478,17 +466,18 @@ def _attention(q: Tensor, ktok: L.Tokens, vtok: L.Tokens, T: int, HKV: int, pos:
     if access is not None:   # which tokens / pages the attention loads (require_cache_statistics)
         L.check(lib.hipattn_mark_attention_access(C.byref(bp), access.data_ptr(), access.stride(0), access.stride(1),
                                                   access.shape[-1], 1 if decode else bsa_block_q, st), "mark_attention_access")
-    n_splits = _decode_splits(B, HKV, K * block_size_k + sink + window) if decode else 1
+    # key ranges: a single query row that is not a decode call keeps one (its heads may have masks of their own)
+    n_splits = lib.hipattn_attention_splits(C.byref(bp)) if decode or TQ > 1 else 1
     bp.n_splits = n_splits
     if n_splits > 1:
-        part_o = torch.empty((B, H, n_splits, D), dtype=torch.float32, device=dev)
-        part_lse = torch.empty((B, H, n_splits), dtype=torch.float32, device=dev)
+        part_o = torch.empty((B, TQ, H, n_splits, D), dtype=torch.float32, device=dev)
+        part_lse = torch.empty((B, TQ, H, n_splits), dtype=torch.float32, device=dev)
         bp.part_o, bp.part_lse = part_o.data_ptr(), part_lse.data_ptr()
         L.check(lib.hipattn_bsa_attention(C.byref(bp), st), "bsa_attention")
         o2 = out.view(B * TQ, H, D)
         if o2.stride(1) != D or o2.stride(0) != H * D:
             raise AssertionError("freshly allocated output must be contiguous")
-        L.check(lib.hipattn_merge_partials(_ptr(part_o), _ptr(part_lse), B * H, n_splits, D, _DT[q.dtype], out.data_ptr(),
+        L.check(lib.hipattn_merge_partials(_ptr(part_o), _ptr(part_lse), B * TQ * H, n_splits, D, _DT[q.dtype], out.data_ptr(),
                                            D, _ptr(lse), st), "merge_partials")
     else:
         bp.lse_out = _ptr(lse)

@@ -210,9 +210,10 @@ int hipattn_finalize_indices(const int32_t* score_max, const int32_t* left_heads
  * block_sparse_attention_cuda_step (attention_extend_bsa.py:511-565).
  *
  * n_splits == 1: writes out [B, TQ, H, D] in the element type.
- * n_splits  > 1: (decode, TQ == 1) the key set is cut into n_splits ranges; split s writes the
- *   normalised partial output part_o [B, H, n_splits, D] fp32 and its base-2 log-sum-exp part_lse
- *   [B, H, n_splits] (-inf for an empty range), to be combined by hipattn_merge_partials.
+ * n_splits  > 1: every block's key list is cut into n_splits ranges; range s writes the normalised partial
+ *   output part_o [B, TQ, H, n_splits, D] fp32 and its base-2 log-sum-exp part_lse [B, TQ, H, n_splits]
+ *   (-inf for an empty range), to be combined by hipattn_merge_partials.  hipattn_attention_splits
+ *   gives a good number for the call.
  * lse_out (optional) [B, TQ, H] fp32 receives the base-2 log-sum-exp of every row (n_splits == 1).
  */
 typedef struct hipattn_bsa_params {
@@ -250,6 +251,13 @@ typedef struct hipattn_bsa_params {
 } hipattn_bsa_params_t;
 
 int hipattn_bsa_attention(const hipattn_bsa_params_t* p, void* stream);
+
+/*
+ * How many key ranges (n_splits, 1..64) fill the GPU best for this call; reads the shapes, the mask geometry and the
+ * addresses and strides of `out`, launches nothing.  HIPATTN_DECODE_SPLITS / HIPATTN_PREFILL_SPLITS in the environment fix
+ * it for calls with one query row / more.
+ */
+int32_t hipattn_attention_splits(const hipattn_bsa_params_t* p);
 
 /*
  * Access statistics of the attention (the `sa` counter of require_cache_statistics): writes 1 into counter
