@@ -326,6 +326,7 @@ int dispatch_dim(const hipattn_scan_params_t& p, cudaStream_t stream) {
 int scan_stage_mma(const hipattn_scan_params_t& p, cudaStream_t stream, bool* handled);
 int scan_stage_tcgen05(const hipattn_scan_params_t& p, cudaStream_t stream, bool* handled);
 int scan_chunks_strict(const hipattn_scan_params_t& p, cudaStream_t stream, bool* handled);
+int scan_chunks_mma(const hipattn_scan_params_t& p, cudaStream_t stream, bool* handled);
 int scan_prepare_keys(const hipattn_tokens_t& k, int dtype, int D, int B, int T, int HKV, float k_scale, float* key_abs,
                       void* k_scaled, uint32_t* status, cudaStream_t stream, const void* rope_cos = nullptr,
                       const void* rope_sin = nullptr, int64_t rope_stride = 0, int rope_rows = 0, int rope_position = 0);
@@ -364,6 +365,8 @@ extern "C" int hipattn_scan_stage(const hipattn_scan_params_t* p, void* stream) 
     HIPATTN_REQUIRE(((uintptr_t)p->rope_cos % 16) == 0 && ((uintptr_t)p->rope_sin % 16) == 0 && p->rope_stride % ra == 0 &&
                         p->rope_stride >= p->D / 2,
                     HIPATTN_ERR_INVALID, "scan stage: cos / sin rows must start on 16-byte boundaries and hold D / 2 columns");
+    rc = scan_chunks_mma(*p, s, &handled);   // decode, small chunks
+    if (handled) return rc;
     if (p->rope_mode == HIPATTN_ROPE_STREAMING) {   // decode: every token of a chunk is rotated to the chunk's index
       rc = scan_chunks_strict(*p, s, &handled);
       if (handled) return rc;
@@ -375,6 +378,8 @@ extern "C" int hipattn_scan_stage(const hipattn_scan_params_t* p, void* stream) 
       if (handled) return rc;
     }
   } else {
+  rc = scan_chunks_mma(*p, s, &handled);
+  if (handled) return rc;
   rc = scan_chunks_strict(*p, s, &handled);
   if (handled) return rc;
   rc = scan_stage_tcgen05(*p, s, &handled);
