@@ -1,19 +1,22 @@
-"""Build libhipattn_sm100.so in-tree with nvcc (sm_100a only).
+"""Build libhipattn_sm100.so in-tree with nvcc (sm_100a only), and the host extension over it with g++.
 
     python -m hip_attention_b200.build [--force] [--verbose]
 """
 from __future__ import annotations
 
 import os
+import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libhipattn_sm100.so")
-SOURCES = ["capi.cu", "scan_stage.cu", "scan_stage_mma.cu", "scan_stage_tcgen05.cu", "scan_chunks_strict.cu", "scan_chunks_mma.cu", "select.cu", "bsa_generic.cu", "bsa_mma.cu", "bsa_tcgen05.cu", "bsa_decode.cu", "decode_noalloc.cu"]
-HEADERS = ["common.cuh", "bsa_common.cuh", "scan_common.cuh", "mma_common.cuh", "tcgen05_common.cuh", "rope.cuh", os.path.join("..", "..", "include", "hipattn.h")]
+HOST = os.path.join(PKG, "_host.so")   # CPython extension: the host path of a call, linked to LIB
+SOURCES = ["capi.cu", "scan_stage.cu", "scan_stage_mma.cu", "scan_stage_tcgen05.cu", "scan_chunks_strict.cu", "scan_chunks_mma.cu", "select.cu", "bsa_generic.cu", "bsa_mma.cu", "bsa_tcgen05.cu", "bsa_decode.cu", "decode_noalloc.cu", "host_kernels.cu"]
+HEADERS = ["common.cuh", "host_kernels.h", "bsa_common.cuh", "scan_common.cuh", "mma_common.cuh", "tcgen05_common.cuh", "rope.cuh", os.path.join("..", "..", "include", "hipattn.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "--use_fast_math=false"]
 
@@ -58,6 +61,17 @@ def build(force: bool = False, verbose: bool = False) -> str:
                 print(out)
     if jobs or force or _stale(LIB, objs):
         run([nvcc, "-shared", "-o", LIB, *objs, "-gencode", "arch=compute_100a,code=sm_100a", "-lcudart"])
+    host_src = os.path.join(CSRC, "host.cpp")
+    if force or jobs or _stale(HOST, [host_src, os.path.join(CSRC, "host_kernels.h"), hdrs[-1], LIB]):
+        import torch
+        root = os.path.dirname(torch.__file__)
+        cuda = os.path.dirname(os.path.dirname(os.path.realpath(shutil.which(nvcc) or nvcc)))
+        run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", host_src, "-o", HOST,
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+             *(f"-I{d}" for d in (os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+                                  sysconfig.get_paths()["include"], os.path.join(cuda, "include"))),
+             f"-L{PKG}", "-l:libhipattn_sm100.so", "-Wl,-rpath,$ORIGIN",
+             f"-L{os.path.join(root, 'lib')}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch_python"])
     return LIB
 
 

@@ -5,6 +5,7 @@
 // composite 64-bit keys (inverted score image << 32 | position), which makes the order total:
 // higher score first, lower chunk position first among equal scores.
 #include "common.cuh"
+#include "host_kernels.h"
 
 namespace hipattn {
 namespace {
@@ -60,7 +61,9 @@ __global__ void __launch_bounds__(kSortThreads) select_stage_kernel(const int32_
                                                                     int k_keep, int k_pad, int sink, int c_prev,
                                                                     int c_next, int32_t* __restrict__ next_left,
                                                                     int32_t* __restrict__ next_right,
-                                                                    int32_t* __restrict__ next_score_max) {
+                                                                    int32_t* __restrict__ next_score_max,
+                                                                    int64_t* __restrict__ next_left64,
+                                                                    int64_t* __restrict__ next_right64) {
   extern __shared__ __align__(16) unsigned char smem[];
   unsigned long long* keys = reinterpret_cast<unsigned long long*>(smem);
   const int64_t row = blockIdx.x;
@@ -91,8 +94,11 @@ __global__ void __launch_bounds__(kSortThreads) select_stage_kernel(const int32_
     const int ra = la + c_prev;
     // attention_extend.py:2133-2165: chunk sizes and offsets go through fp32
     const float w = fmaxf(__fdiv_rn((float)(ra - la), (float)s), 0.f);
-    next_left[row * out_n + o] = la + (int)floorf(__fmul_rn((float)i, w));
-    next_right[row * out_n + o] = ra - (int)floorf(__fmul_rn((float)(s - 1 - i), w));
+    const int nl = la + (int)floorf(__fmul_rn((float)i, w)), nr = ra - (int)floorf(__fmul_rn((float)(s - 1 - i), w));
+    next_left[row * out_n + o] = nl;
+    next_right[row * out_n + o] = nr;
+    if (next_left64) next_left64[row * out_n + o] = nl;
+    if (next_right64) next_right64[row * out_n + o] = nr;
     next_score_max[row * out_n + o] = init;
   }
 }
@@ -198,9 +204,9 @@ extern "C" int hipattn_init_chunks(int32_t* left, int32_t* right, int32_t* score
   return check_launch("init_chunks_kernel");
 }
 
-extern "C" int hipattn_select_stage(const int32_t* score_max, const int32_t* left, int64_t rows, int32_t n, int32_t k_keep,
-                                    int32_t sink, int32_t c_prev, int32_t c_next, int32_t* next_left,
-                                    int32_t* next_right, int32_t* next_score_max, void* stream) {
+int hipattn::select_stage(const int32_t* score_max, const int32_t* left, int64_t rows, int32_t n, int32_t k_keep, int32_t sink,
+                          int32_t c_prev, int32_t c_next, int32_t* next_left, int32_t* next_right, int32_t* next_score_max,
+                          int64_t* next_left64, int64_t* next_right64, cudaStream_t stream) {
   HIPATTN_REQUIRE(score_max && left && next_left && next_right && next_score_max, HIPATTN_ERR_INVALID,
                   "select_stage: null pointer");
   HIPATTN_REQUIRE(rows > 0 && n > 0 && k_keep > 0 && k_keep <= n, HIPATTN_ERR_INVALID,
@@ -212,9 +218,17 @@ extern "C" int hipattn_select_stage(const int32_t* score_max, const int32_t* lef
   const int n_pad = next_pow2(n < 2 ? 2 : n), k_pad = next_pow2(k_keep < 2 ? 2 : k_keep);
   const size_t smem = (size_t)n_pad * sizeof(unsigned long long);
   HIPATTN_CUDA_OK(cudaFuncSetAttribute(select_stage_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  select_stage_kernel<<<(unsigned)rows, kSortThreads, smem, (cudaStream_t)stream>>>(
-      score_max, left, n, n_pad, k_keep, k_pad, sink, c_prev, c_next, next_left, next_right, next_score_max);
+  select_stage_kernel<<<(unsigned)rows, kSortThreads, smem, stream>>>(
+      score_max, left, n, n_pad, k_keep, k_pad, sink, c_prev, c_next, next_left, next_right, next_score_max,
+      next_left64, next_right64);
   return check_launch("select_stage_kernel");
+}
+
+extern "C" int hipattn_select_stage(const int32_t* score_max, const int32_t* left, int64_t rows, int32_t n, int32_t k_keep,
+                                    int32_t sink, int32_t c_prev, int32_t c_next, int32_t* next_left,
+                                    int32_t* next_right, int32_t* next_score_max, void* stream) {
+  return select_stage(score_max, left, rows, n, k_keep, sink, c_prev, c_next, next_left, next_right, next_score_max, nullptr, nullptr,
+                      (cudaStream_t)stream);
 }
 
 extern "C" int hipattn_finalize_indices(const int32_t* score_max, const int32_t* left_heads, int64_t left_row_stride,

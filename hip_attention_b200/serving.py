@@ -19,7 +19,7 @@ import torch
 from torch import Tensor
 
 from .metadata import (HiPAttentionArgs, HiPAttentionOutputMetadata, HiPAttentionStageInputCache, ScanStage)
-from .operator import hip_attention_12
+from .operator import hip_attention_12, host
 
 
 def _default_stages() -> List[ScanStage]:
@@ -181,6 +181,9 @@ class HiPMetadataCache:
                                           mask_cache_statistics=None, sa_cache_statistics=None, stage_caches=caches)
 
 
+_POOL_TYPES = (torch.int64, torch.int32, torch.uint32, torch.float32, torch.bfloat16)
+
+
 class _PoolBuffer:
     """One preallocated buffer of the metadata pool (hip_memory_pool.py:20-53): ``per_head`` buffers are
     [max_batch * heads, ...] and sliced by batch * heads rows, the others are [max_batch, 1, heads, ...]; values are
@@ -204,6 +207,18 @@ class _PoolBuffer:
         view = self.buffer[:batch_size * heads] if self.per_head else self.buffer[:batch_size, :, :heads]
         return view.to(self.dtype, copy=True)
 
+    def get_rows(self, batch_size: int, heads: int) -> int:
+        """Leading rows of the buffer that a read returns, all of them contiguous; checks the batch size."""
+        rows = batch_size * heads if self.per_head else batch_size
+        self._check(rows, "the requested batch")
+        return rows
+
+    def takes_whole(self, value: Tensor) -> bool:
+        """Whether ``value`` fills whole leading rows of the buffer with numbers one launch can convert; checks the rows."""
+        self._check(value.shape[0], "the stored value")
+        return value.is_cuda and value.device == self.buffer.device and value.shape[1:] == self.buffer.shape[1:] and \
+            value.is_floating_point() == self.buffer.is_floating_point() and value.dtype in _POOL_TYPES
+
     def set(self, value: Tensor) -> None:
         self._check(value.shape[0], "the stored value")
         dst = self.buffer[:value.shape[0]] if self.per_head else self.buffer[:value.shape[0], :, :value.shape[2]]
@@ -222,6 +237,7 @@ class HiPMetadataCachePool:
     HIP_DEBUG_ADD_DELAY_WINDOW, HIP_DEBUG_DELAYED_STAGE0) are not built."""
 
     _COUNTERS = ("access_count", "unique_access_count", "cache_miss_count")
+    _STAGE_NAMES = ("indices_left", "indices_right", "out_scores")
 
     def __init__(self, max_total_num_tokens: int, query_head_num: int, layer_num: int, context_length: int, device,
                  hip_config: HiPAttentionConfig) -> None:
@@ -271,6 +287,30 @@ class HiPMetadataCachePool:
     def set_buffer(self, layer_idx: int, name: str, value: Tensor) -> None:
         self._buffer(layer_idx, name).set(value)
 
+    def _get_buffers(self, layer_idx: int, names: Sequence[str], batch_size: int) -> List[Tensor]:
+        """Several reads; on the GPU one launch for all of them (a dozen small copies cost more than the step's attention)."""
+        bufs = [self._buffer(layer_idx, name) for name in names]
+        if not bufs[0].buffer.is_cuda:
+            return [b.get(batch_size, self.head_num) for b in bufs]
+        return host().pool_read([(b.buffer, b.get_rows(batch_size, self.head_num)) for b in bufs])
+
+    def _set_buffers(self, layer_idx: int, items: Sequence) -> None:
+        """Several writes ((name, value); None: zeros in the first ``max_batch_size`` rows), one launch on the GPU."""
+        together = []
+        for name, value in items:
+            b = self._buffer(layer_idx, name)
+            if value is None:
+                if b.buffer.is_cuda:
+                    together.append((b.buffer, None, self.max_batch_size))
+                else:
+                    b.buffer[:self.max_batch_size].zero_()
+            elif b.takes_whole(value):
+                together.append((b.buffer, value, 0))
+            else:
+                b.set(value)
+        if together:
+            host().pool_write(together)
+
     def get_hip_metadata_cache(self, layer_id: int, size: int, batch_size: int,
                                cached_stages: Optional[int]) -> Optional[HiPAttentionOutputMetadata]:
         """What a step may reuse: the mask (``cached_stages`` None or the number of stages), nothing (0, or -1 for the
@@ -279,18 +319,15 @@ class HiPMetadataCachePool:
             raise ValueError("the pool serves decode steps: one query token per request")
         n_stages = len(self.layer_configs[layer_id].stages)
         if cached_stages is None or cached_stages == n_stages:
-            return HiPAttentionOutputMetadata(
-                indices=self.get_buffer(layer_id, "indices", batch_size), ks=self.get_buffer(layer_id, "ks", batch_size),
-                ks_count=self.get_buffer(layer_id, "ks_count", batch_size), ks_start_end=self.get_buffer(layer_id, "ks_start_end", batch_size),
-                mask_cache_statistics=None, sa_cache_statistics=None, stage_caches=None)
+            indices, ks, ks_count, ks_start_end = self._get_buffers(layer_id, ("indices", "ks", "ks_count", "ks_start_end"), batch_size)
+            return HiPAttentionOutputMetadata(indices=indices, ks=ks, ks_count=ks_count, ks_start_end=ks_start_end,
+                                              mask_cache_statistics=None, sa_cache_statistics=None, stage_caches=None)
         if cached_stages <= 0:
             return None
         caches = [HiPAttentionStageInputCache(indices_left=None, indices_right=None, out_scores=None)]
-        for i_stage in range(1, cached_stages + 1):
-            caches.append(HiPAttentionStageInputCache(
-                indices_left=self.get_buffer(layer_id, f"stage_{i_stage}_indices_left", batch_size),
-                indices_right=self.get_buffer(layer_id, f"stage_{i_stage}_indices_right", batch_size),
-                out_scores=self.get_buffer(layer_id, f"stage_{i_stage}_out_scores", batch_size)))
+        got = self._get_buffers(layer_id, [f"stage_{i}_{name}" for i in range(1, cached_stages + 1) for name in self._STAGE_NAMES], batch_size)
+        for i in range(0, len(got), 3):
+            caches.append(HiPAttentionStageInputCache(indices_left=got[i], indices_right=got[i + 1], out_scores=got[i + 2]))
         return HiPAttentionOutputMetadata(indices=None, ks=None, ks_count=None, ks_start_end=None, mask_cache_statistics=None,
                                           sa_cache_statistics=None, stage_caches=caches)
 
@@ -298,20 +335,16 @@ class HiPMetadataCachePool:
         """Store what a step returned.  Stage inputs are only overwritten when the step recomputed them."""
         if size != batch_size:
             raise ValueError("the pool serves decode steps: one query token per request")
-        for name in ("indices", "ks", "ks_count", "ks_start_end"):
-            self.set_buffer(layer_id, name, getattr(metadata, name))
+        items = [(name, getattr(metadata, name)) for name in ("indices", "ks", "ks_count", "ks_start_end")]
         for prefix, stats in (("sa", metadata.sa_cache_statistics), ("mask", metadata.mask_cache_statistics)):
             counts = stats.compute_statistics() if stats is not None else {}
             for c in self._COUNTERS:
                 v = counts.get(c)
-                v = torch.zeros((1,), dtype=torch.int64, device=self.device) if v is None else v
-                self.set_buffer(layer_id, f"{prefix}_{c}", v.view(1, 1).expand(self.max_batch_size, 1))
+                items.append((f"{prefix}_{c}", v if v is None else v.view(1, 1).expand(self.max_batch_size, 1)))
         for i_stage, cache in enumerate(metadata.stage_caches or []):
-            if i_stage == 0:
-                continue
-            self.set_buffer(layer_id, f"stage_{i_stage}_indices_left", cache.indices_left)
-            self.set_buffer(layer_id, f"stage_{i_stage}_indices_right", cache.indices_right)
-            self.set_buffer(layer_id, f"stage_{i_stage}_out_scores", cache.out_scores)
+            if i_stage > 0:
+                items += [(f"stage_{i_stage}_{name}", getattr(cache, name)) for name in self._STAGE_NAMES]
+        self._set_buffers(layer_id, items)
 
     def compute_cache_statistics(self, batch_size: int) -> dict:
         """Access / miss totals over all layers and the hit ratio (0 / 0 when the steps gathered no statistics)."""
