@@ -51,6 +51,7 @@ int bsa_mma(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled);
 int bsa_decode(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled);
 int bsa_tcgen05(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled);
 int64_t bsa_tcgen05_ctas(const hipattn_bsa_params_t& p, int* resident, int* tile_keys);
+bool decode_on_tensor_cores(const hipattn_bsa_params_t& p);
 int64_t bsa_mma_ctas(const hipattn_bsa_params_t& p, int* resident, int* tile_keys);
 int bounded_wait_probe(uint32_t* status, cudaStream_t stream);
 
@@ -198,6 +199,7 @@ extern "C" int32_t hipattn_attention_splits(const hipattn_bsa_params_t* p) {
   const int64_t keys = (int64_t)(p->sink < p->T ? p->sink : p->T) + (int64_t)p->K * p->block_size_k +
                        ((int64_t)p->window + p->block_size_q - 1 < p->T ? (int64_t)p->window + p->block_size_q - 1 : p->T);
   if (p->TQ == 1) {
+    if (decode_on_tensor_cores(*p)) return 1;   // that kernel spreads a key list over the CTAs of a cluster itself
     // Decode: one range when the batch alone fills the GPU; otherwise enough ranges for two CTAs per multiprocessor,
     // each at least four tiles (256 keys) long.
     const int64_t units = (int64_t)p->B * p->HKV;
