@@ -237,7 +237,8 @@ __global__ void __launch_bounds__(128, NR <= 32 ? (STREAM ? 5 : 6) : (NR <= 64 ?
     float score = HIPATTN_SCORE_INIT;
     // The candidate that won the previous round and its score.  When the halved chunk proposes the same key again
     // (always in the last round, for one of the two candidates in the round before it) the score is known: the same
-    // key against the same pooled queries, so the row is neither fetched nor multiplied again.
+    // key against the same pooled queries, so the row is neither fetched nor multiplied again.  (-1: the winner's score
+    // was left between two values, see below.)
     int won_t = -1;
     float won_score = 0.f;
 
@@ -353,35 +354,51 @@ __global__ void __launch_bounds__(128, NR <= 32 ? (STREAM ? 5 : 6) : (NR <= 64 ?
         }
         x = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
       }
+      // The rounded score lies between lo and hi.  A comparison that these bounds settle needs no more; where they overlap,
+      // or where the winner may raise the chunk's best score and its own is not certain, the key is scored by the
+      // strict definition, which costs its warp 600 cycles.  (Scoring every key whose bounds differ: 0.3 % of the keys in
+      // bf16, 2.5 % in fp16, three per round and CTA.)
       const float e_ = eps_q * s_abs * 1.01f;
-      float sc = Elem<DT>::round(x);
-      const bool sure = Elem<DT>::round(x - e_) == Elem<DT>::round(x + e_);
-      if (known) sc = won_score;
-      unsigned need = __ballot_sync(0xffffffffu, idx >= 0 && ok && (!sure || check));
-      while (need) {
-        const int owner = __ffs(need) - 1;
-        need &= need - 1;
-        const float rawv = strict_score(warp * 32 + owner);
-        const float ex = Elem<DT>::round(rawv);
-        if (lane == owner) {
-          if (check) {
-            if (sure && sc != ex) ++st_wrong;
-            if (e_ > 0.f) st_ratio = fmaxf(st_ratio, fabsf(x - rawv) / e_);
+      float lo = Elem<DT>::round(x - e_), hi = Elem<DT>::round(x + e_);
+      if (known) lo = hi = won_score;
+      const bool fetched = idx >= 0 && ok;
+      if (fetched && lo != hi) ++st_fb;
+      bool certain = lo == hi && !check;   // (check mode: every key by both definitions)
+      const int other_t = __shfl_xor_sync(0xffffffffu, tk_asked, 1);   // the other candidate of the same chunk
+      const bool same = (!roped || STREAM) && other_t == tk_asked;      // a key does not beat itself
+      bool win, mine;
+      float wlo, whi;
+      for (;;) {
+        const float olo = __shfl_xor_sync(0xffffffffu, lo, 1), ohi = __shfl_xor_sync(0xffffffffu, hi, 1);
+        const float llo = side ? olo : lo, lhi = side ? ohi : hi, rlo = side ? lo : olo, rhi = side ? hi : ohi;
+        win = llo > rhi && !same;
+        const bool open = !win && !(lhi <= rlo) && !same;
+        wlo = win ? llo : rlo;
+        whi = win ? lhi : rhi;
+        mine = win != (side != 0);
+        unsigned need = __ballot_sync(0xffffffffu, act && fetched && !certain && (open || check || (mine && whi > score)));
+        if (!need) break;
+        while (need) {
+          const int owner = __ffs(need) - 1;
+          need &= need - 1;
+          const float rawv = strict_score(warp * 32 + owner);
+          if (lane == owner) {
+            const float ex = Elem<DT>::round(rawv);
+            if (check) {
+              if (lo == hi && hi != ex) ++st_wrong;
+              if (e_ > 0.f) st_ratio = fmaxf(st_ratio, fabsf(x - rawv) / e_);
+            }
+            lo = hi = ex;
+            certain = true;
           }
-          if (!sure) ++st_fb;
-          sc = ex;
         }
       }
-      const float other = __shfl_xor_sync(0xffffffffu, sc, 1);   // the other candidate of the same chunk
-      const int other_t = __shfl_xor_sync(0xffffffffu, tk_asked, 1);
       if (act) {
         if (idx >= 0) st_keys += 1;
-        const float sl = side ? other : sc, sr = side ? sc : other;
-        const bool win = sl > sr;
         if (win) right = mid; else left = mid;
-        score = fmaxf(score, win ? sl : sr);
-        won_t = (win != (side != 0)) ? tk_asked : other_t;    // left candidate when it won, else the right one
-        won_score = win ? sl : sr;
+        score = fmaxf(score, wlo);   // certain when it matters: a winner whose upper bound exceeds the best was scored strictly
+        won_t = wlo == whi ? (mine ? tk_asked : other_t) : -1;
+        won_score = wlo;
       }
     }
 
