@@ -89,10 +89,6 @@ __host__ __device__ __forceinline__ uint32_t decode_score_bits(int32_t code) {
 }
 __device__ __forceinline__ int32_t encode_score(float s) { return encode_score_bits(__float_as_uint(s)); }
 __device__ __forceinline__ float decode_score(int32_t c) { return __uint_as_float(decode_score_bits(c)); }
-// ascending sort key: best score first, lower position first among equal scores
-__device__ __forceinline__ unsigned long long score_sort_key(int32_t code, unsigned position) {
-  return ((unsigned long long)(~((uint32_t)code ^ 0x80000000u)) << 32) | position;
-}
 
 // ---------------------------------------------------------------------------------------------
 // token addressing: dense K[b, t, h, :] or paged cache[block_table[b, t / P], t % P, h, :]
