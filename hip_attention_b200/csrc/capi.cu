@@ -7,6 +7,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "host_kernels.h"
 
 namespace hipattn {
 
@@ -65,8 +66,10 @@ bool tcgen05_prefill() {
 
 template <int DT>
 __global__ void merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse, int n_parts, int D,
-                             typename Elem<DT>::type* __restrict__ out, int64_t out_stride, float* __restrict__ lse_out) {
+                             typename Elem<DT>::type* __restrict__ out, int64_t out_stride, float* __restrict__ lse_out, int64_t rows_per_group,
+                             int64_t group_stride) {
   const int64_t row = blockIdx.x;
+  out += row / rows_per_group * (group_stride - rows_per_group * out_stride);   // (rows of a group lie out_stride apart)
   const float* lse = part_lse + row * n_parts;
   float m = -INFINITY;
   for (int s = 0; s < n_parts; ++s) m = fmaxf(m, lse[s]);
@@ -82,13 +85,15 @@ __global__ void merge_kernel(const float* __restrict__ part_o, const float* __re
   if (lse_out && threadIdx.x == 0) lse_out[row] = tot > 0.f ? m + log2f(tot) : -INFINITY;
 }
 
-// Access statistics of the attention: one CTA per (batch, KV head, attention block) marks the tokens the reference's
+// Access statistics of the attention: `parts` CTAs per (batch, KV head, attention block) mark the tokens the reference's
 // kernels load for that block (see hipattn_mark_attention_access in the header).
 __global__ void mark_attention_access_kernel(const hipattn_bsa_params_t p, int32_t* counter, int64_t stride_b, int64_t stride_h,
-                                             int n, int window_block_rows) {
+                                             int n, int window_block_rows, int parts) {
   __shared__ int s_pmax;
   const int NBLK = cdiv(p.TQ, p.block_size_q);
   int64_t bid = blockIdx.x;
+  const int part = (int)(bid % parts); bid /= parts;
+  const int first = part * blockDim.x + threadIdx.x, step = parts * blockDim.x;
   const int d = (int)(bid % NBLK); bid /= NBLK;
   const int hkv = (int)(bid % p.HKV); bid /= p.HKV;
   const int b = (int)bid;
@@ -110,13 +115,13 @@ __global__ void mark_attention_access_kernel(const hipattn_bsa_params_t p, int32
   long long ks = p.ks[nrow * p.ks_stride_n + (int64_t)d_idx * p.ks_stride_d];
   ks = ks < 0 ? 0 : (ks > p.K ? p.K : ks);
   const int64_t* idx = p.indices + nrow * p.idx_stride_n + (int64_t)d_idx * p.idx_stride_d;
-  for (int t = threadIdx.x; t < min(p.sink, cur); t += blockDim.x) mark_access(counter, stride_b, stride_h, n, p.k, b, hkv, t);
-  for (int j = threadIdx.x; j < (int)ks * p.block_size_k; j += blockDim.x) {
+  for (int t = first; t < min(p.sink, cur); t += step) mark_access(counter, stride_b, stride_h, n, p.k, b, hkv, t);
+  for (int j = first; j < (int)ks * p.block_size_k; j += step) {
     const long long t = idx[j / p.block_size_k] + j % p.block_size_k;
     if (t >= p.sink && t < cur && t < p.T) mark_access(counter, stride_b, stride_h, n, p.k, b, hkv, t);
   }
   if (p.window > 0)
-    for (int t = max(0, cur - p.window - window_block_rows) + threadIdx.x; t < cur; t += blockDim.x)
+    for (int t = max(0, cur - p.window - window_block_rows) + first; t < cur; t += step)
       mark_access(counter, stride_b, stride_h, n, p.k, b, hkv, t);
 }
 
@@ -137,9 +142,17 @@ extern "C" int hipattn_mark_attention_access(const hipattn_bsa_params_t* p, int3
   if (p->k.cache != nullptr)
     HIPATTN_REQUIRE(p->k.block_table && p->k.cache_seq_lens && p->k.page_size > 0, HIPATTN_ERR_INVALID,
                     "mark_attention_access: paged keys without block_table / cache_seq_lens");
-  const int64_t grid = (int64_t)p->B * p->HKV * cdiv(p->TQ, p->block_size_q);
+  const int64_t units = (int64_t)p->B * p->HKV * cdiv(p->TQ, p->block_size_q);
+  // a token is two dependent reads (block start, page) and a store; with few blocks their lists are shared out, four tokens a
+  // thread, until the GPU holds eight CTAs per multiprocessor (the last 64 queries of a chunk at 90112 tokens, eight CTAs:
+  // 128 us, 9 with the split; five decode sequences, 40 CTAs: 18 us, 7)
+  const int64_t most = (int64_t)(p->sink < p->T ? p->sink : p->T) + (int64_t)p->K * p->block_size_k + (p->window < p->T ? p->window : p->T);
+  int64_t parts = (148 * 8 + units - 1) / units;
+  if (parts > (most + 1023) / 1024) parts = (most + 1023) / 1024;
+  if (parts < 1) parts = 1;
+  const int64_t grid = units * parts;
   HIPATTN_REQUIRE(grid < 0x7fffffffLL, HIPATTN_ERR_INVALID, "mark_attention_access: grid of %lld blocks", (long long)grid);
-  mark_attention_access_kernel<<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(*p, counter, stride_b, stride_h, n, window_block_rows);
+  mark_attention_access_kernel<<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(*p, counter, stride_b, stride_h, n, window_block_rows, (int)parts);
   return check_launch("mark_attention_access_kernel");
 }
 
@@ -241,19 +254,23 @@ extern "C" int32_t hipattn_attention_splits(const hipattn_bsa_params_t* p) {
 
 extern "C" int hipattn_merge_partials(const float* part_o, const float* part_lse, int64_t rows, int32_t n_parts, int32_t D,
                                       int32_t dtype, void* out, int64_t out_stride, float* lse_out, void* stream) {
+  return merge_partials(part_o, part_lse, rows, n_parts, D, dtype, out, out_stride, lse_out, rows, rows * out_stride, (cudaStream_t)stream);
+}
+
+int hipattn::merge_partials(const float* part_o, const float* part_lse, int64_t rows, int n_parts, int D, int dtype, void* out, int64_t out_stride,
+                            float* lse_out, int64_t rows_per_group, int64_t group_stride, cudaStream_t s) {
   HIPATTN_REQUIRE(part_o && part_lse && out, HIPATTN_ERR_INVALID, "merge_partials: null pointer");
   HIPATTN_REQUIRE(rows > 0 && n_parts > 0 && D > 0, HIPATTN_ERR_INVALID, "merge_partials: bad sizes");
   const int threads = D >= 128 ? 128 : 64;
-  cudaStream_t s = (cudaStream_t)stream;
   switch (dtype) {
     case HIPATTN_F32:
-      merge_kernel<HIPATTN_F32><<<(unsigned)rows, threads, 0, s>>>(part_o, part_lse, n_parts, D, (float*)out, out_stride, lse_out);
+      merge_kernel<HIPATTN_F32><<<(unsigned)rows, threads, 0, s>>>(part_o, part_lse, n_parts, D, (float*)out, out_stride, lse_out, rows_per_group, group_stride);
       break;
     case HIPATTN_F16:
-      merge_kernel<HIPATTN_F16><<<(unsigned)rows, threads, 0, s>>>(part_o, part_lse, n_parts, D, (__half*)out, out_stride, lse_out);
+      merge_kernel<HIPATTN_F16><<<(unsigned)rows, threads, 0, s>>>(part_o, part_lse, n_parts, D, (__half*)out, out_stride, lse_out, rows_per_group, group_stride);
       break;
     case HIPATTN_BF16:
-      merge_kernel<HIPATTN_BF16><<<(unsigned)rows, threads, 0, s>>>(part_o, part_lse, n_parts, D, (__nv_bfloat16*)out, out_stride, lse_out);
+      merge_kernel<HIPATTN_BF16><<<(unsigned)rows, threads, 0, s>>>(part_o, part_lse, n_parts, D, (__nv_bfloat16*)out, out_stride, lse_out, rows_per_group, group_stride);
       break;
     default: set_error("merge_partials: unknown dtype %d", dtype); return HIPATTN_ERR_INVALID;
   }

@@ -314,6 +314,21 @@ struct Call {
   Device dv{c10::Device(at::kCUDA, 0)};
   cudaStream_t stream;
   uint32_t* status;
+  // Calls that a prefill chunk is split into read the same keys: what they prepare from them is handed on in this dict
+  // (None: a call of its own), valid for the positions it names.
+  PyObject* shared = Py_None;
+  hipattn::QueryPositions where{};   // positions that prepared tables and keys have to reach
+  at::Tensor last_pos;               // [B] largest of them
+
+  at::Tensor shared_get(const char* name) const {
+    PyObject* v = shared == Py_None ? nullptr : PyDict_GetItemString(shared, name);
+    return v ? tensor_of(v, name) : at::Tensor();
+  }
+  void shared_set(const char* name, const at::Tensor& t) const {
+    if (shared == Py_None || !t.defined()) return;
+    Ref v = checked(wrap(t));
+    if (PyDict_SetItemString(shared, name, v.get()) < 0) throw PyError{};
+  }
 
   void mark(const char* name) {
     if (timer == Py_None) return;
@@ -413,6 +428,16 @@ void check_inputs(Call& c, const at::Tensor& q_mask, const at::Tensor& k_mask) {
   if (c.k_cache.defined() && !c.v_cache.defined()) VALUE_ERROR("k_cache without v_cache");
 }
 
+const int32_t* last_positions(Call& c) {
+  if (!c.last_pos.defined()) c.last_pos = c.shared_get("last_pos");
+  if (!c.last_pos.defined()) {
+    c.last_pos = c.dv.empty({c.where.B}, at::kInt);
+    check(hipattn::last_positions(c.where, c.last_pos.data_ptr<int32_t>(), c.stream), "last_positions");
+    c.shared_set("last_pos", c.last_pos);
+  }
+  return c.last_pos.data_ptr<int32_t>();
+}
+
 // cos / sin [rows, >= D / 2] in q's element type, rows of whole 16-byte pieces (the kernels cast the tables to the
 // element type before use, attention_extend.py:308-321; doing it once here is the same arithmetic)
 at::Tensor rope_table(const Call& c, const at::Tensor& given) {
@@ -429,6 +454,48 @@ at::Tensor rope_table(const Call& c, const at::Tensor& given) {
     }
   }
   return t;
+}
+
+// The call's rope tables.  fp32 tables with 16-bit queries, the usual case, are converted as far as the call can reach into
+// them: a query or key is never rotated to a position beyond the largest query position, except by the scan, whose
+// positions end at the number of chunks of a stage + the window.
+void set_rope_tables(Call& c, int64_t restart_chunks) {
+  c.rope_cos = c.shared_get("rope_cos");
+  c.rope_sin = c.shared_get("rope_sin");
+  if (c.rope_cos.defined()) return;
+  const at::Tensor cos = attr_tensor(c.args, N.rope_cos, "rope_cos"), sin = attr_tensor(c.args, N.rope_sin, "rope_sin");
+  auto plain = [&](const at::Tensor& t) {
+    return t.defined() && t.dim() == 2 && t.size(1) >= c.D / 2 && t.scalar_type() == at::kFloat && t.device() == c.q.device() && t.stride(1) == 1 &&
+           t.stride(0) % 4 == 0 && (uintptr_t)t.data_ptr() % 16 == 0 && t.size(0) > 0 && t.size(0) < (1 << 30);
+  };
+  if (c.dt == HIPATTN_F32 || c.D % 16 || !plain(cos) || !plain(sin) || cos.size(0) != sin.size(0) || cos.stride(0) != sin.stride(0)) {
+    c.rope_cos = rope_table(c, cos);
+    c.rope_sin = rope_table(c, sin);
+  } else {
+    const int64_t c0 = c.stages[0].chunk;
+    int64_t n = cdiv(std::max<int64_t>(0, c.T - c.sink - c.sw), c0), most = std::max(n, restart_chunks);
+    for (size_t i = 1; i < c.stages.size(); ++i) {
+      n = std::min(c.stages[i].k / c.stages[i - 1].chunk, n) * (c.stages[i - 1].chunk / c.stages[i].chunk);
+      most = std::max(most, n);
+    }
+    at::Tensor both = c.dv.empty({2, cos.size(0), c.D / 2}, c.q.scalar_type());
+    hipattn::RopeTables t{};
+    t.cos = cos.data_ptr<float>();
+    t.sin = sin.data_ptr<float>();
+    t.row_stride = cos.stride(0);
+    t.rows = (int)cos.size(0);
+    t.cols = (int)c.D / 2;
+    t.dtype = c.dt;
+    t.floor = (int)std::min<int64_t>(most + std::max<int64_t>(0, c.sw - c0) + 1, 1 << 30);
+    t.q = c.where;
+    if (c.last_pos.defined() || c.where.B * (int64_t)c.where.TQ > 2048) t.last_pos = last_positions(c);
+    t.dst = both.data_ptr();
+    check(hipattn::convert_rope_tables(t, c.stream), "convert_rope_tables");
+    c.rope_cos = both.select(0, 0);
+    c.rope_sin = both.select(0, 1);
+  }
+  c.shared_set("rope_cos", c.rope_cos);
+  c.shared_set("rope_sin", c.rope_sin);
 }
 
 struct Mask {
@@ -500,21 +567,26 @@ Mask estimate_mask(Call& c, const hipattn_tokens_t& ktok, int64_t first, at::Ten
   }
   if (tensor_scan || want_plain) {
     c.mark("start");
-    if (tensor_scan) {
-      key_abs = dv.empty({sides, c.B, c.HKV, c.T}, at::kFloat);
-      if (sides * key_rows < limit) k_scaled = dv.empty({sides, c.B, c.HKV, c.T, c.D}, c.q.scalar_type());
-      void* ks_ptr = k_scaled.defined() ? k_scaled.data_ptr() : nullptr;
-      if (!c.using_extend)
-        check(hipattn_scan_prepare_keys(&ktok, c.dt, c.D, c.B, c.T, c.HKV, k_scale, key_abs.data_ptr<float>(), ks_ptr, c.status, c.stream), "scan_prepare_keys");
-      else   // position -1: both copies (table positions 0 and 1) from one read of the keys
-        check(hipattn_scan_prepare_keys_rope(&ktok, c.dt, c.D, c.B, c.T, c.HKV, k_scale, c.rope_cos.data_ptr(), c.rope_sin.data_ptr(), c.rope_cos.stride(0),
-                                             (int)c.rope_cos.size(0), -1, key_abs.data_ptr<float>(), ks_ptr, c.status, c.stream), "scan_prepare_keys_rope");
-    }
-    if (want_plain) {   // scale 1: the copy holds the keys' own values
-      key_abs_plain = dv.empty({c.B, c.HKV, c.T}, at::kFloat);
-      k_plain = dv.empty({c.B, c.HKV, c.T, c.D}, c.q.scalar_type());
-      check(hipattn_scan_prepare_keys(&ktok, c.dt, c.D, c.B, c.T, c.HKV, 1.0f, key_abs_plain.data_ptr<float>(), k_plain.data_ptr(), c.status, c.stream), "scan_prepare_keys");
-    }
+    // Tokens up to the last query position and the rest of its chunk (a server hands over its model's whole context length);
+    // a restart's first list is the caller's, so all of them.
+    check(hipattn::validate_tokens(ktok, 2, (int)c.D, "k"), "scan_prepare_keys");
+    auto prepare = [&](const char* abs_name, const char* copy_name, at::Tensor& abs, at::Tensor& copy, int copies, bool rope, float scale) {
+      abs = c.shared_get(abs_name);
+      copy = c.shared_get(copy_name);
+      if (abs.defined()) return;
+      abs = dv.empty({copies, c.B, c.HKV, c.T}, at::kFloat);
+      if (copies * key_rows < limit) copy = dv.empty({copies, c.B, c.HKV, c.T, c.D}, c.q.scalar_type());
+      // (table position -1: both copies, rotated to positions 0 and 1, from one read of the keys)
+      check(hipattn::scan_prepare_keys(ktok, c.dt, (int)c.D, (int)c.B, (int)c.T, (int)c.HKV, scale, abs.data_ptr<float>(),
+                                       copy.defined() ? copy.data_ptr() : nullptr, c.status, c.stream, rope ? c.rope_cos.data_ptr() : nullptr,
+                                       rope ? c.rope_sin.data_ptr() : nullptr, rope ? c.rope_cos.stride(0) : 0, rope ? (int)c.rope_cos.size(0) : 0, -1,
+                                       first == 0 ? last_positions(c) : nullptr, (int)c0), "scan_prepare_keys");
+      c.shared_set(abs_name, abs);
+      c.shared_set(copy_name, copy);
+    };
+    if (tensor_scan) prepare("key_abs", "k_scaled", key_abs, k_scaled, sides, c.using_extend, k_scale);
+    // scale 1: the copy holds the keys' own values
+    if (want_plain) prepare("key_abs_plain", "k_plain", key_abs_plain, k_plain, 1, false, 1.0f);
     c.mark("prep");
   }
 
@@ -656,7 +728,7 @@ struct AttentionArgs {
 void attention(Call& c, const hipattn_tokens_t& ktok, const hipattn_tokens_t& vtok, const at::Tensor& indices, const at::Tensor& ks,
                const AttentionArgs& a, const at::Tensor& access, at::Tensor& out, at::Tensor& lse) {
   const Device& dv = c.dv;
-  out = dv.empty({c.B, c.TQ, c.H, c.D}, c.q_attn.scalar_type());
+  if (!out.defined()) out = dv.empty({c.B, c.TQ, c.H, c.D}, c.q_attn.scalar_type());
   if (a.want_lse) lse = dv.empty({c.B, c.TQ, c.H}, at::kFloat);
   const int64_t Kk = indices.size(2);
   hipattn_bsa_params_t bp;
@@ -694,8 +766,8 @@ void attention(Call& c, const hipattn_tokens_t& ktok, const hipattn_tokens_t& vt
     bp.part_o = part.data_ptr<float>();
     bp.part_lse = bp.part_o + rows * bp.n_splits * c.D;
     check(hipattn_bsa_attention(&bp, c.stream), "bsa_attention");
-    check(hipattn_merge_partials(bp.part_o, bp.part_lse, rows, bp.n_splits, (int)c.D, c.dt, out.data_ptr(), c.D,
-                                 lse.defined() ? lse.data_ptr<float>() : nullptr, c.stream), "merge_partials");
+    check(hipattn::merge_partials(bp.part_o, bp.part_lse, rows, bp.n_splits, (int)c.D, c.dt, out.data_ptr(), c.D,
+                                  lse.defined() ? lse.data_ptr<float>() : nullptr, c.TQ * c.H, out.stride(0), c.stream), "merge_partials");
   } else {
     bp.lse_out = lse.defined() ? lse.data_ptr<float>() : nullptr;
     check(hipattn_bsa_attention(&bp, c.stream), "bsa_attention");
@@ -756,6 +828,8 @@ PyObject* forward(PyObject* const* argv) {
   c.reduce = argv[7];
   c.timer = argv[8];
   PyObject* v_ready = argv[9];
+  c.shared = argv[10];
+  at::Tensor context = tensor_of(argv[11], "out");
 
   if (!THPVariable_Check(q_obj) || THPVariable_Unpack(q_obj).dim() != 4) VALUE_ERROR("q must be a tensor [B, TQ, H, D]");
   c.q = THPVariable_Unpack(q_obj);
@@ -818,10 +892,15 @@ PyObject* forward(PyObject* const* argv) {
     begin.pos0 = c.T - c.TQ;
     c.pos = row.as_strided({c.B, c.TQ}, {0, 1});
   }
-  if (c.using_extend) {
-    c.rope_cos = rope_table(c, attr_tensor(c.args, N.rope_cos, "rope_cos"));
-    c.rope_sin = rope_table(c, attr_tensor(c.args, N.rope_sin, "rope_sin"));
+  {
+    const at::Tensor all = c.shared_get("positions");   // of the whole chunk
+    const at::Tensor& w = all.defined() ? all : c.pos;
+    const bool given = all.defined() || !own_pos;
+    c.where = {given ? w.data_ptr<int64_t>() : nullptr, given ? w.stride(0) : 0, given ? w.stride(1) : 0, c.T - c.TQ, (int)c.B, given ? (int)w.size(1) : (int)c.TQ};
   }
+  if (context.defined() && (context.sizes() != c.q_attn.sizes() || context.scalar_type() != c.q_attn.scalar_type() || context.stride(3) != 1 ||
+                            context.stride(2) != c.D || context.stride(1) != c.H * c.D))
+    VALUE_ERROR("out must have q's shape and type, its rows contiguous");
   const int64_t bq = c.stages.back().bq, BDST = cdiv(c.TQ, bq), rows = c.B * BDST;
   const int64_t c0 = c.stages[0].chunk, c_last = c.stages.back().chunk;
   int64_t sw_attn = std::max<int64_t>(0, c.sw - c0) + c0;   // attention_extend.py:1976-1978, 2901
@@ -874,6 +953,7 @@ PyObject* forward(PyObject* const* argv) {
         restart_inputs(c, entry.get(), rows, left, right);
       }
     }
+    if (c.using_extend) set_rope_tables(c, first > 0 ? left.size(1) : 0);
     // scan reads dense K when it is given, else the page pool (attention_extend.py:2524)
     const hipattn_tokens_t kscan = c.k_scan.defined() ? tokens(c.k_scan, undef, undef, undef, "k") : ktok;
     Mask m = estimate_mask(c, kscan, first, left, right, !stage_caches.none(), mask_stats, begin);
@@ -895,6 +975,7 @@ PyObject* forward(PyObject* const* argv) {
     if (attr_true(c.args, N.mask_only)) return PyTuple_Pack(2, Py_None, Py_None);
   } else {
     if (own_pos) check(hipattn::begin_call(begin, c.stream), "begin_call");
+    if (c.using_extend) set_rope_tables(c, 0);
     const at::Tensor ci = attr_tensor(cached, N.indices, "indices"), cks = attr_tensor(cached, N.ks, "ks"),
                      ckc = attr_tensor(cached, N.ks_count, "ks_count"), cse = attr_tensor(cached, N.ks_start_end, "ks_start_end");
     if (!cks.defined() || !ckc.defined() || !cse.defined()) VALUE_ERROR("cached metadata with indices needs ks, ks_count and ks_start_end");
@@ -950,7 +1031,7 @@ PyObject* forward(PyObject* const* argv) {
     Ref s = checked(PyObject_CallMethodOneArg(K.torch_cuda, N.current_stream, dev.get()));
     Ref r = checked(PyObject_CallMethodOneArg(s.get(), N.wait_event, v_ready));
   }
-  at::Tensor context, lse;
+  at::Tensor lse;
   attention(c, ktok, vtok, indices, ks, a, sa_stats, context, lse);
   c.mark("attention");
 
@@ -1071,11 +1152,33 @@ PyObject* guarded(F f) {
 }
 
 PyObject* py_forward(PyObject*, PyObject* const* argv, Py_ssize_t n) {
-  if (n != 10) {
-    PyErr_SetString(PyExc_TypeError, "forward takes ten arguments");
+  if (n != 12) {
+    PyErr_SetString(PyExc_TypeError, "forward takes twelve arguments");
     return nullptr;
   }
   return guarded([&] { return forward(argv); });
+}
+// gather_table(table [*, width], rows [n], lens [n]) -> [n, width]: the rows' first lens[i] entries (the rest is not written)
+PyObject* gather_table(PyObject* const* argv) {
+  const at::Tensor table = tensor_of(argv[0], "req_to_tokens"), rows = tensor_of(argv[1], "req_pool_indices"), lens = tensor_of(argv[2], "seq_lens");
+  auto ints = [](const at::Tensor& t) { return t.defined() && (t.scalar_type() == at::kInt || t.scalar_type() == at::kLong); };
+  if (!ints(table) || !ints(rows) || !ints(lens) || !table.is_cuda() || rows.device() != table.device() || lens.device() != table.device() ||
+      table.dim() != 2 || rows.dim() != 1 || lens.dim() != 1 || lens.size(0) != rows.size(0) || table.stride(1) != 1 || !rows.is_contiguous() ||
+      !lens.is_contiguous() || rows.size(0) > 65535 || table.size(0) < 1)
+    Py_RETURN_NONE;
+  const c10::cuda::CUDAGuard guard(table.device());
+  at::Tensor out = at::detail::empty_cuda({rows.size(0), table.size(1)}, table.scalar_type(), table.device(), c10::nullopt);
+  check(hipattn::gather_table(table.data_ptr(), table.size(0), table.stride(0), (uint32_t*)status_word(table.device().index()).data_ptr(), (int)table.element_size(), rows.data_ptr(), rows.scalar_type() == at::kLong, lens.data_ptr(),
+                              lens.scalar_type() == at::kLong, (int)rows.size(0), (int)table.size(1), out.data_ptr(),
+                              c10::cuda::getCurrentCUDAStream(table.device().index()).stream()), "gather_table");
+  return wrap(out);
+}
+PyObject* py_gather_table(PyObject*, PyObject* const* argv, Py_ssize_t n) {
+  if (n != 3) {
+    PyErr_SetString(PyExc_TypeError, "gather_table takes three arguments");
+    return nullptr;
+  }
+  return guarded([&] { return gather_table(argv); });
 }
 PyObject* py_status_word(PyObject*, PyObject* index) {
   return guarded([&] { return wrap(status_word((int)PyLong_AsLong(index))); });
@@ -1098,7 +1201,8 @@ PyObject* py_bind(PyObject*, PyObject* const* argv, Py_ssize_t n) {
 }
 
 PyMethodDef methods[] = {
-    {"forward", (PyCFunction)(void*)py_forward, METH_FASTCALL, "q, k, v, args, cached_metadata, return_lse, debug, score_reduce, timer, v_ready"},
+    {"forward", (PyCFunction)(void*)py_forward, METH_FASTCALL, "q, k, v, args, cached_metadata, return_lse, debug, score_reduce, timer, v_ready, shared, out"},
+    {"gather_table", (PyCFunction)(void*)py_gather_table, METH_FASTCALL, "table, rows, lens -> rows of the table, or None when it does not take them"},
     {"status_word", py_status_word, METH_O, "device index -> int32 tensor [1]"},
     {"pool_read", py_pool_read, METH_O, "[(buffer, rows), ...] -> list of tensors"},
     {"pool_write", py_pool_write, METH_O, "[(buffer, value or None, rows), ...]"},

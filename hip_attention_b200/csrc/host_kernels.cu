@@ -23,6 +23,75 @@ __global__ void begin_call_kernel(const BeginCall c) {
   for (int64_t i = first; i < c.n_const; i += step) c.consts[i] = HIPATTN_SCORE_INIT;
 }
 
+__device__ __forceinline__ int clamp_position(int64_t x) { return (int)(x < 0 ? 0 : (x > 0x3fffffff ? 0x3fffffff : x)); }
+
+__global__ void last_positions_kernel(const QueryPositions q, int32_t* last_pos) {
+  __shared__ int s_max;
+  if (threadIdx.x == 0) s_max = 0;
+  __syncthreads();
+  int m = 0;
+  if (q.q_pos == nullptr) m = clamp_position(q.pos0 + q.TQ - 1);
+  else
+    for (int i = threadIdx.x; i < q.TQ; i += blockDim.x) m = max(m, clamp_position(q.q_pos[blockIdx.x * q.stride_b + i * q.stride_t]));
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) atomicMax(&s_max, m);
+  __syncthreads();
+  if (threadIdx.x == 0) last_pos[blockIdx.x] = s_max;
+}
+
+// Four elements per thread and step.  A call touches table rows up to its largest position, and only the first half of the
+// columns (the tables repeat): a server's 131072-row tables cost 38 us when they were converted whole on every call.
+template <int DT>
+__global__ void __launch_bounds__(256) convert_rope_tables_kernel(const RopeTables t) {
+  __shared__ int s_max;
+  if (threadIdx.x == 0) s_max = t.floor;
+  __syncthreads();
+  int m = t.floor;
+  if (t.last_pos) {
+    for (int i = threadIdx.x; i < t.q.B; i += 256) m = max(m, t.last_pos[i]);
+  } else if (t.q.q_pos == nullptr) {
+    m = max(m, clamp_position(t.q.pos0 + t.q.TQ - 1));
+  } else {
+    for (int i = threadIdx.x; i < t.q.B * t.q.TQ; i += 256) m = max(m, clamp_position(t.q.q_pos[i / t.q.TQ * t.q.stride_b + i % t.q.TQ * t.q.stride_t]));
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) atomicMax(&s_max, m);
+  __syncthreads();
+  const int rows = min(t.rows, s_max + 1), q4 = t.cols / 4;
+  const int64_t total = (int64_t)rows * q4, side = (int64_t)t.rows * t.cols;
+  for (int64_t i = blockIdx.x * 256LL + threadIdx.x; i < total; i += gridDim.x * 256LL) {
+    const int r = (int)(i / q4), c = (int)(i - (int64_t)r * q4) * 4;
+#pragma unroll
+    for (int sd = 0; sd < 2; ++sd) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>((sd ? t.sin : t.cos) + r * t.row_stride + c));
+      *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(t.dst) + sd * side + (int64_t)r * t.cols + c) = make_uint2(pack2<DT>(v.x, v.y), pack2<DT>(v.z, v.w));
+    }
+  }
+}
+
+template <typename E>
+__global__ void __launch_bounds__(256) gather_table_kernel(const E* __restrict__ table, int64_t table_rows, int64_t row_stride, uint32_t* status, const void* rows, int rows_i64, const void* lens,
+                                                           int lens_i64, int width, E* __restrict__ dst) {
+  const int i = blockIdx.y;
+  int64_t row = rows_i64 ? ((const int64_t*)rows)[i] : (int64_t)((const int32_t*)rows)[i];
+  if (row < 0 || row >= table_rows) {
+    if (threadIdx.x == 0) atomicOr(status, HIPATTN_STATUS_PAGE_RANGE);
+    row = 0;
+  }
+  int n = width;
+  if (lens) {
+    const int64_t l = lens_i64 ? ((const int64_t*)lens)[i] : (int64_t)((const int32_t*)lens)[i];
+    n = (int)min((int64_t)width, max(l, (int64_t)0));
+  }
+  const E* src = table + row * row_stride;
+  E* out = dst + (int64_t)i * width;
+  constexpr int V = 16 / sizeof(E);
+  const bool vec = ((uintptr_t)src % 16) == 0 && ((uintptr_t)out % 16) == 0;
+  const int nv = vec ? n / V : 0, first = blockIdx.x * 256 + threadIdx.x, step = gridDim.x * 256;
+  for (int j = first; j < nv; j += step) reinterpret_cast<uint4*>(out)[j] = __ldg(reinterpret_cast<const uint4*>(src) + j);
+  for (int j = nv * V + first; j < n; j += step) out[j] = src[j];
+}
+
 __device__ __forceinline__ int64_t load_int(const CopySeg& s, int64_t at) {
   switch (s.src_type) {
     case COPY_I64: return ((const int64_t*)s.src)[at];
@@ -68,6 +137,35 @@ int begin_call(const BeginCall& c, cudaStream_t stream) {
   if (grid > 148 * 8) grid = 148 * 8;
   begin_call_kernel<<<(unsigned)grid, 256, 0, stream>>>(c);
   return check_launch("begin_call_kernel");
+}
+
+int last_positions(const QueryPositions& q, int32_t* last_pos, cudaStream_t stream) {
+  last_positions_kernel<<<(unsigned)q.B, q.TQ > 256 ? 1024 : 256, 0, stream>>>(q, last_pos);
+  return check_launch("last_positions_kernel");
+}
+
+int convert_rope_tables(const RopeTables& t, cudaStream_t stream) {
+  int64_t grid = ((int64_t)t.rows * (t.cols / 4) + 1023) / 1024;
+  if (grid > 148 * 8) grid = 148 * 8;
+  if (grid < 1) grid = 1;
+  if (t.dtype == HIPATTN_BF16) convert_rope_tables_kernel<HIPATTN_BF16><<<(unsigned)grid, 256, 0, stream>>>(t);
+  else convert_rope_tables_kernel<HIPATTN_F16><<<(unsigned)grid, 256, 0, stream>>>(t);
+  return check_launch("convert_rope_tables_kernel");
+}
+
+int gather_table(const void* table, int64_t table_rows, int64_t row_stride, uint32_t* status, int entry_bytes, const void* rows, int rows_i64, const void* lens, int lens_i64, int n,
+                 int width, void* dst, cudaStream_t stream) {
+  if (n <= 0 || width <= 0) return HIPATTN_OK;
+  int64_t gx = ((int64_t)width * entry_bytes / 16 + 255) / 256;
+  const int64_t most = (148 * 8 + n - 1) / n;
+  if (gx > most) gx = most;
+  if (gx < 1) gx = 1;
+  HIPATTN_REQUIRE(n <= 65535, HIPATTN_ERR_INVALID, "gather_table: %d rows", n);
+  if (entry_bytes == 8)
+    gather_table_kernel<int64_t><<<dim3((unsigned)gx, (unsigned)n), 256, 0, stream>>>((const int64_t*)table, table_rows, row_stride, status, rows, rows_i64, lens, lens_i64, width, (int64_t*)dst);
+  else
+    gather_table_kernel<int32_t><<<dim3((unsigned)gx, (unsigned)n), 256, 0, stream>>>((const int32_t*)table, table_rows, row_stride, status, rows, rows_i64, lens, lens_i64, width, (int32_t*)dst);
+  return check_launch("gather_table_kernel");
 }
 
 int zero_memory(void* ptr, int64_t bytes, cudaStream_t stream) {

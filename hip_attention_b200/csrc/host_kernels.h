@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "../../include/hipattn.h"
+
 namespace hipattn {
 
 struct BeginCall {
@@ -35,6 +37,39 @@ struct CopyList {
 };
 int multi_copy(const CopyList& list, cudaStream_t stream);
 
+// Largest query position of every batch element, clamped to [0, 2^30): q_pos [B, TQ], or pos0 + TQ - 1 when q_pos is null.
+struct QueryPositions {
+  const int64_t* q_pos;
+  int64_t stride_b, stride_t, pos0;
+  int B, TQ;
+};
+int last_positions(const QueryPositions& q, int32_t* last_pos, cudaStream_t stream);
+
+// The rows of two fp32 cos / sin tables that a call can touch, converted to the 16-bit element type: rows up to the larger of
+// `floor` and the largest query position; dst [2][rows][cols].
+struct RopeTables {
+  const float *cos, *sin;
+  int64_t row_stride;
+  int rows, cols, dtype, floor;
+  QueryPositions q;         // few positions: read by every block
+  const int32_t* last_pos;  // [q.B] when given: read instead of the positions
+  void* dst;
+};
+int convert_rope_tables(const RopeTables& t, cudaStream_t stream);
+
+// rows[i] of table [table_rows, width] -> dst [n, width], only the first lens[i] entries of a row when lens is given; a row
+// outside the table reads row 0 and sets HIPATTN_STATUS_PAGE_RANGE
+int gather_table(const void* table, int64_t table_rows, int64_t row_stride, uint32_t* status, int entry_bytes, const void* rows, int rows_i64, const void* lens, int lens_i64, int n,
+                 int width, void* dst, cudaStream_t stream);
+
+// hipattn_scan_prepare_keys[_rope] for live tokens only: those at most `reach` behind last_pos[b]
+int scan_prepare_keys(const hipattn_tokens_t& k, int dtype, int D, int B, int T, int HKV, float k_scale, float* key_abs, void* k_scaled,
+                      uint32_t* status, cudaStream_t stream, const void* rope_cos, const void* rope_sin, int64_t rope_stride, int rope_rows,
+                      int rope_position, const int32_t* last_pos, int reach);
+int validate_tokens(const hipattn_tokens_t& t, int elem_bytes, int D, const char* name);
+// hipattn_merge_partials into rows of `rows_per_group`, the groups group_stride apart
+int merge_partials(const float* part_o, const float* part_lse, int64_t rows, int n_parts, int D, int dtype, void* out, int64_t out_stride,
+                   float* lse_out, int64_t rows_per_group, int64_t group_stride, cudaStream_t stream);
 int zero_memory(void* ptr, int64_t bytes, cudaStream_t stream);
 
 // hipattn_select_stage that also writes the next stage's bounds as int64 (either pointer may be null)

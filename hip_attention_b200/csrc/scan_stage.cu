@@ -329,7 +329,8 @@ int scan_chunks_strict(const hipattn_scan_params_t& p, cudaStream_t stream, bool
 int scan_chunks_mma(const hipattn_scan_params_t& p, cudaStream_t stream, bool* handled);
 int scan_prepare_keys(const hipattn_tokens_t& k, int dtype, int D, int B, int T, int HKV, float k_scale, float* key_abs,
                       void* k_scaled, uint32_t* status, cudaStream_t stream, const void* rope_cos = nullptr,
-                      const void* rope_sin = nullptr, int64_t rope_stride = 0, int rope_rows = 0, int rope_position = 0);
+                      const void* rope_sin = nullptr, int64_t rope_stride = 0, int rope_rows = 0, int rope_position = 0,
+                      const int32_t* last_pos = nullptr, int reach = 0);
 
 }  // namespace hipattn
 

@@ -473,84 +473,113 @@ struct PrepareRope {      // rotate every key to one fixed table position before
   int rows, position;
 };
 
-template <int DT>
-__global__ void scan_prepare_keys_kernel(const hipattn_tokens_t k, int D, int B, int T, int HKV, float k_scale, float* key_abs,
-                                         unsigned char* k_scaled, uint32_t* status, const PrepareRope rope) {
-  const int pieces = D * 2 / 16;
-  const int rows_per_block = blockDim.x / pieces;
-  const int sub = threadIdx.x / pieces, piece = threadIdx.x % pieces;
+// Sixteen (head dim 64: eight) lanes per row, UNROLL rows of a lane in flight: the kernel is bound by memory once the
+// look-ups and loads of several rows overlap (90112 tokens of 8 heads through a page table of one token each, both rotated
+// copies: 213 us with one row at a time, 122 now).  Rows are dealt token by token, so that the heads of a token, which lie
+// next to each other in the cache, are read together.  last_pos: the largest query position of every batch element (or
+// null); tokens more than `reach` behind it belong to no chunk that is ever active and are left out.
+constexpr int kPrepareUnroll = 4;
+
+template <int DT, int PIECES, bool ROPE>
+__global__ void __launch_bounds__(256) scan_prepare_keys_kernel(const hipattn_tokens_t k, int B, int T, int HKV, float k_scale, float* key_abs,
+                                                                unsigned char* k_scaled, uint32_t* status, const PrepareRope rope, int ctas_per_seq,
+                                                                const int32_t* last_pos, int reach) {
+  using P = typename Pair16<DT>::type;
+  constexpr int RB = 256 / PIECES, ROWB = PIECES * 16, U = kPrepareUnroll, HALF = PIECES / 2;
+  const int sub = threadIdx.x / PIECES, piece = threadIdx.x % PIECES;
+  const int b = blockIdx.x / ctas_per_seq, part = blockIdx.x % ctas_per_seq;
   const int64_t total = (int64_t)B * T * HKV;
+  int live = T;
+  if (last_pos) live = min((int64_t)T, (int64_t)max(last_pos[b], 0) + reach + 1);
+  const int rows = live * HKV;
   const uint32_t kscale2 = pack_scalar2<DT>(k_scale);
-  for (int64_t r = (int64_t)blockIdx.x * rows_per_block + sub; r < total; r += (int64_t)gridDim.x * rows_per_block) {
-    const int hkv = (int)(r % HKV);
-    const int64_t bt = r / HKV;
-    const int t = (int)(bt % T), b = (int)(bt / T);
-    const char* src = token_row(k, b, t, hkv, 2, status);
-    const uint4 w = k.fp8_e5m2 ? widen_fp8_e5m2<DT>(*reinterpret_cast<const uint2*>(src + piece * 8))
-                               : *reinterpret_cast<const uint4*>(src + piece * 16);
-    const int64_t ro = ((int64_t)b * HKV + hkv) * T + t;     // head-major: the tokens of a KV head are contiguous
-    // scales a piece, sums its magnitude over the row and stores both into copy `side`
-    auto emit = [&](uint32_t* v, int side) {
-      float s = 0.f;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        v[i] = mul2<DT>(v[i], kscale2);
-        const uint32_t m = v[i] & 0x7fff7fffu;
-        s += lo_f32<DT>(m) + hi_f32<DT>(m);
-      }
-      const int64_t rs = ro + (int64_t)side * total;
-      if (k_scaled) *reinterpret_cast<uint4*>(k_scaled + rs * (int64_t)(D * 2) + piece * 16) = make_uint4(v[0], v[1], v[2], v[3]);
-      for (int o = pieces >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (piece == 0 && key_abs) key_abs[rs] = s;
-    };
-    if (rope.cos != nullptr) {
-      const int half = pieces >> 1, pr = piece < half ? piece + half : piece - half;
-      const uint4 wr = k.fp8_e5m2 ? widen_fp8_e5m2<DT>(*reinterpret_cast<const uint2*>(src + pr * 8))
-                                  : *reinterpret_cast<const uint4*>(src + pr * 16);
-      // rotation on packed 16-bit pairs: products and sum round once to the element type, as the scalar form does
-      using P = typename Pair16<DT>::type;
-      const uint32_t xv[4] = {w.x, w.y, w.z, w.w}, rv[4] = {wr.x, wr.y, wr.z, wr.w};
-      // position -1: both copies of the "relative" backend (table positions 0 and 1) from one read of the row
-      const int n_pos = rope.position < 0 ? 2 : 1;
-      for (int sd = 0; sd < n_pos; ++sd) {
-        const int pos = rope.position < 0 ? sd : rope.position;
-        const uint4 tc = rope_table_raw(rope.cos, rope.stride, rope.rows, pos, piece % half);
-        const uint4 ts = rope_table_raw(rope.sin, rope.stride, rope.rows, pos, piece % half);
-        const uint32_t cv[4] = {tc.x, tc.y, tc.z, tc.w}, sv[4] = {ts.x, ts.y, ts.z, ts.w};
-        uint32_t v[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const P xp = *reinterpret_cast<const P*>(&xv[i]), rp = *reinterpret_cast<const P*>(&rv[i]);
-          const P cp = *reinterpret_cast<const P*>(&cv[i]), sp = *reinterpret_cast<const P*>(&sv[i]);
-          const P rot = __hadd2_rn(__hmul2_rn(xp, cp), __hmul2_rn(piece < half ? __hneg2(rp) : rp, sp));
-          v[i] = *reinterpret_cast<const uint32_t*>(&rot);
-        }
-        emit(v, sd);
-      }
-    } else {
-      uint32_t v[4] = {w.x, w.y, w.z, w.w};
-      emit(v, 0);
+  auto as_p = [](uint32_t w) { return *reinterpret_cast<const P*>(&w); };
+  // table pieces of the one or two positions (position -1: both copies of the "relative" backend, table positions 0 and 1)
+  const int n_pos = ROPE && rope.position < 0 ? 2 : 1;
+  uint4 tc[ROPE ? 2 : 1], ts[ROPE ? 2 : 1];
+  if constexpr (ROPE) {
+    for (int sd = 0; sd < n_pos; ++sd) {
+      const int pos = rope.position < 0 ? sd : rope.position;
+      tc[sd] = rope_table_raw(rope.cos, rope.stride, rope.rows, pos, piece % HALF);
+      ts[sd] = rope_table_raw(rope.sin, rope.stride, rope.rows, pos, piece % HALF);
     }
   }
+  for (int base = part * RB * U; base < rows; base += ctas_per_seq * RB * U) {
+    uint4 w[U];
+    int64_t ro[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int r = min(base + u * RB + sub, rows - 1);   // (the tail repeats the last row)
+      const int t = r / HKV, hkv = r - t * HKV;
+      const char* src = token_row(k, b, t, hkv, 2, status);
+      w[u] = k.fp8_e5m2 ? widen_fp8_e5m2<DT>(__ldg(reinterpret_cast<const uint2*>(src + piece * 8))) : __ldg(reinterpret_cast<const uint4*>(src + piece * 16));
+      ro[u] = ((int64_t)b * HKV + hkv) * T + t;     // head-major: the tokens of a KV head are contiguous
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t xv[4] = {w[u].x, w[u].y, w[u].z, w[u].w};
+      uint32_t rv[4];
+      if constexpr (ROPE) {   // the piece half a row away, with the sign of rotate_half
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          rv[i] = __shfl_xor_sync(0xffffffffu, xv[i], HALF);
+          if (piece < HALF) rv[i] ^= 0x80008000u;
+        }
+      }
+#pragma unroll
+      for (int sd = 0; sd < (ROPE ? 2 : 1); ++sd) {
+        if (sd >= n_pos) break;
+        uint32_t v[4];
+        float s = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          v[i] = xv[i];
+          if constexpr (ROPE) {
+            // rotation on packed 16-bit pairs: products and sum round once to the element type, as the scalar form does
+            const uint32_t cv[4] = {tc[sd].x, tc[sd].y, tc[sd].z, tc[sd].w}, sv[4] = {ts[sd].x, ts[sd].y, ts[sd].z, ts[sd].w};
+            const P rot = __hadd2_rn(__hmul2_rn(as_p(xv[i]), as_p(cv[i])), __hmul2_rn(as_p(rv[i]), as_p(sv[i])));
+            v[i] = *reinterpret_cast<const uint32_t*>(&rot);
+          }
+          v[i] = mul2<DT>(v[i], kscale2);
+          const uint32_t m = v[i] & 0x7fff7fffu;
+          s += lo_f32<DT>(m) + hi_f32<DT>(m);
+        }
+        const int64_t rs = ro[u] + (int64_t)sd * total;
+        if (k_scaled) *reinterpret_cast<uint4*>(k_scaled + rs * ROWB + piece * 16) = make_uint4(v[0], v[1], v[2], v[3]);
+#pragma unroll
+        for (int o = PIECES >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (piece == 0 && key_abs) key_abs[rs] = s;
+      }
+    }
+  }
+}
+
+template <int DT, int PIECES>
+int launch_prepare(const hipattn_tokens_t& k, int B, int T, int HKV, float k_scale, float* key_abs, void* k_scaled, uint32_t* status,
+                   const PrepareRope& rope, const int32_t* last_pos, int reach, cudaStream_t stream) {
+  const int64_t per_cta = 256 / PIECES * kPrepareUnroll, rows = (int64_t)T * HKV;
+  int64_t ctas = (rows + per_cta - 1) / per_cta;
+  const int64_t most = (148 * 16 + B - 1) / B;   // two waves of eight resident CTAs
+  if (ctas > most) ctas = most;
+  HIPATTN_REQUIRE(rows < 0x7fffffffLL && ctas * B < 0x7fffffffLL, HIPATTN_ERR_INVALID, "scan_prepare_keys: %lld rows per sequence", (long long)rows);
+  auto kern = rope.cos ? scan_prepare_keys_kernel<DT, PIECES, true> : scan_prepare_keys_kernel<DT, PIECES, false>;
+  kern<<<(unsigned)(ctas * B), 256, 0, stream>>>(k, B, T, HKV, k_scale, key_abs, (unsigned char*)k_scaled, status, rope, (int)ctas, last_pos, reach);
+  return check_launch("scan_prepare_keys_kernel");
 }
 
 }  // namespace
 
 int scan_prepare_keys(const hipattn_tokens_t& k, int dtype, int D, int B, int T, int HKV, float k_scale, float* key_abs,
                       void* k_scaled, uint32_t* status, cudaStream_t stream, const void* rope_cos, const void* rope_sin,
-                      int64_t rope_stride, int rope_rows, int rope_position) {
+                      int64_t rope_stride, int rope_rows, int rope_position, const int32_t* last_pos, int reach) {
   const PrepareRope rope{rope_cos, rope_sin, rope_stride, rope_rows, rope_position};
   HIPATTN_REQUIRE(dtype == HIPATTN_BF16 || dtype == HIPATTN_F16, HIPATTN_ERR_UNSUPPORTED, "scan_prepare_keys: 16-bit element types only");
   HIPATTN_REQUIRE(D == 64 || D == 128, HIPATTN_ERR_UNSUPPORTED, "scan_prepare_keys: head dimension %d is not built (64, 128)", D);
-  const int64_t total = (int64_t)B * T * HKV;
-  const int rows_per_block = 256 / (D * 2 / 16);
-  int64_t grid = (total + rows_per_block - 1) / rows_per_block;
-  if (grid > 148 * 32) grid = 148 * 32;
   if (dtype == HIPATTN_BF16)
-    scan_prepare_keys_kernel<HIPATTN_BF16><<<(unsigned)grid, 256, 0, stream>>>(k, D, B, T, HKV, k_scale, key_abs, (unsigned char*)k_scaled, status, rope);
-  else
-    scan_prepare_keys_kernel<HIPATTN_F16><<<(unsigned)grid, 256, 0, stream>>>(k, D, B, T, HKV, k_scale, key_abs, (unsigned char*)k_scaled, status, rope);
-  return check_launch("scan_prepare_keys_kernel");
+    return D == 128 ? launch_prepare<HIPATTN_BF16, 16>(k, B, T, HKV, k_scale, key_abs, k_scaled, status, rope, last_pos, reach, stream)
+                    : launch_prepare<HIPATTN_BF16, 8>(k, B, T, HKV, k_scale, key_abs, k_scaled, status, rope, last_pos, reach, stream);
+  return D == 128 ? launch_prepare<HIPATTN_F16, 16>(k, B, T, HKV, k_scale, key_abs, k_scaled, status, rope, last_pos, reach, stream)
+                  : launch_prepare<HIPATTN_F16, 8>(k, B, T, HKV, k_scale, key_abs, k_scaled, status, rope, last_pos, reach, stream);
 }
 
 // Takes 16-bit prefill shapes (16 to 128 pooled rows in multiples of 16, head dim 64 or 128) when the

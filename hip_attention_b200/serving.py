@@ -19,7 +19,7 @@ import torch
 from torch import Tensor
 
 from .metadata import (HiPAttentionArgs, HiPAttentionOutputMetadata, HiPAttentionStageInputCache, ScanStage)
-from .operator import hip_attention_12, host
+from .operator import hip_attention_12, hip_attention_impl, host
 
 
 def _default_stages() -> List[ScanStage]:
@@ -419,7 +419,10 @@ def forward_paged_hip(query: Tensor, sm_scale: float, batch_size: int, k_cache: 
         v_cache = v_cache.view(v_cache.shape[0], 1, v_cache.shape[1], hidden)
     elif k is None:
         raise ValueError("neither k_cache nor k was given")
-    block_table = req_to_tokens.index_select(0, req_pool_indices)
+    # the table's rows of this batch, as far as the sequences reach (entries beyond them are never read)
+    block_table = host().gather_table(req_to_tokens, req_pool_indices, seq_lens) if req_to_tokens.is_cuda else None
+    if block_table is None:
+        block_table = req_to_tokens.index_select(0, req_pool_indices)
     if block_table.shape[0] != batch_size:
         raise ValueError("req_pool_indices must name one request per batch entry")
     head_dim = k_cache.shape[-1] if k_cache is not None else k.shape[-1]
@@ -449,8 +452,14 @@ def forward_paged_hip(query: Tensor, sm_scale: float, batch_size: int, k_cache: 
         return context.to(query.dtype), metadata
     if query_for_mask is not None:
         raise ValueError("query_for_mask cannot be combined with the split of a prefill chunk")
-    sparse, _ = hip_attention_12((query[:, :-LAST_DENSE] * sm_scale).to(query.dtype), k, v,
-                                 args=make_args(pos[:, :-LAST_DENSE], layer.sliding_window_size), cached_metadata=cached_metadata)
-    dense, metadata = hip_attention_12((query[:, -LAST_DENSE:] * sm_scale).to(query.dtype), k, v,
-                                       args=make_args(pos[:, -LAST_DENSE:], 777), cached_metadata=cached_metadata)
-    return torch.cat([sparse.to(query.dtype), dense.to(query.dtype)], dim=1), metadata
+    scaled = (query * sm_scale).to(query.dtype)
+    parts = (slice(None, -LAST_DENSE), layer.sliding_window_size), (slice(-LAST_DENSE, None), 777)
+    if cached_metadata is not None or not scaled.is_cuda:
+        sparse, _ = hip_attention_12(scaled[:, parts[0][0]], k, v, args=make_args(pos[:, parts[0][0]], parts[0][1]), cached_metadata=cached_metadata)
+        dense, metadata = hip_attention_12(scaled[:, parts[1][0]], k, v, args=make_args(pos[:, parts[1][0]], parts[1][1]), cached_metadata=cached_metadata)
+        return torch.cat([sparse.to(query.dtype), dense.to(query.dtype)], dim=1), metadata
+    # both parts read the same keys (prepared once, for the chunk's positions) and write their rows of one output
+    shared, context = {"positions": pos.to(torch.int64)}, torch.empty_like(scaled)
+    for rows, window in parts:
+        _, metadata = hip_attention_impl(scaled[:, rows], k, v, make_args(pos[:, rows], window), None, shared=shared, out=context[:, rows])
+    return context, metadata
