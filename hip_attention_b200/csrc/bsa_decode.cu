@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(kDecodeWarps<ROPE, F8> * 32, 2) bsa_decode_mma
       const int t = key_position_at(kl, j, start, &w);
       if (admits(pq, t, w, p.window)) {
         tok = t;
-        if (ROPE) rp = rope_key_position(kl, j, t, p.window);
+        if (ROPE) rp = rope_key_position(kl, j, t);
         page = 0;
         if (paged && t < reach) {
           const int64_t o = (int64_t)b * p.k.table_stride_b + (page_shift >= 0 ? (t >> page_shift) : (t / page_size));

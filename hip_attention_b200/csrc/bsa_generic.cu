@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kThreads) bsa_generic_kernel(const hipattn_bsa
           float xr[VEC], tc[VEC], ts[VEC];
           const int pr = pc < HALF ? pc + HALF : pc - HALF;
           widen16<DT>(k8 ? widen_fp8_e5m2<KDT>(*reinterpret_cast<const uint2*>(kr + pr * 8)) : *reinterpret_cast<const uint4*>(kr + pr * 16), xr);
-          const int new_t = rope_key_position(kl, j0 + kk, t, p.window);
+          const int new_t = rope_key_position(kl, j0 + kk, t);
           rope_table_piece<DT>(p.rope_cos, p.rope_stride, p.rope_rows, new_t, pc % HALF, tc);
           rope_table_piece<DT>(p.rope_sin, p.rope_stride, p.rope_rows, new_t, pc % HALF, ts);
           rope_rotate_piece<DT, VEC>(kv, xr, tc, ts, pc < HALF);

@@ -103,7 +103,8 @@ __global__ void __launch_bounds__(M * 2) bsa_mma_kernel(const hipattn_bsa_params
   }
   const int pmin = s_mm[0], pmax = s_mm[1];
   const int rmin = s_mm[2], rmax = s_mm[3];
-  const KeyList kl = make_key_list(p, b, h0, d, pmin, pmax);
+  KeyList kl = make_key_list(p, b, h0, d, pmin, pmax);
+  trim_selected(kl, rmax, p.window);
   // the tiles of this CTA's key range (all of them unless the caller asked for key splits)
   const int all_tiles = cdiv(kl.total, TKM);
   const int per_split = cdiv(all_tiles, p.n_splits);
@@ -133,7 +134,7 @@ __global__ void __launch_bounds__(M * 2) bsa_mma_kernel(const hipattn_bsa_params
       }
       m.koff[tid] = ko;
       m.voff[tid] = vo;
-      m.rpos[tid] = (t >= 0 && p.rope_cos) ? rope_key_position(kl, j, t, p.window) : -1;
+      m.rpos[tid] = (t >= 0 && p.rope_cos) ? rope_key_position(kl, j, t) : -1;
       const bool far_ok = t >= 0 && !w && t <= rmin - p.window;
       const bool win_ok = t >= 0 && w && t > rmax - p.window && t <= rmin;
       const int f = __all_sync(0xffffffffu, far_ok), g = __all_sync(0xffffffffu, win_ok);

@@ -297,7 +297,8 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
   __syncthreads();
   const int pmin = s_mm[0], pmax = s_mm[1];
   const int rmin = s_mm[2], rmax = s_mm[3];
-  const KeyList kl = make_key_list(p, b, h0, d, pmin, pmax);
+  KeyList kl = make_key_list(p, b, h0, d, pmin, pmax);
+  trim_selected(kl, rmax, p.window);
   // the tiles of this CTA's key range (all of them unless the caller asked for key splits)
   const int all_tiles = cdiv(kl.total, TK5);
   const int per_split = SPLIT ? cdiv(all_tiles, p.n_splits) : all_tiles;
@@ -368,7 +369,7 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
     }
     m.kptr[e] = ko >= 0 ? kbase + ko : reinterpret_cast<const char*>(g_zero_row);
     m.vptr[e] = vo >= 0 ? vbase + vo : reinterpret_cast<const char*>(g_zero_row);
-    if (ROPE) ms.rpos[e] = t >= 0 ? rope_key_position(kl, j, t, p.window) : -1;
+    if (ROPE) ms.rpos[e] = t >= 0 ? rope_key_position(kl, j, t) : -1;
     const bool far_ok = t >= 0 && !w && t <= rmin - p.window;
     const bool win_ok = t >= 0 && w && t > rmax - p.window && t <= rmin;
     const int f = __all_sync(0xffffffffu, far_ok), g = __all_sync(0xffffffffu, win_ok);
