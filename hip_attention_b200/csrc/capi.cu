@@ -85,6 +85,28 @@ __global__ void merge_kernel(const float* __restrict__ part_o, const float* __re
   if (lse_out && threadIdx.x == 0) lse_out[row] = tot > 0.f ? m + log2f(tot) : -INFINITY;
 }
 
+// The same merge over shard outputs in the element type, part-major.
+template <int DT>
+__global__ void merge_shards_kernel(const typename Elem<DT>::type* __restrict__ outs, const float* __restrict__ lses, int64_t rows, int parts, int D,
+                                    typename Elem<DT>::type* __restrict__ out) {
+  const int64_t row = blockIdx.x;
+  float m = -INFINITY;
+  for (int s = 0; s < parts; ++s) m = fmaxf(m, __ldg(lses + s * rows + row));
+  float tot = 0.f;
+  for (int s = 0; s < parts; ++s) {
+    const float l = __ldg(lses + s * rows + row);
+    if (l > -INFINITY) tot += exp2f(l - m);
+  }
+  for (int e = threadIdx.x; e < D; e += blockDim.x) {
+    float acc = 0.f;
+    for (int s = 0; s < parts; ++s) {
+      const float l = __ldg(lses + s * rows + row);
+      if (l > -INFINITY) acc += exp2f(l - m) * Elem<DT>::to_f32(outs[(s * rows + row) * D + e]);
+    }
+    out[row * D + e] = Elem<DT>::from_f32(tot > 0.f ? acc / tot : 0.f);
+  }
+}
+
 // Access statistics of the attention: `parts` CTAs per (batch, KV head, attention block) mark the tokens the reference's
 // kernels load for that block (see hipattn_mark_attention_access in the header).
 __global__ void mark_attention_access_kernel(const hipattn_bsa_params_t p, int32_t* counter, int64_t stride_b, int64_t stride_h,
@@ -275,6 +297,16 @@ int hipattn::merge_partials(const float* part_o, const float* part_lse, int64_t 
     default: set_error("merge_partials: unknown dtype %d", dtype); return HIPATTN_ERR_INVALID;
   }
   return check_launch("merge_kernel");
+}
+
+int hipattn::merge_shards(const void* outs, const float* lses, int64_t rows, int parts, int D, int dtype, void* out, cudaStream_t s) {
+  HIPATTN_REQUIRE(rows > 0 && rows < 0x7fffffffLL && parts > 0 && D > 0, HIPATTN_ERR_INVALID, "merge_shards: bad sizes");
+  switch (dtype) {
+    case HIPATTN_F32: merge_shards_kernel<HIPATTN_F32><<<(unsigned)rows, 128, 0, s>>>((const float*)outs, lses, rows, parts, D, (float*)out); break;
+    case HIPATTN_F16: merge_shards_kernel<HIPATTN_F16><<<(unsigned)rows, 128, 0, s>>>((const __half*)outs, lses, rows, parts, D, (__half*)out); break;
+    default: merge_shards_kernel<HIPATTN_BF16><<<(unsigned)rows, 128, 0, s>>>((const __nv_bfloat16*)outs, lses, rows, parts, D, (__nv_bfloat16*)out);
+  }
+  return check_launch("merge_shards_kernel");
 }
 
 extern "C" int32_t hipattn_encode_score(float score) {

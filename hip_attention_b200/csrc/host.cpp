@@ -179,7 +179,70 @@ float round_to(float x, int dt) {
 
 struct Device {
   c10::Device dev;
-  at::Tensor empty(at::IntArrayRef sizes, at::ScalarType t) const { return at::detail::empty_cuda(sizes, t, dev, c10::nullopt); }
+  std::vector<at::Tensor>* keep = nullptr;   // a call beside the current stream: holds its memory until the streams have joined
+  at::Tensor empty(at::IntArrayRef sizes, at::ScalarType t) const {
+    at::Tensor x = at::detail::empty_cuda(sizes, t, dev, c10::nullopt);
+    if (keep) keep->push_back(x);
+    return x;
+  }
+};
+
+// Calls that do not depend on one another run beside the current stream: fork() marks the point they start from, forward()
+// with the fork launches on a stream of the pool, join() makes the current stream wait for all of them.  Memory still
+// belongs to the current stream; what the calls allocate is held until the join, so nothing is reused under them.
+struct Fork {
+  c10::Device dev{at::kCUDA, 0};
+  c10::cuda::CUDAStream main;
+  cudaEvent_t start = nullptr;
+  std::vector<cudaEvent_t> done;
+  std::vector<at::Tensor> keep;
+  explicit Fork(c10::Device d) : dev(d), main(c10::cuda::getCurrentCUDAStream(d.index())) {}
+  ~Fork() {
+    join();
+    if (start) cudaEventDestroy(start);
+  }
+  void join() {
+    for (cudaEvent_t e : done) {
+      cudaStreamWaitEvent(main.stream(), e, 0);
+      cudaEventDestroy(e);
+    }
+    done.clear();
+    keep.clear();
+  }
+};
+void cuda_ok(cudaError_t e, const char* what) {
+  if (e != cudaSuccess) fail(PyExc_RuntimeError, "%s: %s", what, cudaGetErrorString(e));
+}
+const char* kForkName = "hip_attention_b200.fork";
+void drop_fork(PyObject* o) { delete (Fork*)PyCapsule_GetPointer(o, kForkName); }
+// the launches of one call on a stream of the pool; the end is marked however the call ends
+struct Beside {
+  Fork* fork = nullptr;
+  cudaStream_t stream = nullptr;
+  void begin(Fork* f) {
+    stream = c10::cuda::getStreamFromPool(false, f->dev.index()).stream();
+    cuda_ok(cudaStreamWaitEvent(stream, f->start, 0), "cudaStreamWaitEvent");
+    fork = f;
+  }
+  // work given to the current stream in between comes first
+  void after_current() {
+    if (!fork) return;
+    cudaEvent_t e;
+    cuda_ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+    cudaEventRecord(e, fork->main.stream());
+    cudaStreamWaitEvent(stream, e, 0);
+    cudaEventDestroy(e);
+  }
+  ~Beside() {
+    if (!fork) return;
+    cudaEvent_t e;
+    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess) {
+      cudaEventRecord(e, stream);
+      fork->done.push_back(e);
+    } else {
+      cudaStreamSynchronize(stream);
+    }
+  }
 };
 
 // Device status word (one int32 per device) the kernels OR their HIPATTN_STATUS_* bits into.
@@ -729,7 +792,7 @@ void attention(Call& c, const hipattn_tokens_t& ktok, const hipattn_tokens_t& vt
                const AttentionArgs& a, const at::Tensor& access, at::Tensor& out, at::Tensor& lse) {
   const Device& dv = c.dv;
   if (!out.defined()) out = dv.empty({c.B, c.TQ, c.H, c.D}, c.q_attn.scalar_type());
-  if (a.want_lse) lse = dv.empty({c.B, c.TQ, c.H}, at::kFloat);
+  if (a.want_lse && !lse.defined()) lse = dv.empty({c.B, c.TQ, c.H}, at::kFloat);
   const int64_t Kk = indices.size(2);
   hipattn_bsa_params_t bp;
   memset(&bp, 0, sizeof(bp));
@@ -829,7 +892,9 @@ PyObject* forward(PyObject* const* argv) {
   c.timer = argv[8];
   PyObject* v_ready = argv[9];
   c.shared = argv[10];
-  at::Tensor context = tensor_of(argv[11], "out");
+  at::Tensor context = tensor_of(argv[11], "out"), lse = tensor_of(argv[12], "lse");
+  Fork* fork = argv[13] == Py_None ? nullptr : (Fork*)PyCapsule_GetPointer(argv[13], kForkName);
+  if (argv[13] != Py_None && !fork) throw PyError{};
 
   if (!THPVariable_Check(q_obj) || THPVariable_Unpack(q_obj).dim() != 4) VALUE_ERROR("q must be a tensor [B, TQ, H, D]");
   c.q = THPVariable_Unpack(q_obj);
@@ -872,6 +937,15 @@ PyObject* forward(PyObject* const* argv) {
   c.stream = c10::cuda::getCurrentCUDAStream(c.q.device().index()).stream();
   at::Tensor status = status_word(c.q.device().index());
   c.status = (uint32_t*)status.data_ptr();
+  Beside beside;
+  // (a decode call with something to scan and no rope tables: nothing on its way is a torch operation)
+  if (fork) {
+    c.dv.keep = &fork->keep;    // (memory that a call on the current stream gives back could be handed to one beside it)
+    if (PyObject_IsTrue(argv[14]) == 1 && c.TQ == 1 && !c.using_extend && c.T - c.sink - c.sw > 0 && c.q.device() == fork->dev) {
+      beside.begin(fork);
+      c.stream = beside.stream;
+    }
+  }
 
   hipattn::BeginCall begin{};
   Ref pos_obj = attr(c.args, N.position_ids);
@@ -884,7 +958,7 @@ PyObject* forward(PyObject* const* argv) {
   } else {
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(c.stream, &capturing);
-    if (capturing != cudaStreamCaptureStatusNone) VALUE_ERROR("position_ids must be given under CUDA graph capture");
+    if (capturing != cudaStreamCaptureStatusNone && c.shared == Py_None) VALUE_ERROR("position_ids must be given under CUDA graph capture");
     own_pos = true;
     at::Tensor row = c.dv.empty({c.TQ}, at::kLong);
     begin.pos = row.data_ptr<int64_t>();
@@ -1003,6 +1077,8 @@ PyObject* forward(PyObject* const* argv) {
     } else {
       indices = ci.clone().to(at::kLong).contiguous(); ks = cks.clone().to(at::kLong).contiguous(); ks_count = ckc.clone(); kse = cse.clone();
       if (indices.device() != c.q.device() || ks.device() != c.q.device()) VALUE_ERROR("cached metadata is on another device than q");
+      beside.after_current();
+      if (c.dv.keep) c.dv.keep->insert(c.dv.keep->end(), {indices, ks});
     }
   }
 
@@ -1031,7 +1107,8 @@ PyObject* forward(PyObject* const* argv) {
     Ref s = checked(PyObject_CallMethodOneArg(K.torch_cuda, N.current_stream, dev.get()));
     Ref r = checked(PyObject_CallMethodOneArg(s.get(), N.wait_event, v_ready));
   }
-  at::Tensor lse;
+  if (lse.defined() && (lse.scalar_type() != at::kFloat || lse.numel() != c.B * c.TQ * c.H || !lse.is_contiguous()))
+    VALUE_ERROR("lse must be a contiguous float32 tensor [B, TQ, H]");
   attention(c, ktok, vtok, indices, ks, a, sa_stats, context, lse);
   c.mark("attention");
 
@@ -1152,8 +1229,8 @@ PyObject* guarded(F f) {
 }
 
 PyObject* py_forward(PyObject*, PyObject* const* argv, Py_ssize_t n) {
-  if (n != 12) {
-    PyErr_SetString(PyExc_TypeError, "forward takes twelve arguments");
+  if (n != 15) {
+    PyErr_SetString(PyExc_TypeError, "forward takes fifteen arguments");
     return nullptr;
   }
   return guarded([&] { return forward(argv); });
@@ -1172,6 +1249,84 @@ PyObject* gather_table(PyObject* const* argv) {
                               lens.scalar_type() == at::kLong, (int)rows.size(0), (int)table.size(1), out.data_ptr(),
                               c10::cuda::getCurrentCUDAStream(table.device().index()).stream()), "gather_table");
   return wrap(out);
+}
+// fork(tensor): the point of the current stream of its device that calls beside it start from
+PyObject* py_fork(PyObject*, PyObject* x) {
+  return guarded([&]() -> PyObject* {
+    const at::Tensor t = tensor_of(x, "q");
+    const c10::cuda::CUDAGuard guard(t.device());
+    status_word(t.device().index());
+    std::unique_ptr<Fork> f(new Fork(t.device()));
+    cuda_ok(cudaEventCreateWithFlags(&f->start, cudaEventDisableTiming), "cudaEventCreate");
+    cuda_ok(cudaEventRecord(f->start, f->main.stream()), "cudaEventRecord");
+    PyObject* o = PyCapsule_New(f.get(), kForkName, drop_fork);
+    if (o) f.release();
+    return o;
+  });
+}
+PyObject* py_join(PyObject*, PyObject* o) {
+  return guarded([&]() -> PyObject* {
+    Fork* f = (Fork*)PyCapsule_GetPointer(o, kForkName);
+    if (!f) return nullptr;
+    const c10::cuda::CUDAGuard guard(f->dev);
+    f->join();
+    Py_RETURN_NONE;
+  });
+}
+// stack_rows([[tensors...], ...]): every list of [rows, ...] tensors one below the other, in one launch
+PyObject* stack_rows(PyObject* lists) {
+  const Py_ssize_t n = PyList_GET_SIZE(lists);
+  Ref out = checked(PyList_New(n));
+  std::unique_ptr<c10::cuda::CUDAGuard> guard;
+  std::unique_ptr<Copies> cp;
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    PyObject* l = PyList_GET_ITEM(lists, i);
+    const Py_ssize_t m = PyList_GET_SIZE(l);
+    const at::Tensor first = tensor_of(PyList_GET_ITEM(l, 0), "rows");
+    if (!cp) {
+      guard.reset(new c10::cuda::CUDAGuard(first.device()));
+      cp.reset(new Copies(c10::cuda::getCurrentCUDAStream(first.device().index()).stream()));
+    }
+    std::vector<int64_t> sizes = first.sizes().vec();
+    int64_t rows = 0;
+    for (Py_ssize_t j = 0; j < m; ++j) {
+      const at::Tensor t = tensor_of(PyList_GET_ITEM(l, j), "rows");
+      if (t.scalar_type() != first.scalar_type() || t.device() != first.device() || t.dim() != first.dim() || t.dim() < 1 || t.sizes().slice(1) != first.sizes().slice(1))
+        VALUE_ERROR("shards of one page pool must have block tables and lengths of the same type and width");
+      rows += t.size(0);
+    }
+    sizes[0] = rows;
+    at::Tensor dst = at::detail::empty_cuda(sizes, first.scalar_type(), first.device(), c10::nullopt);
+    int64_t at_row = 0;
+    for (Py_ssize_t j = 0; j < m; ++j) {
+      const at::Tensor t = tensor_of(PyList_GET_ITEM(l, j), "rows");
+      cp->add(t, dst.narrow(0, at_row, t.size(0)));
+      at_row += t.size(0);
+    }
+    PyList_SET_ITEM(out.get(), i, wrap(dst));
+  }
+  if (cp) cp->flush();
+  return out.release();
+}
+PyObject* py_stack_rows(PyObject*, PyObject* lists) {
+  return guarded([&] { return stack_rows(lists); });
+}
+// merge_shards(outs [S, B, 1, H, D], lses [S, B, 1, H]) -> [B, 1, H, D]
+PyObject* py_merge_shards(PyObject*, PyObject* const* argv, Py_ssize_t n) {
+  if (n != 2) {
+    PyErr_SetString(PyExc_TypeError, "merge_shards takes two arguments");
+    return nullptr;
+  }
+  return guarded([&]() -> PyObject* {
+    const at::Tensor o = tensor_of(argv[0], "outs"), l = tensor_of(argv[1], "lses");
+    if (dtype_of(o.scalar_type()) < 0 || o.dim() != 5 || l.dim() != 4 || !o.is_contiguous() || !l.is_contiguous() || l.numel() * o.size(4) != o.numel())
+      VALUE_ERROR("merge_shards: outs [S, B, 1, H, D] and lses [S, B, 1, H] must be contiguous");
+    const c10::cuda::CUDAGuard guard(o.device());
+    at::Tensor out = at::detail::empty_cuda(o.sizes().slice(1), o.scalar_type(), o.device(), c10::nullopt);
+    check(hipattn::merge_shards(o.data_ptr(), l.data_ptr<float>(), l.numel() / l.size(0), (int)l.size(0), (int)o.size(4), dtype_of(o.scalar_type()),
+                                out.data_ptr(), c10::cuda::getCurrentCUDAStream(o.device().index()).stream()), "merge_shards");
+    return wrap(out);
+  });
 }
 PyObject* py_gather_table(PyObject*, PyObject* const* argv, Py_ssize_t n) {
   if (n != 3) {
@@ -1201,8 +1356,12 @@ PyObject* py_bind(PyObject*, PyObject* const* argv, Py_ssize_t n) {
 }
 
 PyMethodDef methods[] = {
-    {"forward", (PyCFunction)(void*)py_forward, METH_FASTCALL, "q, k, v, args, cached_metadata, return_lse, debug, score_reduce, timer, v_ready, shared, out"},
+    {"forward", (PyCFunction)(void*)py_forward, METH_FASTCALL, "q, k, v, args, cached_metadata, return_lse, debug, score_reduce, timer, v_ready, shared, out, lse, fork, beside"},
     {"gather_table", (PyCFunction)(void*)py_gather_table, METH_FASTCALL, "table, rows, lens -> rows of the table, or None when it does not take them"},
+    {"fork", py_fork, METH_O, "tensor -> fork of the current stream"},
+    {"join", py_join, METH_O, "fork"},
+    {"stack_rows", py_stack_rows, METH_O, "[[tensors], ...] -> [tensor, ...]"},
+    {"merge_shards", (PyCFunction)(void*)py_merge_shards, METH_FASTCALL, "outs, lses -> context"},
     {"status_word", py_status_word, METH_O, "device index -> int32 tensor [1]"},
     {"pool_read", py_pool_read, METH_O, "[(buffer, rows), ...] -> list of tensors"},
     {"pool_write", py_pool_write, METH_O, "[(buffer, value or None, rows), ...]"},

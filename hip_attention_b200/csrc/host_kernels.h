@@ -70,6 +70,8 @@ int validate_tokens(const hipattn_tokens_t& t, int elem_bytes, int D, const char
 // hipattn_merge_partials into rows of `rows_per_group`, the groups group_stride apart
 int merge_partials(const float* part_o, const float* part_lse, int64_t rows, int n_parts, int D, int dtype, void* out, int64_t out_stride,
                    float* lse_out, int64_t rows_per_group, int64_t group_stride, cudaStream_t stream);
+// Log-sum-exp merge of shard outputs in the element type: outs [parts, rows, D], lses [parts, rows] base-2 -> out [rows, D]
+int merge_shards(const void* outs, const float* lses, int64_t rows, int parts, int D, int dtype, void* out, cudaStream_t stream);
 int zero_memory(void* ptr, int64_t bytes, cudaStream_t stream);
 
 // hipattn_select_stage that also writes the next stage's bounds as int64 (either pointer may be null)

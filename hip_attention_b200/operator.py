@@ -131,7 +131,8 @@ class PhaseTimer:
 def hip_attention_impl(q: Tensor, k: Optional[Tensor], v: Optional[Tensor], args: HiPAttentionArgs,
                        cached_metadata: Optional[HiPAttentionOutputMetadata] = None, *, return_lse: bool = False,
                        debug: Optional[dict] = None, score_reduce=None, timer: Optional[PhaseTimer] = None,
-                       v_ready: Optional[torch.cuda.Event] = None, shared: Optional[dict] = None, out: Optional[Tensor] = None):
+                       v_ready: Optional[torch.cuda.Event] = None, shared: Optional[dict] = None, out: Optional[Tensor] = None,
+                       lse: Optional[Tensor] = None, fork=None, beside: bool = False):
     """Implementation behind ``hip_attention_12``.
 
     ``return_lse`` adds the base-2 log-sum-exp [B, TQ, H]; ``score_reduce(score_int32)`` is called after every scan
@@ -140,9 +141,12 @@ def hip_attention_impl(q: Tensor, k: Optional[Tensor], v: Optional[Tensor], args
     mask estimator reads only q and k, so a caller that streams its inputs to the device may issue the call as soon as q
     and k have arrived and pass the event that marks the arrival of v (dense ``v`` or the value cache); the attention
     launch waits for it.  ``shared``: a dict that calls on the same keys hand on, so that key copies and rope tables are
-    prepared once; its entry ``positions`` [B, n] names the query positions of all of them.  ``out`` [B, TQ, H, D] receives
-    the context."""
-    return (_host_module or host()).forward(q, k, v, args, cached_metadata, return_lse, debug, score_reduce, timer, v_ready, shared, out)
+    prepared once; its entry ``positions`` [B, n] names the query positions of all of them.  ``out`` [B, TQ, H, D] and
+    ``lse`` [B, TQ, H] receive the context and its log-sum-exp.  ``fork``: a fork of the current stream (``host().fork``)
+    with calls that do not depend on one another; with ``beside`` a decode call runs beside that stream.  The results may
+    be used after ``host().join``."""
+    return (_host_module or host()).forward(q, k, v, args, cached_metadata, return_lse, debug, score_reduce, timer, v_ready, shared, out,
+                                            lse, fork, beside)
 
 
 def hip_attention_12(q: Tensor, k: Optional[Tensor], v: Optional[Tensor], args: Optional[HiPAttentionArgs] = None,

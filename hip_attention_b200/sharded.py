@@ -108,7 +108,7 @@ def hip_attention_12_sequence_sharded(q: Tensor, shard_kv: Sequence[Tuple], args
     ``(context [B, 1, H, D], list of metadata, one entry per operator call)``; passing that list back as
     ``cached`` reuses the masks.
     """
-    from .operator import hip_attention_impl
+    from .operator import hip_attention_impl, host
     if q.shape[1] != 1:
         raise ValueError("sequence sharding is a decode path (one query row)")
     B = q.shape[0]
@@ -135,42 +135,49 @@ def hip_attention_12_sequence_sharded(q: Tensor, shard_kv: Sequence[Tuple], args
                 e += 1
         groups.append((j, e))
         j = e
-    outs, lses, mds = [], [], []
+    n_local, H, D = len(shard_kv), q.shape[2], q.shape[3]
+    po = torch.empty((n_local, B, 1, H, D), dtype=q.dtype, device=q.device)       # partial outputs and their log-sum-exp
+    pl = torch.empty((n_local, B, 1, H), dtype=torch.float32, device=q.device)
+    mds = [None] * len(groups)
+    ops = host()
+    # what the batched calls need from torch comes before the fork
+    calls = []
     for gi, (j0, j1) in enumerate(groups):
         m = j1 - j0
         if live[j0] == 0:   # beyond the live sequence: an empty partial
-            outs.append(torch.zeros((1,) + tuple(q.shape), dtype=torch.float32, device=q.device))
-            lses.append(torch.full((1, B, 1, q.shape[2]), float("-inf"), dtype=torch.float32, device=q.device))
-            mds.append(None)
+            po[j0:j1].zero_()
+            pl[j0:j1].fill_(float("-inf"))
             continue
         s = first_shard + j0
         a = sequence_shard_args(args, s, n_shards, live[j0], per_shard_k, q.device, owns_window=s == last_live)
-        a.position_ids = torch.full((m * B, 1), live[j0] - 1, dtype=torch.int64, device=q.device)
-        kv = shard_kv[j0]
+        kv, qq, k, v = shard_kv[j0], q, None, None
         if len(kv) == 2:
             k, v = kv
-            qq = q
         else:
-            k = v = None
-            a.k_cache, a.v_cache = kv[0], kv[1]
-            if m == 1:
-                a.block_table, a.cache_seq_lens, qq = kv[2], kv[3], q
-            else:
-                a.block_table = torch.cat([shard_kv[j][2] for j in range(j0, j1)], 0)
-                a.cache_seq_lens = torch.cat([shard_kv[j][3] for j in range(j0, j1)], 0)
-                qq = q.repeat(m, 1, 1, 1)
+            a.k_cache, a.v_cache, a.block_table, a.cache_seq_lens = kv
+            if m > 1:
+                a.block_table, a.cache_seq_lens = ops.stack_rows([[shard_kv[j][i] for j in range(j0, j1)] for i in (2, 3)])
+                qq = q.expand(m, 1, H, D) if B == 1 else q.repeat(m, 1, 1, 1)
             a.update_flags()
-        o, md, lse = hip_attention_impl(qq, k, v, a, None if cached is None else cached[gi], return_lse=True)
-        outs.append(o.float().view(m, B, 1, q.shape[2], q.shape[3]))
-        lses.append(lse.view(m, B, 1, q.shape[2]))
-        mds.append(md)
-    po = torch.cat(outs)   # [S_local, B, 1, H, D]
-    pl = torch.cat(lses)   # [S_local, B, 1, H]
+        calls.append((gi, m, qq, k, v, a, po[j0:j1].view(m * B, 1, H, D), pl[j0:j1].view(m * B, 1, H)))
+    # The groups are independent and each is a chain of short launches: the largest runs on the current stream, the others
+    # beside it (eight shards of 131072 tokens: 0.53 ms one after the other, 0.35 ms).  The query's position is the last
+    # key's, which the operator writes itself.
+    calls.sort(key=lambda c: -c[1])
+    fork = ops.fork(q) if len(calls) > 1 else None
+    try:
+        for i, (gi, m, qq, k, v, a, o, l) in enumerate(calls):
+            mds[gi] = hip_attention_impl(qq, k, v, a, None if cached is None else cached[gi], return_lse=True, shared={}, out=o, lse=l, fork=fork,
+                                         beside=i > 0)[1]
+    finally:
+        if fork is not None:
+            ops.join(fork)
     if dist.is_available() and dist.is_initialized() and dist.get_world_size(group) > 1:
         world = dist.get_world_size(group)
+        po = po.float()
         go = torch.empty((world,) + tuple(po.shape), dtype=po.dtype, device=po.device)
         gl = torch.empty((world,) + tuple(pl.shape), dtype=pl.dtype, device=pl.device)
         dist.all_gather_into_tensor(go, po, group=group)
         dist.all_gather_into_tensor(gl, pl, group=group)
-        po, pl = go.flatten(0, 1), gl.flatten(0, 1)
-    return merge_shard_partials(po, pl, q.dtype), mds
+        return merge_shard_partials(go.flatten(0, 1), gl.flatten(0, 1), q.dtype), mds
+    return ops.merge_shards(po, pl), mds
