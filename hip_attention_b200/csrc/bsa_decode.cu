@@ -659,8 +659,8 @@ int launch_mma(const hipattn_bsa_params_t& p, cudaStream_t stream) {
   const int64_t grid = units * cluster;
   HIPATTN_REQUIRE(grid > 0 && grid < 0x7fffffffLL, HIPATTN_ERR_INVALID, "decode grid of %lld blocks", (long long)grid);
   auto kern = bsa_decode_mma_kernel<DT, D, ROPE, F8>;
-  HIPATTN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  if (cluster > 8) HIPATTN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  HIPATTN_CUDA_OK(allow_smem((const void*)kern, smem));
+  if (cluster > 8) HIPATTN_CUDA_OK(allow_wide_clusters((const void*)kern));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(kDW * 32);
@@ -689,7 +689,7 @@ int launch(const hipattn_bsa_params_t& p, cudaStream_t stream) {
   const int64_t grid = (int64_t)p.B * p.HKV * p.n_splits;
   HIPATTN_REQUIRE(grid > 0 && grid < 0x7fffffffLL, HIPATTN_ERR_INVALID, "decode grid of %lld blocks", (long long)grid);
   auto kern = bsa_decode_kernel<DT, LPR, G>;
-  HIPATTN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  HIPATTN_CUDA_OK(allow_smem((const void*)kern, smem));
   kern<<<(unsigned)grid, kWarps * 32, smem, stream>>>(p);
   return check_launch("bsa_decode_kernel");
 }

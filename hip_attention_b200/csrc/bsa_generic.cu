@@ -321,7 +321,7 @@ int launch(const hipattn_bsa_params_t& p, int packed, int rows_per_head, int n_s
   const int64_t grid = (int64_t)p.B * (packed ? p.HKV : p.H) * NBLK * n_sub * p.n_splits;
   HIPATTN_REQUIRE(grid > 0 && grid < 0x7fffffffLL, HIPATTN_ERR_INVALID, "attention grid of %lld blocks", (long long)grid);
   auto kern = bsa_generic_kernel<DT, D, BM>;
-  HIPATTN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  HIPATTN_CUDA_OK(allow_smem((const void*)kern, smem));
   kern<<<(unsigned)grid, kThreads, smem, stream>>>(p, packed, rows_per_head, n_sub);
   return check_launch("bsa_generic_kernel");
 }

@@ -737,7 +737,7 @@ int launch5_ws(const hipattn_bsa_params_t& p, int BQ, int n_sub, cudaStream_t st
   const int64_t grid = (int64_t)p.B * (p.H / NH) * NBLK * n_sub * p.n_splits;
   HIPATTN_REQUIRE(grid > 0 && grid < 0x7fffffffLL, HIPATTN_ERR_INVALID, "attention grid of %lld blocks", (long long)grid);
   auto kern = bsa_tcgen05_ws_kernel<DT, D, ROPE, KV8, SPLIT>;
-  HIPATTN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  HIPATTN_CUDA_OK(allow_smem((const void*)kern, smem));
   kern<<<(unsigned)grid, 256, smem, stream>>>(p, BQ, n_sub);
   return check_launch("bsa_tcgen05_ws_kernel");
 }

@@ -5,6 +5,9 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
+#include <set>
+#include <utility>
 
 #include "common.cuh"
 #include "host_kernels.h"
@@ -21,6 +24,34 @@ void set_error(const char* fmt, ...) {
   va_start(ap, fmt);
   vsnprintf(g_error, sizeof(g_error), fmt, ap);
   va_end(ap);
+}
+
+cudaError_t allow_smem(const void* kernel, size_t bytes) {
+  static thread_local std::map<std::pair<int, const void*>, size_t> allowed;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  size_t& have = allowed[{dev, kernel}];
+  if (bytes <= have) return cudaSuccess;
+  // all that the kernel's own shared memory leaves of a block's 227 KB: the same value whichever thread or size comes first
+  cudaFuncAttributes attr;
+  e = cudaFuncGetAttributes(&attr, kernel);
+  if (e != cudaSuccess) return e;
+  const size_t most = 227 * 1024 - attr.sharedSizeBytes;
+  if (bytes > most) return cudaErrorInvalidValue;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+  if (e == cudaSuccess) have = most;
+  return e;
+}
+
+cudaError_t allow_wide_clusters(const void* kernel) {
+  static thread_local std::set<std::pair<int, const void*>> allowed;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess || allowed.count({dev, kernel})) return e;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) allowed.insert({dev, kernel});
+  return e;
 }
 
 int validate_tokens(const hipattn_tokens_t& t, int elem_bytes, int D, const char* name) {

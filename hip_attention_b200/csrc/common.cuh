@@ -44,6 +44,11 @@ inline int check_launch(const char* what) {
   return HIPATTN_OK;
 }
 
+// Function attributes are set once per thread, device and kernel (a call into the runtime costs as much as half a launch).
+// allow_smem: at least `bytes` of dynamic shared memory.
+cudaError_t allow_smem(const void* kernel, size_t bytes);
+cudaError_t allow_wide_clusters(const void* kernel);
+
 int validate_tokens(const hipattn_tokens_t& t, int elem_bytes, int D, const char* name);
 
 // ---------------------------------------------------------------------------------------------

@@ -1174,9 +1174,11 @@ PyObject* pool_read(PyObject* list) {
   return out.release();
 }
 
-// pool_write([(buffer, value or None, rows)...]): value into the leading rows of its buffer, zeros for None
+// pool_write([(buffer, value or None, rows)...]): value into the leading rows of its buffer, zeros for None; returns the
+// places in the list of the values it does not take (another layout, type or device, too many rows)
 PyObject* pool_write(PyObject* list) {
   const Py_ssize_t n = PyList_GET_SIZE(list);
+  Ref left = checked(PyList_New(0));
   std::unique_ptr<c10::cuda::CUDAGuard> guard;
   std::unique_ptr<Copies> cp;
   for (Py_ssize_t i = 0; i < n; ++i) {
@@ -1198,11 +1200,19 @@ PyObject* pool_write(PyObject* list) {
       s.plain = 1;
       cp->add(s);
     } else {
-      cp->add(THPVariable_Unpack(val), buf);
+      const at::Tensor v = tensor_of(val, "value");
+      const int ts = copy_type(v.scalar_type()), td = copy_type(buf.scalar_type());
+      if (ts < 0 || (ts >= hipattn::COPY_F32) != (td >= hipattn::COPY_F32) || v.device() != buf.device() || v.dim() != buf.dim() || v.dim() < 1 ||
+          v.size(0) > buf.size(0) || v.sizes().slice(1) != buf.sizes().slice(1)) {
+        Ref at = checked(PyLong_FromSsize_t(i));
+        if (PyList_Append(left.get(), at.get()) < 0) throw PyError{};
+        continue;
+      }
+      cp->add(v, buf);
     }
   }
   if (cp) cp->flush();
-  Py_RETURN_NONE;
+  return left.release();
 }
 
 // ---------------------------------------------------------------------------------------------------------------------

@@ -540,7 +540,7 @@ int launch(const hipattn_scan_params_t& p, int c_log2, int HB, cudaStream_t stre
   const int64_t grid = units * n_split;
   HIPATTN_REQUIRE(grid > 0 && grid < 0x7fffffffLL, HIPATTN_ERR_INVALID, "scan grid of %lld blocks", (long long)grid);
   auto kern = scan_chunks_mma_kernel<DT, D, MODE, F8>;
-  HIPATTN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  HIPATTN_CUDA_OK(allow_smem((const void*)kern, smem));
   kern<<<(unsigned)grid, 128, smem, stream>>>(p, c_log2, HB, n_split, passes_total, p.mode == HIPATTN_SCAN_CHECK ? 1 : 0);
   return check_launch("scan_chunks_mma_kernel");
 }

@@ -292,7 +292,7 @@ int launch(const hipattn_scan_params_t& p, cudaStream_t stream) {
   const int64_t grid = units * nblk;
   HIPATTN_REQUIRE(grid > 0 && grid < 0x7fffffffLL, HIPATTN_ERR_INVALID, "scan grid of %lld blocks", (long long)grid);
   auto kern = scan_stage_kernel<DT, D, RT, EXT>;
-  HIPATTN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  HIPATTN_CUDA_OK(allow_smem((const void*)kern, smem));
   kern<<<(unsigned)grid, 32 * NW, smem, stream>>>(p, nblk, nblk_total, NW);
   return check_launch("scan_stage_kernel");
 }

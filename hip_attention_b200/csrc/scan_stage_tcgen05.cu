@@ -443,7 +443,7 @@ int launch(const hipattn_scan_params_t& p, cudaStream_t stream) {
   const int64_t grid = units * nblk;
   HIPATTN_REQUIRE(grid > 0 && grid < 0x7fffffffLL, HIPATTN_ERR_INVALID, "scan grid of %lld blocks", (long long)grid);
   auto kern = scan_stage_tcgen05_kernel<DT, D, NR, STREAM>;
-  HIPATTN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  HIPATTN_CUDA_OK(allow_smem((const void*)kern, smem));
   kern<<<(unsigned)grid, 128, smem, stream>>>(p, nblk, nblk_total, p.mode == HIPATTN_SCAN_CHECK ? 1 : 0);
   return check_launch("scan_stage_tcgen05_kernel");
 }

@@ -314,7 +314,7 @@ int hipattn::select_stage(const int32_t* score_max, const int32_t* left, int64_t
   const size_t smem = (size_t)k_pad * sizeof(uint32_t);
   return by_row_length(n, [&](auto threads, auto items) -> int {
     auto kern = select_stage_kernel<decltype(threads)::value, decltype(items)::value>;
-    if (smem > 40 * 1024) HIPATTN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 40 * 1024) HIPATTN_CUDA_OK(allow_smem((const void*)kern, smem));
     kern<<<(unsigned)rows, decltype(threads)::value, smem, stream>>>(score_max, left, n, k_keep, k_pad, sink, c_prev, c_next, next_left, next_right,
                                                                     next_score_max, next_left64, next_right64);
     return check_launch("select_stage_kernel");

@@ -181,9 +181,6 @@ class HiPMetadataCache:
                                           mask_cache_statistics=None, sa_cache_statistics=None, stage_caches=caches)
 
 
-_POOL_TYPES = (torch.int64, torch.int32, torch.uint32, torch.float32, torch.bfloat16)
-
-
 class _PoolBuffer:
     """One preallocated buffer of the metadata pool (hip_memory_pool.py:20-53): ``per_head`` buffers are
     [max_batch * heads, ...] and sliced by batch * heads rows, the others are [max_batch, 1, heads, ...]; values are
@@ -212,12 +209,6 @@ class _PoolBuffer:
         rows = batch_size * heads if self.per_head else batch_size
         self._check(rows, "the requested batch")
         return rows
-
-    def takes_whole(self, value: Tensor) -> bool:
-        """Whether ``value`` fills whole leading rows of the buffer with numbers one launch can convert; checks the rows."""
-        self._check(value.shape[0], "the stored value")
-        return value.is_cuda and value.device == self.buffer.device and value.shape[1:] == self.buffer.shape[1:] and \
-            value.is_floating_point() == self.buffer.is_floating_point() and value.dtype in _POOL_TYPES
 
     def set(self, value: Tensor) -> None:
         self._check(value.shape[0], "the stored value")
@@ -296,20 +287,16 @@ class HiPMetadataCachePool:
 
     def _set_buffers(self, layer_idx: int, items: Sequence) -> None:
         """Several writes ((name, value); None: zeros in the first ``max_batch_size`` rows), one launch on the GPU."""
-        together = []
-        for name, value in items:
-            b = self._buffer(layer_idx, name)
-            if value is None:
-                if b.buffer.is_cuda:
-                    together.append((b.buffer, None, self.max_batch_size))
-                else:
-                    b.buffer[:self.max_batch_size].zero_()
-            elif b.takes_whole(value):
-                together.append((b.buffer, value, 0))
+        rows = self.max_batch_size
+        bufs = [self._buffer(layer_idx, name) for name, _ in items]
+        left = range(len(items))
+        if bufs[0].buffer.is_cuda:
+            left = host().pool_write([(b.buffer, value, rows) for b, (_, value) in zip(bufs, items)])
+        for i in left:
+            if items[i][1] is None:
+                bufs[i].buffer[:rows].zero_()
             else:
-                b.set(value)
-        if together:
-            host().pool_write(together)
+                bufs[i].set(items[i][1])
 
     def get_hip_metadata_cache(self, layer_id: int, size: int, batch_size: int,
                                cached_stages: Optional[int]) -> Optional[HiPAttentionOutputMetadata]:
