@@ -60,30 +60,11 @@ __device__ __forceinline__ float pair_hi(uint32_t w) {
   return __half2float(__ushort_as_half((unsigned short)(w >> 16)));
 }
 
-// two-wide fp32 arithmetic (one instruction for a pair of lanes' values): the softmax is bound by instruction issue
-__device__ __forceinline__ unsigned long long f32x2(float lo, float hi) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void f32x2_split(unsigned long long v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long fma_f32x2(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
 // maximum of three values in one instruction
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;\n" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
-}
-__device__ __forceinline__ unsigned long long add_f32x2(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
-  return r;
 }
 
 // Record of a tile for the softmax warps (ring of eight: the copy warps run at most three tiles ahead of the softmax

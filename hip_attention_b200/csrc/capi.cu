@@ -80,6 +80,7 @@ int validate_tokens(const hipattn_tokens_t& t, int elem_bytes, int D, const char
 
 int bsa_generic(const hipattn_bsa_params_t& p, cudaStream_t stream);
 int bsa_mma(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled);
+int bsa_fp32(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled);
 int bsa_decode(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled);
 int bsa_tcgen05(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled);
 int64_t bsa_tcgen05_ctas(const hipattn_bsa_params_t& p, int* resident, int* tile_keys);
@@ -250,6 +251,8 @@ extern "C" int hipattn_bsa_attention(const hipattn_bsa_params_t* p, void* stream
     if (handled) return rc;
   }
   rc = bsa_mma(*p, (cudaStream_t)stream, &handled);
+  if (handled) return rc;
+  rc = bsa_fp32(*p, (cudaStream_t)stream, &handled);
   if (handled) return rc;
   return bsa_generic(*p, (cudaStream_t)stream);
 }

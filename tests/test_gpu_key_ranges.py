@@ -14,6 +14,7 @@ SHAPES = {
     "d64": dict(D=64, H=4, HKV=2, bq=64, dtype="fp16"),
     "mha": dict(D=128, H=2, HKV=2, bq=64, dtype="bf16"),
     "fp32": dict(D=64, H=4, HKV=2, bq=64, dtype="fp32"),
+    "fp32_d128": dict(D=128, H=4, HKV=1, bq=128, dtype="fp32"),
     "fp8_bf16": dict(D=128, H=8, HKV=2, bq=64, dtype="bf16", fp8=True),
     "fp8_fp16_d64": dict(D=64, H=4, HKV=2, bq=64, dtype="fp16", fp8=True),
 }
