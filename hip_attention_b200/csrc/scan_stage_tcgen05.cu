@@ -30,16 +30,11 @@ namespace hipattn {
 namespace {
 
 // the CTA's small shared variables (behind the operand tiles in dynamic shared memory)
-// (kept at 56 bytes: with the 16-row operand tiles six CTAs share a multiprocessor's shared memory to the byte)
 struct ScanShared {
   unsigned long long mbar;
   uint32_t tmem;
   int abort;
-  int g[2][4];      // per-warp largest chunk of the current chunk block, double buffered; during set-up g[1][2] holds the
-                    // block's smallest position and g[1][3] the largest |pooled query| (read before g[1] is first written,
-                    // which happens behind the first chunk block's barrier)
-  unsigned char fetched[4];   // [r % 3]: "some warp fetched rows in round r"
-  int pad_;
+  int p_min, q_max;   // the block's smallest position; the largest |pooled query|, as bits
 };
 constexpr uint32_t kScanSlack = 896;   // padding reserved in front of the tiles
 
@@ -94,8 +89,7 @@ __global__ void __launch_bounds__(128, NR <= 32 ? (STREAM ? 5 : 6) : (NR <= 64 ?
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(mbar));
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     sh.abort = 0;
-    sh.g[1][3] = 0;
-    sh.fetched[0] = sh.fetched[1] = sh.fetched[2] = 0;
+    sh.q_max = 0;
   }
   // The block's query rows go to shared memory (the key tile is free until the first round) with one batch of
   // asynchronous copies, issued before the TMEM allocation so that the trip to DRAM overlaps it: the pooled queries are
@@ -115,7 +109,7 @@ __global__ void __launch_bounds__(128, NR <= 32 ? (STREAM ? 5 : 6) : (NR <= 64 ?
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&sh.tmem)), "r"(TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     const int m = block_min_position(p, b, t0, Rv, lane);
-    if (lane == 0) sh.g[1][2] = m;
+    if (lane == 0) sh.p_min = m;
   }
   cp_async_wait<0>();
   tc_fence_before();
@@ -141,12 +135,12 @@ __global__ void __launch_bounds__(128, NR <= 32 ? (STREAM ? 5 : 6) : (NR <= 64 ?
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) qmax_local = fmaxf(qmax_local, __shfl_xor_sync(0xffffffffu, qmax_local, o));
-  if (lane == 0) atomicMax(&sh.g[1][3], __float_as_int(qmax_local));  // non-negative floats order as ints
+  if (lane == 0) atomicMax(&sh.q_max, __float_as_int(qmax_local));  // non-negative floats order as ints
   fence_async_smem();
   __syncthreads();
 
-  const int pt = max(sh.g[1][2] - p.scan_window, 0);
-  const float eps_q = kEps * __int_as_float(sh.g[1][3]);
+  const int pt = max(sh.p_min - p.scan_window, 0);
+  const float eps_q = kEps * __int_as_float(sh.q_max);
   const int n = p.n_chunks;
   const int64_t row = (int64_t)b * BDST + d;
   const char* kbase = reinterpret_cast<const char*>(p.k_scaled);
@@ -157,8 +151,8 @@ __global__ void __launch_bounds__(128, NR <= 32 ? (STREAM ? 5 : 6) : (NR <= 64 ?
   const int side = tid & 1;
   // in-kernel RoPE, backend "relative": the prepared keys come in two copies (rotated to position 0 / 1 for the left /
   // right candidate), and a key's score depends on the side it is proposed for, so no score is carried over
-  const bool roped = p.rope_mode != HIPATTN_ROPE_NONE;
-  const int side_rows = (roped && !STREAM) ? p.B * p.HKV * p.T : 0;
+  const bool by_side = p.rope_mode != HIPATTN_ROPE_NONE && !STREAM;
+  const int side_rows = by_side ? p.B * p.HKV * p.T : 0;
   unsigned long long st_keys = 0, st_fb = 0, st_wrong = 0;
   float st_ratio = 0.f;
   uint32_t phase = 0;
@@ -193,221 +187,215 @@ __global__ void __launch_bounds__(128, NR <= 32 ? (STREAM ? 5 : 6) : (NR <= 64 ?
     return best;
   };
 
-  bool aborted = Rv == 0;
-  int cbi = 0;
-  int rr = 0;   // rounds executed by this CTA so far (the same number in every thread)
+  // Every warp works through its own chunks: 16 of each chunk block of the CTA, the next block's as soon as these are
+  // settled, whatever the other warps are at.  A round is then nothing but copies, barrier, MMA and decision; a block does not
+  // begin with a barrier over its chunk sizes nor end with a round that only repeats a key (128k prefill, three
+  // stages: 9.25 ms with both, 8.38 ms without).
+  //
+  // The reference runs 32 - clz(largest chunk of the group of block_chunk chunks) rounds.  With one score per key the count
+  // does not matter: a chunk that a round has left with one token proposes it twice more, it neither wins nor loses against
+  // itself and its score is counted already, so the chunk is settled there.  Where the score depends on the side, the
+  // rounds are counted.
+  bool aborted = Rv == 0, done = false, in_range = false;
+  int cb = cblk - nblk, c = 0, it = 0, rounds = 0, left = 0, right = 0;
+  float score = HIPATTN_SCORE_INIT;
+  // The candidate that won the previous round and its score.  When the halved chunk proposes the same key again
+  // (one of the two candidates of a chunk of two tokens) the score is known: the same key against the same pooled
+  // queries, so the row is neither fetched nor multiplied again.  (-1: the winner's score was left between two values, see
+  // below.)
+  int won_t = -1;
+  float won_score = 0.f;
   // the bounds of a thread's chunk are requested one chunk block ahead, so that their latency is not part of the chain
   int next_left = 0, next_right = 0;
-  if (cblk < nblk_total && cblk * 64 + (tid >> 1) < n) {
-    next_left = __ldg(p.left + row * n + cblk * 64 + (tid >> 1));
-    next_right = __ldg(p.right + row * n + cblk * 64 + (tid >> 1));
-  }
-  for (int cb = cblk; cb < nblk_total && !aborted; cb += nblk, ++cbi) {
-    const int c = cb * 64 + (tid >> 1);
-    const bool in_range = c < n;
-    int left = next_left, right = next_right;
+  auto request = [&](int block) {
+    const int cn = block * 64 + (tid >> 1);
     next_left = next_right = 0;
-    {
-      const int cn = c + nblk * 64;
-      if (cb + nblk < nblk_total && cn < n) {
-        next_left = __ldg(p.left + row * n + cn);
-        next_right = __ldg(p.right + row * n + cn);
-      }
+    if (block < nblk_total && cn < n) {
+      next_left = __ldg(p.left + row * n + cn);
+      next_right = __ldg(p.right + row * n + cn);
     }
-    // halving rounds: fixed by the largest chunk of the reference group of block_chunk chunks that
-    // holds this thread's chunk; a warp covers 16 chunks, the CTA 64
-    {
-      int m = in_range ? right - left : 0;
-      if (p.block_chunk > 64) {
-        const int gbase = (cb * 64 / p.block_chunk) * p.block_chunk;
-        for (int i = tid; i < p.block_chunk; i += 128) {
-          const int cc = gbase + i;
-          if (cc < n) m = max(m, p.right[row * n + cc] - p.left[row * n + cc]);
-        }
-      }
-      m = __reduce_max_sync(0xffffffffu, m);
-      if (lane == 0) sh.g[cbi & 1][warp] = m;
-    }
-    __syncthreads();
-    const int cta_max = max(max(sh.g[cbi & 1][0], sh.g[cbi & 1][1]), max(sh.g[cbi & 1][2], sh.g[cbi & 1][3]));
-    const int gmax = p.block_chunk >= 64 ? cta_max
-                     : (p.block_chunk == 32 ? max(sh.g[cbi & 1][warp], sh.g[cbi & 1][warp ^ 1]) : sh.g[cbi & 1][warp]);
-    const int my_rounds = gmax >= 1 ? 32 - __clz(gmax) : 0;
-    const int cta_rounds = cta_max >= 1 ? 32 - __clz(cta_max) : 0;
-    float score = HIPATTN_SCORE_INIT;
-    // The candidate that won the previous round and its score.  When the halved chunk proposes the same key again
-    // (always in the last round, for one of the two candidates in the round before it) the score is known: the same
-    // key against the same pooled queries, so the row is neither fetched nor multiplied again.  (-1: the winner's score
-    // was left between two values, see below.)
-    int won_t = -1;
-    float won_score = 0.f;
+  };
+  request(cblk);
 
-    for (int it = 0; it < cta_rounds; ++it) {
-      // A warp goes straight from its decisions to the copies of its next 32 rows: those rows are its own (only this
-      // warp re-reads them for a strict re-score) and the MMA that read the tile has completed for every warp.  The one
-      // CTA-wide barrier of a round sits between the copies and the MMA; it also carries "is anybody still searching".
-      const bool act = in_range && it < my_rounds && left < right && left <= pt && left >= 0;
-      const int mid = (left + right) >> 1;
-      int tk = side ? ((mid + right) >> 1) : ((left + mid) >> 1);
-      const int tk_asked = tk;
-      const bool known = act && (!roped || STREAM) && tk == won_t;   // (streaming: a chunk's keys keep their rotation from round to round)
-      int idx = -1;
-      if (act && !known) {
-        if (tk < 0 || tk >= p.T) {
-          atomicOr(p.status, HIPATTN_STATUS_TOKEN_RANGE);
-          tk = min(max(tk, 0), p.T - 1);
-        }
-        idx = (b * p.HKV + hkv) * p.T + tk + side * side_rows;   // (second copy: keys rotated for the right candidate)
-        if (p.access_counter) mark_access(p.access_counter, p.access_stride_b, p.access_stride_h, p.access_n, p.k, b, hkv, tk);
+  while (!aborted) {
+    bool act;
+    for (;;) {
+      act = left < right && left <= pt && left >= 0 && (by_side ? it < rounds : it == 0 || right - left > 1);
+      if (done || __any_sync(0xffffffffu, act)) break;
+      if (in_range && side == 0) {
+        if (score > HIPATTN_SCORE_INIT) atomicMax(p.score_max + row * n + c, encode_score(score));
+        const int64_t o = (row * p.H + h) * n + c;
+        if (p.left_out) p.left_out[o] = left;
+        if (p.right_out) p.right_out[o] = right;
+        if (p.score_out) p.score_out[o] = score;
       }
-      // the key's magnitude is needed only after the MMA: requested here, its latency hides behind the row copies
-      float s_abs = (!STREAM && idx >= 0) ? __ldg(p.key_abs + idx) : 0.f;
-      // ---- gather this warp's 32 rows: 8 lanes per row, 128 contiguous bytes per row and instruction ----
-      if (__any_sync(0xffffffffu, idx >= 0)) {   // a warp whose scores are all known (or inactive) copies nothing
-      if (lane == 0) *(volatile unsigned char*)&sh.fetched[rr % 3] = 1;
+      cb += nblk;
+      done = cb >= nblk_total;
+      c = cb * 64 + (tid >> 1);
+      in_range = !done && c < n;
+      left = next_left;
+      right = next_right;
+      request(cb + nblk);
+      if (by_side && !done) {
+        const int c0 = cb * 64 + warp * 16, gbase = c0 / p.block_chunk * p.block_chunk;
+        int m = 0;
+        for (int i = gbase + lane; i < min(gbase + p.block_chunk, n); i += 32) m = max(m, __ldg(p.right + row * n + i) - __ldg(p.left + row * n + i));
+        m = __reduce_max_sync(0xffffffffu, m);
+        rounds = m >= 1 ? 32 - __clz(m) : 0;
+      }
+      it = 0;
+      score = HIPATTN_SCORE_INIT;
+      won_t = -1;
+    }
+    ++it;
+    // A warp goes straight from its decisions to the copies of its next 32 rows: those rows are its own (only this
+    // warp re-reads them for a strict re-score) and the MMA that read the tile has completed for every warp.  The one
+    // CTA-wide barrier of a round sits between the copies and the MMA; it also carries "is anybody still searching".
+    const int mid = (left + right) >> 1;
+    int tk = side ? ((mid + right) >> 1) : ((left + mid) >> 1);
+    const int tk_asked = tk;
+    const bool known = act && !by_side && tk == won_t;   // (streaming: a chunk's keys keep their rotation from round to round)
+    int idx = -1;
+    if (act && !known) {
+      if (tk < 0 || tk >= p.T) {
+        atomicOr(p.status, HIPATTN_STATUS_TOKEN_RANGE);
+        tk = min(max(tk, 0), p.T - 1);
+      }
+      idx = (b * p.HKV + hkv) * p.T + tk + side * side_rows;   // (second copy: keys rotated for the right candidate)
+      if (p.access_counter) mark_access(p.access_counter, p.access_stride_b, p.access_stride_h, p.access_n, p.k, b, hkv, tk);
+    }
+    // the key's magnitude is needed only after the MMA: requested here, its latency hides behind the row copies
+    float s_abs = (!STREAM && idx >= 0) ? __ldg(p.key_abs + idx) : 0.f;
+    // ---- gather this warp's 32 rows: 8 lanes per row, 128 contiguous bytes per row and instruction ----
+    if (!done) {
 #pragma unroll
-      for (int r0 = 0; r0 < 32; r0 += 4) {
-        const int j = r0 + (lane >> 3);
-        const int src = __shfl_sync(0xffffffffu, idx, j);
-        // no branch between the copies: the row of an inactive candidate is a copy of zero source bytes (zero fill)
-        const bool live = src >= 0;
-        const char* gp = kbase + (int64_t)(live ? src : 0) * ROWB + (lane & 7) * 16;
-        const uint32_t sp = sK_u32 + sw128(warp * 32 + j, lane & 7);
+    for (int r0 = 0; r0 < 32; r0 += 4) {
+      const int j = r0 + (lane >> 3);
+      const int src = __shfl_sync(0xffffffffu, idx, j);
+      // no branch between the copies: the row of an inactive candidate is a copy of zero source bytes (zero fill)
+      const bool live = src >= 0;
+      const char* gp = kbase + (int64_t)(live ? src : 0) * ROWB + (lane & 7) * 16;
+      const uint32_t sp = sK_u32 + sw128(warp * 32 + j, lane & 7);
 #pragma unroll
-        for (int kb = 0; kb < KB; ++kb) cp_async16_zfill(sp + kb * K_BLOCK_BYTES, gp + kb * 128, live);
-      }
-      }
-      cp_async_commit();
-      cp_async_wait<0>();
-      if (STREAM) {
-        // the 16 pieces of a row were copied by eight lanes: all of the warp's copies are visible after this point
-        __syncwarp();
-        if (idx >= 0) {
-          if constexpr (D == 128) {
-            const int r = warp * 32 + lane;
-            const uint32_t s2 = pack_scalar2<DT>(p.k_scale);
-#pragma unroll 2
-            for (int pp = 0; pp < 8; ++pp) {
-              const uint32_t a_lo = sK_u32 + sw128(r, pp), a_hi = a_lo + K_BLOCK_BYTES;
-              uint4 lo = lds128(a_lo), hi = lds128(a_hi);
-              rope_rotate_packed<DT>(lo, hi, rope_table_raw(p.rope_cos, p.rope_stride, p.rope_rows, c, pp),
-                                     rope_table_raw(p.rope_sin, p.rope_stride, p.rope_rows, c, pp));
-              uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                w[i] = mul2<DT>(w[i], s2);
-                s_abs += fabsf(lo_f32<DT>(w[i])) + fabsf(hi_f32<DT>(w[i]));
-              }
-              sts128(a_lo, make_uint4(w[0], w[1], w[2], w[3]));
-              sts128(a_hi, make_uint4(w[4], w[5], w[6], w[7]));
-            }
-          }
-        }
-      }
-      fence_async_smem();
-      tc_fence_before();
-      // the barrier's result is one bit (any predicate non-zero): "somebody is still searching, or gave up"
-      if (!__syncthreads_or(act || *(volatile int*)&sh.abort)) break;
-      if (*(volatile int*)&sh.abort) { aborted = true; break; }
-      // somebody fetched a row: the tile is multiplied; else every live score is known from the round before
-      const bool scored = *(volatile unsigned char*)&sh.fetched[rr % 3] != 0;
-      if (tid == 0) *(volatile unsigned char*)&sh.fetched[(rr + 2) % 3] = 0;   // next written two barriers from now
-      ++rr;
-      if (scored && tid == 0) {
-        tc_fence_after();
-        // the descriptors of the K-steps differ from the first one's in the start-address field only (shared-memory
-        // addresses stay below 2^18, so the 14-bit field does not carry): one add each instead of building them anew
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k)
-          umma(tmem, da0 + (uint64_t)(((k >> 2) * K_BLOCK_BYTES + (k & 3) * 32) >> 4),
-               db0 + (uint64_t)(((k >> 2) * Q_BLOCK_BYTES + (k & 3) * 32) >> 4), idesc, k > 0 ? 1u : 0u);
-        umma_commit(mbar);
-      }
+      for (int kb = 0; kb < KB; ++kb) cp_async16_zfill(sp + kb * K_BLOCK_BYTES, gp + kb * 128, live);
+    }
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    if (STREAM) {
+      // the 16 pieces of a row were copied by eight lanes: all of the warp's copies are visible after this point
       __syncwarp();
-      bool ok = true;
-      if (scored) {
-        ok = mbar_wait(mbar, phase, &sh.abort, p.status);
-        phase ^= 1u;
-        ok = __all_sync(0xffffffffu, ok);
-        tc_fence_after();
-      }
-      float x = -INFINITY;
-      if (ok && scored) {
-        // four short maximum chains; the row mask is only paid for by a ragged last query block.  128 pooled rows
-        // are read as two halves of 64 columns so that the live registers stay those of the 64-row variant.
-        constexpr int NLD = NR > 64 ? 64 : NR;
-        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      if (idx >= 0) {
+        if constexpr (D == 128) {
+          const int r = warp * 32 + lane;
+          const uint32_t s2 = pack_scalar2<DT>(p.k_scale);
+#pragma unroll 2
+          for (int pp = 0; pp < 8; ++pp) {
+            const uint32_t a_lo = sK_u32 + sw128(r, pp), a_hi = a_lo + K_BLOCK_BYTES;
+            uint4 lo = lds128(a_lo), hi = lds128(a_hi);
+            rope_rotate_packed<DT>(lo, hi, rope_table_raw(p.rope_cos, p.rope_stride, p.rope_rows, c, pp),
+                                   rope_table_raw(p.rope_sin, p.rope_stride, p.rope_rows, c, pp));
+            uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
-        for (int c0 = 0; c0 < NR; c0 += NLD) {
-          float v[NLD];
-          if (NLD == 16) tmem_ld16(my_tmem + c0, v);
-          else if (NLD == 32) tmem_ld32(my_tmem + c0, v);
-          else tmem_ld64(my_tmem + c0, v);
-          if (Rv >= NR) {
-#pragma unroll
-            for (int j = 0; j < NLD; ++j) m4[j & 3] = fmaxf(m4[j & 3], v[j]);
-          } else {
-#pragma unroll
-            for (int j = 0; j < NLD; ++j)
-              if (c0 + j < Rv) m4[j & 3] = fmaxf(m4[j & 3], v[j]);
-          }
-        }
-        x = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-      }
-      // The rounded score lies between lo and hi.  A comparison that these bounds settle needs no more; where they overlap,
-      // or where the winner may raise the chunk's best score and its own is not certain, the key is scored by the
-      // strict definition, which costs its warp 600 cycles.  (Scoring every key whose bounds differ: 0.3 % of the keys in
-      // bf16, 2.5 % in fp16, three per round and CTA.)
-      const float e_ = eps_q * s_abs * 1.01f;
-      float lo = Elem<DT>::round(x - e_), hi = Elem<DT>::round(x + e_);
-      if (known) lo = hi = won_score;
-      const bool fetched = idx >= 0 && ok;
-      if (fetched && lo != hi) ++st_fb;
-      bool certain = lo == hi && !check;   // (check mode: every key by both definitions)
-      const int other_t = __shfl_xor_sync(0xffffffffu, tk_asked, 1);   // the other candidate of the same chunk
-      const bool same = (!roped || STREAM) && other_t == tk_asked;      // a key does not beat itself
-      bool win, mine;
-      float wlo, whi;
-      for (;;) {
-        const float olo = __shfl_xor_sync(0xffffffffu, lo, 1), ohi = __shfl_xor_sync(0xffffffffu, hi, 1);
-        const float llo = side ? olo : lo, lhi = side ? ohi : hi, rlo = side ? lo : olo, rhi = side ? hi : ohi;
-        win = llo > rhi && !same;
-        const bool open = !win && !(lhi <= rlo) && !same;
-        wlo = win ? llo : rlo;
-        whi = win ? lhi : rhi;
-        mine = win != (side != 0);
-        unsigned need = __ballot_sync(0xffffffffu, act && fetched && !certain && (open || check || (mine && whi > score)));
-        if (!need) break;
-        while (need) {
-          const int owner = __ffs(need) - 1;
-          need &= need - 1;
-          const float rawv = strict_score(warp * 32 + owner);
-          if (lane == owner) {
-            const float ex = Elem<DT>::round(rawv);
-            if (check) {
-              if (lo == hi && hi != ex) ++st_wrong;
-              if (e_ > 0.f) st_ratio = fmaxf(st_ratio, fabsf(x - rawv) / e_);
+            for (int i = 0; i < 8; ++i) {
+              w[i] = mul2<DT>(w[i], s2);
+              s_abs += fabsf(lo_f32<DT>(w[i])) + fabsf(hi_f32<DT>(w[i]));
             }
-            lo = hi = ex;
-            certain = true;
+            sts128(a_lo, make_uint4(w[0], w[1], w[2], w[3]));
+            sts128(a_hi, make_uint4(w[4], w[5], w[6], w[7]));
           }
         }
-      }
-      if (act) {
-        if (idx >= 0) st_keys += 1;
-        if (win) right = mid; else left = mid;
-        score = fmaxf(score, wlo);   // certain when it matters: a winner whose upper bound exceeds the best was scored strictly
-        won_t = wlo == whi ? (mine ? tk_asked : other_t) : -1;
-        won_score = wlo;
       }
     }
-
-    if (in_range && side == 0 && !aborted) {
-      if (score > HIPATTN_SCORE_INIT) atomicMax(p.score_max + row * n + c, encode_score(score));
-      const int64_t o = (row * p.H + h) * n + c;
-      if (p.left_out) p.left_out[o] = left;
-      if (p.right_out) p.right_out[o] = right;
-      if (p.score_out) p.score_out[o] = score;
+    fence_async_smem();
+    tc_fence_before();
+    // the barrier's result is one bit (any predicate non-zero): "somebody is still searching, or gave up"
+    if (!__syncthreads_or(!done || *(volatile int*)&sh.abort)) break;
+    if (*(volatile int*)&sh.abort) { aborted = true; break; }
+    if (tid == 0) {
+      tc_fence_after();
+      // the descriptors of the K-steps differ from the first one's in the start-address field only (shared-memory
+      // addresses stay below 2^18, so the 14-bit field does not carry): one add each instead of building them anew
+#pragma unroll
+      for (int k = 0; k < D / 16; ++k)
+        umma(tmem, da0 + (uint64_t)(((k >> 2) * K_BLOCK_BYTES + (k & 3) * 32) >> 4),
+             db0 + (uint64_t)(((k >> 2) * Q_BLOCK_BYTES + (k & 3) * 32) >> 4), idesc, k > 0 ? 1u : 0u);
+      umma_commit(mbar);
+    }
+    __syncwarp();
+    bool ok = mbar_wait(mbar, phase, &sh.abort, p.status);
+    phase ^= 1u;
+    ok = __all_sync(0xffffffffu, ok);
+    tc_fence_after();
+    if (!ok) done = true;   // the CTA leaves at the next barrier
+    float x = -INFINITY;
+    if (!done) {
+      // four short maximum chains; the row mask is only paid for by a ragged last query block.  128 pooled rows
+      // are read as two halves of 64 columns so that the live registers stay those of the 64-row variant.
+      constexpr int NLD = NR > 64 ? 64 : NR;
+      float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int c0 = 0; c0 < NR; c0 += NLD) {
+        float v[NLD];
+        if (NLD == 16) tmem_ld16(my_tmem + c0, v);
+        else if (NLD == 32) tmem_ld32(my_tmem + c0, v);
+        else tmem_ld64(my_tmem + c0, v);
+        if (Rv >= NR) {
+#pragma unroll
+          for (int j = 0; j < NLD; ++j) m4[j & 3] = fmaxf(m4[j & 3], v[j]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < NLD; ++j)
+            if (c0 + j < Rv) m4[j & 3] = fmaxf(m4[j & 3], v[j]);
+        }
+      }
+      x = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+    }
+    // The rounded score lies between lo and hi.  A comparison that these bounds settle needs no more; where they overlap,
+    // or where the winner may raise the chunk's best score and its own is not certain, the key is scored by the
+    // strict definition, which costs its warp 600 cycles.  (Scoring every key whose bounds differ: 0.3 % of the keys in
+    // bf16, 2.5 % in fp16, three per round and CTA.)
+    const float e_ = eps_q * s_abs * 1.01f;
+    float lo = Elem<DT>::round(x - e_), hi = Elem<DT>::round(x + e_);
+    if (known) lo = hi = won_score;
+    const bool fetched = idx >= 0 && !done;
+    if (fetched && lo != hi) ++st_fb;
+    bool certain = lo == hi && !check;   // (check mode: every key by both definitions)
+    const int other_t = __shfl_xor_sync(0xffffffffu, tk_asked, 1);   // the other candidate of the same chunk
+    const bool same = !by_side && other_t == tk_asked;      // a key does not beat itself
+    bool win, mine;
+    float wlo, whi;
+    for (;;) {
+      const float olo = __shfl_xor_sync(0xffffffffu, lo, 1), ohi = __shfl_xor_sync(0xffffffffu, hi, 1);
+      const float llo = side ? olo : lo, lhi = side ? ohi : hi, rlo = side ? lo : olo, rhi = side ? hi : ohi;
+      win = llo > rhi && !same;
+      const bool open = !win && !(lhi <= rlo) && !same;
+      wlo = win ? llo : rlo;
+      whi = win ? lhi : rhi;
+      mine = win != (side != 0);
+      unsigned need = __ballot_sync(0xffffffffu, act && fetched && !certain && (open || check || (mine && whi > score)));
+      if (!need) break;
+      while (need) {
+        const int owner = __ffs(need) - 1;
+        need &= need - 1;
+        const float rawv = strict_score(warp * 32 + owner);
+        if (lane == owner) {
+          const float ex = Elem<DT>::round(rawv);
+          if (check) {
+            if (lo == hi && hi != ex) ++st_wrong;
+            if (e_ > 0.f) st_ratio = fmaxf(st_ratio, fabsf(x - rawv) / e_);
+          }
+          lo = hi = ex;
+          certain = true;
+        }
+      }
+    }
+    if (act) {
+      if (idx >= 0) st_keys += 1;
+      if (win) right = mid; else left = mid;
+      score = fmaxf(score, wlo);   // certain when it matters: a winner whose upper bound exceeds the best was scored strictly
+      won_t = wlo == whi ? (mine ? tk_asked : other_t) : -1;
+      won_score = wlo;
     }
   }
 
