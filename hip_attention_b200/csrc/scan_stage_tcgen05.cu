@@ -38,14 +38,18 @@ struct ScanShared {
 };
 constexpr uint32_t kScanSlack = 896;   // padding reserved in front of the tiles
 
-// Resident CTAs per multiprocessor the register allocation aims at: six with 16 or 32 pooled rows (80 registers; shared
-// memory holds six 37 KB CTAs; at 92 registers only five are resident and stages 0 and 1 of the 128k prefill take 8 %
-// longer), four with 64, three with 128 (shared memory).
+// Resident CTAs per multiprocessor the register allocation aims at.  Head dim 128: six with 16 or 32 pooled rows (80
+// registers; shared memory holds six 37 KB CTAs; at 92 registers only five are resident and stages 0 and 1 of the 128k
+// prefill take 8 % longer), four with 64, three with 128 (shared memory).  Head dim 64 has half the tile and is bound by
+// registers alone: one more in either case (ragged fp16 prefill, three stages: 571 -> 555 us).
+constexpr int resident_ctas(int D, int NR, bool stream) {
+  return NR <= 32 ? (stream ? 5 : (D == 64 ? 7 : 6)) : (NR <= 64 ? (D == 64 ? 5 : 4) : 3);
+}
 // STREAM = in-kernel RoPE, backend "streaming": the prepared copy holds the keys as they are (head-major, neither scaled
 // nor rotated); every thread rotates the row it asked for to its chunk's index, scales it and sums its magnitude in the
 // operand tile, between the landing of the copies and the round's barrier.
 template <int DT, int D, int NR, bool STREAM>
-__global__ void __launch_bounds__(128, NR <= 32 ? (STREAM ? 5 : 6) : (NR <= 64 ? 4 : 3)) scan_stage_tcgen05_kernel(const hipattn_scan_params_t p, int nblk, int nblk_total, int check) {
+__global__ void __launch_bounds__(128, resident_ctas(D, NR, STREAM)) scan_stage_tcgen05_kernel(const hipattn_scan_params_t p, int nblk, int nblk_total, int check) {
   constexpr int ROWB = D * 2;                 // bytes per key / query row
   constexpr int PIECES = ROWB / 16;
   constexpr int KB = D / 64;                  // 128-byte K-blocks per row
@@ -427,7 +431,7 @@ int launch(const hipattn_scan_params_t& p, cudaStream_t stream) {
   const int BDST = cdiv(p.TQ, p.block_size_q);
   const int nblk_total = cdiv(p.n_chunks, 64);
   const int64_t units = (int64_t)p.B * p.H * BDST;
-  const int nblk = scan_ctas_per_unit(units, nblk_total, 148 * (NR <= 32 ? (STREAM ? 5 : 6) : (NR <= 64 ? 4 : 3)));
+  const int nblk = scan_ctas_per_unit(units, nblk_total, 148 * resident_ctas(D, NR, STREAM));
   const int64_t grid = units * nblk;
   HIPATTN_REQUIRE(grid > 0 && grid < 0x7fffffffLL, HIPATTN_ERR_INVALID, "scan grid of %lld blocks", (long long)grid);
   auto kern = scan_stage_tcgen05_kernel<DT, D, NR, STREAM>;
