@@ -8,6 +8,8 @@
 // bit for bit.  The best score of the surviving halves is reduced over heads with an atomic max on
 // an order-preserving integer image.
 //
+// (fp32 prefill of 32 and more pooled rows forms that score from bounds, see below.)
+//
 // Mapping: one CTA = 32 * NW consecutive chunks of one (batch, query block, head); a lane owns one
 // chunk and both of its candidate keys.  Key rows are gathered with 16-byte cp.async (16 lanes per
 // 256-byte row, fully coalesced) into a per-warp staging area; pooled queries sit in shared memory as
@@ -102,6 +104,9 @@ __global__ void __launch_bounds__(128, RT == 1 ? 7 : 1) scan_stage_kernel(const 
   float* qtile = reinterpret_cast<float*>(smem);                       // [Rpad][D]
   unsigned char* kstage = smem + (size_t)Rpad * D * sizeof(float);     // [NW][2][32][kRowStride]
   __shared__ int s_pmin;
+  constexpr bool kBounds = DT == HIPATTN_F32 && RT >= 32;   // (16 rows: what it saves goes into settling)
+  __shared__ float s_qmax[4];
+  float q_max = 0.f;
 
   // ---- pooled queries (once per CTA) ----
   for (int i = threadIdx.x; i < Rpad * G::kPieces; i += blockDim.x) {
@@ -112,7 +117,16 @@ __global__ void __launch_bounds__(128, RT == 1 ? 7 : 1) scan_stage_kernel(const 
     if (r < Rv) pooled_query_piece<DT>(p, b, h, t0 + r * p.stride_q, pc, v);
 #pragma unroll
     for (int e = 0; e < G::kVec; e += 4)
-      *reinterpret_cast<float4*>(qtile + (size_t)r * D + pc * G::kVec + e) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+      *reinterpret_cast<float4*>(qtile + (size_t)r * D + (kBounds ? pc ^ (r & 3) : pc) * G::kVec + e) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+    if (kBounds) {
+#pragma unroll
+      for (int e = 0; e < G::kVec; ++e) q_max = fmaxf(q_max, fabsf(v[e]));
+    }
+  }
+  if (kBounds) {
+    // (not a number: the comparison below then settles nothing)
+    const int m = __reduce_max_sync(0xffffffffu, __float_as_int(q_max));
+    if (lane == 0) s_qmax[warp] = __int_as_float(m);
   }
   if (warp == 0) {
     const int m = block_min_position(p, b, t0, Rv, lane);
@@ -128,6 +142,10 @@ __global__ void __launch_bounds__(128, RT == 1 ? 7 : 1) scan_stage_kernel(const 
   const unsigned char* my_l = wstage + (size_t)lane * G::kRowStride;
   const unsigned char* my_r = wstage + (size_t)(32 + lane) * G::kRowStride;
   const int ntile = Rpad / RT;
+  if (kBounds) {
+    q_max = 0.f;
+    for (int w = 0; w < (int)blockDim.x >> 5; ++w) q_max = fmaxf(q_max, s_qmax[w]);
+  }
 
   // ---- chunk blocks of this CTA ----
   for (int cb = cblk; cb < nblk_total; cb += nblk) {
@@ -212,7 +230,92 @@ __global__ void __launch_bounds__(128, RT == 1 ? 7 : 1) scan_stage_kernel(const 
     __syncwarp();
 
     float sl = -INFINITY, sr = -INFINITY;
+    auto key_piece = [&](const unsigned char* my, int right_side, int pc, float* out) {
+      if (!EXT || p.rope_mode == HIPATTN_ROPE_NONE) unpack_scaled<DT>(*reinterpret_cast<const uint4*>(my + pc * 16), p.k_scale, out);
+      else   // keys at their chunk's index (streaming) or at 0 / 1 for the left / right candidate (relative)
+        unpack_rope_scaled<DT, D>(my, pc, p.rope_mode == HIPATTN_ROPE_RELATIVE ? right_side : c, p, out);
+    };
     if (act) {
+      if constexpr (kBounds) {
+        // fp32: a strict multiply and add are two roundings and two instructions, and only the largest of the rows' dot
+        // products counts.  All of them are formed with the two-wide fma first; either sum is within (D + 2) 2^-24 of
+        // sum |q||k| of the true one, so rows further than twice the radius below the largest cannot hold the strict
+        // maximum, and the lane forms the strict sum for what is left: one row of 64, seldom two.
+        // (4096 queries, 8 heads, D 64, 64 pooled rows: 212 us with every row strict, 166 us so.)
+        for (int tile = 0; tile < ntile; ++tile) {
+          unsigned long long al[RT], ar[RT];   // even and odd elements' sums
+          float sum_l = 0.f, sum_r = 0.f;
+#pragma unroll
+          for (int r = 0; r < RT; ++r) al[r] = ar[r] = 0ull;
+          const float* qt = qtile + (size_t)tile * RT * D;
+#pragma unroll 1
+          for (int p4 = 0; p4 < G::kPieces; p4 += 4) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              float kl[4], kr[4];
+              key_piece(my_l, 0, p4 + j, kl);
+              key_piece(my_r, 1, p4 + j, kr);
+              const unsigned long long l0 = f32x2(kl[0], kl[1]), l1 = f32x2(kl[2], kl[3]), r0 = f32x2(kr[0], kr[1]), r1 = f32x2(kr[2], kr[3]);
+              sum_l += (fabsf(kl[0]) + fabsf(kl[1])) + (fabsf(kl[2]) + fabsf(kl[3]));
+              sum_r += (fabsf(kr[0]) + fabsf(kr[1])) + (fabsf(kr[2]) + fabsf(kr[3]));
+#pragma unroll
+              for (int r = 0; r < RT; ++r) {
+                const ulonglong2 qv = *reinterpret_cast<const ulonglong2*>(qt + r * D + (p4 + (j ^ (r & 3))) * 4);
+                al[r] = fma_f32x2(qv.x, l0, al[r]);
+                ar[r] = fma_f32x2(qv.x, r0, ar[r]);
+                al[r] = fma_f32x2(qv.y, l1, al[r]);
+                ar[r] = fma_f32x2(qv.y, r1, ar[r]);
+              }
+            }
+          }
+          const int live = min(RT, Rv - tile * RT);
+          // the rows of a side that may hold its maximum
+          auto open_rows = [&](const unsigned long long* a2, float sum, float best) {
+            const float e = fmaf((2 * D + 16) * 0x1p-24f * q_max, sum, 1e-36f);
+            float m = -INFINITY;
+#pragma unroll
+            for (int r = 0; r < RT; ++r) {
+              float lo, hi;
+              f32x2_split(a2[r], lo, hi);
+              if (r < live) m = fmaxf(m, lo + hi);
+            }
+            const float least = fmaxf(m - 2.f * e, best - e);
+            uint32_t rows = 0;
+#pragma unroll
+            for (int r = 0; r < RT; ++r) {
+              float lo, hi;
+              f32x2_split(a2[r], lo, hi);
+              if (r < live && !(lo + hi < least)) rows |= 1u << r;
+            }
+            return rows;
+          };
+          uint32_t rows_l = known_l ? 0u : open_rows(al, sum_l, sl), rows_r = known_r ? 0u : open_rows(ar, sum_r, sr);
+          while (rows_l | rows_r) {   // both sides' sums side by side: each is one chain of dependent additions
+            const int i = rows_l ? __ffs(rows_l) - 1 : 0, j = rows_r ? __ffs(rows_r) - 1 : 0;
+            float a = 0.f, c2 = 0.f;
+#pragma unroll 4
+            for (int pc = 0; pc < G::kPieces; ++pc) {
+              float kl[4], kr[4];
+              key_piece(my_l, 0, pc, kl);
+              key_piece(my_r, 1, pc, kr);
+              const float4 ql = *reinterpret_cast<const float4*>(qt + i * D + (pc ^ (i & 3)) * 4);
+              const float4 qr = *reinterpret_cast<const float4*>(qt + j * D + (pc ^ (j & 3)) * 4);
+              a = mac<DT>(ql.x, kl[0], a);
+              c2 = mac<DT>(qr.x, kr[0], c2);
+              a = mac<DT>(ql.y, kl[1], a);
+              c2 = mac<DT>(qr.y, kr[1], c2);
+              a = mac<DT>(ql.z, kl[2], a);
+              c2 = mac<DT>(qr.z, kr[2], c2);
+              a = mac<DT>(ql.w, kl[3], a);
+              c2 = mac<DT>(qr.w, kr[3], c2);
+            }
+            if (rows_l) sl = fmaxf(sl, a);
+            if (rows_r) sr = fmaxf(sr, c2);
+            rows_l &= rows_l - 1u;      // (0 stays 0: 0 & -1)
+            rows_r &= rows_r - 1u;
+          }
+        }
+      } else
       for (int tile = 0; tile < ntile && !(known_l && known_r); ++tile) {
         float accl[RT], accr[RT];
 #pragma unroll
@@ -221,14 +324,8 @@ __global__ void __launch_bounds__(128, RT == 1 ? 7 : 1) scan_stage_kernel(const 
 #pragma unroll 2
         for (int pc = 0; pc < G::kPieces; ++pc) {
           float kl[G::kVec], kr[G::kVec];
-          if (!EXT || p.rope_mode == HIPATTN_ROPE_NONE) {
-            unpack_scaled<DT>(*reinterpret_cast<const uint4*>(my_l + pc * 16), p.k_scale, kl);
-            unpack_scaled<DT>(*reinterpret_cast<const uint4*>(my_r + pc * 16), p.k_scale, kr);
-          } else {   // keys at their chunk's index (streaming) or at 0 / 1 for the left / right candidate (relative)
-            const bool rel = p.rope_mode == HIPATTN_ROPE_RELATIVE;
-            unpack_rope_scaled<DT, D>(my_l, pc, rel ? 0 : c, p, kl);
-            unpack_rope_scaled<DT, D>(my_r, pc, rel ? 1 : c, p, kr);
-          }
+          key_piece(my_l, 0, pc, kl);
+          key_piece(my_r, 1, pc, kr);
 #pragma unroll
           for (int r = 0; r < RT; ++r) {
 #pragma unroll
@@ -306,7 +403,9 @@ int dispatch_rows(const hipattn_scan_params_t& p, cudaStream_t stream) {
   if (rows <= 1) return ext ? launch<DT, D, 1, true>(p, stream) : launch<DT, D, 1, false>(p, stream);
   if (R <= 16) return ext ? launch<DT, D, 16, true>(p, stream) : launch<DT, D, 16, false>(p, stream);
   if (R <= 32) return ext ? launch<DT, D, 32, true>(p, stream) : launch<DT, D, 32, false>(p, stream);
-  return ext ? launch<DT, D, 64, true>(p, stream) : launch<DT, D, 64, false>(p, stream);
+  // (fp32 keeps two sums per row and key: tiles of 32 rows)
+  constexpr int kTop = DT == HIPATTN_F32 ? 32 : 64;
+  return ext ? launch<DT, D, kTop, true>(p, stream) : launch<DT, D, kTop, false>(p, stream);
 }
 
 template <int DT>
