@@ -88,6 +88,20 @@ __global__ void __launch_bounds__(128, resident_ctas(D, NR, STREAM)) scan_stage_
   if (t0 < p.TQ) Rv = min(R, (p.TQ - t0 + p.stride_q - 1) / p.stride_q);
   const uint32_t mbar = smem_u32(&sh.mbar);
 
+  const int n = p.n_chunks;
+  const int64_t row = (int64_t)b * BDST + d;
+  // the bounds of a thread's chunk are requested one chunk block ahead, so that their latency is not part of the chain
+  int next_left = 0, next_right = 0;
+  auto request = [&](int block) {
+    const int cn = block * 64 + (tid >> 1);
+    next_left = next_right = 0;
+    if (block < nblk_total && cn < n) {
+      next_left = __ldg(p.left + row * n + cn);
+      next_right = __ldg(p.right + row * n + cn);
+    }
+  };
+  request(cblk);   // (the first block's latency hides behind the set-up)
+
   // ---- set-up: barrier, TMEM, pooled queries as the B operand ----
   if (tid == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(mbar));
@@ -112,6 +126,7 @@ __global__ void __launch_bounds__(128, resident_ctas(D, NR, STREAM)) scan_stage_
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&sh.tmem)), "r"(TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  } else if (warp == 1) {   // (beside the allocation)
     const int m = block_min_position(p, b, t0, Rv, lane);
     if (lane == 0) sh.p_min = m;
   }
@@ -145,8 +160,6 @@ __global__ void __launch_bounds__(128, resident_ctas(D, NR, STREAM)) scan_stage_
 
   const int pt = max(sh.p_min - p.scan_window, 0);
   const float eps_q = kEps * __int_as_float(sh.q_max);
-  const int n = p.n_chunks;
-  const int64_t row = (int64_t)b * BDST + d;
   const char* kbase = reinterpret_cast<const char*>(p.k_scaled);
   const uint32_t sK_u32 = smem_u32(sK), sQ_u32 = smem_u32(sQ);
   const uint32_t idesc = make_idesc(DT == HIPATTN_BF16 ? 1 : 0, 128, NR, 0);
@@ -209,18 +222,6 @@ __global__ void __launch_bounds__(128, resident_ctas(D, NR, STREAM)) scan_stage_
   // below.)
   int won_t = -1;
   float won_score = 0.f;
-  // the bounds of a thread's chunk are requested one chunk block ahead, so that their latency is not part of the chain
-  int next_left = 0, next_right = 0;
-  auto request = [&](int block) {
-    const int cn = block * 64 + (tid >> 1);
-    next_left = next_right = 0;
-    if (block < nblk_total && cn < n) {
-      next_left = __ldg(p.left + row * n + cn);
-      next_right = __ldg(p.right + row * n + cn);
-    }
-  };
-  request(cblk);
-
   while (!aborted) {
     bool act;
     for (;;) {
