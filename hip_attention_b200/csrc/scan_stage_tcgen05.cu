@@ -38,12 +38,13 @@ struct ScanShared {
 };
 constexpr uint32_t kScanSlack = 896;   // padding reserved in front of the tiles
 
-// Resident CTAs per multiprocessor the register allocation aims at.  Head dim 128: six with 16 or 32 pooled rows (80
-// registers; shared memory holds six 37 KB CTAs; at 92 registers only five are resident and stages 0 and 1 of the 128k
-// prefill take 8 % longer), four with 64, three with 128 (shared memory).  Head dim 64 has half the tile and is bound by
-// registers alone: one more in either case (ragged fp16 prefill, three stages: 571 -> 555 us).
+// Resident CTAs per multiprocessor the register allocation aims at.  Head dim 128, as shared memory allows: six with 16 pooled
+// rows (80 registers; six 37 KB CTAs; at 92 registers only five are resident and stages 0 and 1 of the 128k prefill take 8 %
+// longer), five with 32, four with 64, three with 128.  Head dim 64 has half the tile and is bound by registers alone: one
+// or two more (ragged fp16 prefill, three stages: 571 -> 555 us).
 constexpr int resident_ctas(int D, int NR, bool stream) {
-  return NR <= 32 ? (stream ? 5 : (D == 64 ? 7 : 6)) : (NR <= 64 ? (D == 64 ? 5 : 4) : 3);
+  if (NR <= 32) return D == 64 ? 7 : (stream || NR == 32 ? 5 : 6);
+  return NR <= 64 ? (D == 64 ? 5 : 4) : 3;
 }
 // STREAM = in-kernel RoPE, backend "streaming": the prepared copy holds the keys as they are (head-major, neither scaled
 // nor rotated); every thread rotates the row it asked for to its chunk's index, scales it and sums its magnitude in the
