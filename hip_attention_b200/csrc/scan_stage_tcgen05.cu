@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(128, resident_ctas(D, NR, STREAM)) scan_stage_
   const uint32_t my_tmem = tmem + ((uint32_t)(warp * 32) << 16);
   const int side = tid & 1;
   // in-kernel RoPE, backend "relative": the prepared keys come in two copies (rotated to position 0 / 1 for the left /
-  // right candidate), and a key's score depends on the side it is proposed for, so no score is carried over
+  // right candidate), and a key's score depends on the side it is proposed for
   const bool by_side = p.rope_mode != HIPATTN_ROPE_NONE && !STREAM;
   const int side_rows = by_side ? p.B * p.HKV * p.T : 0;
   unsigned long long st_keys = 0, st_fb = 0, st_wrong = 0;
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(128, resident_ctas(D, NR, STREAM)) scan_stage_
     const int mid = (left + right) >> 1;
     int tk = side ? ((mid + right) >> 1) : ((left + mid) >> 1);
     const int tk_asked = tk;
-    const bool known = act && !by_side && tk == won_t;   // (streaming: a chunk's keys keep their rotation from round to round)
+    const bool known = act && tk == won_t;   // (streaming: a chunk's keys keep their rotation from round to round)
     int idx = -1;
     if (act && !known) {
       if (tk < 0 || tk >= p.T) {
@@ -367,8 +367,10 @@ __global__ void __launch_bounds__(128, resident_ctas(D, NR, STREAM)) scan_stage_
     const bool fetched = idx >= 0 && !done;
     if (fetched && lo != hi) ++st_fb;
     bool certain = lo == hi && !check;   // (check mode: every key by both definitions)
-    const int other_t = __shfl_xor_sync(0xffffffffu, tk_asked, 1);   // the other candidate of the same chunk
-    const bool same = !by_side && other_t == tk_asked;      // a key does not beat itself
+    // the other candidate of the same chunk; a key does not beat itself.  By side, the same key is another candidate there: its
+    // score is known only to the side that proposed it.
+    const int other_t = by_side ? -1 : __shfl_xor_sync(0xffffffffu, tk_asked, 1);
+    const bool same = other_t == tk_asked;
     bool win, mine;
     float wlo, whi;
     for (;;) {
