@@ -151,13 +151,16 @@ __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64
 // multiplied with V, so that an fp8 cache keeps softmax weights of at least 16 significant bits: the general kernel, which
 // served it before, multiplies fp32 weights.  (2 x 3001 queries, RoPE: 12.2 ms there, 1.43 ms here; output 5e-5 apart.)
 // Head dim 64: the same roles with half the MMAs and copies per tile; 2 x 2999 queries of 16 heads 0.44 ms with mma.sync,
-// 0.24 ms here.
+// 0.27 here.  Its weights go in two terms as well: with one, and the lagging maximum, no weight of a row is exact, while
+// mma.sync has the row's largest at exactly 1 (error against 64 bits before the output is rounded, fp16: 5.7e-5 with
+// mma.sync, 9.5e-5 with one term, 6e-6 with two).
 // SPLIT = the grid may cut key lists into ranges (p.n_splits); the variant without is 2 % faster on grids that need none.
 template <int DT, int D, bool ROPE, bool KV8, bool SPLIT>
 __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bsa_params_t p, int BQ, int n_sub) {
   using T = typename Elem<DT>::type;
   constexpr int NT = 256;
   static_assert(D == 128 || (D == 64 && !ROPE), "in-kernel RoPE pairs the two 128-byte halves of a 256-byte row");
+  constexpr bool TWO = KV8 || D == 64;        // softmax weights in two 16-bit terms
   constexpr int KB = D / 64;                  // 128-byte blocks per row
   constexpr int PIECES = D / 8;               // 16-byte pieces per row
   constexpr int Q_BYTES = KB * 128 * 128;
@@ -541,7 +544,7 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
           umma_ts(tmem_o, tp + kk * 8, dv | (uint64_t)((vb + kk * 128) & 0x3fffu), idesc_o, (it > 0 || kk > 0) ? 1u : 0u);
-        if (KV8) {   // the weights' second terms
+        if (TWO) {   // the weights' second terms
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) umma_ts(tmem_o, tp + 32 + kk * 8, dv | (uint64_t)((vb + kk * 128) & 0x3fffu), idesc_o, 1u);
         }
@@ -622,7 +625,7 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
       // the scaling and the row sum run two values per instruction
       const unsigned long long scale2 = f32x2(kLog2e, kLog2e), nbase2 = f32x2(-base, -base);
       unsigned long long sum2[4] = {0ull, 0ull, 0ull, 0ull};
-      float pk[32], pk2[KV8 ? 32 : 1];
+      float pk[32], pk2[TWO ? 32 : 1];
 #pragma unroll
       for (int j = 0; j < TK5; j += 2) {
         float x0, x1;
@@ -630,7 +633,7 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
         const float e0 = exp2_approx(x0), e1 = exp2_approx(x1);
         const uint32_t w = pack2<DT>(e0, e1);
         pk[j >> 1] = __uint_as_float(w);
-        if constexpr (KV8) {
+        if constexpr (TWO) {
           pk2[j >> 1] = __uint_as_float(pack2<DT>(e0 - pair_lo<DT>(w), e1 - pair_hi<DT>(w)));
           sum2[(j >> 1) & 3] = add_f32x2(sum2[(j >> 1) & 3], f32x2(e0, e1));
           continue;
@@ -645,7 +648,7 @@ __global__ void __launch_bounds__(256, 2) bsa_tcgen05_ws_kernel(const hipattn_bs
         (void)b0; (void)b1;
         l_run += a0 + a1;
       }
-      if constexpr (KV8) tmem_st32<false>(ts + 32, pk2);   // ... and the second terms over the other half
+      if constexpr (TWO) tmem_st32<false>(ts + 32, pk2);   // ... and the second terms over the other half
       tmem_st32(ts, pk);        // P(it) over the first half of S(it)
       tc_fence_before();
       if (__any_sync(0xffffffffu, s_abort != 0)) break;   // warp-uniform: the TMEM accesses are warp-collective

@@ -1,0 +1,54 @@
+"""Attention whose softmax weights go through the tensor cores in two 16-bit terms, against 64 bits on the mask it used: what is
+left besides the rounding of the output itself is small.
+
+The bound: two terms keep 16 (bf16) or 22 (fp16) significant bits of a weight, and a score is a fp32 sum of 64 or 128
+products, so the context before it is rounded is within p = 1.5e-5 of the exact one, relative; the rounding of the output
+alone is r = 1.6e-3 (bf16) or 2.0e-4 (fp16).  The two add in quadrature: sqrt(1 + (p / r)^2) r < 1.003 r.  With single 16-bit
+weights p is 6e-5 to 2.7e-4 and the sum 1.006 r to 1.1 r."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _exact(q, k, v, md, rows, w):
+    """[n, H, D] in 64 bits: queries ``rows`` (index, position) of q [1, TQ, H, D] over sink, selected blocks and window."""
+    H, G, c, window = w["H"], w["H"] // w["HKV"], w["chunks"][-1], max(w["sw"], w["chunks"][0])
+    out = []
+    for r, p in rows:
+        t = torch.arange(w["T"], device=q.device)
+        blocks = md.indices[0, r // w["bq"], :int(md.ks[0, r // w["bq"]])]
+        sel = torch.zeros(w["T"] + c, dtype=torch.bool, device=q.device)
+        sel[(blocks[:, None] + torch.arange(c, device=q.device)).flatten()] = True
+        far = ((t < w["sink"]) | sel[:w["T"]]) & (t <= p - window)
+        t = t[far | ((t > p - window) & (t <= p))]
+        kk, vv = k[0, t].double().repeat_interleave(G, 1), v[0, t].double().repeat_interleave(G, 1)
+        s = torch.einsum("hd,nhd->hn", q[0, r].double(), kk)
+        out.append(torch.einsum("hn,nhd->hd", torch.softmax(s, -1), vv))
+    return torch.stack(out)
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "fp16"])
+@pytest.mark.parametrize("shape", [
+    dict(TQ=201, T=9001, D=64, bq=64),                       # prefill, two heads per CTA
+    dict(TQ=130, T=9001, D=64, bq=128),                      # one head, 128 rows
+])
+def test_error_is_the_rounding_of_the_output(shape, dtype):
+    import bench
+    from hip_attention_b200 import hip_attention_impl, read_status
+    w = dict(bench.WORKLOADS["prefill_128k"], H=8, HKV=2, keep=[4096, 2048, 1024], dtype=dtype)
+    w.update(shape)
+    g = torch.Generator(device="cuda").manual_seed(9)
+    dt = bench._DT[dtype]
+    q, k, v = (torch.randn((1, n, h, w["D"]), generator=g, device="cuda", dtype=dt) for n, h in ((w["TQ"], w["H"]), (w["T"], w["HKV"]), (w["T"], w["HKV"])))
+    q = q * w["D"] ** -0.5
+    k[:, ::100] *= 4
+    read_status("cuda")
+    out, md = hip_attention_impl(q, k, v, bench.make_args(w))
+    assert read_status("cuda") == 0
+    rows = [(r, w["T"] - w["TQ"] + r) for r in range(0, w["TQ"], max(1, w["TQ"] // 24))]
+    ref = _exact(q, k, v, md, rows, w)
+    err = (out[0, [r for r, _ in rows]].double() - ref).norm().item()
+    rounding = (ref.to(dt).double() - ref).norm().item()
+    print(f"{shape} {dtype}: error {err / ref.norm().item():.4e}, rounding alone {rounding / ref.norm().item():.4e}, ratio {err / rounding:.4f}")
+    assert err <= 1.003 * rounding
