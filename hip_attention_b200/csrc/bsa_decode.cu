@@ -269,8 +269,14 @@ __global__ void __launch_bounds__(kWarps * 32, 1) bsa_decode_kernel(const hipatt
 // their own, n_splits.)
 //
 // In-kernel RoPE: the key's pieces i and i + D / 64 hold elements d and d + D / 2, rotated in registers; the table pieces
-// travel with the rows.  fp8 rows are widened in registers, and the softmax weights then go in two 16-bit terms (the general
-// kernel, which served fp8 before, kept them in fp32).
+// travel with the rows.  fp8 rows are widened in registers.
+//
+// With RoPE or fp8 rows the softmax weights go in two 16-bit terms, the rounded weight and what the rounding left: the general
+// kernel, which served fp8 before, kept them in fp32; and a single term is exact for the largest weight of each warp's keys
+// only, so its error grows as fewer warps share a list (12 sequences with RoPE, bf16, error against 64 bits before the
+// output is rounded: 1.4e-4 with sixteen warps to a list, 1.8e-4 with the eight it has here, below 2e-5 with two terms, which
+// cost nothing beside the rotation).  Without RoPE there are six warps and more, not the four of the kernel before, and the
+// second products would cost 6 % of a full batch.
 //
 // Bound: HBM.  32 sequences, 3328 keys each (436 MB): 0.115 ms with a three-stage shared-memory ring and a barrier per
 // 64 keys (3.8 TB/s), 0.080 ms here (5.4 TB/s).  One sequence: 10.8 + 4.7 us (attention, merge), 12.9 us here.  RoPE, 12 sequences:
@@ -310,6 +316,7 @@ __global__ void __launch_bounds__(kDecodeWarps<ROPE, F8> * 32, 2) bsa_decode_mma
   constexpr int NB = D / 64;        // 64-column blocks
   constexpr int MS = D + 2;
   constexpr int EB = F8 ? 1 : 2;
+  constexpr bool TWO = F8 || ROPE;  // softmax weights in two 16-bit terms
   constexpr int kDW = kDecodeWarps<ROPE, F8>;
   using Raw = typename std::conditional<F8, uint2, uint4>::type;
   extern __shared__ __align__(16) float s_merge[];   // [kDW][G][MS], then the CTA's own result [G][MS]
@@ -545,7 +552,7 @@ __global__ void __launch_bounds__(kDecodeWarps<ROPE, F8> * 32, 2) bsa_decode_mma
       // ---- O += P V ----
       uint32_t pa[4] = {pack2<DT>(s[0][0], s[0][1]), 0u, pack2<DT>(s[1][0], s[1][1]), 0u};
       uint32_t pl[4] = {0u, 0u, 0u, 0u};
-      if constexpr (F8) {   // what the rounding of the weights left
+      if constexpr (TWO) {   // what the rounding of the weights left
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
           const float r0 = s[nt][0] - Elem<DT>::round(s[nt][0]), r1 = s[nt][1] - Elem<DT>::round(s[nt][1]);
@@ -565,7 +572,7 @@ __global__ void __launch_bounds__(kDecodeWarps<ROPE, F8> * 32, 2) bsa_decode_mma
           const uint32_t b0 = __byte_perm(v0[t >> 1], v1[t >> 1], sel), b1 = __byte_perm(v8[t >> 1], v9[t >> 1], sel);
           float c[4] = {o[nb * 8 + t][0], o[nb * 8 + t][1], 0.f, 0.f};
           mma16816<DT>(c, pa, b0, b1);
-          if constexpr (F8) mma16816<DT>(c, pl, b0, b1);
+          if constexpr (TWO) mma16816<DT>(c, pl, b0, b1);
           o[nb * 8 + t][0] = c[0];
           o[nb * 8 + t][1] = c[1];
         }
