@@ -659,15 +659,19 @@ int launch_mma(const hipattn_bsa_params_t& p, cudaStream_t stream) {
   const int G = p.H / p.HKV;
   const size_t smem = sizeof(float) * (size_t)(kDW + 1) * G * (D + 2);
   const int64_t units = (int64_t)p.B * p.HKV * p.n_splits;
-  // CTAs per unit: enough to put two on every multiprocessor, as long as every warp has at least sixteen keys
+  // CTAs per unit: as many as put two on every multiprocessor, as long as every warp has at least sixteen keys and the device
+  // holds the clusters of all units at once (a multiprocessor group has room for a whole number of them).  Sizes between the
+  // powers of two count: with 4 for the 40 units of five sequences, where 7 fit, 24 warps shared a list instead of 42, and
+  // the error of their single-term weights was 1.2 to 1.3 times as large.
   const int64_t keys = (p.sink < p.T ? p.sink : p.T) + (int64_t)p.K * p.block_size_k + (p.window < p.T ? p.window : p.T);
-  int cluster = 1;
-  while (cluster < kMaxCluster && units * cluster * 2 <= 148 * 2 && keys / p.n_splits >= (int64_t)cluster * 2 * kDW * 16) cluster *= 2;
-  const int64_t grid = units * cluster;
-  HIPATTN_REQUIRE(grid > 0 && grid < 0x7fffffffLL, HIPATTN_ERR_INVALID, "decode grid of %lld blocks", (long long)grid);
   auto kern = bsa_decode_mma_kernel<DT, D, ROPE, F8>;
   HIPATTN_CUDA_OK(allow_smem((const void*)kern, smem));
-  if (cluster > 8) HIPATTN_CUDA_OK(allow_wide_clusters((const void*)kern));
+  int64_t most = 148 * 2 / units;
+  if (most > keys / p.n_splits / (kDW * 16)) most = keys / p.n_splits / (kDW * 16);
+  int cluster = most < 1 ? 1 : (most > kMaxCluster ? kMaxCluster : (int)most);
+  while (cluster > 1 && resident_clusters((const void*)kern, cluster, kDW * 32, smem) < units) --cluster;
+  const int64_t grid = units * cluster;
+  HIPATTN_REQUIRE(grid > 0 && grid < 0x7fffffffLL, HIPATTN_ERR_INVALID, "decode grid of %lld blocks", (long long)grid);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(kDW * 32);

@@ -6,7 +6,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
-#include <set>
+#include <tuple>
 #include <utility>
 
 #include "common.cuh"
@@ -44,14 +44,30 @@ cudaError_t allow_smem(const void* kernel, size_t bytes) {
   return e;
 }
 
-cudaError_t allow_wide_clusters(const void* kernel) {
-  static thread_local std::set<std::pair<int, const void*>> allowed;
+int resident_clusters(const void* kernel, int cluster, int threads, size_t smem) {
+  static thread_local std::map<std::tuple<int, const void*, int, size_t>, int> known;
   int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess || allowed.count({dev, kernel})) return e;
-  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (e == cudaSuccess) allowed.insert({dev, kernel});
-  return e;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  const auto found = known.find({dev, kernel, cluster, smem});
+  if (found != known.end()) return found->second;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)cluster);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)cluster;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if ((cluster > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
+      cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();   // (a size the device does not take is not an error of the call)
+    n = 0;
+  }
+  known[{dev, kernel, cluster, smem}] = n;
+  return n;
 }
 
 int validate_tokens(const hipattn_tokens_t& t, int elem_bytes, int D, const char* name) {

@@ -45,9 +45,10 @@ inline int check_launch(const char* what) {
 }
 
 // Function attributes are set once per thread, device and kernel (a call into the runtime costs as much as half a launch).
-// allow_smem: at least `bytes` of dynamic shared memory.
+// allow_smem: at least `bytes` of dynamic shared memory.  resident_clusters: clusters of `cluster` CTAs that the device holds at
+// once, 0 when it cannot place one; sizes beyond eight are allowed on the way.
 cudaError_t allow_smem(const void* kernel, size_t bytes);
-cudaError_t allow_wide_clusters(const void* kernel);
+int resident_clusters(const void* kernel, int cluster, int threads, size_t smem);
 
 int validate_tokens(const hipattn_tokens_t& t, int elem_bytes, int D, const char* name);
 

@@ -17,6 +17,9 @@ pytestmark = pytest.mark.gpu
     dict(B=2, H=4, HKV=2, D=64, T=2049),
     dict(B=1, H=2, HKV=2, D=128, T=5003),
     dict(B=40, H=32, HKV=8, D=128, T=1500),               # more units than the GPU has room for
+    dict(B=5, H=32, HKV=8, D=128, T=5003),                # clusters whose size is no power of two
+    dict(B=24, H=16, HKV=4, D=64, T=3001),
+    dict(B=3, H=32, HKV=8, D=128, T=5003),
 ])
 def test_decode_attention_matches_oracle(shape, kv, ranges, monkeypatch):
     import bench
