@@ -33,6 +33,9 @@
 #include "scan_common.cuh"
 
 namespace hipattn {
+
+int strict_chunk_heads(const hipattn_scan_params_t& p);
+
 namespace {
 
 constexpr int kPass = 64;        // rows of a warp's pass
@@ -55,7 +58,7 @@ __device__ __forceinline__ uint2 load_row8(const char* p) {
 // MODE: HIPATTN_ROPE_NONE / _RELATIVE / _STREAMING; F8: e5m2 rows
 template <int DT, int D, int MODE, bool F8>
 __global__ void __launch_bounds__(128, MODE == HIPATTN_ROPE_NONE || F8 ? 4 : 3)
-    scan_chunks_mma_kernel(const hipattn_scan_params_t p, int c_log2, int HB, int n_split, int passes_total, int check) {
+    scan_chunks_mma_kernel(const hipattn_scan_params_t p, int c_log2, int HB, int n_split, int passes_total, int check, int nan_loses) {
   constexpr int PIECES = D / 8, QS = D + kQPad, NL = D / 32;   // pieces of a row; pieces per lane
   constexpr int NV = MODE == HIPATTN_ROPE_RELATIVE ? 2 : 1;    // scores per row and head
   using Raw = typename std::conditional<F8, uint2, uint4>::type;
@@ -130,6 +133,7 @@ __global__ void __launch_bounds__(128, MODE == HIPATTN_ROPE_NONE || F8 ? 4 : 3)
   const uint32_t kscale2 = pack_scalar2<DT>(p.k_scale);
   // this lane's columns of a product: heads (lane % 4) * 2 and + 1
   const int col = (lane & 3) * 2;
+  const uint32_t real_columns = (col < heads ? 0x55555555u : 0u) | (col + 1 < heads ? 0xaaaaaaaau : 0u);   // bits of `unsure`
   // (1.05: the magnitudes are summed in packed 16-bit arithmetic, at most 16 terms each)
   const float eps0 = kEps * 1.05f * s_qmax[col], eps1 = kEps * 1.05f * s_qmax[col + 1];
   const int check_tab = 4 * NV * HB * kTabStride;   // check mode: tables of the raw products and their radii follow
@@ -403,6 +407,9 @@ __global__ void __launch_bounds__(128, MODE == HIPATTN_ROPE_NONE || F8 ? 4 : 3)
           }
         }
       }
+      // A column beyond the heads has neither a table nor a query row.  Its bounds differ where a key's product or magnitude
+      // is not finite (0 * inf is not a number), so it is taken off the list here.
+      unsure &= real_columns;
       __syncwarp();
     }
     // One lane per (chunk, head) replays the search on the bounds.  Where they leave a comparison or a chunk's best score
@@ -433,7 +440,8 @@ __global__ void __launch_bounds__(128, MODE == HIPATTN_ROPE_NONE || F8 ? 4 : 3)
           const int code = s_list[warp][lane], r = code & 63, hh = (code >> 6) & 7, v = code >> 9;
           float2* t = wtab + (v * HB + hh) * kTabStride + r;
           const float raw = strict_score((const char*)s_src[warp][buf][r], hh, c_first + (r >> c_log2), v);
-          const float ex = Elem<DT>::round(raw);
+          float ex = Elem<DT>::round(raw);
+          if (nan_loses) ex = fmaxf(ex, -INFINITY);
           if (check) {
             const float xv = t[check_tab].x, e = t[check_tab].y;
             ++st_keys;
@@ -476,7 +484,8 @@ __global__ void __launch_bounds__(128, MODE == HIPATTN_ROPE_NONE || F8 ? 4 : 3)
           }
           const float2 sl = t0_[ol], sr = t1_[orr];
           const bool win = sl.x > sr.y;
-          if (!exact && !win && !(sl.y <= sr.x) && (NV == 2 || ol != orr)) {   // (a key does not beat itself)
+          // (a key does not beat itself; bounds that are not numbers leave its score open all the same)
+          if (!exact && !win && !(sl.y <= sr.x) && (NV == 2 || ol != orr || !(sl.x <= sl.y))) {
             mine_open = true;
             break;
           }
@@ -541,7 +550,10 @@ int launch(const hipattn_scan_params_t& p, int c_log2, int HB, cudaStream_t stre
   HIPATTN_REQUIRE(grid > 0 && grid < 0x7fffffffLL, HIPATTN_ERR_INVALID, "scan grid of %lld blocks", (long long)grid);
   auto kern = scan_chunks_mma_kernel<DT, D, MODE, F8>;
   HIPATTN_CUDA_OK(allow_smem((const void*)kern, smem));
-  kern<<<(unsigned)grid, 128, smem, stream>>>(p, c_log2, HB, n_split, passes_total, p.mode == HIPATTN_SCAN_CHECK ? 1 : 0);
+  // A score that is not a number: the whole-chunk strict kernel compares it as it is, the kernel that goes by rounds takes it
+  // for the lowest.  Masks are those of the strict mode, whichever of the two that takes.
+  const bool nan_loses = strict_chunk_heads(p) == 0;
+  kern<<<(unsigned)grid, 128, smem, stream>>>(p, c_log2, HB, n_split, passes_total, p.mode == HIPATTN_SCAN_CHECK ? 1 : 0, nan_loses ? 1 : 0);
   return check_launch("scan_chunks_mma_kernel");
 }
 

@@ -314,27 +314,34 @@ int dispatch_dim(const hipattn_scan_params_t& p, int c_log2, int HB, cudaStream_
 
 }  // namespace
 
-// Decode shapes (a single pooled query row) whose chunk size is a known power of two between 4 and 32 and no
-// larger than the number of rows the rounds of the heads sharing the chunk would fetch.
-// HIPATTN_DECODE_SCAN=rounds keeps the round-by-round kernel.
-int scan_chunks_strict(const hipattn_scan_params_t& p, cudaStream_t stream, bool* handled) {
-  *handled = false;
+// Heads per CTA of a call this kernel can take, 0 for any other: decode shapes (a single pooled query row) whose chunk size is
+// a known power of two between 4 and 32 and no larger than the number of rows the rounds of the heads sharing the chunk
+// would fetch.
+int strict_chunk_heads(const hipattn_scan_params_t& p) {
   const int R = p.block_size_q / p.stride_q;
   const int rows = min(R, cdiv(p.TQ, p.stride_q));
-  if (rows > 1 || (p.D != 64 && p.D != 128 && p.D != 256)) return HIPATTN_OK;
-  if (p.k.fp8_e5m2) return HIPATTN_OK;   // an fp8 cache goes through the round-by-round kernel
+  if (rows > 1 || (p.D != 64 && p.D != 128 && p.D != 256)) return 0;
+  if (p.k.fp8_e5m2) return 0;   // an fp8 cache goes through the round-by-round kernel
   // in-kernel RoPE: "streaming" rotates a chunk's tokens alike; "relative" scores a token by the side it is proposed for
-  if (p.rope_mode != HIPATTN_ROPE_NONE && p.rope_mode != HIPATTN_ROPE_STREAMING) return HIPATTN_OK;
+  if (p.rope_mode != HIPATTN_ROPE_NONE && p.rope_mode != HIPATTN_ROPE_STREAMING) return 0;
   const int C = p.chunk_size;
-  if (C < 4 || C > 32 || (C & (C - 1)) != 0) return HIPATTN_OK;
-  const char* v = getenv("HIPATTN_DECODE_SCAN");
-  if (v && strcmp(v, "rounds") == 0) return HIPATTN_OK;
+  if (C < 4 || C > 32 || (C & (C - 1)) != 0) return 0;
   int c_log2 = 0;
   while ((1 << c_log2) < C) ++c_log2;
   const int Gq = p.H / p.HKV;
   int HB = 4;
   while (HB > 1 && Gq % HB != 0) HB >>= 1;
-  if (C > HB * 2 * (c_log2 + 1)) return HIPATTN_OK;
+  return C > HB * 2 * (c_log2 + 1) ? 0 : HB;
+}
+
+// HIPATTN_DECODE_SCAN=rounds keeps the round-by-round kernel.
+int scan_chunks_strict(const hipattn_scan_params_t& p, cudaStream_t stream, bool* handled) {
+  *handled = false;
+  const int HB = strict_chunk_heads(p);
+  const char* v = getenv("HIPATTN_DECODE_SCAN");
+  if (HB == 0 || (v && strcmp(v, "rounds") == 0)) return HIPATTN_OK;
+  int c_log2 = 0;
+  while ((1 << c_log2) < p.chunk_size) ++c_log2;
   *handled = true;
   switch (p.dtype) {
     case HIPATTN_F32: return dispatch_dim<HIPATTN_F32>(p, c_log2, HB, stream);

@@ -49,3 +49,52 @@ def test_decode_chunk_scan_is_exact(shape, kv, rope, monkeypatch):
     assert keys > 0 and wrong == 0 and fallbacks < 0.25 * keys
     assert ratio < 0.5, f"deviation reached {ratio:.3f} of the assumed radius"
     print(f"{shape} {kv} {rope}: keys {keys} fallbacks {fallbacks} ratio {ratio:.3f}")
+
+
+@pytest.mark.parametrize("keys", ["close", "not_finite"])
+@pytest.mark.parametrize("rope", [None, "relative", "streaming"])
+@pytest.mark.parametrize("kv", ["bf16", "fp16", "fp8"])
+@pytest.mark.parametrize("shape", SHAPES + [dict(B=2, H=8, HKV=2, D=128, T=3333, keep=[2048, 1024, 512])])
+def test_search_on_bounds_equals_strict_scores(shape, kv, rope, keys, monkeypatch):
+    """The call as users make it, without per-head outputs, which would have every score computed strictly before the search:
+    neighbouring keys that are equal or one unit in the last place apart leave the bounds open; infinities, NaN, keys whose
+    magnitudes overflow 16 bits and a query head of zeros give bounds that are not numbers."""
+    import bench
+    from cases import rope_tables
+    from hip_attention_b200 import hip_attention_impl, read_status
+    w = dict(bench.WORKLOADS["decode_128k"], kind="prefill", keep=[4096, 2048, 1024], dtype="fp16" if kv == "fp16" else "bf16")
+    w.update(shape)
+    q, k, v = bench.make_qkv(w, "cuda")
+    g = torch.Generator(device="cuda").manual_seed(5)
+    if keys == "close":
+        n = w["T"] // 2
+        k[:, 1:2 * n:2] = k[:, 0:2 * n:2]
+        bits = k.view(torch.int16)
+        bits[:, 1::4, :, 3] ^= 1
+    else:
+        q[:, :, 0] = 0
+        for value in (float("inf"), float("-inf"), float("nan")):
+            t = torch.randint(0, w["T"], (w["T"] // 100,), generator=g, device="cuda")
+            k[:, t, :, 5] = value
+        t = torch.randint(0, w["T"], (w["T"] // 50,), generator=g, device="cuda")
+        k[:, t] = torch.where(k[:, t] > 0, 5e4, -5e4).to(k.dtype)
+    if kv == "fp8":
+        k, v = k.to(torch.float8_e5m2), v.to(torch.float8_e5m2)
+    kw = {}
+    if rope:
+        cos, sin = rope_tables(w["T"] + 8, w["D"], w["theta"])
+        kw = dict(using_extend=True, need_apply_rope=True, rope_cos=torch.from_numpy(cos).cuda(), rope_sin=torch.from_numpy(sin).cuda(),
+                  scan_extend_backend=rope)
+    read_status("cuda")
+    md = {}
+    for mode in ("auto", "strict"):
+        monkeypatch.setenv("HIPATTN_SCAN_MODE", mode)
+        args = bench.make_args(w, **kw)
+        args.require_cache_statistics = True
+        md[mode] = hip_attention_impl(q, k, v, args)[1]
+    assert read_status("cuda") == 0
+    a, b = md["auto"], md["strict"]
+    for i, (x, y) in enumerate(zip(a.stage_caches[1:], b.stage_caches[1:])):
+        assert torch.equal(x.indices_left, y.indices_left) and torch.equal(x.indices_right, y.indices_right), f"stage {i + 1}"
+    assert torch.equal(a.indices, b.indices) and torch.equal(a.ks, b.ks)
+    assert torch.equal(a.mask_cache_statistics.access_counter, b.mask_cache_statistics.access_counter)
