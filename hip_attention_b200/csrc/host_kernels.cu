@@ -100,6 +100,13 @@ __device__ __forceinline__ int64_t load_int(const CopySeg& s, int64_t at) {
     default: return 0;   // COPY_ZERO
   }
 }
+__device__ __forceinline__ float load_float(const CopySeg& s, int64_t at) {
+  switch (s.src_type) {
+    case COPY_F32: return ((const float*)s.src)[at];
+    case COPY_BF16: return __bfloat162float(((const __nv_bfloat16*)s.src)[at]);
+    default: return 0.f;   // COPY_ZERO
+  }
+}
 
 __global__ void multi_copy_kernel(const CopyList list) {
   const CopySeg& s = list.seg[blockIdx.y];
@@ -116,12 +123,8 @@ __global__ void multi_copy_kernel(const CopyList list) {
     switch (s.dst_type) {
       case COPY_I64: ((int64_t*)s.dst)[dof] = load_int(s, so); break;
       case COPY_I32: case COPY_U32: ((uint32_t*)s.dst)[dof] = (uint32_t)load_int(s, so); break;
-      case COPY_F32:
-        ((float*)s.dst)[dof] = s.src_type == COPY_F32 ? ((const float*)s.src)[so] : __bfloat162float(((const __nv_bfloat16*)s.src)[so]);
-        break;
-      case COPY_BF16:
-        ((__nv_bfloat16*)s.dst)[dof] = s.src_type == COPY_F32 ? __float2bfloat16_rn(((const float*)s.src)[so]) : ((const __nv_bfloat16*)s.src)[so];
-        break;
+      case COPY_F32: ((float*)s.dst)[dof] = load_float(s, so); break;
+      case COPY_BF16: ((__nv_bfloat16*)s.dst)[dof] = __float2bfloat16_rn(load_float(s, so)); break;
     }
   }
 }
@@ -176,6 +179,11 @@ int zero_memory(void* ptr, int64_t bytes, cudaStream_t stream) {
 int multi_copy(const CopyList& list, cudaStream_t stream) {
   int64_t most = 0;
   for (int i = 0; i < list.count; ++i) {
+    const CopySeg& s = list.seg[i];
+    const bool to_float = s.dst_type == COPY_F32 || s.dst_type == COPY_BF16, from_float = s.src_type == COPY_F32 || s.src_type == COPY_BF16;
+    HIPATTN_REQUIRE(s.dst && s.dst_type >= 0 && s.dst_type < COPY_ZERO &&
+                        (s.src_type == COPY_ZERO || (s.src && s.src_type >= 0 && s.src_type < COPY_ZERO && from_float == to_float)),
+                    HIPATTN_ERR_INVALID, "multi_copy: segment %d: type %d to type %d", i, s.src_type, s.dst_type);
     const int64_t t = list.seg[i].n0 * list.seg[i].n1 * list.seg[i].n2;
     if (t > most) most = t;
   }

@@ -286,7 +286,7 @@ class HiPMetadataCachePool:
         return host().pool_read([(b.buffer, b.get_rows(batch_size, self.head_num)) for b in bufs])
 
     def _set_buffers(self, layer_idx: int, items: Sequence) -> None:
-        """Several writes ((name, value); None: zeros in the first ``max_batch_size`` rows), one launch on the GPU."""
+        """Several writes ((name, value); None, for a counter: zeros in the first ``max_batch_size`` rows), one launch on the GPU."""
         rows = self.max_batch_size
         bufs = [self._buffer(layer_idx, name) for name, _ in items]
         left = range(len(items))
@@ -323,14 +323,17 @@ class HiPMetadataCachePool:
         if size != batch_size:
             raise ValueError("the pool serves decode steps: one query token per request")
         items = [(name, getattr(metadata, name)) for name in ("indices", "ks", "ks_count", "ks_start_end")]
+        for i_stage, cache in enumerate(metadata.stage_caches or []):
+            if i_stage > 0:
+                items += [(f"stage_{i_stage}_{name}", getattr(cache, name)) for name in self._STAGE_NAMES]
+        for name, value in items:   # (a step with nothing to scan has no stage inputs: nothing a later step could restart from)
+            if value is None:
+                raise ValueError(f"{name} is None: the metadata of this step cannot be stored")
         for prefix, stats in (("sa", metadata.sa_cache_statistics), ("mask", metadata.mask_cache_statistics)):
             counts = stats.compute_statistics() if stats is not None else {}
             for c in self._COUNTERS:
                 v = counts.get(c)
                 items.append((f"{prefix}_{c}", v if v is None else v.view(1, 1).expand(self.max_batch_size, 1)))
-        for i_stage, cache in enumerate(metadata.stage_caches or []):
-            if i_stage > 0:
-                items += [(f"stage_{i_stage}_{name}", getattr(cache, name)) for name in self._STAGE_NAMES]
         self._set_buffers(layer_id, items)
 
     def compute_cache_statistics(self, batch_size: int) -> dict:

@@ -261,6 +261,44 @@ def test_forward_paged_hip_has_the_reference_parameter_list():
         forward_paged_hip(*common, None, *rest, diag_sliding_window_indices=torch.zeros(1))
 
 
+@pytest.mark.parametrize("dev", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+def test_pool_refuses_metadata_without_a_mask_or_stage_inputs(dev):
+    """Counters may be missing (zeros then); a mask or stage inputs that are None are refused before anything is written."""
+    from hip_attention_b200 import (HiPAttentionConfig, HiPAttentionOutputMetadata, HiPAttentionStageInputCache, HiPMetadataCachePool)
+    H, B = 4, 2
+    pool = HiPMetadataCachePool(64, H, 6, 4096, dev, HiPAttentionConfig())
+    bufs = pool.cache[5]
+    for b in bufs.values():
+        b.buffer.fill_(7)
+    n = bufs["indices"].buffer.shape[-1]
+    mask = dict(indices=torch.zeros((B * H, 1, n), dtype=torch.int64, device=dev), ks=torch.zeros((B * H, 1), dtype=torch.int64, device=dev),
+                ks_count=torch.zeros((B * H, 1, 1), dtype=torch.int64, device=dev), ks_start_end=torch.zeros((B * H, 1, 2), dtype=torch.int64, device=dev),
+                mask_cache_statistics=None, sa_cache_statistics=None)
+    none = HiPAttentionStageInputCache(None, None, None)
+    for bad in (dict(mask, stage_caches=[none, none, none]), dict(mask, indices=None, stage_caches=None), dict(mask, ks=None, stage_caches=None)):
+        with pytest.raises(ValueError, match="None"):
+            pool.set_hip_metadata_cache(5, B, B, HiPAttentionOutputMetadata(**bad))
+        assert all(bool((b.buffer.to(torch.float64) == 7).all()) for b in bufs.values())
+    pool.set_hip_metadata_cache(5, B, B, HiPAttentionOutputMetadata(**mask, stage_caches=None))
+    rows = pool.max_batch_size
+    assert bool((bufs["sa_access_count"].buffer[:rows] == 0).all()) and bool((bufs["sa_access_count"].buffer[rows:] == 7).all())
+    assert bool((bufs["indices"].buffer[:B * H].to(torch.int64) == 0).all()) and bool((bufs["indices"].buffer[B * H:].to(torch.int64) == 7).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.int64, torch.int32, torch.uint32, torch.float32, torch.bfloat16])
+def test_pool_zeros_and_copies_of_every_type(dtype):
+    """The copy kernel's zeros for buffers of every stored type, beside a copy in the same launch."""
+    from hip_attention_b200.operator import host
+    buf = torch.full((6, 5), 7, dtype=dtype, device="cuda") if dtype != torch.uint32 else torch.full((6, 5), 7, dtype=torch.int32, device="cuda").view(dtype)
+    src = (torch.arange(15, device="cuda") + 0.25).view(3, 5)
+    other = torch.zeros((6, 5), dtype=torch.bfloat16, device="cuda")
+    assert host().pool_write([(buf, None, 4), (other, src, 6)]) == []
+    got = buf.to(torch.float64)
+    assert bool((got[:4] == 0).all()) and bool((got[4:] == 7).all())
+    assert torch.equal(other[:3], src.to(torch.bfloat16)) and bool((other[3:] == 0).all())
+
+
 @pytest.mark.gpu
 def test_forward_paged_hip_with_in_kernel_rope_matches_the_reference():
     """The serving default ``using_extend``: un-rotated keys in the pool and cos / sin tables handed to the call.  A
