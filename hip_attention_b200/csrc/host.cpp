@@ -330,7 +330,7 @@ struct Copies {
     if (list.count == hipattn::kMaxCopies) flush();
     list.seg[list.count++] = s;
   }
-  // contiguous dst <- src of the same shape (at most three dimensions once outer ones of equal stride are merged)
+  // contiguous dst <- src of the same shape
   void add(const at::Tensor& src, const at::Tensor& dst) {
     hipattn::CopySeg s{};
     s.src = src.data_ptr();
@@ -342,20 +342,33 @@ struct Copies {
       s.n0 = s.n1 = 1;
       s.n2 = src.numel();
       s.plain = 1;
-    } else {
-      // collapse to three dimensions
-      std::vector<int64_t> n, st;
-      for (int64_t i = 0; i < src.dim(); ++i) {
-        if (src.size(i) == 1) continue;
-        if (!n.empty() && st.back() == src.stride(i) * src.size(i)) { n.back() *= src.size(i); st.back() = src.stride(i); }
-        else { n.push_back(src.size(i)); st.push_back(src.stride(i)); }
-      }
-      while (n.size() < 3) { n.insert(n.begin(), 1); st.insert(st.begin(), 0); }
-      if (n.size() > 3) { add(src.contiguous(), dst); return; }
-      s.n0 = n[0]; s.n1 = n[1]; s.n2 = n[2];
-      for (int i = 0; i < 3; ++i) s.src_s[i] = st[i];
-      s.dst_s[0] = n[1] * n[2]; s.dst_s[1] = n[2]; s.dst_s[2] = 1;
+      add(s);
+      return;
     }
+    std::vector<int64_t> n, st;   // outer dimensions of equal stride merged
+    for (int64_t i = 0; i < src.dim(); ++i) {
+      if (src.size(i) == 1) continue;
+      if (!n.empty() && st.back() == src.stride(i) * src.size(i)) { n.back() *= src.size(i); st.back() = src.stride(i); }
+      else { n.push_back(src.size(i)); st.push_back(src.stride(i)); }
+    }
+    while (n.size() < 3) { n.insert(n.begin(), 1); st.insert(st.begin(), 0); }
+    strided(s, src.element_size(), dst.element_size(), n.data(), st.data(), n.size());
+  }
+  // a segment takes three dimensions: more are dealt out slice by slice (no copy in between, which would have to outlive the launch)
+  void strided(hipattn::CopySeg s, int64_t src_bytes, int64_t dst_bytes, const int64_t* n, const int64_t* st, size_t dims) {
+    if (dims > 3) {
+      int64_t inner = 1;
+      for (size_t i = 1; i < dims; ++i) inner *= n[i];
+      for (int64_t i = 0; i < n[0]; ++i) {
+        strided(s, src_bytes, dst_bytes, n + 1, st + 1, dims - 1);
+        s.src = (const char*)s.src + st[0] * src_bytes;
+        s.dst = (char*)s.dst + inner * dst_bytes;
+      }
+      return;
+    }
+    s.n0 = n[0]; s.n1 = n[1]; s.n2 = n[2];
+    for (int i = 0; i < 3; ++i) s.src_s[i] = st[i];
+    s.dst_s[0] = n[1] * n[2]; s.dst_s[1] = n[2]; s.dst_s[2] = 1;
     add(s);
   }
   void flush() {

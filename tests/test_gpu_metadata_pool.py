@@ -37,3 +37,17 @@ def test_pool_on_gpu_equals_pool_on_cpu(batch, layer):
         got[dev] += [t for c in part.stage_caches[1:] for t in (c.indices_left, c.indices_right, c.out_scores)]
     for a, b in zip(got["cpu"], got["cuda"]):
         assert a.dtype == b.dtype and a.shape == b.shape and torch.equal(a.to(torch.float64), b.cpu().to(torch.float64))
+
+
+@pytest.mark.parametrize("order", [(3, 2, 1, 0), (0, 3, 2, 1), (2, 0, 3, 1)])
+def test_values_of_any_stride_in_one_launch(order):
+    """Several values whose dimensions do not merge: each arrives in its own buffer, the rows behind it untouched."""
+    from hip_attention_b200.operator import host
+    g = torch.Generator(device="cuda").manual_seed(sum(i * x for i, x in enumerate(order)))
+    shape = (3, 4, 5, 6)
+    back = [order.index(i) for i in range(4)]
+    vals = [torch.randint(0, 1000, [shape[i] for i in order], generator=g, device="cuda").permute(back) for _ in range(9)]
+    bufs = [torch.full((5, 4, 5, 6), -1, dtype=torch.int32, device="cuda") for _ in vals]
+    assert vals[0].shape == shape and host().pool_write([(b, v, 5) for b, v in zip(bufs, vals)]) == []
+    for b, v in zip(bufs, vals):
+        assert torch.equal(b[:3].long(), v) and bool((b[3:] == -1).all())
