@@ -391,7 +391,7 @@ struct Call {
   cudaStream_t stream;
   uint32_t* status;
   // Calls that a prefill chunk is split into read the same keys: what they prepare from them is handed on in this dict
-  // (None: a call of its own), valid for the positions it names.
+  // (None: a call of its own), valid for the positions and the windows it names.
   PyObject* shared = Py_None;
   hipattn::QueryPositions where{};   // positions that prepared tables and keys have to reach
   at::Tensor last_pos;               // [B] largest of them
@@ -548,11 +548,20 @@ void set_rope_tables(Call& c, int64_t restart_chunks) {
     c.rope_cos = rope_table(c, cos);
     c.rope_sin = rope_table(c, sin);
   } else {
-    const int64_t c0 = c.stages[0].chunk;
-    int64_t n = cdiv(std::max<int64_t>(0, c.T - c.sink - c.sw), c0), most = std::max(n, restart_chunks);
-    for (size_t i = 1; i < c.stages.size(); ++i) {
-      n = std::min(c.stages[i].k / c.stages[i - 1].chunk, n) * (c.stages[i - 1].chunk / c.stages[i].chunk);
-      most = std::max(most, n);
+    auto reach = [&](int64_t sw) {   // last row of a scan with this window
+      const int64_t c0 = c.stages[0].chunk;
+      int64_t n = cdiv(std::max<int64_t>(0, c.T - c.sink - sw), c0), most = std::max(n, restart_chunks);
+      for (size_t i = 1; i < c.stages.size(); ++i) {
+        n = std::min(c.stages[i].k / c.stages[i - 1].chunk, n) * (c.stages[i - 1].chunk / c.stages[i].chunk);
+        most = std::max(most, n);
+      }
+      return most + std::max<int64_t>(0, sw - c0) + 1;
+    };
+    int64_t floor = reach(c.sw);
+    if (PyObject* windows = c.shared == Py_None ? nullptr : PyDict_GetItemString(c.shared, "windows")) {   // of the calls that use these tables
+      Ref all = checked(PySequence_Fast(windows, "windows must be a list"));
+      for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(all.get()); ++i)
+        floor = std::max(floor, reach(as_int(Ref::borrow(PySequence_Fast_GET_ITEM(all.get(), i)))));
     }
     at::Tensor both = c.dv.empty({2, cos.size(0), c.D / 2}, c.q.scalar_type());
     hipattn::RopeTables t{};
@@ -562,7 +571,7 @@ void set_rope_tables(Call& c, int64_t restart_chunks) {
     t.rows = (int)cos.size(0);
     t.cols = (int)c.D / 2;
     t.dtype = c.dt;
-    t.floor = (int)std::min<int64_t>(most + std::max<int64_t>(0, c.sw - c0) + 1, 1 << 30);
+    t.floor = (int)std::min<int64_t>(floor, 1 << 30);
     t.q = c.where;
     if (c.last_pos.defined() || c.where.B * (int64_t)c.where.TQ > 2048) t.last_pos = last_positions(c);
     t.dst = both.data_ptr();

@@ -141,7 +141,8 @@ def hip_attention_impl(q: Tensor, k: Optional[Tensor], v: Optional[Tensor], args
     mask estimator reads only q and k, so a caller that streams its inputs to the device may issue the call as soon as q
     and k have arrived and pass the event that marks the arrival of v (dense ``v`` or the value cache); the attention
     launch waits for it.  ``shared``: a dict that calls on the same keys hand on, so that key copies and rope tables are
-    prepared once; its entry ``positions`` [B, n] names the query positions of all of them.  ``out`` [B, TQ, H, D] and
+    prepared once; its entries ``positions`` [B, n] and ``windows`` name the query positions and the sliding windows of
+    all of them.  ``out`` [B, TQ, H, D] and
     ``lse`` [B, TQ, H] receive the context and its log-sum-exp.  ``fork``: a fork of the current stream (``host().fork``)
     with calls that do not depend on one another; with ``beside`` a decode call runs beside that stream.  The results may
     be used after ``host().join``."""

@@ -68,3 +68,42 @@ def test_split_prefill_equals_two_calls():
             assert torch.equal(md.indices, ref[1][1].indices) and torch.equal(md.ks, ref[1][1].ks)
     finally:
         S.hip_attention_impl = S_impl
+
+
+@pytest.mark.parametrize("backend", ["relative", "streaming"])
+def test_both_windows_of_a_split_chunk_reach_converted_table_rows(backend):
+    """A layer window below the 777 of the last queries, sink 0 and a short prompt: the last queries' scan rotates to rows that
+    the first part does not reach.  Memory the tables are made in is poisoned; masks and the keys the scans load equal those of
+    two calls of their own."""
+    from cases import rope_tables
+    from hip_attention_b200 import HiPAttentionConfig, forward_paged_hip, hip_attention_12
+    from hip_attention_b200.serving import HiPAttentionPerLayerConfig
+    import hip_attention_b200.serving as S
+    g = torch.Generator(device="cuda").manual_seed(4)
+    n, H, HKV, D, width = 200, 8, 2, 128, 2048
+    kc, vc = (torch.randn((n + 5, HKV, D), generator=g, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    q = torch.randn((n, H, D), generator=g, device="cuda", dtype=torch.bfloat16)
+    req = torch.zeros((2, width), dtype=torch.int32, device="cuda")
+    req[1, :n] = torch.randperm(n, generator=g, device="cuda").to(torch.int32)
+    cos, sin = (torch.from_numpy(t).cuda() for t in rope_tables(16384, D, 5e5))
+    layer = HiPAttentionPerLayerConfig(second_stage_k=64, sliding_window_size=512, sink_token_size=0, scan_extend_backend=backend)
+    cfg = HiPAttentionConfig(layers=[layer, layer], prefill_layers=[layer, layer])
+    calls = []
+
+    def record(q_, k_, v_, args, cached=None, **kw):
+        calls.append((q_, args))
+        return impl(q_, k_, v_, args, cached, **kw)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    poison = torch.full((64 << 20,), 0x7fc07fc0, dtype=torch.int32, device="cuda")   # NaN in either 16-bit type
+    del poison
+    impl, S.hip_attention_impl = S.hip_attention_impl, record
+    try:
+        out, md = forward_paged_hip(q, D ** -0.5, 1, kc, vc, None, torch.arange(n, device="cuda"), torch.tensor([n], dtype=torch.int32, device="cuda"),
+                                    req, torch.tensor([1], device="cuda"), cos, sin, 5, 0.0, width, width, True, cfg)
+    finally:
+        S.hip_attention_impl = impl
+    ref = [hip_attention_12(q_, None, None, a) for q_, a in calls]
+    assert torch.equal(out, torch.cat([r[0] for r in ref], 1))
+    assert torch.equal(md.indices, ref[1][1].indices) and torch.equal(md.ks, ref[1][1].ks)
+    assert torch.equal(md.mask_cache_statistics.access_counter, ref[1][1].mask_cache_statistics.access_counter)
