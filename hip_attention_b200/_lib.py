@@ -12,7 +12,7 @@ F32, F16, BF16 = 0, 1, 2
 STATUS_PAGE_RANGE, STATUS_TOKEN_RANGE, STATUS_TIMEOUT, STATUS_CHUNK_SIZE = 1, 2, 4, 8
 MAX_CHUNKS = 16384
 NOALLOC_SCRATCH_BYTES = 16 * 1024 * 1024
-ABI_VERSION = 9
+ABI_VERSION = 10
 SCAN_AUTO, SCAN_STRICT, SCAN_CHECK = 0, 1, 2
 ROPE_NONE, ROPE_RELATIVE, ROPE_STREAMING = 0, 1, 2
 
@@ -51,7 +51,8 @@ class BsaParams(C.Structure):
                 ("dtype", i32), ("D", i32), ("B", i32), ("TQ", i32), ("H", i32), ("HKV", i32), ("T", i32),
                 ("block_size_q", i32), ("index_block_q", i32), ("block_size_k", i32), ("K", i32),
                 ("sink", i32), ("window", i32), ("n_splits", i32), ("heads_share_mask", i32),
-                ("logit_softcap", f32), ("rope_rows", i32), ("rope_cos", vp), ("rope_sin", vp), ("rope_stride", i64)]
+                ("logit_softcap", f32), ("rope_rows", i32), ("rope_cos", vp), ("rope_sin", vp), ("rope_stride", i64),
+                ("indices_ascending", i32), ("reserved_", i32), ("indices_order", vp)]
 
 
 # name -> (restype, argtypes); every symbol include/hipattn.h declares

@@ -52,10 +52,16 @@ __device__ __forceinline__ KeyList make_key_list(const hipattn_bsa_params_t& p, 
   return kl;
 }
 
-// Drops the selected blocks that no row of the tile admits: a selected token counts up to the row's position - window, block
-// starts ascend, and with a context of a few windows a large part of the selection lies inside them (two prompts of 3001
-// tokens, 4096 selected, window 1024, fp8 and RoPE: 1.32 -> 0.77 ms).  Every warp of the CTA calls it with the rows' largest
-// position; two dependent reads.
+// Whether the selected block starts of this call's lists ascend.  (A caller's mask may be in any order; the answer for one comes
+// from a launch of its own.  Looked up in here, list by list, the code alone cost a prefill chunk that makes its own mask 1.3 %.)
+__device__ __forceinline__ bool lists_ascend(const hipattn_bsa_params_t& p) {
+  return p.indices_ascending && (p.indices_order == nullptr || __ldg(p.indices_order) == 0);
+}
+
+// Drops the selected blocks that no row of the tile admits, of a list whose block starts ascend: a selected token counts up to
+// the row's position - window, and with a context of a few windows a large part of the selection lies inside them (two
+// prompts of 3001 tokens, 4096 selected, window 1024, fp8 and RoPE: 1.32 -> 0.77 ms).  Every warp of the CTA calls it with
+// the rows' largest position; two dependent reads.
 __device__ __forceinline__ void trim_selected(KeyList& kl, int rmax, int window) {
   const int lane = threadIdx.x & 31, n = kl.n_sel / kl.block_k;
   const long long limit = (long long)rmax - window;

@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(kThr, 2) bsa_fp32_kernel(const hipattn_bsa_par
   __syncthreads();
   const int rmin = s_mm[2], rmax = s_mm[3];
   KeyList kl = make_key_list(p, b, h, d, s_mm[0], s_mm[1]);
-  trim_selected(kl, rmax, p.window);
+  if (lists_ascend(p)) trim_selected(kl, rmax, p.window);
   const int far_end = kl.n_sink + kl.n_sel;   // entries from here on are the window's
   const int per = cdiv(cdiv(kl.total, p.n_splits), kKeys) * kKeys;
   const int j_begin = split * per, j_end = min(kl.total, j_begin + per);

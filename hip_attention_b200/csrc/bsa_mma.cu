@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(M * 2) bsa_mma_kernel(const hipattn_bsa_params
   const int pmin = s_mm[0], pmax = s_mm[1];
   const int rmin = s_mm[2], rmax = s_mm[3];
   KeyList kl = make_key_list(p, b, h0, d, pmin, pmax);
-  trim_selected(kl, rmax, p.window);
+  if (lists_ascend(p)) trim_selected(kl, rmax, p.window);
   // the tiles of this CTA's key range (all of them unless the caller asked for key splits)
   const int all_tiles = cdiv(kl.total, TKM);
   const int per_split = cdiv(all_tiles, p.n_splits);

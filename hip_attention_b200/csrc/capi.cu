@@ -378,4 +378,4 @@ extern "C" int hipattn_debug_bounded_wait(uint32_t* status, void* stream) {
 
 extern "C" uint64_t hipattn_launch_count(void) { return hipattn::g_launches.load(std::memory_order_relaxed); }
 extern "C" const char* hipattn_error_string(void) { return g_error; }
-extern "C" int hipattn_abi_version(void) { return 9; }
+extern "C" int hipattn_abi_version(void) { return 10; }

@@ -805,7 +805,7 @@ Mask estimate_mask(Call& c, const hipattn_tokens_t& ktok, int64_t first, at::Ten
 
 struct AttentionArgs {
   int64_t window, block_k, bsa_bq, index_bq;
-  bool heads_share, decode, want_lse;
+  bool heads_share, decode, want_lse, own_mask;
   float softcap;
 };
 
@@ -836,6 +836,18 @@ void attention(Call& c, const hipattn_tokens_t& ktok, const hipattn_tokens_t& vt
   bp.sink = (int)c.sink; bp.window = (int)a.window;
   bp.heads_share_mask = a.heads_share || a.decode;
   bp.logit_softcap = a.softcap;
+  at::Tensor order;
+  bp.indices_ascending = 1;
+  if (!a.own_mask) {   // a mask handed in may be a caller's own, its blocks in any order (decode takes them as they come)
+    bp.indices_ascending = c.TQ > 1 && Kk > 0;
+    if (bp.indices_ascending) {
+      order = dv.empty({1}, at::kInt);
+      bp.indices_order = order.data_ptr<int32_t>();
+      check(hipattn::zero_memory(order.data_ptr(), 4, c.stream), "zero_memory");
+      check(hipattn::check_order(bp.indices, bp.idx_stride_n, bp.idx_stride_d, bp.ks, bp.ks_stride_n, bp.ks_stride_d, (int)indices.size(0),
+                                 (int)indices.size(1), (int)Kk, order.data_ptr<int32_t>(), c.stream), "check_order");
+    }
+  }
   if (c.using_extend) {
     bp.rope_cos = c.rope_cos.data_ptr(); bp.rope_sin = c.rope_sin.data_ptr();
     bp.rope_stride = c.rope_cos.stride(0); bp.rope_rows = (int)c.rope_cos.size(0);
@@ -1118,6 +1130,7 @@ PyObject* forward(PyObject* const* argv) {
   a.bsa_bq = bsa_bq;
   a.index_bq = index_bq;
   a.heads_share = heads_share;
+  a.own_mask = fresh;
   a.decode = c.TQ == 1 && !attr_true(c.args, N.disable_flashdecode) && strcmp(env("HIP_DISABLE_FLASHDECODE", "0"), "1");
   a.want_lse = return_lse;
   Ref cap = attr(c.args, N.logit_softcap);

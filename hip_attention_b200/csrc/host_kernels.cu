@@ -92,6 +92,20 @@ __global__ void __launch_bounds__(256) gather_table_kernel(const E* __restrict__
   for (int j = nv * V + first; j < n; j += step) out[j] = src[j];
 }
 
+__global__ void __launch_bounds__(128) check_order_kernel(const int64_t* __restrict__ indices, int64_t stride_n, int64_t stride_d,
+                                                          const int64_t* __restrict__ ks, int64_t ks_stride_n, int64_t ks_stride_d, int64_t rows,
+                                                          int BDST, int K, int32_t* out_of_order) {
+  for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
+    const int64_t n = row / BDST, d = row % BDST;
+    const int64_t* idx = indices + n * stride_n + d * stride_d;
+    const int64_t have = ks[n * ks_stride_n + d * ks_stride_d];
+    const int count = (int)(have < 0 ? 0 : (have > K ? K : have));
+    bool bad = false;
+    for (int j = threadIdx.x + 1; j < count; j += 128) bad |= idx[j] < idx[j - 1];
+    if (bad) *out_of_order = 1;
+  }
+}
+
 __device__ __forceinline__ int64_t load_int(const CopySeg& s, int64_t at) {
   switch (s.src_type) {
     case COPY_I64: return ((const int64_t*)s.src)[at];
@@ -169,6 +183,15 @@ int gather_table(const void* table, int64_t table_rows, int64_t row_stride, uint
   else
     gather_table_kernel<int32_t><<<dim3((unsigned)gx, (unsigned)n), 256, 0, stream>>>((const int32_t*)table, table_rows, row_stride, status, rows, rows_i64, lens, lens_i64, width, (int32_t*)dst);
   return check_launch("gather_table_kernel");
+}
+
+int check_order(const int64_t* indices, int64_t stride_n, int64_t stride_d, const int64_t* ks, int64_t ks_stride_n, int64_t ks_stride_d, int N, int BDST,
+                int K, int32_t* out_of_order, cudaStream_t stream) {
+  const int64_t rows = (int64_t)N * BDST;
+  if (rows <= 0 || K <= 1) return HIPATTN_OK;
+  check_order_kernel<<<(unsigned)(rows > 148 * 16 ? 148 * 16 : rows), 128, 0, stream>>>(indices, stride_n, stride_d, ks, ks_stride_n, ks_stride_d, rows, BDST,
+                                                                                        K, out_of_order);
+  return check_launch("check_order_kernel");
 }
 
 int zero_memory(void* ptr, int64_t bytes, cudaStream_t stream) {

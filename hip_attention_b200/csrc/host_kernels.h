@@ -72,6 +72,9 @@ int merge_partials(const float* part_o, const float* part_lse, int64_t rows, int
                    float* lse_out, int64_t rows_per_group, int64_t group_stride, cudaStream_t stream);
 // Log-sum-exp merge of shard outputs in the element type: outs [parts, rows, D], lses [parts, rows] base-2 -> out [rows, D]
 int merge_shards(const void* outs, const float* lses, int64_t rows, int parts, int D, int dtype, void* out, cudaStream_t stream);
+// Sets *out_of_order (zeroed by the caller) where the first ks[n][d] of the K entries of a row of indices [N, BDST, K] do not ascend.
+int check_order(const int64_t* indices, int64_t stride_n, int64_t stride_d, const int64_t* ks, int64_t ks_stride_n, int64_t ks_stride_d, int N, int BDST,
+                int K, int32_t* out_of_order, cudaStream_t stream);
 int zero_memory(void* ptr, int64_t bytes, cudaStream_t stream);
 
 // hipattn_select_stage that also writes the next stage's bounds as int64 (either pointer may be null)

@@ -95,7 +95,7 @@ class HiPAttentionStageInputCache:
 
 @dataclass
 class HiPAttentionOutputMetadata:
-    indices: Optional[Tensor]        # [B * H, BDST, K] int64, ascending, padded with INT64_MAX
+    indices: Optional[Tensor]        # [B * H, BDST, K] int64, ascending, padded with INT64_MAX (handed back in: any order)
     ks: Optional[Tensor]             # [B * H, BDST] int64
     ks_count: Optional[Tensor]       # [B * H, BDST, 1] int64
     ks_start_end: Optional[Tensor]   # [B * H, BDST, 2] int32

@@ -224,7 +224,7 @@ typedef struct hipattn_bsa_params {
   const int64_t* pos;
   int64_t pos_stride_b, pos_stride_t;
   hipattn_tokens_t k, v;
-  const int64_t* indices;    /* [B * H, BDST, K] */
+  const int64_t* indices;    /* [B * H, BDST, K], any order (see indices_ascending) */
   int64_t idx_stride_n, idx_stride_d;
   const int64_t* ks;         /* [B * H, BDST] */
   int64_t ks_stride_n, ks_stride_d;
@@ -248,6 +248,12 @@ typedef struct hipattn_bsa_params {
   const void* rope_cos;      /* [rope_rows, D] in the element type of q */
   const void* rope_sin;
   int64_t rope_stride;
+  /* 1: the first ks entries of every row of indices ascend, as hipattn_finalize_indices writes them, unless indices_order is
+   * given and points at a device word that is not 0.  Prefill then finds the blocks that lie inside the window by a search
+   * and leaves them out.  0: the rows may be in any order and every block is visited. */
+  int32_t indices_ascending;
+  int32_t reserved_;
+  const int32_t* indices_order;
 } hipattn_bsa_params_t;
 
 int hipattn_bsa_attention(const hipattn_bsa_params_t* p, void* stream);

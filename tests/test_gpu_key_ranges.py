@@ -45,3 +45,32 @@ def test_key_ranges_match_oracle(shape, tq, ranges, monkeypatch):
     err = (out.float().cpu().double() - ref.double()).abs()
     assert err.max().item() <= mx and err.mean().item() <= mean
     assert (lse.cpu().double() - lse_ref).abs().max().item() < 2e-2
+
+
+@pytest.mark.parametrize("kernel", ["tcgen05", "mma"])
+@pytest.mark.parametrize("shape", ["d128", "d64", "d128_wide_block", "fp32", "fp8_bf16"])
+def test_cached_mask_in_any_order(shape, kernel, monkeypatch):
+    """A caller's mask whose blocks do not ascend attends the same keys: a context of a few windows, where part of the selection
+    lies inside the window of some rows only.  The mask as the operator returned it gives the bits of the call that made it."""
+    import bench
+    from hip_attention_b200 import HiPAttentionOutputMetadata, hip_attention_impl, read_status
+    monkeypatch.setenv("HIPATTN_PREFILL_KERNEL", kernel)
+    w = dict(bench.WORKLOADS["prefill_128k"], TQ=201, T=1501, keep=[1024, 1024, 1024], sink=64, sw=256, **SHAPES[shape])
+    fp8 = w.pop("fp8", False)
+    q, k, v = bench.make_qkv(w, "cuda")
+    if fp8:
+        k, v = k.to(torch.float8_e5m2), v.to(torch.float8_e5m2)
+    read_status("cuda")
+    out, md = hip_attention_impl(q, k, v, bench.make_args(w))
+    again, _ = hip_attention_impl(q, k, v, bench.make_args(w), md)
+    assert torch.equal(out, again)
+    n = int(md.ks.min())
+    assert n > 64 and bool((md.ks == n).all())
+    order = torch.randperm(n, generator=torch.Generator().manual_seed(2)).cuda()
+    idx = md.indices.clone()
+    idx[:, :, :n] = md.indices[:, :, :n][:, :, order]
+    mixed, _ = hip_attention_impl(q, k, v, bench.make_args(w), HiPAttentionOutputMetadata(idx, md.ks, md.ks_count, md.ks_start_end, None, None, None))
+    assert read_status("cuda") == 0
+    mx, mean = output_tolerance(q.dtype)
+    err = (mixed.double() - out.double()).abs()
+    assert err.max().item() <= mx and err.mean().item() <= mean
