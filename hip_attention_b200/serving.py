@@ -449,7 +449,8 @@ def forward_paged_hip(query: Tensor, sm_scale: float, batch_size: int, k_cache: 
         dense, metadata = hip_attention_12(scaled[:, parts[1][0]], k, v, args=make_args(pos[:, parts[1][0]], parts[1][1]), cached_metadata=cached_metadata)
         return torch.cat([sparse.to(query.dtype), dense.to(query.dtype)], dim=1), metadata
     # both parts read the same keys (prepared once, for the chunk's positions and both windows) and write their rows of one output
-    shared, context = {"positions": pos.to(torch.int64), "windows": [window for _, window in parts]}, torch.empty_like(scaled)
+    shared = {"positions": pos.to(torch.int64), "windows": [window for _, window in parts]}
+    context = torch.empty(scaled.shape, dtype=scaled.dtype, device=scaled.device)   # (contiguous, whatever the query's strides)
     for rows, window in parts:
         _, metadata = hip_attention_impl(scaled[:, rows], k, v, make_args(pos[:, rows], window), None, shared=shared, out=context[:, rows])
     return context, metadata

@@ -107,3 +107,25 @@ def test_both_windows_of_a_split_chunk_reach_converted_table_rows(backend):
     assert torch.equal(out, torch.cat([r[0] for r in ref], 1))
     assert torch.equal(md.indices, ref[1][1].indices) and torch.equal(md.ks, ref[1][1].ks)
     assert torch.equal(md.mask_cache_statistics.access_counter, ref[1][1].mask_cache_statistics.access_counter)
+
+
+def test_split_prefill_takes_a_query_of_any_strides():
+    """Queries stored head-major, or as columns of a fused projection, against a contiguous copy."""
+    from hip_attention_b200 import HiPAttentionConfig, forward_paged_hip
+    g = torch.Generator(device="cuda").manual_seed(6)
+    n, ctx, H, HKV, D, width = 150, 2000, 8, 2, 128, 4096
+    kc, vc = (torch.randn((ctx, HKV, D), generator=g, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    req = torch.randperm(ctx, generator=g, device="cuda").to(torch.int32).view(1, ctx)
+    req = torch.nn.functional.pad(req, (0, width - ctx))
+    cfg = HiPAttentionConfig(json_or_path='{"using_extend": false}')
+    head_major = torch.randn((H, n, D), generator=g, device="cuda", dtype=torch.bfloat16).permute(1, 0, 2)
+    fused = torch.randn((n, H + 2 * HKV, D), generator=g, device="cuda", dtype=torch.bfloat16)[:, :H]
+
+    def call(q):
+        return forward_paged_hip(q, D ** -0.5, 1, kc, vc, None, torch.arange(ctx - n, ctx, device="cuda"), torch.tensor([ctx], dtype=torch.int32, device="cuda"),
+                                 req, torch.tensor([0], device="cuda"), None, None, 5, 0.0, width, width, True, cfg)
+    for q in (head_major, fused):
+        assert not q.is_contiguous()
+        out, md = call(q)
+        ref, ref_md = call(q.contiguous())
+        assert out.is_contiguous() and torch.equal(out, ref) and torch.equal(md.indices, ref_md.indices)
