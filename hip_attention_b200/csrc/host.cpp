@@ -1334,14 +1334,17 @@ PyObject* stack_rows(PyObject* lists) {
     }
     std::vector<int64_t> sizes = first.sizes().vec();
     int64_t rows = 0;
+    at::ScalarType type = first.scalar_type();      // int32 and int64 side by side: int64
     for (Py_ssize_t j = 0; j < m; ++j) {
       const at::Tensor t = tensor_of(PyList_GET_ITEM(l, j), "rows");
-      if (t.scalar_type() != first.scalar_type() || t.device() != first.device() || t.dim() != first.dim() || t.dim() < 1 || t.sizes().slice(1) != first.sizes().slice(1))
-        VALUE_ERROR("shards of one page pool must have block tables and lengths of the same type and width");
+      if ((t.scalar_type() != at::kInt && t.scalar_type() != at::kLong) || t.device() != first.device() || t.dim() != first.dim() || t.dim() < 1 ||
+          t.sizes().slice(1) != first.sizes().slice(1))
+        VALUE_ERROR("shards of one page pool must have int32 or int64 block tables and lengths of the same width on one device");
+      type = at::promoteTypes(type, t.scalar_type());
       rows += t.size(0);
     }
     sizes[0] = rows;
-    at::Tensor dst = at::detail::empty_cuda(sizes, first.scalar_type(), first.device(), c10::nullopt);
+    at::Tensor dst = at::detail::empty_cuda(sizes, type, first.device(), c10::nullopt);
     int64_t at_row = 0;
     for (Py_ssize_t j = 0; j < m; ++j) {
       const at::Tensor t = tensor_of(PyList_GET_ITEM(l, j), "rows");

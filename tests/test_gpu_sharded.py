@@ -43,6 +43,17 @@ def test_batched_shards_equal_shards_one_by_one():
     assert torch.equal(again, bat)
 
 
+def test_shards_with_tables_of_either_integer_type():
+    """Block tables and lengths that are int32 in one shard and int64 in the next still share a call."""
+    from hip_attention_b200.sharded import hip_attention_12_sequence_sharded
+    S, L = 8, 4096
+    w, q, paged, _, args = _problem(S, L)
+    mixed = [(kc, vc, tb.long() if s % 2 else tb, n.long() if s % 3 else n) for s, (kc, vc, tb, n) in enumerate(paged)]
+    ref, mds = hip_attention_12_sequence_sharded(q, paged, args, n_shards=S, shard_len=L, per_shard_k=256)
+    out, got = hip_attention_12_sequence_sharded(q, mixed, args, n_shards=S, shard_len=L, per_shard_k=256)
+    assert len(got) == 3 and torch.equal(out, ref) and all(torch.equal(a.indices, b.indices) for a, b in zip(got, mds))
+
+
 def test_partly_filled_sequence():
     """A sequence that ends inside shard 5: the window moves to that shard, its position follows its live length,
     shards 6 and 7 contribute nothing; the page-pool form and the form with dense slices of the live lengths agree."""
