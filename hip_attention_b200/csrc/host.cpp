@@ -434,7 +434,7 @@ void read_stages(Call& c) {
     const int is = PyObject_IsInstance(st, K.ScanStage);
     if (is < 0) throw PyError{};
     if (!is) NOT_BUILT("stage %d: only ScanStage is built (%s given)", (int)i, Py_TYPE(st)->tp_name);
-    if (attr_int(st, N.stage_stride) != 1) NOT_BUILT("stage_stride != 1 is not built");
+    if (attr_num(st, N.stage_stride) != 1) NOT_BUILT("stage_stride != 1 is not built");
     // the selection kernel always realigns, resets the scores and sorts by position; the reference does each only when
     // the stage asks for it (attention_extend.py:2075-2090, 2638)
     if (i > 0 && !(attr_true(st, N.require_realign_index) && attr_true(st, N.require_reset_score) && attr_true(st, N.require_post_sort)))
@@ -469,7 +469,7 @@ void reject_unsupported(Call& c) {
     NOT_BUILT("using_extend and need_apply_rope must be set together (rotation of already rotated q / k, attention_extend.py:299-323, is not built)");
   if (attr_num(a, N.low_percent) > 0 && attr_num(a, N.low_k_ratio) < 1) NOT_BUILT("low_percent / low_k_ratio is dead code in the reference and is not built");
   if (!attr_true(a, N.is_causal)) NOT_BUILT("is_causal=False is not built");
-  if (attr_int(a, N.stage_early_terminate) != 1) NOT_BUILT("stage_early_terminate != 1 is not built");
+  if (attr_num(a, N.stage_early_terminate) != 1) NOT_BUILT("stage_early_terminate != 1 is not built");
   if (!attr(a, N.sliding_window_indices).none()) NOT_BUILT("sliding_window_indices is not built");
   if (strcmp(env("HIP_HEAD_REDUCE", "1"), "1")) NOT_BUILT("HIP_HEAD_REDUCE=0 (per-head masks) is not built");
   for (const char* name : {"HIP_DEBUG_TOPKMEAN", "HIP_DEBUG_UNION_HEAD", "HIP_DEBUG_ADD_DELAY_WINDOW", "HIP_DEBUG_SNAP_KV", "APPLY_V_DOT", "HIP_CUMSUM"})
@@ -957,7 +957,8 @@ PyObject* forward(PyObject* const* argv) {
     c.HKV = c.k.size(2);
     if (c.k.size(0) != c.B || c.k.size(3) != c.D) VALUE_ERROR("k shape %s does not match q shape %s", shape_text(c.k).c_str(), shape_text(c.q).c_str());
   } else {
-    c.T = attr_int(c.args, N.extend_context_length);
+    Ref length = attr(c.args, N.extend_context_length);     // (whatever int() takes: configuration files write 1e5)
+    c.T = as_int(checked(PyNumber_Long(length.get())));
     if (c.k_cache.dim() != 4) VALUE_ERROR("k_cache must be [n_pages, page_size, kv_heads, head_dim] with a contiguous last dim");
     c.HKV = c.k_cache.size(2);
     if (c.k_cache.size(3) != c.D) VALUE_ERROR("k_cache head_dim differs from q");

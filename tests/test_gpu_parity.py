@@ -200,6 +200,19 @@ def test_short_context_has_empty_selection():
     assert (out.float() - ref).abs().max().item() < 2e-2
 
 
+def test_numbers_of_another_type_are_taken():
+    """A context length, a stride and a termination step that are floats of whole value, as parsed configuration files hold them."""
+    from hip_attention_b200 import hip_attention_12
+    q, k, v, pos, c, cfg, (kc, vc, table, seq, ext) = case_inputs("paged_decode_fp16")
+    outs = []
+    for number in (int, float):
+        args = make_args(c, pos.cuda(), k_cache=kc.cuda(), v_cache=vc.cuda(), block_table=table.cuda(), cache_seq_lens=seq.cuda(),
+                         extend_context_length=number(ext), stage_early_terminate=number(1))
+        args.stages[0].stage_stride = number(1)
+        outs.append(hip_attention_12(q.cuda(), None, None, args))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1].indices, outs[1][1].indices)
+
+
 def test_invalid_arguments_raise_before_launch():
     from hip_attention_b200 import HiPAttentionArgs, ScanStage, hip_attention_12
     q = torch.zeros(1, 8, 4, 64, device="cuda", dtype=torch.bfloat16)
