@@ -892,7 +892,7 @@ Ref stage_cache(const Call& c, const Mask& m, size_t i, int64_t BDST) {
 
 // the chunk lists a restart begins with (foreign caches, e.g. the reference's: per-head lists are identical under the
 // head max-reduce)
-void restart_inputs(Call& c, PyObject* entry, int64_t rows, at::Tensor& left, at::Tensor& right) {
+void restart_inputs(Call& c, PyObject* entry, int64_t rows, at::Tensor& left, at::Tensor& right, Beside& beside) {
   Ref l32 = attr_opt(entry, N._left32);
   if (!l32.none()) {
     left = tensor_of(l32.get(), "_left32");
@@ -906,9 +906,14 @@ void restart_inputs(Call& c, PyObject* entry, int64_t rows, at::Tensor& left, at
   at::Tensor two = c.dv.empty({2, rows, n}, at::kInt);
   left = two.select(0, 0);
   right = two.select(0, 1);
-  if (copy_type(l.scalar_type()) > hipattn::COPY_U32 || copy_type(r.scalar_type()) > hipattn::COPY_U32 || copy_type(l.scalar_type()) < 0 ||
-      copy_type(r.scalar_type()) < 0 || l.device() != c.q.device() || r.device() != c.q.device())
-    VALUE_ERROR("stage caches must be integer tensors on q's device");
+  if (l.device() != c.q.device() || r.device() != c.q.device()) VALUE_ERROR("stage caches must be on q's device");
+  for (at::Tensor* t : {&l, &r}) {
+    const int type = copy_type(t->scalar_type());
+    if (type >= 0 && type <= hipattn::COPY_U32) continue;
+    *t = t->to(at::kLong);     // (a caller's own type; a torch operation, on the current stream)
+    beside.after_current();
+    if (c.dv.keep) c.dv.keep->push_back(*t);
+  }
   Copies cp(c.stream);
   cp.add(l.select(2, 0), left);
   cp.add(r.select(2, 0), right);
@@ -1059,7 +1064,7 @@ PyObject* forward(PyObject* const* argv) {
         if (have > (Py_ssize_t)c.stages.size()) VALUE_ERROR("more stage caches than stages");
         first = have - 1;
         Ref entry = checked(PySequence_GetItem(stage_caches.get(), first));
-        restart_inputs(c, entry.get(), rows, left, right);
+        restart_inputs(c, entry.get(), rows, left, right, beside);
       }
     }
     if (c.using_extend) set_rope_tables(c, first > 0 ? left.size(1) : 0);

@@ -154,6 +154,19 @@ def test_cached_mask_and_stage_restart(name):
     assert torch.equal(m4.indices, md.indices) and torch.equal(o4, out)
 
 
+@pytest.mark.parametrize("dtype", [torch.int64, torch.int32, torch.uint32, torch.int16, torch.float32])
+def test_restart_from_stage_caches_of_any_number_type(dtype):
+    """Chunk bounds that a caller stored in a type of their own."""
+    from hip_attention_b200 import HiPAttentionOutputMetadata, HiPAttentionStageInputCache, hip_attention_12
+    q, k, v, pos, c, cfg, paged = case_inputs("prefill_fp32")
+    q, k, v, pos = q.cuda(), k.cuda(), v.cuda(), pos.cuda()
+    out, md = hip_attention_12(q, k, v, make_args(c, pos))
+    caches = [HiPAttentionStageInputCache(None, None, None)] + [
+        HiPAttentionStageInputCache(s.indices_left.to(dtype), s.indices_right.to(dtype), s.out_scores) for s in md.stage_caches[1:]]
+    got, again = hip_attention_12(q, k, v, make_args(c, pos), HiPAttentionOutputMetadata(None, None, None, None, None, None, caches))
+    assert torch.equal(again.indices, md.indices) and torch.equal(got, out)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_decode_kernel_equals_prefill_kernel(dtype):
     """Reference check (tests/v1_2/test_attention_decode_bsa.py:104-107): split-KV decode and the
