@@ -381,7 +381,8 @@ __global__ void __launch_bounds__(128, resident_ctas(D, NR, STREAM)) scan_stage_
       wlo = win ? llo : rlo;
       whi = win ? lhi : rhi;
       mine = win != (side != 0);
-      unsigned need = __ballot_sync(0xffffffffu, act && fetched && !certain && (open || check || (mine && whi > score)));
+      // (bounds that are not numbers, of a magnitude that overflows, bound nothing)
+      unsigned need = __ballot_sync(0xffffffffu, act && fetched && !certain && (open || check || (mine && !(whi <= score))));
       if (!need) break;
       while (need) {
         const int owner = __ffs(need) - 1;

@@ -539,6 +539,28 @@ def test_scan_kernels_agree(shape, dtype, monkeypatch):
     assert torch.equal(md_p.indices, ref_md.indices) and torch.equal(md_p.ks, ref_md.ks)
 
 
+def test_scan_scores_a_lone_key_whose_magnitude_overflows(monkeypatch):
+    """A chunk of one token proposes the same key twice.  Queries of zeros and bf16 keys whose magnitudes add up beyond fp32:
+    the radius is 0 * inf, and the score is the strict one all the same."""
+    from hip_attention_b200 import HiPAttentionArgs, ScanStage, hip_attention_impl
+    T, TQ, H, D = 32 * 40 + 1, 70, 4, 128
+    g = torch.Generator(device="cuda").manual_seed(8)
+    k = torch.randn((1, T, 2, D), generator=g, device="cuda", dtype=torch.bfloat16)
+    k[:, -1] = 1e38
+    q = torch.zeros((1, TQ, H, D), device="cuda", dtype=torch.bfloat16)
+    stages = [ScanStage(64, 4, 32, None, 1), ScanStage(64, 1, 8, 512, 1)]
+    got = {}
+    for mode in ("auto", "strict"):
+        monkeypatch.setenv("HIPATTN_SCAN_MODE", mode)
+        args = HiPAttentionArgs(position_ids=torch.full((1, TQ), T - 1, device="cuda"), sink_token_size=0, sliding_window_size=0, second_stage_k=256,
+                                stages=stages)
+        got[mode] = {}
+        hip_attention_impl(q, k, k, args, debug=got[mode])
+    for a, b in zip(got["auto"]["stages"], got["strict"]["stages"]):
+        assert torch.equal(a["score"], b["score"]) and torch.equal(a["score_max"], b["score_max"])
+    assert bool((got["auto"]["stages"][0]["score"][:, :, -1] == 0).all())
+
+
 @pytest.mark.parametrize("kernel", ["tcgen05", "mma"])
 @pytest.mark.parametrize("bq,tq,hkv", [(64, 300, 2), (128, 300, 2), (64, 64, 4), (64, 1024, 1)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
