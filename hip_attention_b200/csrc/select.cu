@@ -152,18 +152,6 @@ __device__ __forceinline__ void sort_padded(uint32_t* a, int n, int n_pad) {
   bitonic_sort(a, n_pad);
 }
 
-__global__ void init_chunks_kernel(int32_t* left, int32_t* right, int32_t* score_max, int64_t total, int n, int sink,
-                                   int chunk, int T, int scan_window) {
-  const int32_t init = encode_score(HIPATTN_SCORE_INIT);
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(i % n);
-    const int l = sink + c * chunk;
-    left[i] = l;
-    right[i] = min(l + chunk, T - scan_window);
-    score_max[i] = init;
-  }
-}
-
 template <int THREADS, int IPT>
 __global__ void __launch_bounds__(THREADS)
     select_stage_kernel(const int32_t* __restrict__ score_max, const int32_t* __restrict__ left, int n, int k_keep, int k_pad, int sink,
@@ -294,9 +282,11 @@ extern "C" int hipattn_init_chunks(int32_t* left, int32_t* right, int32_t* score
   HIPATTN_REQUIRE(rows >= 0 && n >= 0 && chunk > 0 && sink >= 0, HIPATTN_ERR_INVALID, "init_chunks: bad sizes");
   if (rows * n == 0) return HIPATTN_OK;
   HIPATTN_REQUIRE(left && right && score_max, HIPATTN_ERR_INVALID, "init_chunks: null output");
-  init_chunks_kernel<<<grid_for(rows * n, 256), 256, 0, (cudaStream_t)stream>>>(left, right, score_max, rows * n, n, sink,
-                                                                                chunk, T, scan_window);
-  return check_launch("init_chunks_kernel");
+  BeginCall c{};
+  c.left = left; c.right = right; c.score_max = score_max;
+  c.rows = rows; c.n = n;
+  c.sink = sink; c.chunk = chunk; c.T = T; c.scan_window = scan_window;
+  return begin_call(c, (cudaStream_t)stream);
 }
 
 int hipattn::select_stage(const int32_t* score_max, const int32_t* left, int64_t rows, int32_t n, int32_t k_keep, int32_t sink,
