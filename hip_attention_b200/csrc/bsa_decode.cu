@@ -1,6 +1,9 @@
-// Block-sparse attention, decode (one query row per sequence): bandwidth-bound split-KV kernel.
+// Block-sparse attention, decode (one query row per sequence): two kernels, both bound by memory.
 //
-// One CTA owns (batch, KV head, key range).  The G query heads of the KV group share every K / V row
+// bsa_decode_mma_kernel (16-bit and fp8 rows of head dim 64 or 128, up to eight query heads per KV head; described where it
+// begins) is the one that decode calls run on.  bsa_decode_kernel takes the rest: fp32, and 16-bit rows of head dim 256.
+//
+// bsa_decode_kernel: one CTA owns (batch, KV head, key range).  The G query heads of the KV group share every K / V row
 // that is fetched.  A warp walks its part of the key list 32 keys at a time:
 //   lanes resolve 32 list entries to positions, admission and row addresses (page-table lookups);
 //   K rows are read with 16-byte loads, LPR lanes per row (a 256-byte row = 16 lanes), several rows
@@ -717,15 +720,15 @@ int dispatch_group(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* han
   }
 }
 
+// rows of 128, 256 or 512 bytes; 16-bit rows of head dim 64 and 128 are the tensor-core kernel's
 template <int DT>
 int dispatch_row(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled) {
   const int lpr = p.D * Elem<DT>::bytes / 16;
-  switch (lpr) {
-    case 8: return dispatch_group<DT, 8>(p, stream, handled);
-    case 16: return dispatch_group<DT, 16>(p, stream, handled);
-    case 32: return dispatch_group<DT, 32>(p, stream, handled);
-    default: return HIPATTN_OK;
+  if constexpr (DT == HIPATTN_F32) {
+    if (lpr == 8) return dispatch_group<DT, 8>(p, stream, handled);
+    if (lpr == 16) return dispatch_group<DT, 16>(p, stream, handled);
   }
+  return lpr == 32 ? dispatch_group<DT, 32>(p, stream, handled) : HIPATTN_OK;
 }
 
 }  // namespace
@@ -735,7 +738,8 @@ bool decode_on_tensor_cores(const hipattn_bsa_params_t& p) {
   return p.TQ == 1 && p.dtype != HIPATTN_F32 && p.H / p.HKV <= 8 && (p.D == 64 || p.D == 128) && p.k.fp8_e5m2 == p.v.fp8_e5m2;
 }
 
-// Decode shapes: one query row, 1 / 2 / 4 / 8 query heads per KV head, K / V rows of 128, 256 or 512 bytes.
+// Decode shapes: one query row; what the tensor-core kernel does not take, with 1 / 2 / 4 / 8 query heads per KV head and K / V
+// rows of 128, 256 or 512 bytes.
 int bsa_decode(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled) {
   *handled = false;
   if (decode_on_tensor_cores(p)) {
