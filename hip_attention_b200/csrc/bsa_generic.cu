@@ -1,7 +1,8 @@
 // Block-sparse attention, general kernel (any element type, fp32 arithmetic on CUDA cores).
 //
-// Serves what the other kernels do not take: fp32 decode, small blocks and in-kernel RoPE in fp32, head dim 256; decode (one query row per head; the heads of a KV group are packed into one
-// tile so every gathered key / value row is used by all of them) and shapes the tensor-core prefill
+// Serves what the other kernels do not take: fp32 decode with RoPE or odd groups, small blocks, in-kernel RoPE in fp32, head dim
+// 256.  In decode (one query row per head) the heads of a KV group are packed into one tile, so that every gathered key / value
+// row is used by all of them; in prefill it takes the shapes that the tensor-core
 // kernel does not cover.  Decode may split the key list into ranges; each range writes a normalised
 // partial output with its base-2 log-sum-exp.
 //

@@ -998,6 +998,7 @@ PyObject* forward(PyObject* const* argv) {
   } else {
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(c.stream, &capturing);
+    // (the sequence shards hand over a `shared` dict: theirs are the last positions at every replay)
     if (capturing != cudaStreamCaptureStatusNone && c.shared == Py_None) VALUE_ERROR("position_ids must be given under CUDA graph capture");
     own_pos = true;
     at::Tensor row = c.dv.empty({c.TQ}, at::kLong);
@@ -1296,8 +1297,10 @@ PyObject* gather_table(PyObject* const* argv) {
     Py_RETURN_NONE;
   const c10::cuda::CUDAGuard guard(table.device());
   at::Tensor out = at::detail::empty_cuda({rows.size(0), table.size(1)}, table.scalar_type(), table.device(), c10::nullopt);
-  check(hipattn::gather_table(table.data_ptr(), table.size(0), table.stride(0), (uint32_t*)status_word(table.device().index()).data_ptr(), (int)table.element_size(), rows.data_ptr(), rows.scalar_type() == at::kLong, lens.data_ptr(),
-                              lens.scalar_type() == at::kLong, (int)rows.size(0), (int)table.size(1), out.data_ptr(),
+  const at::Tensor status = status_word(table.device().index());
+  check(hipattn::gather_table(table.data_ptr(), table.size(0), table.stride(0), (uint32_t*)status.data_ptr(), (int)table.element_size(),
+                              rows.data_ptr(), rows.scalar_type() == at::kLong, lens.data_ptr(), lens.scalar_type() == at::kLong,
+                              (int)rows.size(0), (int)table.size(1), out.data_ptr(),
                               c10::cuda::getCurrentCUDAStream(table.device().index()).stream()), "gather_table");
   return wrap(out);
 }

@@ -64,14 +64,16 @@ __global__ void __launch_bounds__(256) convert_rope_tables_kernel(const RopeTabl
 #pragma unroll
     for (int sd = 0; sd < 2; ++sd) {
       const float4 v = __ldg(reinterpret_cast<const float4*>((sd ? t.sin : t.cos) + r * t.row_stride + c));
-      *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(t.dst) + sd * side + (int64_t)r * t.cols + c) = make_uint2(pack2<DT>(v.x, v.y), pack2<DT>(v.z, v.w));
+      uint16_t* dst = reinterpret_cast<uint16_t*>(t.dst) + sd * side + (int64_t)r * t.cols + c;
+      *reinterpret_cast<uint2*>(dst) = make_uint2(pack2<DT>(v.x, v.y), pack2<DT>(v.z, v.w));
     }
   }
 }
 
 template <typename E>
-__global__ void __launch_bounds__(256) gather_table_kernel(const E* __restrict__ table, int64_t table_rows, int64_t row_stride, uint32_t* status, const void* rows, int rows_i64, const void* lens,
-                                                           int lens_i64, int width, E* __restrict__ dst) {
+__global__ void __launch_bounds__(256) gather_table_kernel(const E* __restrict__ table, int64_t table_rows, int64_t row_stride, uint32_t* status,
+                                                           const void* rows, int rows_i64, const void* lens, int lens_i64, int width,
+                                                           E* __restrict__ dst) {
   const int i = blockIdx.y;
   int64_t row = rows_i64 ? ((const int64_t*)rows)[i] : (int64_t)((const int32_t*)rows)[i];
   if (row < 0 || row >= table_rows) {
@@ -170,18 +172,21 @@ int convert_rope_tables(const RopeTables& t, cudaStream_t stream) {
   return check_launch("convert_rope_tables_kernel");
 }
 
-int gather_table(const void* table, int64_t table_rows, int64_t row_stride, uint32_t* status, int entry_bytes, const void* rows, int rows_i64, const void* lens, int lens_i64, int n,
-                 int width, void* dst, cudaStream_t stream) {
+int gather_table(const void* table, int64_t table_rows, int64_t row_stride, uint32_t* status, int entry_bytes, const void* rows, int rows_i64,
+                 const void* lens, int lens_i64, int n, int width, void* dst, cudaStream_t stream) {
   if (n <= 0 || width <= 0) return HIPATTN_OK;
   int64_t gx = ((int64_t)width * entry_bytes / 16 + 255) / 256;
   const int64_t most = (148 * 8 + n - 1) / n;
   if (gx > most) gx = most;
   if (gx < 1) gx = 1;
   HIPATTN_REQUIRE(n <= 65535, HIPATTN_ERR_INVALID, "gather_table: %d rows", n);
+  const dim3 grid((unsigned)gx, (unsigned)n);
   if (entry_bytes == 8)
-    gather_table_kernel<int64_t><<<dim3((unsigned)gx, (unsigned)n), 256, 0, stream>>>((const int64_t*)table, table_rows, row_stride, status, rows, rows_i64, lens, lens_i64, width, (int64_t*)dst);
+    gather_table_kernel<int64_t><<<grid, 256, 0, stream>>>((const int64_t*)table, table_rows, row_stride, status, rows, rows_i64, lens, lens_i64, width,
+                                                           (int64_t*)dst);
   else
-    gather_table_kernel<int32_t><<<dim3((unsigned)gx, (unsigned)n), 256, 0, stream>>>((const int32_t*)table, table_rows, row_stride, status, rows, rows_i64, lens, lens_i64, width, (int32_t*)dst);
+    gather_table_kernel<int32_t><<<grid, 256, 0, stream>>>((const int32_t*)table, table_rows, row_stride, status, rows, rows_i64, lens, lens_i64, width,
+                                                           (int32_t*)dst);
   return check_launch("gather_table_kernel");
 }
 

@@ -59,8 +59,8 @@ int convert_rope_tables(const RopeTables& t, cudaStream_t stream);
 
 // rows[i] of table [table_rows, width] -> dst [n, width], only the first lens[i] entries of a row when lens is given; a row
 // outside the table reads row 0 and sets HIPATTN_STATUS_PAGE_RANGE
-int gather_table(const void* table, int64_t table_rows, int64_t row_stride, uint32_t* status, int entry_bytes, const void* rows, int rows_i64, const void* lens, int lens_i64, int n,
-                 int width, void* dst, cudaStream_t stream);
+int gather_table(const void* table, int64_t table_rows, int64_t row_stride, uint32_t* status, int entry_bytes, const void* rows, int rows_i64,
+                 const void* lens, int lens_i64, int n, int width, void* dst, cudaStream_t stream);
 
 // hipattn_scan_prepare_keys[_rope] for live tokens only: those at most `reach` behind last_pos[b]
 int scan_prepare_keys(const hipattn_tokens_t& k, int dtype, int D, int B, int T, int HKV, float k_scale, float* key_abs, void* k_scaled,

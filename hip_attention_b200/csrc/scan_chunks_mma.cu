@@ -418,109 +418,109 @@ __global__ void __launch_bounds__(128, MODE == HIPATTN_ROPE_NONE || F8 ? 4 : 3)
     bool exact = check || p.score_out != nullptr;
     for (;;) {
       if (exact) {
-      // ---- the uncertain scores by the strict definition, one per lane ----
-      while (__any_sync(0xffffffffu, unsure != 0)) {
-        const int mine = __popc(unsure);
-        int at = mine;
+        // ---- the uncertain scores by the strict definition, one per lane ----
+        while (__any_sync(0xffffffffu, unsure != 0)) {
+          const int mine = __popc(unsure);
+          int at = mine;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int y = __shfl_up_sync(0xffffffffu, at, o);
-          if (lane >= o) at += y;
-        }
-        const int total = min(32, __shfl_sync(0xffffffffu, at, 31));
-        at -= mine;
-        while (unsure && at < 32) {
-          const int bit = __ffs(unsure) - 1;
-          unsure &= unsure - 1;
-          const int i = bit & 3, v = (bit >> 2) % NV, mt = (bit >> 2) / NV;
-          s_list[warp][at++] = (unsigned short)((v << 9) | ((col + (i & 1)) << 6) | (mt * 16 + (lane >> 2) + (i >> 1) * 8));
-        }
-        __syncwarp();
-        if (lane < total) {
-          const int code = s_list[warp][lane], r = code & 63, hh = (code >> 6) & 7, v = code >> 9;
-          float2* t = wtab + (v * HB + hh) * kTabStride + r;
-          const float raw = strict_score((const char*)s_src[warp][buf][r], hh, c_first + (r >> c_log2), v);
-          float ex = Elem<DT>::round(raw);
-          if (nan_loses) ex = fmaxf(ex, -INFINITY);
-          if (check) {
-            const float xv = t[check_tab].x, e = t[check_tab].y;
-            ++st_keys;
-            if (t->x != t->y) ++st_fb;
-            else if (t->x != ex) ++st_wrong;
-            if (e > 0.f) st_ratio = fmaxf(st_ratio, fabsf(xv - raw) / e);
+          for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, at, o);
+            if (lane >= o) at += y;
           }
-          *t = make_float2(ex, ex);
+          const int total = min(32, __shfl_sync(0xffffffffu, at, 31));
+          at -= mine;
+          while (unsure && at < 32) {
+            const int bit = __ffs(unsure) - 1;
+            unsure &= unsure - 1;
+            const int i = bit & 3, v = (bit >> 2) % NV, mt = (bit >> 2) / NV;
+            s_list[warp][at++] = (unsigned short)((v << 9) | ((col + (i & 1)) << 6) | (mt * 16 + (lane >> 2) + (i >> 1) * 8));
+          }
+          __syncwarp();
+          if (lane < total) {
+            const int code = s_list[warp][lane], r = code & 63, hh = (code >> 6) & 7, v = code >> 9;
+            float2* t = wtab + (v * HB + hh) * kTabStride + r;
+            const float raw = strict_score((const char*)s_src[warp][buf][r], hh, c_first + (r >> c_log2), v);
+            float ex = Elem<DT>::round(raw);
+            if (nan_loses) ex = fmaxf(ex, -INFINITY);
+            if (check) {
+              const float xv = t[check_tab].x, e = t[check_tab].y;
+              ++st_keys;
+              if (t->x != t->y) ++st_fb;
+              else if (t->x != ex) ++st_wrong;
+              if (e > 0.f) st_ratio = fmaxf(st_ratio, fabsf(xv - raw) / e);
+            }
+            *t = make_float2(ex, ex);
+          }
+          __syncwarp();
         }
         __syncwarp();
-      }
-      __syncwarp();
       }
       bool open = false;
       uint32_t seen0 = 0, seen1 = 0;   // rows the reference's rounds would have loaded
-    const int hb_log2 = 31 - __clz(HB);
-    for (int w0 = 0; w0 < (HB << cpp_log2); w0 += 32) {
-      const int wi = w0 + lane;
-      const int hh = wi & (HB - 1), cw = wi >> hb_log2;
-      const int c = c_first + cw;
-      const int rbase = (cw << c_log2) & (kPass - 1);
-      const int la = __shfl_sync(0xffffffffu, in.l[0], rbase & 31), lb = __shfl_sync(0xffffffffu, in.l[1], rbase & 31);
-      const int ra = __shfl_sync(0xffffffffu, in.rt[0], rbase & 31), rb = __shfl_sync(0xffffffffu, in.rt[1], rbase & 31);
-      const int l = rbase < 32 ? la : lb, rt = rbase < 32 ? ra : rb;
-      const bool walker = hh < heads && cw < (1 << cpp_log2) && c < n;
-      float slo = HIPATTN_SCORE_INIT, shi = HIPATTN_SCORE_INIT;
-      bool mine_open = false;
-      int wl = l, wr = rt;
-      if (walker) {
-        const float2* t0_ = wtab + hh * kTabStride + rbase;
-        const float2* t1_ = t0_ + (NV - 1) * HB * kTabStride;
-        for (int it = 0; it < rounds; ++it) {
-          if (!(wl < wr && wl <= pt && wl >= 0)) break;
-          const int mid = (wl + wr) >> 1, tl = (wl + mid) >> 1, tr = (mid + wr) >> 1;
-          const int ol = min(tl - l, C - 1), orr = min(tr - l, C - 1);
-          if (p.access_counter) {
-            const unsigned long long m = (1ull << (rbase + ol)) | (1ull << (rbase + orr));
-            seen0 |= (uint32_t)m;
-            seen1 |= (uint32_t)(m >> 32);
+      const int hb_log2 = 31 - __clz(HB);
+      for (int w0 = 0; w0 < (HB << cpp_log2); w0 += 32) {
+        const int wi = w0 + lane;
+        const int hh = wi & (HB - 1), cw = wi >> hb_log2;
+        const int c = c_first + cw;
+        const int rbase = (cw << c_log2) & (kPass - 1);
+        const int la = __shfl_sync(0xffffffffu, in.l[0], rbase & 31), lb = __shfl_sync(0xffffffffu, in.l[1], rbase & 31);
+        const int ra = __shfl_sync(0xffffffffu, in.rt[0], rbase & 31), rb = __shfl_sync(0xffffffffu, in.rt[1], rbase & 31);
+        const int l = rbase < 32 ? la : lb, rt = rbase < 32 ? ra : rb;
+        const bool walker = hh < heads && cw < (1 << cpp_log2) && c < n;
+        float slo = HIPATTN_SCORE_INIT, shi = HIPATTN_SCORE_INIT;
+        bool mine_open = false;
+        int wl = l, wr = rt;
+        if (walker) {
+          const float2* t0_ = wtab + hh * kTabStride + rbase;
+          const float2* t1_ = t0_ + (NV - 1) * HB * kTabStride;
+          for (int it = 0; it < rounds; ++it) {
+            if (!(wl < wr && wl <= pt && wl >= 0)) break;
+            const int mid = (wl + wr) >> 1, tl = (wl + mid) >> 1, tr = (mid + wr) >> 1;
+            const int ol = min(tl - l, C - 1), orr = min(tr - l, C - 1);
+            if (p.access_counter) {
+              const unsigned long long m = (1ull << (rbase + ol)) | (1ull << (rbase + orr));
+              seen0 |= (uint32_t)m;
+              seen1 |= (uint32_t)(m >> 32);
+            }
+            const float2 sl = t0_[ol], sr = t1_[orr];
+            const bool win = sl.x > sr.y;
+            // (a key does not beat itself; bounds that are not numbers leave its score open all the same)
+            if (!exact && !win && !(sl.y <= sr.x) && (NV == 2 || ol != orr || !(sl.x <= sl.y))) {
+              mine_open = true;
+              break;
+            }
+            if (win) wr = mid; else wl = mid;
+            slo = fmaxf(slo, win ? sl.x : sr.x);
+            shi = fmaxf(shi, win ? sl.y : sr.y);
           }
-          const float2 sl = t0_[ol], sr = t1_[orr];
-          const bool win = sl.x > sr.y;
-          // (a key does not beat itself; bounds that are not numbers leave its score open all the same)
-          if (!exact && !win && !(sl.y <= sr.x) && (NV == 2 || ol != orr || !(sl.x <= sl.y))) {
-            mine_open = true;
-            break;
+          if (!mine_open) {
+            const int64_t o = (row * p.H + h0 + hh) * n + c;
+            if (p.left_out) p.left_out[o] = wl;
+            if (p.right_out) p.right_out[o] = wr;
+            if (p.score_out) p.score_out[o] = slo;
           }
-          if (win) wr = mid; else wl = mid;
-          slo = fmaxf(slo, win ? sl.x : sr.x);
-          shi = fmaxf(shi, win ? sl.y : sr.y);
         }
-        if (!mine_open) {
-          const int64_t o = (row * p.H + h0 + hh) * n + c;
-          if (p.left_out) p.left_out[o] = wl;
-          if (p.right_out) p.right_out[o] = wr;
-          if (p.score_out) p.score_out[o] = slo;
+        for (int o = 1; o < HB; o <<= 1) {
+          slo = fmaxf(slo, __shfl_xor_sync(0xffffffffu, slo, o));
+          shi = fmaxf(shi, __shfl_xor_sync(0xffffffffu, shi, o));
+          mine_open |= (bool)__shfl_xor_sync(0xffffffffu, (int)mine_open, o);
         }
+        mine_open |= slo != shi;
+        open |= mine_open;
+        if (!mine_open && walker && hh == 0 && slo > HIPATTN_SCORE_INIT) atomicMax(p.score_max + row * n + c, encode_score(slo));
       }
-      for (int o = 1; o < HB; o <<= 1) {
-        slo = fmaxf(slo, __shfl_xor_sync(0xffffffffu, slo, o));
-        shi = fmaxf(shi, __shfl_xor_sync(0xffffffffu, shi, o));
-        mine_open |= (bool)__shfl_xor_sync(0xffffffffu, (int)mine_open, o);
+      if (!exact && __any_sync(0xffffffffu, open)) {
+        exact = true;
+        continue;
       }
-      mine_open |= slo != shi;
-      open |= mine_open;
-      if (!mine_open && walker && hh == 0 && slo > HIPATTN_SCORE_INIT) atomicMax(p.score_max + row * n + c, encode_score(slo));
-    }
-    if (!exact && __any_sync(0xffffffffu, open)) {
-      exact = true;
-      continue;
-    }
-    if (p.access_counter) {
-      seen0 = __reduce_or_sync(0xffffffffu, seen0);
-      seen1 = __reduce_or_sync(0xffffffffu, seen1);
-      int32_t* ctr = p.access_counter + (int64_t)b * p.access_stride_b + (int64_t)hkv * p.access_stride_h;
-      if ((seen0 >> lane & 1) && in.mark[0] >= 0 && in.mark[0] < p.access_n) ctr[in.mark[0]] = 1;
-      if ((seen1 >> lane & 1) && in.mark[1] >= 0 && in.mark[1] < p.access_n) ctr[in.mark[1]] = 1;
-    }
-    break;
+      if (p.access_counter) {
+        seen0 = __reduce_or_sync(0xffffffffu, seen0);
+        seen1 = __reduce_or_sync(0xffffffffu, seen1);
+        int32_t* ctr = p.access_counter + (int64_t)b * p.access_stride_b + (int64_t)hkv * p.access_stride_h;
+        if ((seen0 >> lane & 1) && in.mark[0] >= 0 && in.mark[0] < p.access_n) ctr[in.mark[0]] = 1;
+        if ((seen1 >> lane & 1) && in.mark[1] >= 0 && in.mark[1] < p.access_n) ctr[in.mark[1]] = 1;
+      }
+      break;
     }
     __syncwarp();
   }

@@ -162,7 +162,7 @@ def hip_attention_12_sequence_sharded(q: Tensor, shard_kv: Sequence[Tuple], args
         calls.append((gi, m, qq, k, v, a, po[j0:j1].view(m * B, 1, H, D), pl[j0:j1].view(m * B, 1, H)))
     # The groups are independent and each is a chain of short launches: the largest runs on the current stream, the others
     # beside it (eight shards of 131072 tokens: 0.53 ms one after the other, 0.35 ms).  The query's position is the last
-    # key's, which the operator writes itself.
+    # key's, which the operator writes itself (`shared`: at every replay of a captured call too).
     calls.sort(key=lambda c: -c[1])
     fork = ops.fork(q) if len(calls) > 1 else None
     try:

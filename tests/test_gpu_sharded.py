@@ -54,6 +54,26 @@ def test_shards_with_tables_of_either_integer_type():
     assert len(got) == 3 and torch.equal(out, ref) and all(torch.equal(a.indices, b.indices) for a, b in zip(got, mds))
 
 
+def test_sharded_step_under_graph_capture():
+    """The calls beside the current stream, their fork and their join in one CUDA graph: replays on new queries equal eager calls."""
+    from hip_attention_b200.sharded import hip_attention_12_sequence_sharded
+    S, L = 8, 4096
+    w, q, paged, _, args = _problem(S, L)
+    how = dict(n_shards=S, shard_len=L, per_shard_k=256)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        hip_attention_12_sequence_sharded(q, paged, args, **how)
+    torch.cuda.synchronize()
+    graph, static = torch.cuda.CUDAGraph(), q.clone()
+    with torch.cuda.graph(graph):
+        out, mds = hip_attention_12_sequence_sharded(static, paged, args, **how)
+    for seed in (1, 2):
+        static.copy_(torch.randn(q.shape, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda", dtype=q.dtype) * 0.1)
+        graph.replay()
+        ref, ref_mds = hip_attention_12_sequence_sharded(static, paged, args, **how)
+        assert torch.equal(out, ref) and all(torch.equal(a.indices, b.indices) for a, b in zip(mds, ref_mds))
+
+
 def test_partly_filled_sequence():
     """A sequence that ends inside shard 5: the window moves to that shard, its position follows its live length,
     shards 6 and 7 contribute nothing; the page-pool form and the form with dense slices of the live lengths agree."""
