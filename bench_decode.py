@@ -225,7 +225,7 @@ def run(a, w, dev, rank, world, triton=False):
             "phases_ms": {"refresh_step": ph_refresh, "cached_step": ph_cached},
             # The bytes counted are the key rows the scan kernels request: the stages with small chunks fetch every
             # token of an active chunk once for the heads of a KV head, the others two rows per chunk, head and round.
-            "roofline": {"kernel": "scan_stage_kernel + scan_chunks_strict_kernel (refresh steps)", "bound": "hbm",
+            "roofline": {"kernel": "scan_stage_kernel + scan_chunks_mma_kernel (refresh steps)", "bound": "hbm",
                          "achieved": scan_gbs, "peak": peak, "peak_source": peak_src,
                          "unit": "GB/s", "frac": scan_gbs / peak if scan_gbs else None, "traffic": None,
                          "algorithmic_bytes_per_refresh": fetched,

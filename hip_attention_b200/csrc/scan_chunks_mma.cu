@@ -133,7 +133,6 @@ __global__ void __launch_bounds__(128, MODE == HIPATTN_ROPE_NONE || F8 ? 4 : 3)
   const uint32_t kscale2 = pack_scalar2<DT>(p.k_scale);
   // this lane's columns of a product: heads (lane % 4) * 2 and + 1
   const int col = (lane & 3) * 2;
-  const uint32_t real_columns = (col < heads ? 0x55555555u : 0u) | (col + 1 < heads ? 0xaaaaaaaau : 0u);   // bits of `unsure`
   // (1.05: the magnitudes are summed in packed 16-bit arithmetic, at most 16 terms each)
   const float eps0 = kEps * 1.05f * s_qmax[col], eps1 = kEps * 1.05f * s_qmax[col + 1];
   const int check_tab = 4 * NV * HB * kTabStride;   // check mode: tables of the raw products and their radii follow
@@ -407,9 +406,6 @@ __global__ void __launch_bounds__(128, MODE == HIPATTN_ROPE_NONE || F8 ? 4 : 3)
           }
         }
       }
-      // A column beyond the heads has neither a table nor a query row.  Its bounds differ where a key's product or magnitude
-      // is not finite (0 * inf is not a number), so it is taken off the list here.
-      unsure &= real_columns;
       __syncwarp();
     }
     // One lane per (chunk, head) replays the search on the bounds.  Where they leave a comparison or a chunk's best score
@@ -419,6 +415,10 @@ __global__ void __launch_bounds__(128, MODE == HIPATTN_ROPE_NONE || F8 ? 4 : 3)
     for (;;) {
       if (exact) {
         // ---- the uncertain scores by the strict definition, one per lane ----
+        // (A column beyond the heads has neither a table nor a query row.  Its bounds differ where a key's product or magnitude
+        // is not finite - 0 * inf is not a number -, so it is taken off the list here: bit 0 of an accumulator's number is its
+        // column.)
+        unsure &= (col < heads ? 0x55555555u : 0u) | (col + 1 < heads ? 0xaaaaaaaau : 0u);
         while (__any_sync(0xffffffffu, unsure != 0)) {
           const int mine = __popc(unsure);
           int at = mine;
