@@ -274,12 +274,14 @@ __global__ void __launch_bounds__(kWarps * 32, 1) bsa_decode_kernel(const hipatt
 // In-kernel RoPE: the key's pieces i and i + D / 64 hold elements d and d + D / 2, rotated in registers; the table pieces
 // travel with the rows.  fp8 rows are widened in registers.
 //
-// With RoPE or fp8 rows the softmax weights go in two 16-bit terms, the rounded weight and what the rounding left: the general
-// kernel, which served fp8 before, kept them in fp32; and a single term is exact for the largest weight of each warp's keys
-// only, so its error grows as fewer warps share a list (12 sequences with RoPE, bf16, error against 64 bits before the
-// output is rounded: 1.4e-4 with sixteen warps to a list, 1.8e-4 with the eight it has here, below 2e-5 with two terms, which
-// cost nothing beside the rotation).  Without RoPE there are six warps and more, not the four of the kernel before, and the
-// second products would cost 6 % of a full batch.
+// TWO = the softmax weights go in two 16-bit terms, the rounded weight and what the rounding left.  A single term is exact for
+// the largest weight of each warp's keys only, so its error grows as fewer warps share a list.  fp8 rows: always (the general
+// kernel, which served them before, kept the weights in fp32).  RoPE: always (12 sequences, bf16, error against 64 bits before
+// the output is rounded: 1.4e-4 with the sixteen warps to a list of the kernel before, 1.8e-4 with the eight here, below 2e-5
+// with two terms, which cost nothing beside the rotation).  Else: in clusters of two, whose twelve warps replace the twelve to
+// sixteen of the kernel before (12 sequences, bf16: 1.5e-4 then, 1.9e-4 with one term, 1e-6 with two, 49.4 -> 53.0 us a cached
+// call).  A single CTA has six warps and more where there were four, larger clusters have as many warps as there were: one term
+// (32 sequences: 2.5e-4 then, 2.4e-4 here; two terms would cost 6 % of a full batch).
 //
 // Bound: HBM.  32 sequences, 3328 keys each (436 MB): 0.115 ms with a three-stage shared-memory ring and a barrier per
 // 64 keys (3.8 TB/s), 0.080 ms here (5.4 TB/s).  One sequence: 10.8 + 4.7 us (attention, merge), 12.9 us here.  RoPE, 12 sequences:
@@ -312,14 +314,13 @@ __device__ __forceinline__ float ld_cluster(uint32_t addr) {
   return v;
 }
 
-template <int DT, int D, bool ROPE, bool F8>
+template <int DT, int D, bool ROPE, bool F8, bool TWO>
 __global__ void __launch_bounds__(kDecodeWarps<ROPE, F8> * 32, 2) bsa_decode_mma_kernel(const hipattn_bsa_params_t p, int cluster) {
   using T = typename Elem<DT>::type;
   constexpr int NL = D / 32;        // pieces of a K row per lane
   constexpr int NB = D / 64;        // 64-column blocks
   constexpr int MS = D + 2;
   constexpr int EB = F8 ? 1 : 2;
-  constexpr bool TWO = F8 || ROPE;  // softmax weights in two 16-bit terms
   constexpr int kDW = kDecodeWarps<ROPE, F8>;
   using Raw = typename std::conditional<F8, uint2, uint4>::type;
   extern __shared__ __align__(16) float s_merge[];   // [kDW][G][MS], then the CTA's own result [G][MS]
@@ -667,12 +668,18 @@ int launch_mma(const hipattn_bsa_params_t& p, cudaStream_t stream) {
   // powers of two count: with 4 for the 40 units of five sequences, where 7 fit, 24 warps shared a list instead of 42, and
   // the error of their single-term weights was 1.2 to 1.3 times as large.
   const int64_t keys = (p.sink < p.T ? p.sink : p.T) + (int64_t)p.K * p.block_size_k + (p.window < p.T ? p.window : p.T);
-  auto kern = bsa_decode_mma_kernel<DT, D, ROPE, F8>;
+  auto kern = bsa_decode_mma_kernel<DT, D, ROPE, F8, F8 || ROPE>;
   HIPATTN_CUDA_OK(allow_smem((const void*)kern, smem));
   int64_t most = 148 * 2 / units;
   if (most > keys / p.n_splits / (kDW * 16)) most = keys / p.n_splits / (kDW * 16);
   int cluster = most < 1 ? 1 : (most > kMaxCluster ? kMaxCluster : (int)most);
   while (cluster > 1 && resident_clusters((const void*)kern, cluster, kDW * 32, smem) < units) --cluster;
+  if constexpr (!F8 && !ROPE) {
+    if (cluster == 2) {   // (see TWO)
+      kern = bsa_decode_mma_kernel<DT, D, ROPE, F8, true>;
+      HIPATTN_CUDA_OK(allow_smem((const void*)kern, smem));
+    }
+  }
   const int64_t grid = units * cluster;
   HIPATTN_REQUIRE(grid > 0 && grid < 0x7fffffffLL, HIPATTN_ERR_INVALID, "decode grid of %lld blocks", (long long)grid);
   cudaLaunchConfig_t cfg = {};

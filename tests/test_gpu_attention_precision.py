@@ -1,10 +1,11 @@
 """Attention whose softmax weights go through the tensor cores in two 16-bit terms, against 64 bits on the mask it used: what is
 left besides the rounding of the output itself is small.
 
-The bound: two terms keep 16 (bf16) or 22 (fp16) significant bits of a weight, and a score is a fp32 sum of 64 or 128
-products, so the context before it is rounded is within p = 1.5e-5 of the exact one, relative; the rounding of the output
-alone is r = 1.6e-3 (bf16) or 2.0e-4 (fp16).  The two add in quadrature: sqrt(1 + (p / r)^2) r < 1.003 r.  With single 16-bit
-weights p is 6e-5 to 2.7e-4 and the sum 1.006 r to 1.1 r."""
+The bound: two terms keep 16 (bf16) or 22 (fp16) significant bits of a weight, 1.5e-5 or 2.4e-7, and a score is a fp32 sum of 64
+or 128 products, good to a few 1e-6 after the exponential: the context before it is rounded is within p = 4e-5 (bf16) or 8e-6
+(fp16) of the exact one, relative.  The rounding of the output alone is r = 1.6e-3 or 2.0e-4, and the two add in quadrature:
+sqrt(1 + (p / r)^2) r < 1.0005 r and 1.001 r.  With single 16-bit weights p is 1e-4 to 9e-4 in bf16 and 1.2e-5 to 1e-4 in fp16, and
+the sum 1.0018 r to 1.08 r on all of these shapes but the ones a whole cluster or fp32 weights served."""
 import pytest
 import torch
 
@@ -49,6 +50,8 @@ def _exact(q, k, v, md, rows, w, tables):
     dict(TQ=130, T=9001, D=64, bq=128),                      # one head, 128 rows
     dict(TQ=1, T=20011, D=128, bq=64, fp8=True),             # decode, a list shared by a whole cluster
     dict(TQ=1, T=20011, D=64, bq=64, rope=True),
+    dict(TQ=1, T=20011, D=128, bq=64, B=12, H=32, HKV=8),    # by two CTAs
+    dict(TQ=1, T=20011, D=64, bq=64, B=12, H=32, HKV=8),
     dict(TQ=1, T=5003, D=128, bq=64, B=40, rope=True),       # by one CTA
     dict(TQ=1, T=5003, D=128, bq=64, B=40, H=16, rope=True, fp8=True),   # eight heads per KV head
 ])
@@ -77,4 +80,4 @@ def test_error_is_the_rounding_of_the_output(shape, dtype):
     err = (out[[b for b, _, _ in rows], [r for _, r, _ in rows]].double() - ref).norm().item()
     rounding = (ref.to(dt).double() - ref).norm().item()
     print(f"{shape} {dtype}: error {err / ref.norm().item():.4e}, rounding alone {rounding / ref.norm().item():.4e}, ratio {err / rounding:.4f}")
-    assert err <= 1.003 * rounding
+    assert err <= (1.0005 if dtype == "bf16" else 1.001) * rounding
