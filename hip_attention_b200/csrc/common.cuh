@@ -136,18 +136,18 @@ __device__ __forceinline__ const char* token_row(const hipattn_tokens_t& tk, int
 
 // Access statistics: 1 at the position (dense) or page (paged: the block-table entry, page 0 beyond the sequence) of
 // token t in counter [B, HKV, n] (uvm_gpu_cache.py:846-909 stores the same 1 on every load).
+// access_index: the index of token t, which the counter may not have.
+__device__ __forceinline__ int64_t access_index(const hipattn_tokens_t& tk, int b, int64_t t) {
+  if (tk.cache == nullptr) return t;
+  const int64_t seq = tk.seq_lens_is_i64 ? ((const int64_t*)tk.cache_seq_lens)[b] : (int64_t)((const int32_t*)tk.cache_seq_lens)[b];
+  const int64_t pi = (int)t / tk.page_size;
+  if (!(t >= 0 && t < seq && pi < tk.table_width)) return 0;
+  const int64_t o = (int64_t)b * tk.table_stride_b + pi;
+  return tk.table_is_i64 ? ((const int64_t*)tk.block_table)[o] : (int64_t)((const int32_t*)tk.block_table)[o];
+}
 __device__ __forceinline__ void mark_access(int32_t* counter, int64_t stride_b, int64_t stride_h, int n, const hipattn_tokens_t& tk,
                                             int b, int hkv, int64_t t) {
-  int64_t i = t;
-  if (tk.cache != nullptr) {
-    const int64_t seq = tk.seq_lens_is_i64 ? ((const int64_t*)tk.cache_seq_lens)[b] : (int64_t)((const int32_t*)tk.cache_seq_lens)[b];
-    const int64_t pi = (int)t / tk.page_size;
-    i = 0;
-    if (t >= 0 && t < seq && pi < tk.table_width) {
-      const int64_t o = (int64_t)b * tk.table_stride_b + pi;
-      i = tk.table_is_i64 ? ((const int64_t*)tk.block_table)[o] : (int64_t)((const int32_t*)tk.block_table)[o];
-    }
-  }
+  const int64_t i = access_index(tk, b, t);
   if (i >= 0 && i < n) counter[(int64_t)b * stride_b + (int64_t)hkv * stride_h + i] = 1;
 }
 

@@ -579,6 +579,8 @@ int scan_prepare_keys(const hipattn_tokens_t& k, int dtype, int D, int B, int T,
                   : launch_prepare<HIPATTN_F16, 8>(k, B, T, HKV, k_scale, key_abs, k_scaled, status, rope, last_pos, reach, stream);
 }
 
+int scan_query_tiles(const hipattn_scan_params_t& p, cudaStream_t stream, bool* handled);
+
 // Takes 16-bit prefill shapes (16 to 128 pooled rows in multiples of 16, head dim 64 or 128) when the
 // caller supplies the prepared keys; anything else is left to the other scan kernels.
 int scan_stage_tcgen05(const hipattn_scan_params_t& p, cudaStream_t stream, bool* handled) {
@@ -594,6 +596,10 @@ int scan_stage_tcgen05(const hipattn_scan_params_t& p, cudaStream_t stream, bool
   if (p.rope_mode == HIPATTN_ROPE_STREAMING && !(p.k_scaled_sides == 1 && p.D == 128)) return HIPATTN_OK;
   const char* v = getenv("HIPATTN_SCAN_KERNEL");
   if (v && strcmp(v, "mma") == 0) return HIPATTN_OK;
+  if (!(v && strcmp(v, "rounds") == 0)) {   // (for comparisons)
+    const int rc = scan_query_tiles(p, stream, handled);
+    if (*handled) return rc;
+  }
   *handled = true;
   if (p.dtype == HIPATTN_BF16) return p.D == 128 ? dispatch_rows<HIPATTN_BF16, 128>(p, stream) : dispatch_rows<HIPATTN_BF16, 64>(p, stream);
   return p.D == 128 ? dispatch_rows<HIPATTN_F16, 128>(p, stream) : dispatch_rows<HIPATTN_F16, 64>(p, stream);

@@ -1,0 +1,115 @@
+"""Prefill scans that score whole tiles of keys: masks, later stages' lists and access counters equal the strict kernel's, where every
+bound is settled at once and where strict scores are needed."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = {
+    "heads4": dict(T=9001, TQ=1100),                                                   # 4 heads x 64 rows: a full accumulator
+    "heads4_d64": dict(T=6007, TQ=1217, D=64, dtype="fp16"),
+    "heads8_rows16": dict(T=5003, TQ=2100, H=8, HKV=1, strides=[4, 4, 4]),             # half of an accumulator
+    "heads8_rows128": dict(T=9001, TQ=2200, H=16, bq=128),                             # two passes, two CTAs a unit
+    "heads20": dict(T=5003, TQ=1030, H=20, HKV=1),                                     # a CTA with part of its heads
+    "heads3": dict(T=5003, TQ=1030, H=6),
+    "heads2_rows128": dict(T=7001, TQ=2200, H=4, bq=128, B=2),
+    "odd_sink": dict(T=5003, TQ=1100, sink=101),                                       # narrowed bounds per head
+    "short_window": dict(T=4099, TQ=1100, sink=64, sw=128),                            # chunks that end beyond the keys
+    "few_kept": dict(T=2049, TQ=1100, keep=[1024, 512, 256], sw=512, sink=0),
+}
+
+
+def problem(shape, keys, rope):
+    import bench
+    from cases import rope_tables
+    w = dict(bench.WORKLOADS["prefill_128k"], H=8, HKV=2, keep=[4096, 1024, 512])
+    w.update(SHAPES[shape])
+    q, k, v = bench.make_qkv(w, "cuda")
+    g = torch.Generator(device="cuda").manual_seed(5)
+    if keys == "close":      # neighbours that are equal or one unit in the last place apart
+        n = w["T"] // 2
+        k[:, 1:2 * n:2] = k[:, 0:2 * n:2]
+        k.view(torch.int16)[:, 1::4, :, 3] ^= 1
+    elif keys == "not_finite":
+        q[:, :, 0] = 0
+        for value in (float("inf"), float("-inf"), float("nan")):
+            k[:, torch.randint(0, w["T"], (w["T"] // 100,), generator=g, device="cuda"), :, 5] = value
+        t = torch.randint(0, w["T"], (w["T"] // 50,), generator=g, device="cuda")
+        k[:, t] = torch.where(k[:, t] > 0, 5e4, -5e4).to(k.dtype)
+    kw = {}
+    if rope:
+        cos, sin = rope_tables(w["T"] + 8, w["D"], w["theta"])
+        kw = dict(using_extend=True, need_apply_rope=True, rope_cos=torch.from_numpy(cos).cuda(), rope_sin=torch.from_numpy(sin).cuda(),
+                  scan_extend_backend=rope)
+    args = bench.make_args(w, **kw)
+    args.require_cache_statistics = True
+    return (q, k, v), args
+
+
+@pytest.mark.parametrize("rope", [None, "relative"])
+@pytest.mark.parametrize("keys", ["random", "close", "not_finite"])
+@pytest.mark.parametrize("shape", list(SHAPES))
+def test_masks_equal_strict(shape, keys, rope, monkeypatch):
+    from hip_attention_b200 import hip_attention_impl
+    qkv, args = problem(shape, keys, rope)
+    md = {}
+    for mode in ("auto", "strict"):
+        monkeypatch.setenv("HIPATTN_SCAN_MODE", mode)
+        md[mode] = hip_attention_impl(*qkv, args)[1]
+    a, b = md["auto"], md["strict"]
+    for i, (x, y) in enumerate(zip(a.stage_caches[1:], b.stage_caches[1:])):
+        assert torch.equal(x.indices_left, y.indices_left) and torch.equal(x.indices_right, y.indices_right), f"stage {i + 1}"
+    assert torch.equal(a.indices, b.indices) and torch.equal(a.ks, b.ks)
+    assert torch.equal(a.mask_cache_statistics.access_counter, b.mask_cache_statistics.access_counter)
+
+
+@pytest.mark.parametrize("keys", ["random", "close", "not_finite"])
+@pytest.mark.parametrize("shape", ["heads4", "heads8_rows128", "heads20", "heads3", "odd_sink", "short_window"])
+def test_bounds_and_scores_per_head_equal_strict(shape, keys, monkeypatch):
+    from hip_attention_b200 import hip_attention_impl
+    qkv, args = problem(shape, keys, None)
+    got = {}
+    stats = torch.zeros(4, dtype=torch.int64, device="cuda")
+    for mode in ("auto", "strict", "check"):
+        monkeypatch.setenv("HIPATTN_SCAN_MODE", mode)
+        dbg = {"scan_stats": stats} if mode == "check" else {}
+        hip_attention_impl(*qkv, args, debug=dbg)
+        got[mode] = dbg["stages"]
+    for mode in ("auto", "check"):
+        for i, (a, b) in enumerate(zip(got[mode], got["strict"])):
+            for key in ("left", "right", "score", "score_max"):
+                assert torch.equal(a[key], b[key]), f"{mode} stage {i} {key}"
+    assert int(stats[2]) == 0, "a score taken without the strict definition is wrong"
+
+
+@pytest.mark.parametrize("rope", [None, "relative"])
+@pytest.mark.parametrize("change", ["longer", "shorter", "moved", "shuffled"])
+def test_restart_from_lists_of_a_callers_own(change, rope, monkeypatch):
+    """Chunks that are longer than the stage's size, empty, off the grid, in no order: each restarted stage as in strict mode."""
+    from hip_attention_b200 import HiPAttentionOutputMetadata, hip_attention_impl
+    from hip_attention_b200.metadata import HiPAttentionStageInputCache
+    qkv, args = problem("heads4", "random", rope)
+    md = hip_attention_impl(*qkv, args)[1]
+    caches = list(md.stage_caches)
+    for stage in (1, 2):
+        c = caches[stage]
+        l, r = c.indices_left.clone(), c.indices_right.clone()
+        if change == "longer":
+            r[..., ::3] += 13
+        elif change == "shorter":
+            r[..., ::2] = torch.maximum(l[..., ::2], r[..., ::2] - 5)
+            r[..., ::7] = l[..., ::7]
+        elif change == "moved":
+            l, r = (l + 3).clamp(max=8990), (r + 3).clamp(max=8999)
+        else:
+            p = torch.randperm(l.shape[-1], device="cuda")
+            l, r = l[..., p], r[..., p]
+        got = {}
+        for mode in ("auto", "strict"):
+            monkeypatch.setenv("HIPATTN_SCAN_MODE", mode)
+            # (a call completes the list of stage inputs that it is given)
+            part = HiPAttentionOutputMetadata(None, None, None, None, None, None, caches[:stage] + [HiPAttentionStageInputCache(l, r, c.out_scores)])
+            got[mode] = hip_attention_impl(*qkv, args, cached_metadata=part)[1]
+        a, b = got["auto"], got["strict"]
+        assert torch.equal(a.indices, b.indices) and torch.equal(a.ks, b.ks), f"stage {stage}"
+        assert torch.equal(a.mask_cache_statistics.access_counter, b.mask_cache_statistics.access_counter), f"stage {stage}"
