@@ -15,7 +15,7 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libhipattn_sm100.so")
 HOST = os.path.join(PKG, "_host.so")   # CPython extension: the host path of a call, linked to LIB
-SOURCES = ["capi.cu", "scan_stage.cu", "scan_stage_mma.cu", "scan_stage_tcgen05.cu", "scan_query_tiles.cu", "scan_chunks_strict.cu", "scan_chunks_mma.cu", "select.cu", "bsa_generic.cu", "bsa_mma.cu", "bsa_fp32.cu", "bsa_tcgen05.cu", "bsa_decode.cu", "decode_noalloc.cu", "host_kernels.cu"]
+SOURCES = ["capi.cu", "scan_stage.cu", "scan_stage_mma.cu", "scan_stage_tcgen05.cu", "scan_query_tiles.cu", "scan_key_tiles.cu", "scan_chunks_strict.cu", "scan_chunks_mma.cu", "select.cu", "bsa_generic.cu", "bsa_mma.cu", "bsa_fp32.cu", "bsa_tcgen05.cu", "bsa_decode.cu", "decode_noalloc.cu", "host_kernels.cu"]
 HEADERS = ["common.cuh", "host_kernels.h", "bsa_common.cuh", "scan_common.cuh", "scan_tiles.cuh", "mma_common.cuh", "tcgen05_common.cuh", "rope.cuh", os.path.join("..", "..", "include", "hipattn.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "--use_fast_math=false"]

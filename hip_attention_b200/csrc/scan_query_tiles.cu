@@ -107,9 +107,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) scan_query_tiles_kernel(const
 #pragma unroll
       for (int e = 0; e < 8; ++e) m = fmaxf(m, fabsf(v[e]));
       // the pieces of a warp belong to one head: 32 divides a head's R * PIECES pieces
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-      if (lane == 0) atomicMax(&s_qmax[hh], __float_as_int(m));   // non-negative floats order as ints
+      const int top = __reduce_max_sync(0xffffffffu, __float_as_int(m));   // (non-negative floats order as ints)
+      if (lane == 0) atomicMax(&s_qmax[hh], top);
     };
     const int total = heads * R * PIECES;
     if (p.stride_q == 1 && p.rope_mode == HIPATTN_ROPE_NONE) {
@@ -411,7 +410,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) scan_query_tiles_kernel(const
           const float so_far = decode_score(code);
           int off = cc * CHUNK;
           asked = 0;
-          bool closed = search_whole<DT, 1, CHUNK>(tab + g * kTabStride, 0, off, slo, shi, asked);
+          bool closed = search_whole<DT, CHUNK>(tab + g * kTabStride, off, slo, shi, asked);
           if (!valid) slo = shi = HIPATTN_SCORE_INIT;
           else seen |= asked;
           float best = fmaxf(slo, so_far);
@@ -439,12 +438,11 @@ __global__ void __launch_bounds__(kTileThreads, 1) scan_query_tiles_kernel(const
           t.known = decode_score(__shfl_sync(0xffffffffu, known, cc * CHUNK));
           t.valid = cw < CPW && g < ng && c0 + cc < n;
           t.pt = pt;
-          t.rounds = 0;
           t.tab = tab + g * kTabStride;
           t.slo = compared ? slo : HIPATTN_SCORE_INIT;
           t.shi = compared ? shi : HIPATTN_SCORE_INIT;
-          search_chunks<DT, 1, CHUNK>(t, p.T, 0, NG, compared, p.score_out != nullptr,
-              [&](int tk, int, int owner) { return strict_of(tk, (w0 + owner) % NG); },
+          search_chunks<DT, CHUNK>(t, p.T, NG, compared, p.score_out != nullptr,
+              [&](int tk, int owner) { return strict_of(tk, (w0 + owner) % NG); },
               [&](int tk) { if (counting) mark_access(p.access_counter, p.access_stride_b, p.access_stride_h, p.access_n, p.k, b, hkv, tk); });
           const int h = head0 + j * NG + g, c = c0 + cc;
           if (t.valid) {

@@ -1,8 +1,8 @@
 // Search of whole chunks on score bounds: the part that the tensor-core scans which score every token of a chunk share
-// (scan_query_tiles.cu).
+// (scan_query_tiles.cu, scan_key_tiles.cu).
 //
 // A warp holds the scores of 32 consecutive rows of a key tile (TMEM lanes) against some groups of pooled queries (a group = the
-// pooled rows of one head and query block), as bounds lo <= rounded score <= hi packed in one word per (side, group, row) in
+// pooled rows of one head and query block), as bounds lo <= rounded score <= hi packed in one word per (group, row) in
 // shared memory.  One lane per (chunk, group) replays the halving search of the reference (attention_extend.py:413-1249) on
 // the bounds; where they leave a comparison open, or the chunk's best score uncertain, the lane asks for the strict score of
 // one key and the whole warp computes it, so that bounds and scores are those of the strict kernel.
@@ -12,7 +12,7 @@
 
 namespace hipattn {
 
-constexpr int kTabStride = 33;   // words of a (side, group): 32 rows, the odd stride spreads the banks
+constexpr int kTabStride = 33;   // words of a group: 32 rows, the odd stride spreads the banks
 
 // largest of three
 __device__ __forceinline__ float max3(float a, float b, float c) {
@@ -68,7 +68,7 @@ __device__ __forceinline__ bool mbar_test(uint32_t mbar, uint32_t parity) {
                : "=r"(done) : "r"(mbar), "r"(parity) : "memory");
   return done != 0;
 }
-__device__ __noinline__ bool mbar_wait_slow(uint32_t mbar, uint32_t parity, volatile int* abort_flag, uint32_t* status) {
+static __device__ __noinline__ bool mbar_wait_slow(uint32_t mbar, uint32_t parity, volatile int* abort_flag, uint32_t* status) {
   return mbar_wait(mbar, parity, abort_flag, status);
 }
 __device__ __forceinline__ bool mbar_wait_quick(uint32_t mbar, uint32_t parity, volatile int* abort_flag, uint32_t* status) {
@@ -81,15 +81,15 @@ __device__ __forceinline__ bool mbar_wait_quick(uint32_t mbar, uint32_t parity, 
 // The search of a lane's chunk where every chunk of the warp is whole and active to its last token, as all of a step's chunks but
 // the last few are: rounds without conditions.  Returns false where a comparison is open; slo / shi: bounds of the best
 // winner.  off: the first row on entry, the row that is left on return.
-template <int DT, int NV, int CHUNK>
-__device__ __forceinline__ bool search_whole(const uint32_t* tab, int side_words, int& off, float& slo, float& shi, uint32_t& seen) {
+template <int DT, int CHUNK>
+__device__ __forceinline__ bool search_whole(const uint32_t* tab, int& off, float& slo, float& shi, uint32_t& seen) {
   bool open = false;
   slo = shi = HIPATTN_SCORE_INIT;
 #pragma unroll
-  for (int s = CHUNK; s >= (NV == 2 ? 1 : 2); s >>= 1) {
+  for (int s = CHUNK; s >= 2; s >>= 1) {
     const int il = off + s / 4, ir = off + s / 2 + s / 4;
     seen |= 1u << il | 1u << ir;
-    const uint32_t bl = tab[il], br = tab[(NV - 1) * side_words + ir];
+    const uint32_t bl = tab[il], br = tab[ir];
     const float llo = lo_f32<DT>(bl), lhi = hi_f32<DT>(bl), rlo = lo_f32<DT>(br), rhi = hi_f32<DT>(br);
     const bool win = llo > rhi;
     open |= !win && !(lhi <= rlo);
@@ -106,18 +106,17 @@ struct ChunkTask {
   bool valid;            // the lane has a task
   int l, r;              // the chunk's bounds; the search narrows them
   int pt;                // chunks that begin beyond pt are not active
-  int rounds;            // halving rounds, where a key has a score per side
   int first;             // token of the chunk's first row in the table
   int row0;              // that row
   float known;           // a score that the chunk has for certain (of any head)
-  uint32_t* tab;         // bounds of this group, left candidates (right ones: + side_words)
+  uint32_t* tab;         // bounds of this group
   float score;           // result: the chunk's score
   float slo, shi;        // bounds of the best winner, where the comparisons are settled already
   uint32_t seen;         // result: rows that the rounds ask for
   bool out_of_range;     // result: a round asked for a token beyond the keys
 };
 
-// Runs the searches of a warp, whatever its chunks are like.  strict(token, side, owner) is called by the whole warp with uniform
+// Runs the searches of a warp, whatever its chunks are like.  strict(token, owner) is called by the whole warp with uniform
 // arguments and returns the strict score, before rounding, of a token for the group of lane `owner`; mark(token) records a token
 // outside the table's rows (of a chunk longer than CHUNK, which only a caller's own list can hold).
 //
@@ -125,8 +124,8 @@ struct ChunkTask {
 // upper bound exceeds every certain one of its chunk, those of other CTAs' heads included (`every`: a chunk's score is wanted
 // for each head).  A strict score costs a warp more than the whole search, and the slowest of the four warps of an accumulator
 // sets the pace.
-template <int DT, int NV, int CHUNK, typename Strict, typename Mark>
-__device__ __forceinline__ void search_chunks(ChunkTask& t, int T, int side_words, int width, bool settled, bool every, Strict strict, Mark mark) {
+template <int DT, int CHUNK, typename Strict, typename Mark>
+__device__ __forceinline__ void search_chunks(ChunkTask& t, int T, int width, bool settled, bool every, Strict strict, Mark mark) {
   const int lane = threadIdx.x & 31;
   const int l0 = t.l, r0 = t.r;
   float slo = t.slo, shi = t.shi;
@@ -149,19 +148,19 @@ __device__ __forceinline__ void search_chunks(ChunkTask& t, int T, int side_word
     }
     const bool mine = live;
     const bool big = r0 - l0 > CHUNK;
-    int wl = l0, wr = r0, it = 0, tl = 0, tr = 0;
-    bool loaded = false;
+    int wl = l0, wr = r0, tl = 0, tr = 0;
+    bool loaded = false, first = true;
     float llo = 0.f, lhi = 0.f, rlo = 0.f, rhi = 0.f, nlo = HIPATTN_SCORE_INIT, nhi = HIPATTN_SCORE_INIT;
     for (;;) {
       int need = -1;   // side of the key whose strict score is wanted
       while (live) {
         const int mid = (wl + wr) >> 1;
         if (!loaded) {
-          if (!(wl < wr && wl <= t.pt && wl >= 0 && (NV == 2 ? it < t.rounds : it == 0 || wr - wl > 1))) {
+          if (!(wl < wr && wl <= t.pt && wl >= 0 && (first || wr - wl > 1))) {
             live = false;
             break;
           }
-          ++it;
+          first = false;
           tl = (wl + mid) >> 1;
           tr = (mid + wr) >> 1;
           t.out_of_range |= tr >= T;
@@ -174,14 +173,13 @@ __device__ __forceinline__ void search_chunks(ChunkTask& t, int T, int side_word
             // (tokens beyond the keys are the last one, whose row a chunk that begins beyond them holds throughout)
             const int il = t.row0 + max(0, min(tl, T - 1) - t.first), ir = t.row0 + max(0, min(tr, T - 1) - t.first);
             t.seen |= 1u << il | 1u << ir;
-            const uint32_t bl = t.tab[il], br = t.tab[(NV - 1) * side_words + ir];
+            const uint32_t bl = t.tab[il], br = t.tab[ir];
             llo = lo_f32<DT>(bl); lhi = hi_f32<DT>(bl);
             rlo = lo_f32<DT>(br); rhi = hi_f32<DT>(br);
           }
           loaded = true;
         }
-        // a key does not beat itself (where it has a score per side, the other side's is another candidate)
-        const bool same = NV == 1 && tl == tr;
+        const bool same = tl == tr;   // a key does not beat itself
         const bool win = llo > rhi && !same;
         const float wlo = win ? llo : rlo, whi = win ? lhi : rhi;
         if (!win && !(lhi <= rlo) && !same) {   // open: the left key's score first, where it is not certain
@@ -204,11 +202,11 @@ __device__ __forceinline__ void search_chunks(ChunkTask& t, int T, int side_word
         todo &= todo - 1;
         const int side = __shfl_sync(0xffffffffu, need, owner);
         const int tk = min(__shfl_sync(0xffffffffu, need == 0 ? tl : tr, owner), T - 1);
-        const float raw = strict(tk, NV == 2 ? side : 0, owner);
+        const float raw = strict(tk, owner);
         if (lane == owner) {
           const float ex = Elem<DT>::round(raw);
           if (side == 0) llo = lhi = ex; else rlo = rhi = ex;
-          if (!big) t.tab[(NV == 2 && side ? side_words : 0) + t.row0 + max(0, tk - t.first)] = pack2<DT>(ex, ex);
+          if (!big) t.tab[t.row0 + max(0, tk - t.first)] = pack2<DT>(ex, ex);
         }
       }
     }

@@ -5,17 +5,21 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
+# (the second stage's kernel wants 64 / heads query blocks for a chunk of the first)
 SHAPES = {
-    "heads4": dict(T=9001, TQ=1100),                                                   # 4 heads x 64 rows: a full accumulator
-    "heads4_d64": dict(T=6007, TQ=1217, D=64, dtype="fp16"),
+    "heads4": dict(T=9001, TQ=2300),                                                   # 4 heads x 64 rows: a full accumulator
+    "heads4_d64": dict(T=6007, TQ=1517, D=64, dtype="fp16"),
     "heads8_rows16": dict(T=5003, TQ=2100, H=8, HKV=1, strides=[4, 4, 4]),             # half of an accumulator
     "heads8_rows128": dict(T=9001, TQ=2200, H=16, bq=128),                             # two passes, two CTAs a unit
     "heads20": dict(T=5003, TQ=1030, H=20, HKV=1),                                     # a CTA with part of its heads
     "heads3": dict(T=5003, TQ=1030, H=6),
     "heads2_rows128": dict(T=7001, TQ=2200, H=4, bq=128, B=2),
-    "odd_sink": dict(T=5003, TQ=1100, sink=101),                                       # narrowed bounds per head
+    "heads2": dict(T=3000, TQ=3000, H=4, sw=256, sink=0),
+    "heads1": dict(T=4500, TQ=4500, H=2, sw=256, sink=0, keep=[8192, 1024, 512]),
+    "chunks512": dict(T=9001, TQ=2300, chunks=[512, 32, 8], keep=[8192, 1024, 512]),   # two tiles of keys a chunk
+    "odd_sink": dict(T=5003, TQ=1410, sink=101),                                       # narrowed bounds per head
     "short_window": dict(T=4099, TQ=1100, sink=64, sw=128),                            # chunks that end beyond the keys
-    "few_kept": dict(T=2049, TQ=1100, keep=[1024, 512, 256], sw=512, sink=0),
+    "few_kept": dict(T=2049, TQ=2049, keep=[1536, 512, 256], sw=512, sink=0),
 }
 
 
