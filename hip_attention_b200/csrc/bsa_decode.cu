@@ -655,10 +655,13 @@ __global__ void __launch_bounds__(kDecodeWarps<ROPE, F8> * 32, 2) bsa_decode_mma
     }
     cluster_sync();   // no CTA leaves while another reads its shared memory
   }
+  // Launched beside the kernel before it: that one has ended, and its writes are visible, before this one ends, so that what follows
+  // on the stream finds both (nothing to wait for otherwise).
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
 }
 
 template <int DT, int D, bool ROPE, bool F8>
-int launch_mma(const hipattn_bsa_params_t& p, cudaStream_t stream) {
+int launch_mma(const hipattn_bsa_params_t& p, cudaStream_t stream, bool beside) {
   constexpr int kDW = kDecodeWarps<ROPE, F8>;
   const int G = p.H / p.HKV;
   const size_t smem = sizeof(float) * (size_t)(kDW + 1) * G * (D + 2);
@@ -687,20 +690,24 @@ int launch_mma(const hipattn_bsa_params_t& p, cudaStream_t stream) {
   cfg.blockDim = dim3(kDW * 32);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = (unsigned)cluster;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  // Beside the copies of the cached mask, which the launch before makes for the caller and the attention does not read: a cached call
+  // of one sequence 18.5 -> 16.0 us, of 32 sequences 86.3 -> 84.8.
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = beside ? 2 : 1;
   HIPATTN_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, p, cluster));
   return check_launch("bsa_decode_mma_kernel");
 }
 
 template <int DT, int D>
-int dispatch_mma(const hipattn_bsa_params_t& p, cudaStream_t stream) {
-  if (p.k.fp8_e5m2) return p.rope_cos ? launch_mma<DT, D, true, true>(p, stream) : launch_mma<DT, D, false, true>(p, stream);
-  return p.rope_cos ? launch_mma<DT, D, true, false>(p, stream) : launch_mma<DT, D, false, false>(p, stream);
+int dispatch_mma(const hipattn_bsa_params_t& p, cudaStream_t stream, bool beside) {
+  if (p.k.fp8_e5m2) return p.rope_cos ? launch_mma<DT, D, true, true>(p, stream, beside) : launch_mma<DT, D, false, true>(p, stream, beside);
+  return p.rope_cos ? launch_mma<DT, D, true, false>(p, stream, beside) : launch_mma<DT, D, false, false>(p, stream, beside);
 }
 
 template <int DT, int LPR, int G>
@@ -747,12 +754,12 @@ bool decode_on_tensor_cores(const hipattn_bsa_params_t& p) {
 
 // Decode shapes: one query row; what the tensor-core kernel does not take, with 1 / 2 / 4 / 8 query heads per KV head and K / V
 // rows of 128, 256 or 512 bytes.
-int bsa_decode(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled) {
+int bsa_decode(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled, bool beside) {
   *handled = false;
   if (decode_on_tensor_cores(p)) {
     *handled = true;
-    if (p.dtype == HIPATTN_BF16) return p.D == 128 ? dispatch_mma<HIPATTN_BF16, 128>(p, stream) : dispatch_mma<HIPATTN_BF16, 64>(p, stream);
-    return p.D == 128 ? dispatch_mma<HIPATTN_F16, 128>(p, stream) : dispatch_mma<HIPATTN_F16, 64>(p, stream);
+    if (p.dtype == HIPATTN_BF16) return p.D == 128 ? dispatch_mma<HIPATTN_BF16, 128>(p, stream, beside) : dispatch_mma<HIPATTN_BF16, 64>(p, stream, beside);
+    return p.D == 128 ? dispatch_mma<HIPATTN_F16, 128>(p, stream, beside) : dispatch_mma<HIPATTN_F16, 64>(p, stream, beside);
   }
   // an fp8 cache and in-kernel RoPE: only the tensor-core kernel above; the rest is the general kernel's
   if (p.TQ != 1 || p.k.fp8_e5m2 || p.v.fp8_e5m2 || p.rope_cos) return HIPATTN_OK;

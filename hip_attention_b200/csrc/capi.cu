@@ -97,7 +97,7 @@ int validate_tokens(const hipattn_tokens_t& t, int elem_bytes, int D, const char
 int bsa_generic(const hipattn_bsa_params_t& p, cudaStream_t stream);
 int bsa_mma(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled);
 int bsa_fp32(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled);
-int bsa_decode(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled);
+int bsa_decode(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled, bool beside);
 int bsa_tcgen05(const hipattn_bsa_params_t& p, cudaStream_t stream, bool* handled);
 int64_t bsa_tcgen05_ctas(const hipattn_bsa_params_t& p, int* resident, int* tile_keys);
 bool decode_on_tensor_cores(const hipattn_bsa_params_t& p);
@@ -226,7 +226,9 @@ extern "C" int hipattn_mark_attention_access(const hipattn_bsa_params_t* p, int3
   return check_launch("mark_attention_access_kernel");
 }
 
-extern "C" int hipattn_bsa_attention(const hipattn_bsa_params_t* p, void* stream) {
+extern "C" int hipattn_bsa_attention(const hipattn_bsa_params_t* p, void* stream) { return hipattn::bsa_attention(p, (cudaStream_t)stream, false); }
+
+int hipattn::bsa_attention(const hipattn_bsa_params_t* p, cudaStream_t stream, bool beside) {
   HIPATTN_REQUIRE(p != nullptr, HIPATTN_ERR_INVALID, "attention params are null");
   HIPATTN_REQUIRE(p->q && p->pos && p->indices && p->ks && p->status, HIPATTN_ERR_INVALID,
                   "attention: q, pos, indices, ks and status are required");
@@ -260,17 +262,17 @@ extern "C" int hipattn_bsa_attention(const hipattn_bsa_params_t* p, void* stream
   // In-kernel RoPE: the mma.sync decode and prefill kernels and (head dim 128) the tcgen05 prefill kernel.  An fp8 KV
   // cache: the tcgen05 prefill kernel.  What none of them takes is the general kernel's.
   bool handled = false;
-  rc = bsa_decode(*p, (cudaStream_t)stream, &handled);
+  rc = bsa_decode(*p, stream, &handled, beside);
   if (handled) return rc;
   if (tcgen05_prefill()) {
-    rc = bsa_tcgen05(*p, (cudaStream_t)stream, &handled);
+    rc = bsa_tcgen05(*p, stream, &handled);
     if (handled) return rc;
   }
-  rc = bsa_mma(*p, (cudaStream_t)stream, &handled);
+  rc = bsa_mma(*p, stream, &handled);
   if (handled) return rc;
-  rc = bsa_fp32(*p, (cudaStream_t)stream, &handled);
+  rc = bsa_fp32(*p, stream, &handled);
   if (handled) return rc;
-  return bsa_generic(*p, (cudaStream_t)stream);
+  return bsa_generic(*p, stream);
 }
 
 // Key ranges for hipattn_bsa_attention.

@@ -371,8 +371,8 @@ struct Copies {
     s.dst_s[0] = n[1] * n[2]; s.dst_s[1] = n[2]; s.dst_s[2] = 1;
     add(s);
   }
-  void flush() {
-    if (list.count) check(hipattn::multi_copy(list, stream), "multi_copy");
+  void flush(bool early = false) {
+    if (list.count) check(hipattn::multi_copy(list, stream, early), "multi_copy");
     list.count = 0;
   }
 };
@@ -813,6 +813,7 @@ Mask estimate_mask(Call& c, const hipattn_tokens_t& ktok, int64_t first, at::Ten
 struct AttentionArgs {
   int64_t window, block_k, bsa_bq, index_bq;
   bool heads_share, decode, want_lse, own_mask;
+  bool beside;   // the launch before is an early multi_copy that the attention does not depend on
   float softcap;
 };
 
@@ -874,7 +875,7 @@ void attention(Call& c, const hipattn_tokens_t& ktok, const hipattn_tokens_t& vt
                                   lse.defined() ? lse.data_ptr<float>() : nullptr, c.TQ * c.H, out.stride(0), c.stream), "merge_partials");
   } else {
     bp.lse_out = lse.defined() ? lse.data_ptr<float>() : nullptr;
-    check(hipattn_bsa_attention(&bp, c.stream), "bsa_attention");
+    check(hipattn::bsa_attention(&bp, c.stream, a.beside), "bsa_attention");
   }
 }
 
@@ -1055,8 +1056,8 @@ PyObject* forward(PyObject* const* argv) {
     miss = all.as_strided({c.B, c.HKV, slots}, {0, 0, 0}, sets * per);
   }
 
-  at::Tensor indices, ks, ks_count, kse;
-  bool heads_share;
+  at::Tensor indices, ks, ks_count, kse, read_indices, read_ks;
+  bool heads_share, copies_first = false;
   int64_t index_bq;
   Ref bsq = attr(c.args, N.block_sparse_block_size_q);
   int64_t bsa_bq = bsq.none() ? bq : as_int(bsq);
@@ -1121,7 +1122,12 @@ PyObject* forward(PyObject* const* argv) {
       indices = like(ci, at::kLong); ks = like(cks, at::kLong); ks_count = like(ckc, ckc.scalar_type()); kse = like(cse, cse.scalar_type());
       Copies cp(c.stream);
       cp.add(ci, indices); cp.add(cks, ks); cp.add(ckc, ks_count); cp.add(cse, kse);
-      cp.flush();
+      // A decode call's attention may read the mask that it was given and run beside the copies, as long as nothing else comes
+      // between the two on the stream.
+      copies_first = cp.list.count > 0 && c.TQ == 1 && ci.scalar_type() == at::kLong && cks.scalar_type() == at::kLong && ci.stride(2) == 1 &&
+                     v_ready == Py_None && c.debug == Py_None && !sa_stats.defined();
+      if (copies_first) { read_indices = ci; read_ks = cks; }
+      cp.flush(copies_first);
     } else {
       indices = ci.clone().to(at::kLong).contiguous(); ks = cks.clone().to(at::kLong).contiguous(); ks_count = ckc.clone(); kse = cse.clone();
       if (indices.device() != c.q.device() || ks.device() != c.q.device()) VALUE_ERROR("cached metadata is on another device than q");
@@ -1150,6 +1156,7 @@ PyObject* forward(PyObject* const* argv) {
   Ref cap = attr(c.args, N.logit_softcap);
   a.softcap = cap.none() ? 0.f : (float)PyFloat_AsDouble(cap.get());
   if (PyErr_Occurred()) throw PyError{};
+  a.beside = copies_first && a.decode;
   c.mark("start");
   if (v_ready != Py_None) {
     Ref dev = checked(PyLong_FromLong(c.q.device().index()));
@@ -1158,7 +1165,7 @@ PyObject* forward(PyObject* const* argv) {
   }
   if (lse.defined() && (lse.scalar_type() != at::kFloat || lse.numel() != c.B * c.TQ * c.H || !lse.is_contiguous()))
     VALUE_ERROR("lse must be a contiguous float32 tensor [B, TQ, H]");
-  attention(c, ktok, vtok, indices, ks, a, sa_stats, context, lse);
+  attention(c, ktok, vtok, a.beside ? read_indices : indices, a.beside ? read_ks : ks, a, sa_stats, context, lse);
   c.mark("attention");
 
   if (fresh && cdiv(c.TQ, bsa_bq) != BDST) {

@@ -124,7 +124,10 @@ __device__ __forceinline__ float load_float(const CopySeg& s, int64_t at) {
   }
 }
 
+// EARLY: a kernel behind this one that was launched for it (hipattn::bsa_attention, beside) may begin at once.
+template <bool EARLY>
 __global__ void multi_copy_kernel(const CopyList list) {
+  if (EARLY) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   const CopySeg& s = list.seg[blockIdx.y];
   const int64_t total = s.n0 * s.n1 * s.n2;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -204,7 +207,7 @@ int zero_memory(void* ptr, int64_t bytes, cudaStream_t stream) {
   return HIPATTN_OK;
 }
 
-int multi_copy(const CopyList& list, cudaStream_t stream) {
+int multi_copy(const CopyList& list, cudaStream_t stream, bool early) {
   int64_t most = 0;
   for (int i = 0; i < list.count; ++i) {
     const CopySeg& s = list.seg[i];
@@ -218,7 +221,8 @@ int multi_copy(const CopyList& list, cudaStream_t stream) {
   if (most <= 0) return HIPATTN_OK;
   int64_t grid = (most + 1023) / 1024;
   if (grid > 148 * 4) grid = 148 * 4;
-  multi_copy_kernel<<<dim3((unsigned)grid, (unsigned)list.count), 256, 0, stream>>>(list);
+  auto kern = early ? multi_copy_kernel<true> : multi_copy_kernel<false>;
+  kern<<<dim3((unsigned)grid, (unsigned)list.count), 256, 0, stream>>>(list);
   return check_launch("multi_copy_kernel");
 }
 

@@ -35,7 +35,11 @@ struct CopyList {
   CopySeg seg[kMaxCopies];
   int count;
 };
-int multi_copy(const CopyList& list, cudaStream_t stream);
+int multi_copy(const CopyList& list, cudaStream_t stream, bool early = false);
+
+// hipattn_bsa_attention; beside: the launch before this one on the stream is a multi_copy with `early` whose outputs the attention does
+// not read, and the two may run side by side (decode on the tensor cores; other kernels wait for the copies as usual).
+int bsa_attention(const hipattn_bsa_params_t* p, cudaStream_t stream, bool beside);
 
 // Largest query position of every batch element, clamped to [0, 2^30): q_pos [B, TQ], or pos0 + TQ - 1 when q_pos is null.
 struct QueryPositions {
