@@ -63,7 +63,7 @@ WORKLOADS = {
 _DT = {"bf16": torch.bfloat16, "fp16": torch.float16, "fp32": torch.float32}
 # dram__bytes_read.sum + dram__bytes_write.sum per scan launch (mean of the three stages) from one ncu capture of
 # this command; a capture is valid for the (workload, GPUs, queries) it was taken on only, hence the key
-NCU_DRAM_BYTES_PER_SCAN_LAUNCH = {("prefill_128k", 1, 32768): (563160320 + 582162688 + 357693696) / 3}
+NCU_DRAM_BYTES_PER_SCAN_LAUNCH = {("prefill_128k", 1, 32768): (568252672 + 320165376 + 360078592) / 3}
 NCU_TRAFFIC_SOURCE = "ncu capture (dram__bytes_read.sum + dram__bytes_write.sum), prefill_128k, 1 GPU, 32768 queries only"
 
 
@@ -129,9 +129,9 @@ def oracle_config(w: dict):
 
 def scan_bytes(w: dict, heads: int, fetched: bool = False) -> float:
     """Algorithmic bytes of the scan stages of one call: active chunks x (log2(chunk) + 1) rounds x 2 key
-    rows x D x element size, summed over (batch, query block, head, stage).  ``fetched``: the rows the kernels
-    actually gather -- a candidate that repeats the previous round's winner is not fetched again, which removes
-    three of the 2 (log2(chunk) + 1) rows of a chunk."""
+    rows x D x element size, summed over (batch, query block, head, stage).  ``fetched``: the rows that the
+    round-by-round kernels gather -- a candidate that repeats the previous round's winner is not fetched again, which
+    removes three of the 2 (log2(chunk) + 1) rows of a chunk."""
     eb = 4 if w["dtype"] == "fp32" else 2
     B, TQ, T, D, bq = w["B"], w["TQ"], w["T"], w["D"], w["bq"]
     c0 = w["chunks"][0]
@@ -596,7 +596,8 @@ def run_prefill(a, w, dev, rank, world):
                  "traffic_source": NCU_TRAFFIC_SOURCE if (a.workload, world, w["TQ"]) in NCU_DRAM_BYTES_PER_SCAN_LAUNCH else None,
                  "flops_per_launch": sf / max(1, n_scan), "launch_ms": scan_ms / max(1, n_scan),
                  "algorithm": "flops and bytes of the reference's rounds (two key rows per chunk, head and round); the "
-                              "kernels skip rows whose score is already known, see the *_executed figures",
+                              "*_executed and gather figures are those of the rounds without the rows whose score is known "
+                              "already; stages that score whole tiles of keys gather fewer bytes and multiply more",
                  "flops_executed_per_launch": scan_flops(w, heads_local, True) / max(1, n_scan),
                  "executed_tflops": scan_flops(w, heads_local, True) / 1e12 / (scan_ms / 1e3) if scan_ms > 0 else None,
                  "gathered_bytes_per_launch": scan_bytes(w, heads_local, True) / max(1, n_scan),
