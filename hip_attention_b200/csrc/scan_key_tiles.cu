@@ -190,8 +190,8 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
     // ---- pooled queries: one bulk copy per entry ----
     if (lane == 0) {
       const unsigned char* src = t.pooled + bh * BDST * entry_bytes;
-      int slot = 0, use = 0, next = __ldg(&entries[0].x);
-      for (int k = 0, e = 0; k < stages_total; ++k) {
+      int slot = 0, use = 0, next = __ldg(&entries[0].x), k = 0;
+      for (int e = 0; k < stages_total; ++k) {
         if (use > 0 && !mbar_wait_quick(smem_u32(&s_empty[slot]), (use - 1) & 1, &s_abort, p.status)) break;
         const int ne = min(EB, count - k * EB);
         const uint32_t bar = smem_u32(&s_full[slot]), dst = smem_u32(sQ) + slot * Q_STAGE;
@@ -204,6 +204,8 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
         }
         if (++slot == STAGES) { slot = 0; ++use; }
       }
+      if (*(volatile int*)&s_abort)
+        for (int i = max(0, k - STAGES); i < k; ++i) mbar_drain(smem_u32(&s_full[i % STAGES]), (i / STAGES) & 1);
     }
     __syncwarp();
   } else if (warp == 2 || warp == 3) {
@@ -211,8 +213,8 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
     const int acc = warp - 2;
     if (lane == 0) {
       const uint64_t da0 = make_desc(smem_u32(sA) + acc * A_TILE, 16, 1024), db0 = make_desc(smem_u32(sQ), 16, KB * 1024);
-      int slot = 0, use = 0, set = acc;
-      for (int k = 0; k < stages_total; ++k) {
+      int slot = 0, use = 0, set = acc, k = 0, last = 0;
+      for (; k < stages_total; ++k) {
         if (!mbar_wait_quick(smem_u32(&s_full[slot]), use & 1, &s_abort, p.status)) break;
         if (k > 0 && !mbar_wait_quick(smem_u32(&s_acce[acc]), (k - 1) & 1, &s_abort, p.status)) break;
         tc_fence_after();
@@ -222,12 +224,15 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
         for (int q = 0; q < D / 16; ++q)
           umma(tmem + acc * COLS, da0 + (uint64_t)(((q >> 2) * A_BLOCK + (q & 3) * 32) >> 4), db + (uint64_t)(((q >> 2) * 1024 + (q & 3) * 32) >> 4), idesc,
                q > 0 ? 1u : 0u);
-        umma_commit(smem_u32(&s_accf[set][acc]));
         umma_commit(smem_u32(&s_empty[slot]));
+        umma_commit(smem_u32(&s_accf[set][acc]));   // (last: the searches wait for it before the CTA may end)
+        last = set;
         set += 2;
         if (set >= kSearchSets) set -= kSearchSets;
         if (++slot == STAGES) { slot = 0; ++use; }
       }
+      // (every third accumulator of a thread is a set's)
+      if (*(volatile int*)&s_abort && k > 0) mbar_drain(smem_u32(&s_accf[last][acc]), ((k - 1) / kSearchSets) & 1);
     }
     __syncwarp();
   } else if (warp >= kFirstSearchWarp) {

@@ -231,7 +231,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) scan_query_tiles_kernel(const
         }
       };
       if (acc) advance();
-      for (int k = 0; it < mine; ++k) {
+      int k = 0, last = 0;
+      for (; it < mine; ++k) {
         if (!mbar_wait_quick(smem_u32(&s_full[slot]), use & 1, &s_abort, p.status)) break;
         if (k > 0 && !mbar_wait_quick(smem_u32(&s_acce[acc]), (k - 1) & 1, &s_abort, p.status)) break;
         tc_fence_after();
@@ -241,13 +242,16 @@ __global__ void __launch_bounds__(kTileThreads, 1) scan_query_tiles_kernel(const
         for (int q = 0; q < D / 16; ++q)
           umma(tmem + acc * COLS, da + (uint64_t)(((q >> 2) * A_BLOCK + (q & 3) * 32) >> 4),
                db + (uint64_t)(((q >> 2) * Q_BLOCK + (q & 3) * 32) >> 4), idesc, q > 0 ? 1u : 0u);
-        umma_commit(smem_u32(&s_accf[set][acc]));
         umma_commit(smem_u32(&s_empty[slot]));
+        umma_commit(smem_u32(&s_accf[set][acc]));   // (last: the searches wait for it before the CTA may end)
+        last = set;
         set += 2;
         if (set >= kSearchSets) set -= kSearchSets;
         advance();
         advance();
       }
+      // (every third accumulator of a thread is a set's)
+      if (*(volatile int*)&s_abort && k > 0) mbar_drain(smem_u32(&s_accf[last][acc]), ((k - 1) / kSearchSets) & 1);
     }
     __syncwarp();
   } else if (warp >= kFirstSearchWarp) {

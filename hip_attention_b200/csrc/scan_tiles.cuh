@@ -21,6 +21,15 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   return r;
 }
 
+// After a time-out: waits, with a limit of its own, for an operation that is in flight, so that a CTA leaves none behind.
+static __device__ __noinline__ void mbar_drain(uint32_t mbar, uint32_t parity) {
+  const long long t0 = clock64();
+  uint32_t done = 0;
+  while (!done && clock64() - t0 < kWaitCycles)
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+                 : "=r"(done) : "r"(mbar), "r"(parity) : "memory");
+}
+
 // Row maxima of a thread's accumulator columns: NG groups of R columns from column `taddr`, 64 columns per TMEM load.  Groups at
 // `ng` and beyond are skipped in steps of whole loads.
 template <int R, int NG>
