@@ -35,6 +35,7 @@ struct KeyTiles {
   const int2* entries;           // [B, n_grid, BDST]: query block, position of the chunk in its list of kept ones
   const int32_t* counts;         // [B, n_grid]
   int n_grid, sink, c_prev;      // chunks of the stage before: grid of c_prev tokens from `sink`
+  int tries;                     // wait_tries()
 };
 
 // ---- pooled queries of a (batch, KV head, query block), rows beyond the last one repeat the first ----
@@ -192,7 +193,7 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
       const unsigned char* src = t.pooled + bh * BDST * entry_bytes;
       int slot = 0, use = 0, next = __ldg(&entries[0].x), k = 0;
       for (int e = 0; k < stages_total; ++k) {
-        if (use > 0 && !mbar_wait_quick(smem_u32(&s_empty[slot]), (use - 1) & 1, &s_abort, p.status)) break;
+        if (use > 0 && !mbar_wait_quick(smem_u32(&s_empty[slot]), (use - 1) & 1, &s_abort, p.status, t.tries)) break;
         const int ne = min(EB, count - k * EB);
         const uint32_t bar = smem_u32(&s_full[slot]), dst = smem_u32(sQ) + slot * Q_STAGE;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(ne * entry_bytes) : "memory");
@@ -204,8 +205,7 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
         }
         if (++slot == STAGES) { slot = 0; ++use; }
       }
-      if (*(volatile int*)&s_abort)
-        for (int i = max(0, k - STAGES); i < k; ++i) mbar_drain(smem_u32(&s_full[i % STAGES]), (i / STAGES) & 1);
+      for (int i = max(0, k - STAGES); i < k; ++i) mbar_drain(smem_u32(&s_full[i % STAGES]), (i / STAGES) & 1);
     }
     __syncwarp();
   } else if (warp == 2 || warp == 3) {
@@ -215,8 +215,8 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
       const uint64_t da0 = make_desc(smem_u32(sA) + acc * A_TILE, 16, 1024), db0 = make_desc(smem_u32(sQ), 16, KB * 1024);
       int slot = 0, use = 0, set = acc, k = 0, last = 0;
       for (; k < stages_total; ++k) {
-        if (!mbar_wait_quick(smem_u32(&s_full[slot]), use & 1, &s_abort, p.status)) break;
-        if (k > 0 && !mbar_wait_quick(smem_u32(&s_acce[acc]), (k - 1) & 1, &s_abort, p.status)) break;
+        if (!mbar_wait_quick(smem_u32(&s_full[slot]), use & 1, &s_abort, p.status, t.tries)) break;
+        if (k > 0 && !mbar_wait_quick(smem_u32(&s_acce[acc]), (k - 1) & 1, &s_abort, p.status, t.tries)) break;
         tc_fence_after();
         const uint32_t idesc = make_idesc(DT == HIPATTN_BF16 ? 1 : 0, 128, min(EB, count - k * EB) * Gq * R, 0);
         const uint64_t db = db0 + (uint64_t)((slot * Q_STAGE) >> 4);
@@ -225,14 +225,14 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
           umma(tmem + acc * COLS, da0 + (uint64_t)(((q >> 2) * A_BLOCK + (q & 3) * 32) >> 4), db + (uint64_t)(((q >> 2) * 1024 + (q & 3) * 32) >> 4), idesc,
                q > 0 ? 1u : 0u);
         umma_commit(smem_u32(&s_empty[slot]));
-        umma_commit(smem_u32(&s_accf[set][acc]));   // (last: the searches wait for it before the CTA may end)
+        umma_commit(smem_u32(&s_accf[set][acc]));   // (last: waited for before the role ends)
         last = set;
         set += 2;
         if (set >= kSearchSets) set -= kSearchSets;
         if (++slot == STAGES) { slot = 0; ++use; }
       }
       // (every third accumulator of a thread is a set's)
-      if (*(volatile int*)&s_abort && k > 0) mbar_drain(smem_u32(&s_accf[last][acc]), ((k - 1) / kSearchSets) & 1);
+      if (k > 0) mbar_drain(smem_u32(&s_accf[last][acc]), ((k - 1) / kSearchSets) & 1);
     }
     __syncwarp();
   } else if (warp >= kFirstSearchWarp) {
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
       const int ng = min(EB, count - (u >> 1) * EB) * Gq;
       const int l = base + acc * 128 + quarter * 32;   // the warp's chunk: CHUNK tokens from here
       const bool valid = walker && cur.d >= 0;
-      ok = __all_sync(0xffffffffu, mbar_wait_quick(smem_u32(&s_accf[set][acc]), phase >> acc & 1, &s_abort, p.status));
+      ok = __all_sync(0xffffffffu, mbar_wait_quick(smem_u32(&s_accf[set][acc]), phase >> acc & 1, &s_abort, p.status, t.tries));
       if (!ok) break;
       phase ^= 1u << acc;
       tc_fence_after();
@@ -439,7 +439,7 @@ int scan_key_tiles(const hipattn_scan_params_t& p, int sink, int c_prev, void* s
   int32_t* last = (int32_t*)take((int64_t)p.B * BDST * 4);
   int2* entries = (int2*)take((int64_t)p.B * n_grid * BDST * 8);
   int32_t* counts = (int32_t*)take((int64_t)p.B * n_grid * 4);
-  const KeyTiles t{pooled, q_max, last, entries, counts, n_grid, sink, c_prev};
+  const KeyTiles t{pooled, q_max, last, entries, counts, n_grid, sink, c_prev, wait_tries()};
   if (p.dtype == HIPATTN_BF16)
     return p.D == 128 ? run<HIPATTN_BF16, 128>(p, t, pooled, q_max, last, entries, counts, stream) : run<HIPATTN_BF16, 64>(p, t, pooled, q_max, last, entries, counts, stream);
   return p.D == 128 ? run<HIPATTN_F16, 128>(p, t, pooled, q_max, last, entries, counts, stream) : run<HIPATTN_F16, 64>(p, t, pooled, q_max, last, entries, counts, stream);

@@ -33,6 +33,7 @@ struct QueryTiles {
   int stages;        // key tiles in the ring
   int split;         // CTAs that share out the key tiles
   int check;
+  int tries;         // wait_tries()
 };
 
 template <int DT, int D, int R>
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) scan_query_tiles_kernel(const
           cp_async_wait<0>();
           report();
         }
-        ok = __all_sync(0xffffffffu, mbar_wait_quick(smem_u32(&s_empty[slot]), (use - 1) & 1, &s_abort, p.status));
+        ok = __all_sync(0xffffffffu, mbar_wait_quick(smem_u32(&s_empty[slot]), (use - 1) & 1, &s_abort, p.status, cfg.tries));
         if (!ok) break;
       }
       const uint32_t dst = sA_u32 + slot * A_STAGE;
@@ -233,8 +234,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) scan_query_tiles_kernel(const
       if (acc) advance();
       int k = 0, last = 0;
       for (; it < mine; ++k) {
-        if (!mbar_wait_quick(smem_u32(&s_full[slot]), use & 1, &s_abort, p.status)) break;
-        if (k > 0 && !mbar_wait_quick(smem_u32(&s_acce[acc]), (k - 1) & 1, &s_abort, p.status)) break;
+        if (!mbar_wait_quick(smem_u32(&s_full[slot]), use & 1, &s_abort, p.status, cfg.tries)) break;
+        if (k > 0 && !mbar_wait_quick(smem_u32(&s_acce[acc]), (k - 1) & 1, &s_abort, p.status, cfg.tries)) break;
         tc_fence_after();
         const uint32_t idesc = make_idesc(DT == HIPATTN_BF16 ? 1 : 0, 128, min(NG, heads - j * NG) * R, 0);
         const uint64_t da = da0 + (uint64_t)((slot * A_STAGE) >> 4), db = db0 + (uint64_t)((j * Q_PASS) >> 4);
@@ -243,7 +244,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) scan_query_tiles_kernel(const
           umma(tmem + acc * COLS, da + (uint64_t)(((q >> 2) * A_BLOCK + (q & 3) * 32) >> 4),
                db + (uint64_t)(((q >> 2) * Q_BLOCK + (q & 3) * 32) >> 4), idesc, q > 0 ? 1u : 0u);
         umma_commit(smem_u32(&s_empty[slot]));
-        umma_commit(smem_u32(&s_accf[set][acc]));   // (last: the searches wait for it before the CTA may end)
+        umma_commit(smem_u32(&s_accf[set][acc]));   // (last: waited for before the role ends)
         last = set;
         set += 2;
         if (set >= kSearchSets) set -= kSearchSets;
@@ -251,7 +252,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) scan_query_tiles_kernel(const
         advance();
       }
       // (every third accumulator of a thread is a set's)
-      if (*(volatile int*)&s_abort && k > 0) mbar_drain(smem_u32(&s_accf[last][acc]), ((k - 1) / kSearchSets) & 1);
+      if (k > 0) mbar_drain(smem_u32(&s_accf[last][acc]), ((k - 1) / kSearchSets) & 1);
     }
     __syncwarp();
   } else if (warp >= kFirstSearchWarp) {
@@ -319,7 +320,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) scan_query_tiles_kernel(const
       float eps[NG];   // radius per unit of key magnitude
 #pragma unroll
       for (int g = 0; g < NG; ++g) eps[g] = s_eps[j * NG + g];
-      ok = __all_sync(0xffffffffu, mbar_wait_quick(smem_u32(&s_accf[set][acc]), phase >> acc & 1, &s_abort, p.status));
+      ok = __all_sync(0xffffffffu, mbar_wait_quick(smem_u32(&s_accf[set][acc]), phase >> acc & 1, &s_abort, p.status, cfg.tries));
       if (!ok) break;
       phase ^= 1u << acc;
       tc_fence_after();
@@ -507,6 +508,7 @@ int launch(const hipattn_scan_params_t& p, cudaStream_t stream) {
   const TilePlan plan = plan_tiles(p);
   QueryTiles cfg;
   cfg.check = p.mode == HIPATTN_SCAN_CHECK ? 1 : 0;
+  cfg.tries = wait_tries();
   cfg.passes = plan.passes;
   cfg.head_groups = plan.head_groups;
   // (an even number of slots: with one pass a tile, a slot's phases are then all waited for by one of the two MMA threads)

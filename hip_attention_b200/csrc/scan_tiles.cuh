@@ -7,6 +7,9 @@
 // the bounds; where they leave a comparison open, or the chunk's best score uncertain, the lane asks for the strict score of
 // one key and the whole warp computes it, so that bounds and scores are those of the strict kernel.
 #pragma once
+#include <cstdlib>
+#include <cstring>
+
 #include "scan_common.cuh"
 #include "tcgen05_common.cuh"
 
@@ -21,7 +24,8 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   return r;
 }
 
-// After a time-out: waits, with a limit of its own, for an operation that is in flight, so that a CTA leaves none behind.
+// At the end of a role: waits, with a limit of its own, for what the role issued last, so that a CTA leaves nothing in flight however
+// its other roles ended (a role that has issued all it had may be gone before another one's wait runs out).
 static __device__ __noinline__ void mbar_drain(uint32_t mbar, uint32_t parity) {
   const long long t0 = clock64();
   uint32_t done = 0;
@@ -77,14 +81,24 @@ __device__ __forceinline__ bool mbar_test(uint32_t mbar, uint32_t parity) {
                : "=r"(done) : "r"(mbar), "r"(parity) : "memory");
   return done != 0;
 }
-static __device__ __noinline__ bool mbar_wait_slow(uint32_t mbar, uint32_t parity, volatile int* abort_flag, uint32_t* status) {
-  return mbar_wait(mbar, parity, abort_flag, status);
+// (tries: wait_tries(); with none of them a barrier that is not ready counts as a wait that ran out)
+static __device__ __noinline__ bool mbar_wait_slow(uint32_t mbar, uint32_t parity, volatile int* abort_flag, uint32_t* status, int tries) {
+  if (tries > 0) return mbar_wait(mbar, parity, abort_flag, status);
+  if (mbar_test(mbar, parity)) return true;
+  *abort_flag = 1;
+  atomicOr(status, HIPATTN_STATUS_TIMEOUT);
+  return false;
 }
-__device__ __forceinline__ bool mbar_wait_quick(uint32_t mbar, uint32_t parity, volatile int* abort_flag, uint32_t* status) {
+__device__ __forceinline__ bool mbar_wait_quick(uint32_t mbar, uint32_t parity, volatile int* abort_flag, uint32_t* status, int tries) {
 #pragma unroll 1
-  for (int i = 0; i < 64; ++i)
+  for (int i = 0; i < tries; ++i)
     if (mbar_try(mbar, parity)) return true;
-  return mbar_wait_slow(mbar, parity, abort_flag, status);
+  return mbar_wait_slow(mbar, parity, abort_flag, status, tries);
+}
+// HIPATTN_SCAN_WAIT=none lets a test take the kernels' ways out of a wait that has run out.
+inline int wait_tries() {
+  const char* v = getenv("HIPATTN_SCAN_WAIT");
+  return v && strcmp(v, "none") == 0 ? 0 : 64;
 }
 
 // The search of a lane's chunk where every chunk of the warp is whole and active to its last token, as all of a step's chunks but

@@ -117,3 +117,22 @@ def test_restart_from_lists_of_a_callers_own(change, rope, monkeypatch):
         a, b = got["auto"], got["strict"]
         assert torch.equal(a.indices, b.indices) and torch.equal(a.ks, b.ks), f"stage {stage}"
         assert torch.equal(a.mask_cache_statistics.access_counter, b.mask_cache_statistics.access_counter), f"stage {stage}"
+
+
+def test_waits_that_run_out_are_reported_and_leave_nothing(monkeypatch):
+    """Every wait of both kernels that is not over at once counts as one that ran out: the call ends, says so, and the next one, which
+    needs all of the tensor memory, is right."""
+    from hip_attention_b200 import _lib, hip_attention_impl, read_status
+    qkv, args = problem("heads4", "random", None)
+    read_status("cuda")
+    want = hip_attention_impl(*qkv, args)[1]
+    assert read_status("cuda") == 0
+    for _ in range(3):
+        monkeypatch.setenv("HIPATTN_SCAN_WAIT", "none")
+        hip_attention_impl(*qkv, args)
+        torch.cuda.synchronize()
+        assert read_status("cuda") & _lib.STATUS_TIMEOUT
+        monkeypatch.delenv("HIPATTN_SCAN_WAIT")
+        md = hip_attention_impl(*qkv, args)[1]
+        assert read_status("cuda") == 0
+        assert torch.equal(md.indices, want.indices) and torch.equal(md.ks, want.ks)
