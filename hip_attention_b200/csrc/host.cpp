@@ -745,8 +745,14 @@ Mask estimate_mask(Call& c, const hipattn_tokens_t& ktok, int64_t first, at::Ten
     c.mark("start");
     // (a caller's own list, which a restart begins with, may hold a chunk twice, and so may what is selected from it)
     const int64_t scratch_bytes = i > 0 && first == 0 ? hipattn::scan_key_tiles_scratch(sp, (int)c.sink, (int)c.stages[i - 1].chunk) : 0;
+    at::Tensor scratch;
     if (scratch_bytes > 0) {
-      at::Tensor scratch = dv.empty({scratch_bytes}, at::kByte);
+      try {
+        scratch = dv.empty({scratch_bytes}, at::kByte);
+      } catch (const c10::OutOfMemoryError&) {   // the general scan needs none
+      }
+    }
+    if (scratch.defined()) {
       check(hipattn::scan_key_tiles(sp, (int)c.sink, (int)c.stages[i - 1].chunk, scratch.data_ptr(), c.stream), ("scan_stage[" + std::to_string(i) + "]").c_str());
     } else {
       check(hipattn_scan_stage(&sp, c.stream), ("scan_stage[" + std::to_string(i) + "]").c_str());

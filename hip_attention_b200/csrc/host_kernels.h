@@ -87,8 +87,8 @@ int select_stage(const int32_t* score_max, const int32_t* left, int64_t rows, in
                  int64_t* next_right64, cudaStream_t stream);
 
 // The scan stage for a list that select_stage has made, from whole chunks of c_prev tokens on the grid from `sink`, each at most once in
-// a row (few pooled rows, see scan_key_tiles.cu).  scratch: device memory of scan_key_tiles_scratch bytes; 0 bytes where the
-// stage is hipattn_scan_stage's.
+// a row (few pooled rows, see scan_key_tiles.cu).  scratch: device memory of scan_key_tiles_scratch bytes, at most 128 MB
+// or what one query block needs; 0 bytes where the stage is hipattn_scan_stage's.
 int64_t scan_key_tiles_scratch(const hipattn_scan_params_t& p, int sink, int c_prev);
 int scan_key_tiles(const hipattn_scan_params_t& p, int sink, int c_prev, void* scratch, cudaStream_t stream);
 

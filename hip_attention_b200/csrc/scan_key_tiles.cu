@@ -28,12 +28,14 @@ constexpr int kThreads = (kFirstSearchWarp + kSearchWarps) * 32;
 constexpr int kRows = 16, kChunk = 32;   // pooled rows of a head, tokens of a chunk
 constexpr int kTile = 256;               // tokens of a CTA
 
+// A launch takes a slice of the query blocks, nd of them from d0 on, of nb sequences from b0 on.
 struct KeyTiles {
-  const unsigned char* pooled;   // [B, HKV, BDST][rows / 8][D / 64][8 rows][128 B], swizzled; rows = heads of a KV head x pooled rows
-  const float* q_max;            // [B, H, BDST] largest |pooled query|
-  const int32_t* last;           // [B, BDST] chunks that begin beyond this position are not active
-  const int2* entries;           // [B, n_grid, BDST]: query block, position of the chunk in its list of kept ones
-  const int32_t* counts;         // [B, n_grid]
+  unsigned char* pooled;         // [nb, HKV, nd][rows / 8][D / 64][8 rows][128 B], swizzled; rows = heads of a KV head x pooled rows
+  float* q_max;                  // [nb, H, nd] largest |pooled query|
+  int32_t* last;                 // [nb, nd] chunks that begin beyond this position are not active
+  int2* entries;                 // [nb, n_grid, nd]: query block of the slice, position of the chunk in its list of kept ones
+  int32_t* counts;               // [nb, n_grid]
+  int b0, nb, d0, nd;
   int n_grid, sink, c_prev;      // chunks of the stage before: grid of c_prev tokens from `sink`
   int tries;                     // wait_tries()
 };
@@ -42,18 +44,18 @@ struct KeyTiles {
 // (All query rows of a piece are requested before the first is added up: one after the other 150 us for the 268 MB of the 128k
 // prefill, 61 here.)
 template <int DT, int D>
-__global__ void __launch_bounds__(256) pool_queries_kernel(const hipattn_scan_params_t p, unsigned char* pooled, float* q_max, int32_t* last) {
+__global__ void __launch_bounds__(256) pool_queries_kernel(const hipattn_scan_params_t p, const KeyTiles kt) {
   using T = typename Elem<DT>::type;
   constexpr int PIECES = D / 8, KB = D / 64, BATCH = 4;
-  const int Gq = p.H / p.HKV, BDST = cdiv(p.TQ, p.block_size_q);
+  const int Gq = p.H / p.HKV;
   int64_t bid = blockIdx.x;
-  const int d = (int)(bid % BDST); bid /= BDST;
-  const int hkv = (int)(bid % p.HKV), b = (int)(bid / p.HKV);
-  const int t0 = d * p.block_size_q, Rv = min(kRows, (p.TQ - t0 + p.stride_q - 1) / p.stride_q);
+  const int d = (int)(bid % kt.nd); bid /= kt.nd;
+  const int hkv = (int)(bid % p.HKV), bl = (int)(bid / p.HKV), b = kt.b0 + bl;
+  const int t0 = (kt.d0 + d) * p.block_size_q, Rv = min(kRows, (p.TQ - t0 + p.stride_q - 1) / p.stride_q);
   __shared__ int s_max[16];
   if (threadIdx.x < 16) s_max[threadIdx.x] = 0;
   __syncthreads();
-  unsigned char* dst = pooled + (((int64_t)b * p.HKV + hkv) * BDST + d) * Gq * kRows * D * 2;
+  unsigned char* dst = kt.pooled + (((int64_t)bl * p.HKV + hkv) * kt.nd + d) * Gq * kRows * D * 2;
   for (int i = threadIdx.x; i < Gq * kRows * PIECES; i += 256) {
     const int pc = i % PIECES, rr = i / PIECES, hh = rr / kRows, r = rr % kRows;
     const int t = t0 + (r < Rv ? r : 0) * p.stride_q;
@@ -87,26 +89,25 @@ __global__ void __launch_bounds__(256) pool_queries_kernel(const hipattn_scan_pa
   }
   if (threadIdx.x < 32 && hkv == 0) {
     const int m = block_min_position(p, b, t0, Rv, threadIdx.x);
-    if (threadIdx.x == 0) last[b * BDST + d] = max(m - p.scan_window, 0);
+    if (threadIdx.x == 0) kt.last[bl * kt.nd + d] = max(m - p.scan_window, 0);
   }
   __syncthreads();
-  if (threadIdx.x < Gq) q_max[((int64_t)b * p.H + hkv * Gq + threadIdx.x) * BDST + d] = __int_as_float(s_max[threadIdx.x]);
+  if (threadIdx.x < Gq) kt.q_max[((int64_t)bl * p.H + hkv * Gq + threadIdx.x) * kt.nd + d] = __int_as_float(s_max[threadIdx.x]);
 }
 
 // ---- the query blocks whose list holds a chunk of the grid, and where; blocks it is not active for are left out ----
-__global__ void __launch_bounds__(256) list_queries_kernel(const int32_t* __restrict__ left, int n, int per, int BDST, int n_grid, int sink, int c_prev,
-                                                           const int32_t* __restrict__ last, int2* entries, int32_t* counts) {
-  const int g = blockIdx.x % n_grid, b = blockIdx.x / n_grid;
-  const int want = sink + g * c_prev, kept = n / per, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(256) list_queries_kernel(const int32_t* __restrict__ left, int n, int per, int BDST, const KeyTiles kt) {
+  const int g = blockIdx.x % kt.n_grid, bl = blockIdx.x / kt.n_grid;
+  const int want = kt.sink + g * kt.c_prev, kept = n / per, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   __shared__ int s_warp[8];
-  int2* out = entries + ((int64_t)b * n_grid + g) * BDST;
+  int2* out = kt.entries + ((int64_t)bl * kt.n_grid + g) * kt.nd;
   int total = 0;
-  for (int d0 = 0; d0 < BDST; d0 += 256) {
+  for (int d0 = 0; d0 < kt.nd; d0 += 256) {
     const int d = d0 + threadIdx.x;
     int lo = 0;
     bool in = false;
-    if (d < BDST && want <= __ldg(last + b * BDST + d)) {
-      const int32_t* row = left + ((int64_t)b * BDST + d) * n;   // the kept chunks ascend; each is `per` entries
+    if (d < kt.nd && want <= __ldg(kt.last + bl * kt.nd + d)) {
+      const int32_t* row = left + ((int64_t)(kt.b0 + bl) * BDST + kt.d0 + d) * n;   // the kept chunks ascend; each is `per` entries
       int hi = kept;
       while (lo < hi) {
         const int mid = (lo + hi) >> 1;
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(256) list_queries_kernel(const int32_t* __rest
     total += all;
     __syncthreads();
   }
-  if (threadIdx.x == 0) counts[b * n_grid + g] = total;
+  if (threadIdx.x == 0) kt.counts[bl * kt.n_grid + g] = total;
 }
 
 template <int DT, int D>
@@ -153,13 +154,13 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
   int64_t bid = blockIdx.x;
   const int part = (int)(bid % parts); bid /= parts;
   const int gi = (int)(bid % t.n_grid); bid /= t.n_grid;
-  const int hkv = (int)(bid % p.HKV), b = (int)(bid / p.HKV);
-  const int count = __ldg(t.counts + b * t.n_grid + gi);
+  const int hkv = (int)(bid % p.HKV), bl = (int)(bid / p.HKV), b = t.b0 + bl;
+  const int count = __ldg(t.counts + bl * t.n_grid + gi);
   if (count == 0) return;
   const int base = t.sink + gi * t.c_prev + part * kTile;   // the CTA's first token
-  const int2* entries = t.entries + ((int64_t)b * t.n_grid + gi) * BDST;
+  const int2* entries = t.entries + ((int64_t)bl * t.n_grid + gi) * t.nd;
   const int stages_total = cdiv(count, EB);
-  const int64_t bh = (int64_t)b * p.HKV + hkv;
+  const int64_t bh = (int64_t)b * p.HKV + hkv, slice = (int64_t)bl * p.HKV + hkv;
   const int entry_bytes = Gq * R * ROWB;
   const char* kbase = reinterpret_cast<const char*>(p.k_scaled) + bh * p.T * ROWB;
 
@@ -190,7 +191,7 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
   if (warp == 0) {
     // ---- pooled queries: one bulk copy per entry ----
     if (lane == 0) {
-      const unsigned char* src = t.pooled + bh * BDST * entry_bytes;
+      const unsigned char* src = t.pooled + slice * t.nd * entry_bytes;
       int slot = 0, use = 0, next = __ldg(&entries[0].x), k = 0;
       for (int e = 0; k < stages_total; ++k) {
         if (use > 0 && !mbar_wait_quick(smem_u32(&s_empty[slot]), (use - 1) & 1, &s_abort, p.status, t.tries)) break;
@@ -241,6 +242,7 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
     uint32_t* tab = tabs + (warp - kFirstSearchWarp) * TAB_WORDS;
     const uint32_t my_tmem = tmem + ((uint32_t)(quarter * 32) << 16);
     const int per = t.c_prev / CHUNK, n = p.n_chunks;
+    const int64_t row0 = (int64_t)b * BDST + t.d0;   // row of the slice's first block
     const bool counting = p.access_counter != nullptr;
     int32_t* counter = counting ? p.access_counter + (int64_t)b * p.access_stride_b + (int64_t)hkv * p.access_stride_h : nullptr;
     // this lane's key of each tile: magnitudes and the slot of the access counter
@@ -248,7 +250,8 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
     const float abs0 = __ldg(p.key_abs + bh * p.T + tk0), abs1 = __ldg(p.key_abs + bh * p.T + tk1);
     const int64_t mark0 = counting ? access_index(p.k, b, tk0) : (int64_t)-1, mark1 = counting ? access_index(p.k, b, tk1) : (int64_t)-1;
     // this lane's task: group g (entry g / Gq of the stage, head g % Gq) of the warp's chunk; the upper half of the warp has none
-    const int g = lane % NG, eg = g / Gq, hg = hkv * Gq + g % Gq;
+    const int g = lane % NG, eg = g / Gq;
+    const float* q_max = t.q_max + ((int64_t)bl * p.H + hkv * Gq + g % Gq) * t.nd;
     const bool walker = lane < NG;
     // What a round needs from memory is requested ahead: a lane's entry two rounds, what hangs on it one.
     struct Next {
@@ -263,9 +266,9 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
     auto details = [&](int u, int2 e) {
       Next x{e.x, 0, 0, 0.f};
       if (e.x >= 0) {
-        x.pt = __ldg(t.last + b * BDST + e.x);
-        x.q_max = __ldg(t.q_max + ((int64_t)b * p.H + hg) * BDST + e.x);
-        x.code = __ldcg(p.score_max + ((int64_t)b * BDST + e.x) * n + chunk_of(u, e.y));
+        x.pt = __ldg(t.last + bl * t.nd + e.x);
+        x.q_max = __ldg(q_max + e.x);
+        x.code = __ldcg(p.score_max + (row0 + e.x) * n + chunk_of(u, e.y));
       }
       return x;
     };
@@ -299,7 +302,7 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
         tab[i * kTabStride + lane] = pack2<DT>(x[i] - e_, x[i] + e_);
       }
       __syncwarp();
-      const int64_t row = (int64_t)b * BDST + cur.d;
+      const int64_t row = row0 + cur.d;
       const int c = chunk_of(u, j);
       const float so_far = decode_score(cur.code);
       uint32_t seen = 0;
@@ -331,7 +334,7 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
               // one pooled row per lane, from the operand's copy in memory (its stage may hold other queries by now)
               const int d = __shfl_sync(0xffffffffu, d_mine, owner), rr = owner % NG % Gq * R + lane % R;
               const uint4* kp = reinterpret_cast<const uint4*>(kbase + (int64_t)tk * ROWB);
-              const unsigned char* qp = t.pooled + (bh * BDST + d) * (int64_t)entry_bytes + (rr >> 3) * (KB * 1024);
+              const unsigned char* qp = t.pooled + (slice * t.nd + d) * (int64_t)entry_bytes + (rr >> 3) * (KB * 1024);
               float a = 0.f;
 #pragma unroll 1
               for (int p0 = 0; p0 < PIECES; p0 += 8) {
@@ -381,18 +384,15 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
 }
 
 template <int DT, int D>
-int run(const hipattn_scan_params_t& p, const KeyTiles& t, unsigned char* pooled, float* q_max, int32_t* last, int2* entries, int32_t* counts,
-        cudaStream_t stream) {
-  const int BDST = cdiv(p.TQ, p.block_size_q);
-  pool_queries_kernel<DT, D><<<(unsigned)(p.B * p.HKV * BDST), 256, 0, stream>>>(p, pooled, q_max, last);
+int run(const hipattn_scan_params_t& p, const KeyTiles& t, cudaStream_t stream) {
+  pool_queries_kernel<DT, D><<<(unsigned)(t.nb * p.HKV * t.nd), 256, 0, stream>>>(p, t);
   int rc = check_launch("pool_queries_kernel");
   if (rc) return rc;
-  list_queries_kernel<<<(unsigned)(p.B * t.n_grid), 256, 0, stream>>>(p.left, p.n_chunks, t.c_prev / kChunk, BDST, t.n_grid, t.sink, t.c_prev, last, entries,
-                                                                      counts);
+  list_queries_kernel<<<(unsigned)(t.nb * t.n_grid), 256, 0, stream>>>(p.left, p.n_chunks, t.c_prev / kChunk, cdiv(p.TQ, p.block_size_q), t);
   rc = check_launch("list_queries_kernel");
   if (rc) return rc;
   const size_t smem = 1024 + (size_t)kTile * D * 2 + 2 * (size_t)256 * D * 2 + (size_t)kSearchWarps * (256 / kRows) * kTabStride * 4;
-  const int64_t grid = (int64_t)p.B * p.HKV * t.n_grid * (t.c_prev / kTile);
+  const int64_t grid = (int64_t)t.nb * p.HKV * t.n_grid * (t.c_prev / kTile);
   HIPATTN_REQUIRE(grid > 0 && grid < 0x7fffffffLL, HIPATTN_ERR_INVALID, "scan grid of %lld blocks", (long long)grid);
   auto kern = scan_key_tiles_kernel<DT, D>;
   HIPATTN_CUDA_OK(allow_smem((const void*)kern, smem));
@@ -400,7 +400,37 @@ int run(const hipattn_scan_params_t& p, const KeyTiles& t, unsigned char* pooled
   return check_launch("scan_key_tiles_kernel");
 }
 
-int64_t align16(int64_t x) { return (x + 15) / 16 * 16; }
+// Scratch of a launch, and how a call is cut so that no launch needs more than kMaxScratch (a single query block may): whole
+// sequences as long as one fits, else query blocks of one sequence in equal parts.  The lists alone are 8 bytes a grid chunk and
+// query block, which grows with the square of the length (a million tokens on themselves: 2.1 GB of pooled queries of 32 heads, 0.5 GB
+// of lists).  A launch of that size fetches each key once for hundreds of query blocks.
+constexpr int64_t kMaxScratch = 128ll << 20;
+struct Slices {
+  int n_grid, nb, nd;   // chunks of the grid, most sequences and query blocks of a launch
+  int64_t pooled, q_max, last, entries, counts;   // bytes
+  int64_t bytes() const { return pooled + q_max + last + entries + counts; }
+};
+Slices plan_slices(const hipattn_scan_params_t& p, int sink, int c_prev) {
+  const int BDST = cdiv(p.TQ, p.block_size_q);
+  auto align16 = [](int64_t x) { return (x + 15) / 16 * 16; };
+  Slices s;
+  s.n_grid = cdiv(p.T - sink, c_prev);
+  auto size = [&](int nb, int nd) {
+    s.nb = nb;
+    s.nd = nd;
+    const int64_t blocks = (int64_t)nb * nd;
+    s.pooled = blocks * p.H * kRows * p.D * 2;
+    s.q_max = align16(blocks * p.H * 4);
+    s.last = align16(blocks * 4);
+    s.entries = align16(blocks * s.n_grid * 8);
+    s.counts = align16((int64_t)nb * s.n_grid * 4);
+    return s.bytes();
+  };
+  const int64_t one = size(1, BDST);
+  if (one <= kMaxScratch) size((int)min((int64_t)p.B, kMaxScratch / one), BDST);
+  else size(1, cdiv(BDST, (int)min((int64_t)BDST, (one + kMaxScratch - 1) / kMaxScratch)));
+  return s;
+}
 
 }  // namespace
 
@@ -420,29 +450,41 @@ int64_t scan_key_tiles_scratch(const hipattn_scan_params_t& p, int sink, int c_p
   if (v && (strcmp(v, "mma") == 0 || strcmp(v, "rounds") == 0)) return 0;
   const int64_t n_grid = cdiv(p.T - sink, c_prev), kept = p.n_chunks / (c_prev / kChunk);
   if (BDST * kept * G < 64 * n_grid) return 0;
-  return align16((int64_t)p.B * p.H * BDST * R * p.D * 2) + align16((int64_t)p.B * p.H * BDST * 4) + align16((int64_t)p.B * BDST * 4) +
-         align16(p.B * n_grid * BDST * 8) + align16(p.B * n_grid * 4);
+  return plan_slices(p, sink, c_prev).bytes();
 }
 
 // The scan stage on a list that select_stage has made from chunks of c_prev tokens (kept chunks on the grid from `sink`, ascending,
-// each cut into whole chunks of p.chunk_size); scratch: 16-byte aligned.
+// each cut into whole chunks of p.chunk_size); scratch: 16-byte aligned, used by one launch after the other.
 int scan_key_tiles(const hipattn_scan_params_t& p, int sink, int c_prev, void* scratch, cudaStream_t stream) {
-  const int R = p.block_size_q / p.stride_q, BDST = cdiv(p.TQ, p.block_size_q), n_grid = cdiv(p.T - sink, c_prev);
+  const Slices s = plan_slices(p, sink, c_prev);
+  KeyTiles t;
   unsigned char* at = (unsigned char*)scratch;
   auto take = [&](int64_t bytes) {
     unsigned char* x = at;
-    at += align16(bytes);
+    at += bytes;
     return x;
   };
-  unsigned char* pooled = take((int64_t)p.B * p.H * BDST * R * p.D * 2);
-  float* q_max = (float*)take((int64_t)p.B * p.H * BDST * 4);
-  int32_t* last = (int32_t*)take((int64_t)p.B * BDST * 4);
-  int2* entries = (int2*)take((int64_t)p.B * n_grid * BDST * 8);
-  int32_t* counts = (int32_t*)take((int64_t)p.B * n_grid * 4);
-  const KeyTiles t{pooled, q_max, last, entries, counts, n_grid, sink, c_prev, wait_tries()};
-  if (p.dtype == HIPATTN_BF16)
-    return p.D == 128 ? run<HIPATTN_BF16, 128>(p, t, pooled, q_max, last, entries, counts, stream) : run<HIPATTN_BF16, 64>(p, t, pooled, q_max, last, entries, counts, stream);
-  return p.D == 128 ? run<HIPATTN_F16, 128>(p, t, pooled, q_max, last, entries, counts, stream) : run<HIPATTN_F16, 64>(p, t, pooled, q_max, last, entries, counts, stream);
+  t.pooled = take(s.pooled);
+  t.q_max = (float*)take(s.q_max);
+  t.last = (int32_t*)take(s.last);
+  t.entries = (int2*)take(s.entries);
+  t.counts = (int32_t*)take(s.counts);
+  t.n_grid = s.n_grid;
+  t.sink = sink;
+  t.c_prev = c_prev;
+  t.tries = wait_tries();
+  const int BDST = cdiv(p.TQ, p.block_size_q);
+  for (t.b0 = 0; t.b0 < p.B; t.b0 += s.nb) {
+    t.nb = min(s.nb, p.B - t.b0);
+    for (t.d0 = 0; t.d0 < BDST; t.d0 += s.nd) {
+      t.nd = min(s.nd, BDST - t.d0);
+      int rc;
+      if (p.dtype == HIPATTN_BF16) rc = p.D == 128 ? run<HIPATTN_BF16, 128>(p, t, stream) : run<HIPATTN_BF16, 64>(p, t, stream);
+      else rc = p.D == 128 ? run<HIPATTN_F16, 128>(p, t, stream) : run<HIPATTN_F16, 64>(p, t, stream);
+      if (rc) return rc;
+    }
+  }
+  return HIPATTN_OK;
 }
 
 }  // namespace hipattn

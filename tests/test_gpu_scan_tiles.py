@@ -27,7 +27,7 @@ def problem(shape, keys, rope):
     import bench
     from cases import rope_tables
     w = dict(bench.WORKLOADS["prefill_128k"], H=8, HKV=2, keep=[4096, 1024, 512])
-    w.update(SHAPES[shape])
+    w.update(shape if isinstance(shape, dict) else SHAPES[shape])
     q, k, v = bench.make_qkv(w, "cuda")
     g = torch.Generator(device="cuda").manual_seed(5)
     if keys == "close":      # neighbours that are equal or one unit in the last place apart
@@ -48,6 +48,16 @@ def problem(shape, keys, rope):
     args = bench.make_args(w, **kw)
     args.require_cache_statistics = True
     return (q, k, v), args
+
+
+def launches(call):
+    """Names of the scan kernels that a call launches, in order."""
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events() if "scan_" in e.name and "_kernel" in e.name and "prepare" not in e.name]
+    return [n.split("scan_")[1].split("_kernel")[0] for n in names]
 
 
 @pytest.mark.parametrize("rope", [None, "relative"])
@@ -136,3 +146,49 @@ def test_waits_that_run_out_are_reported_and_leave_nothing(monkeypatch):
         md = hip_attention_impl(*qkv, args)[1]
         assert read_status("cuda") == 0
         assert torch.equal(md.indices, want.indices) and torch.equal(md.ks, want.ks)
+
+
+@pytest.mark.parametrize("shape", [dict(T=33001, TQ=33001, H=64, HKV=8), dict(T=9001, TQ=9001, H=64, HKV=8, B=5)], ids=["blocks", "sequences"])
+def test_key_tiles_in_several_launches(shape, monkeypatch):
+    """More query blocks, or sequences, than one launch has scratch for (258 KB a block here, 128 MB in all: 516 blocks of one sequence,
+    141 of five)."""
+    from hip_attention_b200 import hip_attention_impl
+    qkv, args = problem(shape, "random", None)
+    md = {}
+    for mode in ("auto", "strict"):
+        monkeypatch.setenv("HIPATTN_SCAN_MODE", mode)
+        if mode == "auto":
+            assert launches(lambda: hip_attention_impl(*qkv, args)).count("key_tiles") == 2
+        md[mode] = hip_attention_impl(*qkv, args)[1]
+    a, b = md["auto"], md["strict"]
+    assert torch.equal(a.stage_caches[2].indices_left, b.stage_caches[2].indices_left)
+    assert torch.equal(a.indices, b.indices) and torch.equal(a.ks, b.ks)
+    assert torch.equal(a.mask_cache_statistics.access_counter, b.mask_cache_statistics.access_counter)
+
+
+def test_without_memory_for_the_scratch():
+    """The rounds need none: a call that finds no room for the key tiles' scratch (68 MB here) goes by them."""
+    from hip_attention_b200 import hip_attention_impl
+    qkv, args = problem(dict(T=16500, TQ=16500, H=64, HKV=8), "random", None)
+    want = hip_attention_impl(*qkv, args)[1]
+    total = torch.cuda.mem_get_info()[1]
+    calls, held = [], []
+
+    def after_stage(score):    # (called after each scan stage; the second one asks for scratch)
+        calls.append(1)
+        if len(calls) == 1:
+            torch.cuda.empty_cache()
+            torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (16 << 20)) / total)
+            with pytest.raises(torch.OutOfMemoryError):
+                while True:
+                    held.append(torch.empty(32 << 20, dtype=torch.uint8, device="cuda"))
+        else:
+            held.clear()
+            torch.cuda.set_per_process_memory_fraction(1.0)
+
+    try:
+        md = hip_attention_impl(*qkv, args, score_reduce=after_stage)[1]
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert len(calls) == 3
+    assert torch.equal(md.indices, want.indices) and torch.equal(md.ks, want.ks)
