@@ -14,9 +14,6 @@
 // Bound: as scan_query_tiles.cu, the chain from an accumulator's MMAs to its release.  128k prefill, second stage (chunk
 // 32, 4 heads x 16 rows): 3135 us by rounds, which were bound by their gathers (10.7 TB/s from L2), 1740 and 73 for the
 // pooled queries and the lists; ragged fp16 prefill 189 -> 117 us.
-#include <cstdlib>
-#include <cstring>
-
 #include "host_kernels.h"
 #include "scan_tiles.cuh"
 
@@ -432,13 +429,34 @@ Slices plan_slices(const hipattn_scan_params_t& p, int sink, int c_prev) {
   return s;
 }
 
+// Whether the keys are worth keeping.  A CTA's keys, operands and start cost 5 us, its list runs as one chain, and CTAs are few where
+// heads and chunks are; the rounds pay per (query block, head) instead.  In units of 14 ns, what the rounds lose on a
+// list entry of 16 groups (head, block): they take `listed` of them and a fifth per block and head, the key tiles 50 per
+// entry of the longest list, that of a chunk which every block keeps, and 400 per CTA of a multiprocessor.  Entries are counted for
+// queries that are the last TQ of T, without the blocks that a chunk is not active for.  On 1235 random calls (1 to 16 heads a KV
+// head, 1 to 16 KV heads, 200 to 16384 queries of 1400 to 100000 tokens, 8 to 128 kept chunks) the stage took 379 ms by rounds, 247.4 by
+// the better of the two, 248.2 by this rule, 24 calls slower than by rounds by more than 3 %, 1.5 times at most (65 -> 97 us: three
+// chunks of 2595 tokens).  A threshold of 64 groups a chunk, whatever its blocks and CTAs, had 253.2, 208 calls and 3.8 times at
+// most (16 heads of one KV head and 2309 tokens: 16 us by rounds, 59 here, on nine CTAs).
+bool worth_turning(const hipattn_scan_params_t& p, int sink, int c_prev) {
+  const int G = p.H / p.HKV, BDST = cdiv(p.TQ, p.block_size_q), kept = p.n_chunks / (c_prev / kChunk);
+  int64_t listed = 0, longest = 0, chunks = 0;
+  for (int d = 0; d < BDST; ++d) {
+    const int64_t reach = (int64_t)p.T - p.TQ + (int64_t)d * p.block_size_q - p.scan_window - sink;
+    if (reach < 0) continue;
+    chunks = reach / c_prev + 1;
+    listed += min((int64_t)kept, chunks);
+    ++longest;
+  }
+  const double pairs = (double)p.B * p.HKV * (c_prev / kTile), entries = G / 16.0;
+  return pairs * listed * entries + p.B * (double)p.H * BDST / 5 > 50 * longest * entries + 400 * fmax(1.0, pairs * chunks / 148);
+}
+
 }  // namespace
 
 // Bytes of scratch that scan_key_tiles needs for this call, 0 where it does not take it: chunks of 32 cut from chunks of whole key
-// tiles, 16 pooled rows a head, no in-kernel RoPE, no per-head results.  Each CTA has its keys to fetch, so its list has to be
-// worth it: time against the rounds (4096 queries and fewer, 8192 to 131072 tokens), by heads and query blocks per chunk: 4 heads
-// 64 blocks 0.64, 32 0.70 to 0.92, 16 0.85 to 0.95, 10 1.08 to 1.19, 5 1.5; 8 heads 8 blocks 0.90; 2 heads 32 blocks 0.84, 16
-// 1.09; 1 head 64 blocks 0.84, 32 1.13.  With 32 pooled rows 0.99 (64 blocks) to 1.4, "relative" 0.92 (128 blocks) to 1.6.
+// tiles, 16 pooled rows a head, no in-kernel RoPE, no per-head results.  With 32 pooled rows the tiles took 0.99 to 1.4 of the rounds'
+// time, "relative" 0.92 to 1.6.
 int64_t scan_key_tiles_scratch(const hipattn_scan_params_t& p, int sink, int c_prev) {
   const int R = p.block_size_q / p.stride_q, G = p.H / p.HKV, BDST = cdiv(p.TQ, p.block_size_q);
   if (p.mode != HIPATTN_SCAN_AUTO || p.dtype == HIPATTN_F32 || (p.D != 64 && p.D != 128) || p.key_abs == nullptr || p.k_scaled == nullptr) return 0;
@@ -446,10 +464,8 @@ int64_t scan_key_tiles_scratch(const hipattn_scan_params_t& p, int sink, int c_p
   if (R != kRows || (G & (G - 1)) != 0 || G > 16 || p.TQ <= p.stride_q) return 0;
   if (p.chunk_size != kChunk || c_prev % kTile != 0 || p.n_chunks % (c_prev / kChunk) != 0 || p.T <= sink) return 0;
   if ((int64_t)p.B * p.T * p.HKV >= 0x7fffffffLL || (int64_t)p.B * p.HKV * BDST >= 0x7fffffffLL) return 0;
-  const char* v = getenv("HIPATTN_SCAN_KERNEL");
-  if (v && (strcmp(v, "mma") == 0 || strcmp(v, "rounds") == 0)) return 0;
-  const int64_t n_grid = cdiv(p.T - sink, c_prev), kept = p.n_chunks / (c_prev / kChunk);
-  if (BDST * kept * G < 64 * n_grid) return 0;
+  const ScanChoice choice = scan_choice();
+  if (choice == SCAN_BY_MMA || choice == SCAN_BY_ROUNDS || (choice != SCAN_BY_TILES && !worth_turning(p, sink, c_prev))) return 0;
   return plan_slices(p, sink, c_prev).bytes();
 }
 

@@ -95,6 +95,14 @@ __device__ __forceinline__ bool mbar_wait_quick(uint32_t mbar, uint32_t parity, 
     if (mbar_try(mbar, parity)) return true;
   return mbar_wait_slow(mbar, parity, abort_flag, status, tries);
 }
+// HIPATTN_SCAN_KERNEL, for comparisons: the prefill scans on mma.sync, by rounds, or on whole tiles wherever these can be had, whether
+// they are the faster ones or not.
+enum ScanChoice { SCAN_BY_RULE, SCAN_BY_MMA, SCAN_BY_ROUNDS, SCAN_BY_TILES };
+inline ScanChoice scan_choice() {
+  const char* v = getenv("HIPATTN_SCAN_KERNEL");
+  if (!v) return SCAN_BY_RULE;
+  return strcmp(v, "mma") == 0 ? SCAN_BY_MMA : strcmp(v, "rounds") == 0 ? SCAN_BY_ROUNDS : strcmp(v, "tiles") == 0 ? SCAN_BY_TILES : SCAN_BY_RULE;
+}
 // HIPATTN_SCAN_WAIT=none lets a test take the kernels' ways out of a wait that has run out.
 inline int wait_tries() {
   const char* v = getenv("HIPATTN_SCAN_WAIT");

@@ -1,11 +1,20 @@
 """Prefill scans that score whole tiles of keys: masks, later stages' lists and access counters equal the strict kernel's, where every
 bound is settled at once and where strict scores are needed."""
+import re
+
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
-# (the second stage's kernel wants 64 / heads query blocks for a chunk of the first)
+
+@pytest.fixture(autouse=True)
+def tiles(monkeypatch, request):
+    """The whole-tile kernels wherever they can be had: the calls here are smaller than what they are chosen for."""
+    if "by_rule" not in request.keywords:
+        monkeypatch.setenv("HIPATTN_SCAN_KERNEL", "tiles")
+
+
 SHAPES = {
     "heads4": dict(T=9001, TQ=2300),                                                   # 4 heads x 64 rows: a full accumulator
     "heads4_d64": dict(T=6007, TQ=1517, D=64, dtype="fp16"),
@@ -56,8 +65,14 @@ def launches(call):
     with profile(activities=[ProfilerActivity.CUDA]) as prof:
         call()
         torch.cuda.synchronize()
-    names = [e.name for e in prof.events() if "scan_" in e.name and "_kernel" in e.name and "prepare" not in e.name]
-    return [n.split("scan_")[1].split("_kernel")[0] for n in names]
+    names = [re.search(r"scan_(\w+)_kernel", e.name) for e in prof.events()]
+    return [n.group(1) for n in names if n and n.group(1) != "prepare_keys"]
+
+
+def expected(args, H, HKV):
+    """What this file's calls launch in the second stage: key tiles as far as their shapes allow it."""
+    G, rows = H // HKV, args.stages[1].stage_block_size_q // args.stages[1].stage_block_stride_q
+    return "key_tiles" if not args.using_extend and rows == 16 and G in (1, 2, 4, 8, 16) else "stage_tcgen05"
 
 
 @pytest.mark.parametrize("rope", [None, "relative"])
@@ -69,6 +84,8 @@ def test_masks_equal_strict(shape, keys, rope, monkeypatch):
     md = {}
     for mode in ("auto", "strict"):
         monkeypatch.setenv("HIPATTN_SCAN_MODE", mode)
+        if mode == "auto" and keys == "random":
+            assert launches(lambda: hip_attention_impl(*qkv, args))[1] == expected(args, qkv[0].shape[2], qkv[1].shape[2])
         md[mode] = hip_attention_impl(*qkv, args)[1]
     a, b = md["auto"], md["strict"]
     for i, (x, y) in enumerate(zip(a.stage_caches[1:], b.stage_caches[1:])):
@@ -192,3 +209,32 @@ def test_without_memory_for_the_scratch():
         torch.cuda.set_per_process_memory_fraction(1.0)
     assert len(calls) == 3
     assert torch.equal(md.indices, want.indices) and torch.equal(md.ks, want.ks)
+
+
+# heads, KV heads, query rows of a block, pooling strides, queries, tokens, kept -> kernel of the second stage
+RULE = [
+    # (few CTAs, one with a list of all blocks: 2.4 to 2.5 times the rounds' time by key tiles)
+    (32, 2, 64, (4, 4, 1), 3000, 3000, (32768, 8192, 2048), "stage_tcgen05"),
+    (16, 1, 64, (4, 4, 1), 4202, 7692, (32768, 8192, 2048), "stage_tcgen05"),
+    # (blocks listed, but few active)
+    (32, 8, 64, (4, 4, 1), 2500, 2500, (32768, 8192, 2048), "stage_tcgen05"),
+    (64, 8, 64, (4, 4, 1), 2048, 2048, (32768, 8192, 2048), "stage_tcgen05"),
+    (32, 8, 64, (4, 4, 1), 4096, 4096, (32768, 8192, 2048), "key_tiles"),
+    (16, 4, 64, (4, 4, 1), 2999, 20011, (32768, 8192, 2048), "key_tiles"),
+    (64, 8, 64, (4, 4, 1), 1100, 8192, (32768, 8192, 2048), "key_tiles"),
+]
+
+
+@pytest.mark.by_rule
+@pytest.mark.parametrize("H,HKV,bq,strides,TQ,T,keep,want", RULE)
+def test_tiles_where_they_are_faster(H, HKV, bq, strides, TQ, T, keep, want, monkeypatch):
+    """Kernels that the rules choose, on calls whose times with either are far apart."""
+    from hip_attention_b200 import hip_attention_impl
+    import bench
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q = torch.randn((1, TQ, H, 128), generator=g, device="cuda", dtype=torch.bfloat16) * 128 ** -0.5
+    k = torch.randn((1, T, HKV, 128), generator=g, device="cuda", dtype=torch.bfloat16)
+    args = bench.make_args(dict(chunks=(256, 32, 8), bq=bq, strides=strides, keep=keep, sink=256, sw=1024))
+    assert launches(lambda: hip_attention_impl(q, k, k, args))[1] == want
+    monkeypatch.setenv("HIPATTN_SCAN_KERNEL", "rounds")
+    assert launches(lambda: hip_attention_impl(q, k, k, args)) == ["stage_tcgen05"] * 3
