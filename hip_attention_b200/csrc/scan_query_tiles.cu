@@ -542,13 +542,27 @@ int dispatch_rows(const hipattn_scan_params_t& p, cudaStream_t stream) {
 // but 4 x 16 1.11, 2 x 64 0.93 (head dim 64: 1.05), 1 x 128 1.05.  Chunks of 16 would take 0.78 (8 x 32) to 1.25 of the rounds'
 // time, of 32 1.14 to 1.8; "relative", whose every key has two scores, 0.78 (8 x 32) to 1.2.  With fewer than 32 units the
 // rounds, whose CTAs are smaller, spread better: 16 units 1.09 to 1.16, 32 units 0.89 to 0.98.
+//
+// A CTA puts 64 to 128 KB of pooled queries in place before its first tile, so its list has to be worth that: three steps (a key
+// tile against 256 columns), seven per 64 query rows where a pooled row is the mean of several, and ten steps per multiprocessor in
+// all.  On 1330 random calls (2 to 16 heads a KV head, 1 to 16 KV heads, 200 to 16384 queries of 1400 to 100000 tokens, 32 to 1024
+// chunks) the stage took 414 ms by rounds, 306.0 by the better of the two, 307.5 by this rule, with 52 calls slower than by rounds by
+// more than 3 %, 1.32 times at most; with the units alone 310.7, 337 calls and 2.4 times at most (8 x 32 rows, 64 chunks, 48 units:
+// 15 us by rounds, 35 here).
 int scan_query_tiles(const hipattn_scan_params_t& p, cudaStream_t stream, bool* handled) {
   *handled = false;
   const int R = p.block_size_q / p.stride_q, G = p.H / p.HKV;
   if (p.rope_mode != HIPATTN_ROPE_NONE || (R != 16 && R != 32 && R != 64 && R != 128)) return HIPATTN_OK;
-  if (p.chunk_size != kTileChunk || p.T < kTileChunk) return HIPATTN_OK;
-  if (G * R < 128 || (G < 4 && G * R < 192) || G < 2) return HIPATTN_OK;
-  if ((int64_t)p.B * p.HKV * cdiv(p.TQ, p.block_size_q) * plan_tiles(p).head_groups < 32) return HIPATTN_OK;
+  if (p.chunk_size != kTileChunk || p.T < kTileChunk || G < 2 || G * R < 128) return HIPATTN_OK;
+  const ScanChoice choice = scan_choice();
+  if (choice == SCAN_BY_ROUNDS) return HIPATTN_OK;
+  if (choice != SCAN_BY_TILES) {
+    if (G < 4 && G * R < 192) return HIPATTN_OK;
+    const int64_t blocks = (int64_t)p.B * p.HKV * cdiv(p.TQ, p.block_size_q), ctas = plan_tiles(p).head_groups;
+    const int64_t steps = (int64_t)cdiv(p.n_chunks, 128 / kTileChunk) * cdiv(G, 256 / R);   // of a query block and KV head
+    if (blocks * ctas < 32 || blocks * steps < 10 * 148) return HIPATTN_OK;
+    if (p.stride_q == 1 ? steps < ctas * 3 : steps * 64 < ctas * 7 * p.block_size_q) return HIPATTN_OK;
+  }
   *handled = true;
   if (p.dtype == HIPATTN_BF16) return p.D == 128 ? dispatch_rows<HIPATTN_BF16, 128>(p, stream) : dispatch_rows<HIPATTN_BF16, 64>(p, stream);
   return p.D == 128 ? dispatch_rows<HIPATTN_F16, 128>(p, stream) : dispatch_rows<HIPATTN_F16, 64>(p, stream);

@@ -599,10 +599,8 @@ int scan_stage_tcgen05(const hipattn_scan_params_t& p, cudaStream_t stream, bool
   if (p.rope_mode == HIPATTN_ROPE_STREAMING && !(p.k_scaled_sides == 1 && p.D == 128)) return HIPATTN_OK;
   const char* v = getenv("HIPATTN_SCAN_KERNEL");
   if (v && strcmp(v, "mma") == 0) return HIPATTN_OK;
-  if (!(v && strcmp(v, "rounds") == 0)) {   // (for comparisons)
-    const int rc = scan_query_tiles(p, stream, handled);
-    if (*handled) return rc;
-  }
+  const int rc = scan_query_tiles(p, stream, handled);
+  if (*handled) return rc;
   *handled = true;
   if (p.dtype == HIPATTN_BF16) return p.D == 128 ? dispatch_rows<HIPATTN_BF16, 128>(p, stream) : dispatch_rows<HIPATTN_BF16, 64>(p, stream);
   return p.D == 128 ? dispatch_rows<HIPATTN_F16, 128>(p, stream) : dispatch_rows<HIPATTN_F16, 64>(p, stream);

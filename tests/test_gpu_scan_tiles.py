@@ -70,9 +70,12 @@ def launches(call):
 
 
 def expected(args, H, HKV):
-    """What this file's calls launch in the second stage: key tiles as far as their shapes allow it."""
-    G, rows = H // HKV, args.stages[1].stage_block_size_q // args.stages[1].stage_block_stride_q
-    return "key_tiles" if not args.using_extend and rows == 16 and G in (1, 2, 4, 8, 16) else "stage_tcgen05"
+    """What this file's calls launch: whole tiles in the second and third stage as far as their shapes allow it."""
+    G, rows = H // HKV, [s.stage_block_size_q // s.stage_block_stride_q for s in args.stages]
+    if args.using_extend:
+        return ["stage_tcgen05"] * 3
+    return ["stage_tcgen05", "key_tiles" if rows[1] == 16 and G in (1, 2, 4, 8, 16) else "stage_tcgen05",
+            "query_tiles" if G >= 2 and G * rows[2] >= 128 else "stage_tcgen05"]
 
 
 @pytest.mark.parametrize("rope", [None, "relative"])
@@ -85,7 +88,7 @@ def test_masks_equal_strict(shape, keys, rope, monkeypatch):
     for mode in ("auto", "strict"):
         monkeypatch.setenv("HIPATTN_SCAN_MODE", mode)
         if mode == "auto" and keys == "random":
-            assert launches(lambda: hip_attention_impl(*qkv, args))[1] == expected(args, qkv[0].shape[2], qkv[1].shape[2])
+            assert launches(lambda: hip_attention_impl(*qkv, args)) == expected(args, qkv[0].shape[2], qkv[1].shape[2])
         md[mode] = hip_attention_impl(*qkv, args)[1]
     a, b = md["auto"], md["strict"]
     for i, (x, y) in enumerate(zip(a.stage_caches[1:], b.stage_caches[1:])):
@@ -211,17 +214,22 @@ def test_without_memory_for_the_scratch():
     assert torch.equal(md.indices, want.indices) and torch.equal(md.ks, want.ks)
 
 
-# heads, KV heads, query rows of a block, pooling strides, queries, tokens, kept -> kernel of the second stage
+# heads, KV heads, query rows of a block, pooling strides, queries, tokens, kept -> kernels of the second and third stage
 RULE = [
     # (few CTAs, one with a list of all blocks: 2.4 to 2.5 times the rounds' time by key tiles)
-    (32, 2, 64, (4, 4, 1), 3000, 3000, (32768, 8192, 2048), "stage_tcgen05"),
-    (16, 1, 64, (4, 4, 1), 4202, 7692, (32768, 8192, 2048), "stage_tcgen05"),
+    (32, 2, 64, (4, 4, 1), 3000, 3000, (32768, 8192, 2048), ("stage_tcgen05", "query_tiles")),
+    (16, 1, 64, (4, 4, 1), 4202, 7692, (32768, 8192, 2048), ("stage_tcgen05", "query_tiles")),
     # (blocks listed, but few active)
-    (32, 8, 64, (4, 4, 1), 2500, 2500, (32768, 8192, 2048), "stage_tcgen05"),
-    (64, 8, 64, (4, 4, 1), 2048, 2048, (32768, 8192, 2048), "stage_tcgen05"),
-    (32, 8, 64, (4, 4, 1), 4096, 4096, (32768, 8192, 2048), "key_tiles"),
-    (16, 4, 64, (4, 4, 1), 2999, 20011, (32768, 8192, 2048), "key_tiles"),
-    (64, 8, 64, (4, 4, 1), 1100, 8192, (32768, 8192, 2048), "key_tiles"),
+    (32, 8, 64, (4, 4, 1), 2500, 2500, (32768, 8192, 2048), ("stage_tcgen05", "query_tiles")),
+    (64, 8, 64, (4, 4, 1), 2048, 2048, (32768, 8192, 2048), ("stage_tcgen05", "query_tiles")),
+    (32, 8, 64, (4, 4, 1), 4096, 4096, (32768, 8192, 2048), ("key_tiles", "query_tiles")),
+    (16, 4, 64, (4, 4, 1), 2999, 20011, (32768, 8192, 2048), ("key_tiles", "query_tiles")),
+    (64, 8, 64, (4, 4, 1), 1100, 8192, (32768, 8192, 2048), ("key_tiles", "query_tiles")),
+    # (short lists: 2.4, 1.8 and 1.5 times the rounds' time by query tiles)
+    (64, 8, 64, (4, 4, 2), 357, 16723, (4096, 512, 256), ("stage_tcgen05", "stage_tcgen05")),
+    (8, 1, 64, (4, 4, 1), 2652, 73875, (4096, 512, 256), ("stage_tcgen05", "stage_tcgen05")),
+    (32, 8, 64, (4, 4, 2), 16384, 32938, (4096, 512, 256), ("key_tiles", "stage_tcgen05")),
+    (64, 8, 128, (4, 4, 1), 2000, 32768, (65536, 16384, 4096), ("stage_tcgen05", "query_tiles")),
 ]
 
 
@@ -235,6 +243,6 @@ def test_tiles_where_they_are_faster(H, HKV, bq, strides, TQ, T, keep, want, mon
     q = torch.randn((1, TQ, H, 128), generator=g, device="cuda", dtype=torch.bfloat16) * 128 ** -0.5
     k = torch.randn((1, T, HKV, 128), generator=g, device="cuda", dtype=torch.bfloat16)
     args = bench.make_args(dict(chunks=(256, 32, 8), bq=bq, strides=strides, keep=keep, sink=256, sw=1024))
-    assert launches(lambda: hip_attention_impl(q, k, k, args))[1] == want
+    assert tuple(launches(lambda: hip_attention_impl(q, k, k, args))[1:]) == want
     monkeypatch.setenv("HIPATTN_SCAN_KERNEL", "rounds")
     assert launches(lambda: hip_attention_impl(q, k, k, args)) == ["stage_tcgen05"] * 3
