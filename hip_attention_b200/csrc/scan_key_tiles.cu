@@ -128,7 +128,19 @@ __global__ void __launch_bounds__(256) list_queries_kernel(const int32_t* __rest
   if (threadIdx.x == 0) kt.counts[bl * kt.n_grid + g] = total;
 }
 
-template <int DT, int D>
+// ---- per-head results of chunks that no list holds: not active, so as they came ----
+__global__ void __launch_bounds__(256) untouched_heads_kernel(const hipattn_scan_params_t p, int64_t total) {
+  const int64_t per_row = (int64_t)p.H * p.n_chunks;
+  for (int64_t i = blockIdx.x * 256LL + threadIdx.x; i < total; i += gridDim.x * 256LL) {
+    const int64_t c = i / per_row * p.n_chunks + i % p.n_chunks;
+    p.left_out[i] = p.left[c];
+    p.right_out[i] = p.right[c];
+    p.score_out[i] = HIPATTN_SCORE_INIT;
+  }
+}
+
+// CHECKED: per-head results, statistics, and in check mode every score by both definitions.
+template <int DT, int D, bool CHECKED>
 __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipattn_scan_params_t p, const KeyTiles t) {
   constexpr int ROWB = D * 2, PIECES = ROWB / 16, KB = D / 64;
   constexpr int R = kRows, CHUNK = kChunk, COLS = 256, NG = COLS / R;   // columns of a stage, groups (query block, head)
@@ -271,6 +283,9 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
     };
     int2 ent = entry_of(set), ent2 = entry_of(set + kSearchSets);
     Next nx = details(set, ent);
+    const bool per_head = CHECKED && p.left_out != nullptr;
+    unsigned st_keys = 0, st_fb = 0, st_wrong = 0;
+    float st_ratio = 0.f;
     uint32_t phase = 0;
     bool ok = true;
     for (int u = set; u < stages_total * 2 && ok; u += kSearchSets) {
@@ -299,6 +314,59 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
         tab[i * kTabStride + lane] = pack2<DT>(x[i] - e_, x[i] + e_);
       }
       __syncwarp();
+      // strict score of a token for the group of lane `owner`
+      const int d_mine = cur.d;
+      auto strict_of = [&](int tk, int owner) -> float {
+        // one pooled row per lane, from the operand's copy in memory (its stage may hold other queries by now)
+        const int d = __shfl_sync(0xffffffffu, d_mine, owner), rr = owner % NG % Gq * R + lane % R;
+        const uint4* kp = reinterpret_cast<const uint4*>(kbase + (int64_t)tk * ROWB);
+        const unsigned char* qp = t.pooled + (slice * t.nd + d) * (int64_t)entry_bytes + (rr >> 3) * (KB * 1024);
+        float a = 0.f;
+#pragma unroll 1
+        for (int p0 = 0; p0 < PIECES; p0 += 8) {
+          uint4 kw[8], qw[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            kw[e] = __ldg(kp + p0 + e);
+            qw[e] = __ldg(reinterpret_cast<const uint4*>(qp + (p0 >> 3) * 1024 + sw128(rr & 7, e)));
+          }
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            a = fmaf(lo_f32<DT>(qw[e].x), lo_f32<DT>(kw[e].x), a);
+            a = fmaf(hi_f32<DT>(qw[e].x), hi_f32<DT>(kw[e].x), a);
+            a = fmaf(lo_f32<DT>(qw[e].y), lo_f32<DT>(kw[e].y), a);
+            a = fmaf(hi_f32<DT>(qw[e].y), hi_f32<DT>(kw[e].y), a);
+            a = fmaf(lo_f32<DT>(qw[e].z), lo_f32<DT>(kw[e].z), a);
+            a = fmaf(hi_f32<DT>(qw[e].z), hi_f32<DT>(kw[e].z), a);
+            a = fmaf(lo_f32<DT>(qw[e].w), lo_f32<DT>(kw[e].w), a);
+            a = fmaf(hi_f32<DT>(qw[e].w), hi_f32<DT>(kw[e].w), a);
+          }
+        }
+        float top = fmaxf(a, -INFINITY);   // (a score that is not a number is the lowest)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        return top;
+      };
+      if constexpr (CHECKED) {
+#pragma unroll 1
+        for (int i = 0; i < ng; ++i) {
+          uint32_t* w = tab + i * kTabStride + lane;
+          ++st_keys;
+          if (lo_f32<DT>(*w) != hi_f32<DT>(*w)) ++st_fb;
+          if (p.mode != HIPATTN_SCAN_CHECK) continue;
+          const float e_ = __shfl_sync(0xffffffffu, unit, i) * s_abs;
+#pragma unroll 1
+          for (int o = 0; o < 32; ++o) {
+            const float raw = strict_of(min(l + o, p.T - 1), i), ex = Elem<DT>::round(raw);
+            if (lane == o) {
+              if (lo_f32<DT>(*w) == hi_f32<DT>(*w) && hi_f32<DT>(*w) != ex) ++st_wrong;
+              if (e_ > 0.f) st_ratio = fmaxf(st_ratio, fabsf(x[i] - raw) / e_);
+              *w = pack2<DT>(ex, ex);
+            }
+          }
+        }
+        __syncwarp();
+      }
       const int64_t row = row0 + cur.d;
       const int c = chunk_of(u, j);
       const float so_far = decode_score(cur.code);
@@ -312,7 +380,7 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
       for (int o = 1; o < Gq; o <<= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
       // a score that may raise the chunk's best has to be certain
       closed |= !valid;
-      const bool compared = plain && __all_sync(0xffffffffu, closed);
+      const bool compared = plain && !per_head && __all_sync(0xffffffffu, closed);
       if (!compared || __any_sync(0xffffffffu, shi > slo && shi > best)) {
         ChunkTask task;
         task.valid = valid;
@@ -325,41 +393,14 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
         task.tab = tab + g * kTabStride;
         task.slo = compared ? slo : HIPATTN_SCORE_INIT;
         task.shi = compared ? shi : HIPATTN_SCORE_INIT;
-        const int d_mine = cur.d;
-        search_chunks<DT, CHUNK>(task, p.T, Gq, compared, false,
-            [&](int tk, int owner) -> float {
-              // one pooled row per lane, from the operand's copy in memory (its stage may hold other queries by now)
-              const int d = __shfl_sync(0xffffffffu, d_mine, owner), rr = owner % NG % Gq * R + lane % R;
-              const uint4* kp = reinterpret_cast<const uint4*>(kbase + (int64_t)tk * ROWB);
-              const unsigned char* qp = t.pooled + (slice * t.nd + d) * (int64_t)entry_bytes + (rr >> 3) * (KB * 1024);
-              float a = 0.f;
-#pragma unroll 1
-              for (int p0 = 0; p0 < PIECES; p0 += 8) {
-                uint4 kw[8], qw[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                  kw[e] = __ldg(kp + p0 + e);
-                  qw[e] = __ldg(reinterpret_cast<const uint4*>(qp + (p0 >> 3) * 1024 + sw128(rr & 7, e)));
-                }
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                  a = fmaf(lo_f32<DT>(qw[e].x), lo_f32<DT>(kw[e].x), a);
-                  a = fmaf(hi_f32<DT>(qw[e].x), hi_f32<DT>(kw[e].x), a);
-                  a = fmaf(lo_f32<DT>(qw[e].y), lo_f32<DT>(kw[e].y), a);
-                  a = fmaf(hi_f32<DT>(qw[e].y), hi_f32<DT>(kw[e].y), a);
-                  a = fmaf(lo_f32<DT>(qw[e].z), lo_f32<DT>(kw[e].z), a);
-                  a = fmaf(hi_f32<DT>(qw[e].z), hi_f32<DT>(kw[e].z), a);
-                  a = fmaf(lo_f32<DT>(qw[e].w), lo_f32<DT>(kw[e].w), a);
-                  a = fmaf(hi_f32<DT>(qw[e].w), hi_f32<DT>(kw[e].w), a);
-                }
-              }
-              float top = fmaxf(a, -INFINITY);   // (a score that is not a number is the lowest)
-#pragma unroll
-              for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-              return top;
-            },
-            [](int) {});
+        search_chunks<DT, CHUNK>(task, p.T, Gq, compared, per_head, strict_of, [](int) {});
         if (task.valid && task.out_of_range) atomicOr(p.status, HIPATTN_STATUS_TOKEN_RANGE);
+        if (per_head && valid) {
+          const int64_t o = (row * p.H + hkv * Gq + g % Gq) * n + c;
+          p.left_out[o] = task.l;
+          p.right_out[o] = task.r;
+          p.score_out[o] = task.score;
+        }
         seen = compared ? seen : (valid ? task.seen : 0);
         best = fmaxf(task.score, so_far);
         for (int o = 1; o < Gq; o <<= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
@@ -371,6 +412,13 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
         if ((seen >> lane & 1) && m >= 0 && m < p.access_n) counter[m] = 1;
       }
       __syncwarp();   // the table is written anew
+    }
+    if (CHECKED && p.stats) {
+      unsigned long long* st = reinterpret_cast<unsigned long long*>(p.stats);
+      if (st_keys) atomicAdd(st + ST_KEYS, (unsigned long long)st_keys);
+      if (st_fb) atomicAdd(st + ST_FALLBACK, (unsigned long long)st_fb);
+      if (st_wrong) atomicAdd(st + ST_WRONG, (unsigned long long)st_wrong);
+      atomicMax(reinterpret_cast<unsigned int*>(p.stats + ST_RATIO_BITS), __float_as_uint(st_ratio));
     }
   }
   tc_fence_before();
@@ -391,7 +439,7 @@ int run(const hipattn_scan_params_t& p, const KeyTiles& t, cudaStream_t stream) 
   const size_t smem = 1024 + (size_t)kTile * D * 2 + 2 * (size_t)256 * D * 2 + (size_t)kSearchWarps * (256 / kRows) * kTabStride * 4;
   const int64_t grid = (int64_t)t.nb * p.HKV * t.n_grid * (t.c_prev / kTile);
   HIPATTN_REQUIRE(grid > 0 && grid < 0x7fffffffLL, HIPATTN_ERR_INVALID, "scan grid of %lld blocks", (long long)grid);
-  auto kern = scan_key_tiles_kernel<DT, D>;
+  auto kern = p.left_out || p.stats || p.mode == HIPATTN_SCAN_CHECK ? scan_key_tiles_kernel<DT, D, true> : scan_key_tiles_kernel<DT, D, false>;
   HIPATTN_CUDA_OK(allow_smem((const void*)kern, smem));
   kern<<<(unsigned)grid, kThreads, smem, stream>>>(p, t);
   return check_launch("scan_key_tiles_kernel");
@@ -455,12 +503,13 @@ bool worth_turning(const hipattn_scan_params_t& p, int sink, int c_prev) {
 }  // namespace
 
 // Bytes of scratch that scan_key_tiles needs for this call, 0 where it does not take it: chunks of 32 cut from chunks of whole key
-// tiles, 16 pooled rows a head, no in-kernel RoPE, no per-head results.  With 32 pooled rows the tiles took 0.99 to 1.4 of the rounds'
+// tiles, 16 pooled rows a head, no in-kernel RoPE, all of the per-head results or none.  With 32 pooled rows the tiles took 0.99 to 1.4 of the rounds'
 // time, "relative" 0.92 to 1.6.
 int64_t scan_key_tiles_scratch(const hipattn_scan_params_t& p, int sink, int c_prev) {
   const int R = p.block_size_q / p.stride_q, G = p.H / p.HKV, BDST = cdiv(p.TQ, p.block_size_q);
-  if (p.mode != HIPATTN_SCAN_AUTO || p.dtype == HIPATTN_F32 || (p.D != 64 && p.D != 128) || p.key_abs == nullptr || p.k_scaled == nullptr) return 0;
-  if (p.rope_mode != HIPATTN_ROPE_NONE || p.left_out || p.right_out || p.score_out || p.stats) return 0;
+  const bool heads = p.left_out && p.right_out && p.score_out;
+  if (p.mode == HIPATTN_SCAN_STRICT || p.dtype == HIPATTN_F32 || (p.D != 64 && p.D != 128) || p.key_abs == nullptr || p.k_scaled == nullptr) return 0;
+  if (p.rope_mode != HIPATTN_ROPE_NONE || (!heads && (p.left_out || p.right_out || p.score_out))) return 0;
   if (R != kRows || (G & (G - 1)) != 0 || G > 16 || p.TQ <= p.stride_q) return 0;
   if (p.chunk_size != kChunk || c_prev % kTile != 0 || p.n_chunks % (c_prev / kChunk) != 0 || p.T <= sink) return 0;
   if ((int64_t)p.B * p.T * p.HKV >= 0x7fffffffLL || (int64_t)p.B * p.HKV * BDST >= 0x7fffffffLL) return 0;
@@ -490,6 +539,12 @@ int scan_key_tiles(const hipattn_scan_params_t& p, int sink, int c_prev, void* s
   t.c_prev = c_prev;
   t.tries = wait_tries();
   const int BDST = cdiv(p.TQ, p.block_size_q);
+  if (p.left_out) {
+    const int64_t total = (int64_t)p.B * BDST * p.H * p.n_chunks;
+    untouched_heads_kernel<<<(unsigned)min((total + 255) / 256, (int64_t)148 * 16), 256, 0, stream>>>(p, total);
+    const int rc = check_launch("untouched_heads_kernel");
+    if (rc) return rc;
+  }
   for (t.b0 = 0; t.b0 < p.B; t.b0 += s.nb) {
     t.nb = min(s.nb, p.B - t.b0);
     for (t.d0 = 0; t.d0 < BDST; t.d0 += s.nd) {

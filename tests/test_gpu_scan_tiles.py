@@ -98,8 +98,11 @@ def test_masks_equal_strict(shape, keys, rope, monkeypatch):
 
 
 @pytest.mark.parametrize("keys", ["random", "close", "not_finite"])
-@pytest.mark.parametrize("shape", ["heads4", "heads8_rows128", "heads20", "heads3", "odd_sink", "short_window"])
+@pytest.mark.parametrize("shape", ["heads4", "heads4_d64", "heads8_rows16", "heads8_rows128", "heads20", "heads3", "heads1", "odd_sink", "short_window",
+                                   "chunks512"])
 def test_bounds_and_scores_per_head_equal_strict(shape, keys, monkeypatch):
+    """Check mode scores every key by both definitions, in both kernels: none may be taken for certain that is not, and the error
+    radius is twice what is needed or more."""
     from hip_attention_b200 import hip_attention_impl
     qkv, args = problem(shape, keys, None)
     got = {}
@@ -107,13 +110,17 @@ def test_bounds_and_scores_per_head_equal_strict(shape, keys, monkeypatch):
     for mode in ("auto", "strict", "check"):
         monkeypatch.setenv("HIPATTN_SCAN_MODE", mode)
         dbg = {"scan_stats": stats} if mode == "check" else {}
-        hip_attention_impl(*qkv, args, debug=dbg)
+        names = launches(lambda: hip_attention_impl(*qkv, args, debug=dbg))
+        assert mode == "strict" or names == expected(args, qkv[0].shape[2], qkv[1].shape[2])
         got[mode] = dbg["stages"]
     for mode in ("auto", "check"):
         for i, (a, b) in enumerate(zip(got[mode], got["strict"])):
             for key in ("left", "right", "score", "score_max"):
                 assert torch.equal(a[key], b[key]), f"{mode} stage {i} {key}"
-    assert int(stats[2]) == 0, "a score taken without the strict definition is wrong"
+    keys_seen, uncertain, wrong, ratio = stats.tolist()
+    assert 0 < uncertain < keys_seen and wrong == 0, "a score taken without the strict definition is wrong"
+    if keys == "random":
+        assert torch.tensor([ratio & 0xffffffff], dtype=torch.int64).to(torch.int32).view(torch.float32).item() < 0.5
 
 
 @pytest.mark.parametrize("rope", [None, "relative"])
