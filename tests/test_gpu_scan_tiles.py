@@ -156,6 +156,58 @@ def test_restart_from_lists_of_a_callers_own(change, rope, monkeypatch):
         assert torch.equal(a.mask_cache_statistics.access_counter, b.mask_cache_statistics.access_counter), f"stage {stage}"
 
 
+@pytest.mark.parametrize("form", ["dense", "dense_d64", "paged", "q_by_heads", "positions_falling", "heads16", "heads16_paged"])
+def test_sequences_of_their_own(form, monkeypatch):
+    """Two sequences whose queries end at different tokens, nothing but NaN behind the last chunk that they reach: whole tiles, rounds
+    and the strict kernel give the same lists, masks and counters, through a page table too."""
+    import bench
+    from hip_attention_b200 import hip_attention_impl, read_status
+    B, T, TQ, live, page = 2, 8200, 3200, 7003, 16
+    w = dict(bench.WORKLOADS["prefill_128k"], B=B, TQ=TQ, T=T, H=8, HKV=2, keep=[4096, 1024, 512], sink=64, sw=320)
+    if form.startswith("heads16"):
+        w["H"] = 32
+    if form == "dense_d64":
+        w.update(D=64, dtype="fp16")
+    q, k, v = bench.make_qkv(w, "cuda")
+    k[:, live + 512:], v[:, live + 512:] = float("nan"), float("nan")
+    pos = (torch.arange(TQ) + torch.tensor([[live - TQ], [live - 1300 - TQ]])).cuda()
+    if form == "positions_falling":
+        pos = pos.flip(1)
+    if form == "q_by_heads":
+        q = q.permute(0, 2, 1, 3).contiguous().permute(0, 2, 1, 3)
+    args = bench.make_args(w, position_ids=pos)
+    args.require_cache_statistics = True
+    if form.endswith("paged"):
+        g = torch.Generator(device="cuda").manual_seed(9)
+        n = -(-T // page)
+        table = torch.randperm(B * n + 3, generator=g, device="cuda")[:B * n].view(B, n).to(torch.int32)
+        pools = []
+        for x in (k, v):
+            x = torch.nn.functional.pad(x, (0, 0, 0, 0, 0, n * page - T)).view(B * n, page, w["HKV"], -1)
+            pool = torch.full((B * n + 3, *x.shape[1:]), float("nan"), dtype=x.dtype, device="cuda")
+            pool[table.view(-1).long()] = x
+            pools.append(pool)
+        args.k_cache, args.v_cache = pools
+        args.block_table, args.cache_seq_lens, args.extend_context_length = table, torch.full((B,), T, dtype=torch.int32, device="cuda"), T
+        args.update_flags()
+        k = v = None
+    md = {}
+    for name in ("tiles", "rounds", "strict"):
+        monkeypatch.setenv("HIPATTN_SCAN_MODE", "strict" if name == "strict" else "auto")
+        monkeypatch.setenv("HIPATTN_SCAN_KERNEL", name)
+        read_status("cuda")
+        names = launches(lambda: md.update({name: hip_attention_impl(q, k, v, args)[1]}))
+        assert read_status("cuda") == 0
+        assert name == "strict" or names == (["stage_tcgen05", "key_tiles", "query_tiles"] if name == "tiles" else ["stage_tcgen05"] * 3)
+    for name in ("tiles", "rounds"):
+        a, b = md[name], md["strict"]
+        for i, (x, y) in enumerate(zip(a.stage_caches[1:], b.stage_caches[1:])):
+            assert torch.equal(x.indices_left, y.indices_left), f"{name} stage {i + 1}"
+        assert torch.equal(a.indices, b.indices) and torch.equal(a.ks, b.ks), name
+        assert torch.equal(a.mask_cache_statistics.access_counter, b.mask_cache_statistics.access_counter), name
+    assert int(md["tiles"].mask_cache_statistics.access_counter.sum()) > 0
+
+
 def test_waits_that_run_out_are_reported_and_leave_nothing(monkeypatch):
     """Every wait of both kernels that is not over at once counts as one that ran out: the call ends, says so, and the next one, which
     needs all of the tensor memory, is right."""
