@@ -170,6 +170,15 @@ def scan_flops(w: dict, heads: int, fetched: bool = False) -> float:
     return total
 
 
+def first_stage_rates(w: dict, heads: int, ms: float) -> dict:
+    """What the first scan stage executes: it goes by rounds whatever its size, and fetches every row but those whose score
+    is known.  The kernels of the later stages depend on their shapes."""
+    first = dict(w, chunks=w["chunks"][:1], keep=w["keep"][:1])
+    flops, gathered = scan_flops(first, heads, True), scan_bytes(first, heads, True)
+    return {"launch_ms": ms, "flops_executed": flops, "executed_tflops": flops / 1e12 / (ms / 1e3) if ms > 0 else None,
+            "gathered_bytes": gathered, "gather_gbs": gathered / 1e9 / (ms / 1e3) if ms > 0 else None}
+
+
 def attention_flops(w: dict, heads: int) -> float:
     return 4.0 * w["D"] * w["B"] * heads * w["TQ"] * (w["keep"][-1] + w["sink"] + w["sw"])
 
@@ -588,20 +597,17 @@ def run_prefill(a, w, dev, rank, world):
     scan_tf = sf / 1e12 / (scan_ms / 1e3) if scan_ms > 0 else None
     att_tf = af / 1e12 / (att_ms / 1e3) if att_ms > 0 else None
     # The scan launches are the larger share of the step.  Their key-row gathers are served by L2 (one KV head's keys are
-    # swept by all its query blocks; the DRAM traffic measured under ncu is about 1 % of the gathered bytes), so the bound
-    # that applies is the tensor pipe their dot products run on; the gather rate and the DRAM traffic are side figures.
+    # swept by all its query blocks; the DRAM traffic measured under ncu is 3 % of what the launches gather and stream), so
+    # the bound that applies is the tensor pipe their dot products run on; the gather rate and the DRAM traffic are side figures.
     scan_roof = {"kernel": "scan stage kernels (%d launches per step)" % n_scan, "bound": "tensor", "achieved": scan_tf,
                  "peak": tc_peak, "peak_source": peak_src, "unit": "TFLOP/s", "frac": scan_tf / tc_peak if scan_tf else None,
                  "traffic": NCU_DRAM_BYTES_PER_SCAN_LAUNCH.get((a.workload, world, w["TQ"])),
                  "traffic_source": NCU_TRAFFIC_SOURCE if (a.workload, world, w["TQ"]) in NCU_DRAM_BYTES_PER_SCAN_LAUNCH else None,
                  "flops_per_launch": sf / max(1, n_scan), "launch_ms": scan_ms / max(1, n_scan),
-                 "algorithm": "flops and bytes of the reference's rounds (two key rows per chunk, head and round); the "
-                              "*_executed and gather figures are those of the rounds without the rows whose score is known "
-                              "already; stages that score whole tiles of keys gather fewer bytes and multiply more",
-                 "flops_executed_per_launch": scan_flops(w, heads_local, True) / max(1, n_scan),
-                 "executed_tflops": scan_flops(w, heads_local, True) / 1e12 / (scan_ms / 1e3) if scan_ms > 0 else None,
-                 "gathered_bytes_per_launch": scan_bytes(w, heads_local, True) / max(1, n_scan),
-                 "gather_gbs": scan_bytes(w, heads_local, True) / 1e9 / (scan_ms / 1e3) if scan_ms > 0 else None,
+                 "algorithm": "flops of the reference's rounds (two key rows per chunk, head and round); what is executed "
+                              "differs by stage: rows whose score is known are skipped, and stages that score whole tiles "
+                              "of keys gather fewer bytes and multiply more",
+                 "first_stage": first_stage_rates(w, heads_local, phases.get("scan0", 0.0)),
                  "gather_served_by": "L2; the gather rate is not an HBM figure and may exceed the HBM copy peak",
                  "hbm_peak_gbs": hbm_peak}
     att_roof = {"kernel": "bsa_tcgen05 prefill attention kernel", "bound": "tensor", "achieved": att_tf, "peak": tc_peak,

@@ -43,3 +43,14 @@ def test_workload_table_holds_the_benchmark_configurations():
     assert w["decode_1m"]["T"] == 1 << 20 and w["decode_1m"]["shards"] == 8
     for name, c in w.items():
         assert len(c["chunks"]) == len(c["keep"]) == len(c["strides"]), name
+
+
+def test_first_stage_rates_count_the_rows_that_rounds_fetch():
+    """15 of 18 rows a chunk of 256 and head; the 15 chunks in front of the window are active for both query blocks."""
+    w = dict(bench.WORKLOADS["prefill_128k"], TQ=128, T=4096, sink=0, sw=256)
+    r = bench.first_stage_rates(w, 32, 2.0)
+    chunks = 2 * 15
+    assert r["gathered_bytes"] == chunks * 15 * 128 * 2 * 32
+    assert r["flops_executed"] == chunks * 15 * 32 * 2 * 16 * 128
+    assert r["gather_gbs"] == r["gathered_bytes"] / 1e9 / 2e-3 and r["executed_tflops"] == r["flops_executed"] / 1e12 / 2e-3
+    assert bench.first_stage_rates(w, 32, 0.0)["gather_gbs"] is None
