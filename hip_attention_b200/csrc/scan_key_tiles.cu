@@ -331,16 +331,7 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
             qw[e] = __ldg(reinterpret_cast<const uint4*>(qp + (p0 >> 3) * 1024 + sw128(rr & 7, e)));
           }
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            a = fmaf(lo_f32<DT>(qw[e].x), lo_f32<DT>(kw[e].x), a);
-            a = fmaf(hi_f32<DT>(qw[e].x), hi_f32<DT>(kw[e].x), a);
-            a = fmaf(lo_f32<DT>(qw[e].y), lo_f32<DT>(kw[e].y), a);
-            a = fmaf(hi_f32<DT>(qw[e].y), hi_f32<DT>(kw[e].y), a);
-            a = fmaf(lo_f32<DT>(qw[e].z), lo_f32<DT>(kw[e].z), a);
-            a = fmaf(hi_f32<DT>(qw[e].z), hi_f32<DT>(kw[e].z), a);
-            a = fmaf(lo_f32<DT>(qw[e].w), lo_f32<DT>(kw[e].w), a);
-            a = fmaf(hi_f32<DT>(qw[e].w), hi_f32<DT>(kw[e].w), a);
-          }
+          for (int e = 0; e < 8; ++e) a = strict_piece<DT>(qw[e], kw[e], a);
         }
         float top = fmaxf(a, -INFINITY);   // (a score that is not a number is the lowest)
 #pragma unroll
@@ -413,13 +404,7 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
       }
       __syncwarp();   // the table is written anew
     }
-    if (CHECKED && p.stats) {
-      unsigned long long* st = reinterpret_cast<unsigned long long*>(p.stats);
-      if (st_keys) atomicAdd(st + ST_KEYS, (unsigned long long)st_keys);
-      if (st_fb) atomicAdd(st + ST_FALLBACK, (unsigned long long)st_fb);
-      if (st_wrong) atomicAdd(st + ST_WRONG, (unsigned long long)st_wrong);
-      atomicMax(reinterpret_cast<unsigned int*>(p.stats + ST_RATIO_BITS), __float_as_uint(st_ratio));
-    }
+    if (CHECKED && p.stats) add_stats(p.stats, st_keys, st_fb, st_wrong, st_ratio);
   }
   tc_fence_before();
   __syncthreads();

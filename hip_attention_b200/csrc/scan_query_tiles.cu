@@ -366,16 +366,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) scan_query_tiles_kernel(const
 #pragma unroll
           for (int e = 0; e < BATCH; ++e)
 #pragma unroll
-            for (int i = 0; i < RL; ++i) {
-              a[i] = fmaf(lo_f32<DT>(qw[e][i].x), lo_f32<DT>(kw[e].x), a[i]);
-              a[i] = fmaf(hi_f32<DT>(qw[e][i].x), hi_f32<DT>(kw[e].x), a[i]);
-              a[i] = fmaf(lo_f32<DT>(qw[e][i].y), lo_f32<DT>(kw[e].y), a[i]);
-              a[i] = fmaf(hi_f32<DT>(qw[e][i].y), hi_f32<DT>(kw[e].y), a[i]);
-              a[i] = fmaf(lo_f32<DT>(qw[e][i].z), lo_f32<DT>(kw[e].z), a[i]);
-              a[i] = fmaf(hi_f32<DT>(qw[e][i].z), hi_f32<DT>(kw[e].z), a[i]);
-              a[i] = fmaf(lo_f32<DT>(qw[e][i].w), lo_f32<DT>(kw[e].w), a[i]);
-              a[i] = fmaf(hi_f32<DT>(qw[e][i].w), hi_f32<DT>(kw[e].w), a[i]);
-            }
+            for (int i = 0; i < RL; ++i) a[i] = strict_piece<DT>(qw[e][i], kw[e], a[i]);
         }
         float best = -INFINITY;
 #pragma unroll
@@ -470,13 +461,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) scan_query_tiles_kernel(const
       }
       __syncwarp();   // the table is written anew
     }
-    if (p.stats) {
-      unsigned long long* st = reinterpret_cast<unsigned long long*>(p.stats);
-      if (st_keys) atomicAdd(st + ST_KEYS, (unsigned long long)st_keys);
-      if (st_fb) atomicAdd(st + ST_FALLBACK, (unsigned long long)st_fb);
-      if (st_wrong) atomicAdd(st + ST_WRONG, (unsigned long long)st_wrong);
-      atomicMax(reinterpret_cast<unsigned int*>(p.stats + ST_RATIO_BITS), __float_as_uint(st_ratio));
-    }
+    if (p.stats) add_stats(p.stats, st_keys, st_fb, st_wrong, st_ratio);
   }
   tc_fence_before();
   __syncthreads();

@@ -65,6 +65,28 @@ __device__ __forceinline__ void group_maxima(uint32_t taddr, int ng, float* x) {
   }
 }
 
+// The strict definition's sum over the eight elements of a piece: fused multiply-adds in ascending order.
+template <int DT>
+__device__ __forceinline__ float strict_piece(const uint4& q, const uint4& k, float a) {
+  a = fmaf(lo_f32<DT>(q.x), lo_f32<DT>(k.x), a);
+  a = fmaf(hi_f32<DT>(q.x), hi_f32<DT>(k.x), a);
+  a = fmaf(lo_f32<DT>(q.y), lo_f32<DT>(k.y), a);
+  a = fmaf(hi_f32<DT>(q.y), hi_f32<DT>(k.y), a);
+  a = fmaf(lo_f32<DT>(q.z), lo_f32<DT>(k.z), a);
+  a = fmaf(hi_f32<DT>(q.z), hi_f32<DT>(k.z), a);
+  a = fmaf(lo_f32<DT>(q.w), lo_f32<DT>(k.w), a);
+  return fmaf(hi_f32<DT>(q.w), hi_f32<DT>(k.w), a);
+}
+
+// Adds what a thread counted to the statistics words.
+__device__ __forceinline__ void add_stats(uint64_t* stats, unsigned keys, unsigned fallback, unsigned wrong, float ratio) {
+  unsigned long long* st = reinterpret_cast<unsigned long long*>(stats);
+  if (keys) atomicAdd(st + ST_KEYS, (unsigned long long)keys);
+  if (fallback) atomicAdd(st + ST_FALLBACK, (unsigned long long)fallback);
+  if (wrong) atomicAdd(st + ST_WRONG, (unsigned long long)wrong);
+  atomicMax(reinterpret_cast<unsigned int*>(st + ST_RATIO_BITS), __float_as_uint(ratio));
+}
+
 // An mbarrier's phase: tried a few times, and waited for out of line.  The roles of these kernels go through long straight code, each
 // warp its own, so that instructions come from beyond the first-level caches and cost five to six cycles apiece: the way through a
 // barrier that is ready is kept short.
