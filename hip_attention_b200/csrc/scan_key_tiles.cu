@@ -34,7 +34,6 @@ struct KeyTiles {
   int32_t* counts;               // [nb, n_grid]
   int b0, nb, d0, nd;
   int n_grid, sink, c_prev;      // chunks of the stage before: grid of c_prev tokens from `sink`
-  int tries;                     // wait_tries()
 };
 
 // ---- pooled queries of a (batch, KV head, query block), rows beyond the last one repeat the first ----
@@ -140,7 +139,7 @@ __global__ void __launch_bounds__(256) untouched_heads_kernel(const hipattn_scan
 }
 
 // CHECKED: per-head results, statistics, and in check mode every score by both definitions.
-template <int DT, int D, bool CHECKED>
+template <int DT, int D, bool CHECKED, bool PATIENT>
 __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipattn_scan_params_t p, const KeyTiles t) {
   constexpr int ROWB = D * 2, PIECES = ROWB / 16, KB = D / 64;
   constexpr int R = kRows, CHUNK = kChunk, COLS = 256, NG = COLS / R;   // columns of a stage, groups (query block, head)
@@ -203,7 +202,7 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
       const unsigned char* src = t.pooled + slice * t.nd * entry_bytes;
       int slot = 0, use = 0, next = __ldg(&entries[0].x), k = 0;
       for (int e = 0; k < stages_total; ++k) {
-        if (use > 0 && !mbar_wait_quick(smem_u32(&s_empty[slot]), (use - 1) & 1, &s_abort, p.status, t.tries)) break;
+        if (use > 0 && !mbar_wait_quick<PATIENT>(smem_u32(&s_empty[slot]), (use - 1) & 1, &s_abort, p.status)) break;
         const int ne = min(EB, count - k * EB);
         const uint32_t bar = smem_u32(&s_full[slot]), dst = smem_u32(sQ) + slot * Q_STAGE;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(ne * entry_bytes) : "memory");
@@ -225,8 +224,8 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
       const uint64_t da0 = make_desc(smem_u32(sA) + acc * A_TILE, 16, 1024), db0 = make_desc(smem_u32(sQ), 16, KB * 1024);
       int slot = 0, use = 0, set = acc, k = 0, last = 0;
       for (; k < stages_total; ++k) {
-        if (!mbar_wait_quick(smem_u32(&s_full[slot]), use & 1, &s_abort, p.status, t.tries)) break;
-        if (k > 0 && !mbar_wait_quick(smem_u32(&s_acce[acc]), (k - 1) & 1, &s_abort, p.status, t.tries)) break;
+        if (!mbar_wait_quick<PATIENT>(smem_u32(&s_full[slot]), use & 1, &s_abort, p.status)) break;
+        if (k > 0 && !mbar_wait_quick<PATIENT>(smem_u32(&s_acce[acc]), (k - 1) & 1, &s_abort, p.status)) break;
         tc_fence_after();
         const uint32_t idesc = make_idesc(DT == HIPATTN_BF16 ? 1 : 0, 128, min(EB, count - k * EB) * Gq * R, 0);
         const uint64_t db = db0 + (uint64_t)((slot * Q_STAGE) >> 4);
@@ -297,7 +296,7 @@ __global__ void __launch_bounds__(kThreads, 1) scan_key_tiles_kernel(const hipat
       const int ng = min(EB, count - (u >> 1) * EB) * Gq;
       const int l = base + acc * 128 + quarter * 32;   // the warp's chunk: CHUNK tokens from here
       const bool valid = walker && cur.d >= 0;
-      ok = __all_sync(0xffffffffu, mbar_wait_quick(smem_u32(&s_accf[set][acc]), phase >> acc & 1, &s_abort, p.status, t.tries));
+      ok = __all_sync(0xffffffffu, mbar_wait_quick<PATIENT>(smem_u32(&s_accf[set][acc]), phase >> acc & 1, &s_abort, p.status));
       if (!ok) break;
       phase ^= 1u << acc;
       tc_fence_after();
@@ -424,7 +423,9 @@ int run(const hipattn_scan_params_t& p, const KeyTiles& t, cudaStream_t stream) 
   const size_t smem = 1024 + (size_t)kTile * D * 2 + 2 * (size_t)256 * D * 2 + (size_t)kSearchWarps * (256 / kRows) * kTabStride * 4;
   const int64_t grid = (int64_t)t.nb * p.HKV * t.n_grid * (t.c_prev / kTile);
   HIPATTN_REQUIRE(grid > 0 && grid < 0x7fffffffLL, HIPATTN_ERR_INVALID, "scan grid of %lld blocks", (long long)grid);
-  auto kern = p.left_out || p.stats || p.mode == HIPATTN_SCAN_CHECK ? scan_key_tiles_kernel<DT, D, true> : scan_key_tiles_kernel<DT, D, false>;
+  auto kern = p.left_out || p.stats || p.mode == HIPATTN_SCAN_CHECK ? scan_key_tiles_kernel<DT, D, true, true> : scan_key_tiles_kernel<DT, D, false, true>;
+  if constexpr (DT == HIPATTN_BF16 && D == 128)
+    if (without_patience()) kern = scan_key_tiles_kernel<DT, D, false, false>;
   HIPATTN_CUDA_OK(allow_smem((const void*)kern, smem));
   kern<<<(unsigned)grid, kThreads, smem, stream>>>(p, t);
   return check_launch("scan_key_tiles_kernel");
@@ -522,7 +523,6 @@ int scan_key_tiles(const hipattn_scan_params_t& p, int sink, int c_prev, void* s
   t.n_grid = s.n_grid;
   t.sink = sink;
   t.c_prev = c_prev;
-  t.tries = wait_tries();
   const int BDST = cdiv(p.TQ, p.block_size_q);
   if (p.left_out) {
     const int64_t total = (int64_t)p.B * BDST * p.H * p.n_chunks;

@@ -33,10 +33,9 @@ struct QueryTiles {
   int stages;        // key tiles in the ring
   int split;         // CTAs that share out the key tiles
   int check;
-  int tries;         // wait_tries()
 };
 
-template <int DT, int D, int R>
+template <int DT, int D, int R, bool PATIENT>
 __global__ void __launch_bounds__(kTileThreads, 1) scan_query_tiles_kernel(const hipattn_scan_params_t p, const QueryTiles cfg) {
   constexpr int ROWB = D * 2, PIECES = ROWB / 16, KB = D / 64;
   constexpr int COLS = 256, NG = COLS / R;                 // columns and heads of a pass
@@ -188,7 +187,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) scan_query_tiles_kernel(const
           cp_async_wait<0>();
           report();
         }
-        ok = __all_sync(0xffffffffu, mbar_wait_quick(smem_u32(&s_empty[slot]), (use - 1) & 1, &s_abort, p.status, cfg.tries));
+        ok = __all_sync(0xffffffffu, mbar_wait_quick<PATIENT>(smem_u32(&s_empty[slot]), (use - 1) & 1, &s_abort, p.status));
         if (!ok) break;
       }
       const uint32_t dst = sA_u32 + slot * A_STAGE;
@@ -234,8 +233,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) scan_query_tiles_kernel(const
       if (acc) advance();
       int k = 0, last = 0;
       for (; it < mine; ++k) {
-        if (!mbar_wait_quick(smem_u32(&s_full[slot]), use & 1, &s_abort, p.status, cfg.tries)) break;
-        if (k > 0 && !mbar_wait_quick(smem_u32(&s_acce[acc]), (k - 1) & 1, &s_abort, p.status, cfg.tries)) break;
+        if (!mbar_wait_quick<PATIENT>(smem_u32(&s_full[slot]), use & 1, &s_abort, p.status)) break;
+        if (k > 0 && !mbar_wait_quick<PATIENT>(smem_u32(&s_acce[acc]), (k - 1) & 1, &s_abort, p.status)) break;
         tc_fence_after();
         const uint32_t idesc = make_idesc(DT == HIPATTN_BF16 ? 1 : 0, 128, min(NG, heads - j * NG) * R, 0);
         const uint64_t da = da0 + (uint64_t)((slot * A_STAGE) >> 4), db = db0 + (uint64_t)((j * Q_PASS) >> 4);
@@ -320,7 +319,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) scan_query_tiles_kernel(const
       float eps[NG];   // radius per unit of key magnitude
 #pragma unroll
       for (int g = 0; g < NG; ++g) eps[g] = s_eps[j * NG + g];
-      ok = __all_sync(0xffffffffu, mbar_wait_quick(smem_u32(&s_accf[set][acc]), phase >> acc & 1, &s_abort, p.status, cfg.tries));
+      ok = __all_sync(0xffffffffu, mbar_wait_quick<PATIENT>(smem_u32(&s_accf[set][acc]), phase >> acc & 1, &s_abort, p.status));
       if (!ok) break;
       phase ^= 1u << acc;
       tc_fence_after();
@@ -493,7 +492,6 @@ int launch(const hipattn_scan_params_t& p, cudaStream_t stream) {
   const TilePlan plan = plan_tiles(p);
   QueryTiles cfg;
   cfg.check = p.mode == HIPATTN_SCAN_CHECK ? 1 : 0;
-  cfg.tries = wait_tries();
   cfg.passes = plan.passes;
   cfg.head_groups = plan.head_groups;
   // (an even number of slots: with one pass a tile, a slot's phases are then all waited for by one of the two MMA threads)
@@ -503,7 +501,9 @@ int launch(const hipattn_scan_params_t& p, cudaStream_t stream) {
   cfg.split = scan_ctas_per_unit(units * 8, cdiv(p.n_chunks, 128 / kTileChunk));   // (one CTA a multiprocessor, a wave of them)
   const int64_t grid = units * cfg.split;
   HIPATTN_REQUIRE(grid > 0 && grid < 0x7fffffffLL, HIPATTN_ERR_INVALID, "scan grid of %lld blocks", (long long)grid);
-  auto kern = scan_query_tiles_kernel<DT, D, R>;
+  auto kern = scan_query_tiles_kernel<DT, D, R, true>;
+  if constexpr (DT == HIPATTN_BF16 && D == 128 && R == 64)
+    if (without_patience()) kern = scan_query_tiles_kernel<DT, D, R, false>;
   HIPATTN_CUDA_OK(allow_smem((const void*)kern, smem));
   kern<<<(unsigned)grid, kTileThreads, smem, stream>>>(p, cfg);
   return check_launch("scan_query_tiles_kernel");
