@@ -12,8 +12,9 @@
 // pool_queries_kernel writes the pooled queries in operand layout, list_queries_kernel the blocks that kept a chunk.
 //
 // Bound: as scan_query_tiles.cu, the chain from an accumulator's MMAs to its release.  128k prefill, second stage (chunk
-// 32, 4 heads x 16 rows): 3135 us by rounds, which were bound by their gathers (10.7 TB/s from L2), 1740 and 73 for the
-// pooled queries and the lists; ragged fp16 prefill 189 -> 117 us.
+// 32, 4 heads x 16 rows): 3146 us by rounds, which were bound by their gathers (10.7 TB/s from L2), 1862 here (1740 on
+// another board) and 74 for the pooled queries and the lists; ragged fp16 prefill 179 -> 97 us and less
+// than 20.
 #include "host_kernels.h"
 #include "scan_tiles.cuh"
 
