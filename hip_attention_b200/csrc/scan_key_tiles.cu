@@ -13,8 +13,7 @@
 //
 // Bound: as scan_query_tiles.cu, the chain from an accumulator's MMAs to its release.  128k prefill, second stage (chunk
 // 32, 4 heads x 16 rows): 3146 us by rounds, which were bound by their gathers (10.7 TB/s from L2), 1862 here (1740 on
-// another board) and 74 for the pooled queries and the lists; ragged fp16 prefill 179 -> 97 us and less
-// than 20.
+// another board) and 74 for the pooled queries and the lists; ragged fp16 prefill 179 -> 97 us and less than 20.
 #include "host_kernels.h"
 #include "scan_tiles.cuh"
 
@@ -490,8 +489,8 @@ bool worth_turning(const hipattn_scan_params_t& p, int sink, int c_prev) {
 }  // namespace
 
 // Bytes of scratch that scan_key_tiles needs for this call, 0 where it does not take it: chunks of 32 cut from chunks of whole key
-// tiles, 16 pooled rows a head, no in-kernel RoPE, all of the per-head results or none.  With 32 pooled rows the tiles took 0.99 to 1.4 of the rounds'
-// time, "relative" 0.92 to 1.6.
+// tiles, 16 pooled rows a head, no in-kernel RoPE, all of the per-head results or none.  With 32 pooled rows the tiles
+// took 0.99 to 1.4 of the rounds' time, "relative" 0.92 to 1.6.
 int64_t scan_key_tiles_scratch(const hipattn_scan_params_t& p, int sink, int c_prev) {
   const int R = p.block_size_q / p.stride_q, G = p.H / p.HKV, BDST = cdiv(p.TQ, p.block_size_q);
   const bool heads = p.left_out && p.right_out && p.score_out;

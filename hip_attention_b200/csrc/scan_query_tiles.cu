@@ -15,7 +15,8 @@
 // Shared memory is the reason why the links are long: the MMAs read 96 of its 128 bytes a cycle (half accumulators of 128
 // columns all 128, and were slower) and the loads of everyone else queue behind them.  128k prefill, third stage
 // (chunk 8, 4 heads x 64 rows): 2750 us by rounds, 1985 here (1820 on another board); 131072 queries of 64 heads (8 x 128 rows): 28.8
-// -> 23.6 ms.  On the way, on the board of the 1820: two sets 2190, one MMA thread 2080, strict scores that read shared memory piece by piece 2030.
+// -> 23.6 ms.  On the way, on the board of the 1820: two sets 2190, one MMA thread 2080, strict scores that read shared memory
+// piece by piece 2030.
 #include "scan_tiles.cuh"
 
 namespace hipattn {
