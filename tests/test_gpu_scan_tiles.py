@@ -273,6 +273,28 @@ def test_without_memory_for_the_scratch():
     assert torch.equal(md.indices, want.indices) and torch.equal(md.ks, want.ks)
 
 
+def test_under_capture():
+    """Lists, pooled queries and scratch are made anew at every replay."""
+    from hip_attention_b200 import hip_attention_impl, read_status
+    (q, k, v), args = problem("heads4", "random", None)
+    args.position_ids = (torch.arange(q.shape[1], device="cuda") + k.shape[1] - q.shape[1])[None]
+    other = torch.randn_like(q) * 128 ** -0.5
+    want = hip_attention_impl(other, k, v, args)
+    assert not torch.equal(want[1].indices, hip_attention_impl(q, k, v, args)[1].indices)
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        out, md = hip_attention_impl(q, k, v, args)
+    q.copy_(other)
+    for _ in range(2):
+        out.zero_(), md.indices.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want[0]) and torch.equal(md.indices, want[1].indices) and torch.equal(md.ks, want[1].ks)
+        assert torch.equal(md.mask_cache_statistics.access_counter, want[1].mask_cache_statistics.access_counter)
+    assert read_status("cuda") == 0
+
+
 # heads, KV heads, query rows of a block, pooling strides, queries, tokens, kept -> kernels of the second and third stage
 RULE = [
     # (few CTAs, one with a list of all blocks: 2.4 to 2.5 times the rounds' time by key tiles)
